@@ -18,6 +18,7 @@
 #include <cuda.h>
 
 #include "seq_common.cuh"
+#include "tc_pair.cuh"
 
 namespace b200seq {
 
@@ -232,35 +233,133 @@ __global__ void __launch_bounds__(128) linear_tc_kernel(const __grid_constant__ 
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(tmem) : "memory");
 }
 
-typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                             CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// ---- epilogues of the paired-SM kernel (tc_pair.cuh): v[j] = acc[n][m + j] ----
+struct EpiF32 {
+    float* y;
+    int64_t ldy;
+    int N, silu_lo, silu_hi;
+    __device__ __forceinline__ void store(float (&v)[32], int n, int m, int m_end, int) const {
+        if (n >= N) return;
+        if (n >= silu_lo && n < silu_hi) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = siluf_acc(v[j]);
+        }
+        float* o = y + (int64_t)m * ldy + n;
+        if (m + 32 <= m_end) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) o[(int64_t)j * ldy] = v[j];
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                if (m + j < m_end) o[(int64_t)j * ldy] = v[j];
+        }
+    }
+};
+struct EpiPlainAct {
+    void* out;
+    int64_t ldo;
+    int N, dtype, kind;
+    __device__ __forceinline__ void store(float (&v)[32], int n, int m, int m_end, int) const {
+        if (n >= N) return;
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            if (m + j < m_end) store_act(out, dtype, (int64_t)(m + j) * ldo + n, act_plain(kind, v[j]));
+    }
+};
+// rows alternate (gate j, up j): an even lane holds the gates, the odd lane beside it the ups of the same 32 tokens.  They trade halves, so
+// that the even lane computes tokens 0 .. 15 and the odd one 16 .. 31 (one activation per lane and token instead of one per lane pair).
+// pack: bf16 output with 4-byte aligned pairs of columns -- lanes two apart trade again and store two columns at once
+// Activations that leave as bf16 take the division without its branches (reciprocal approximation and one Newton step, 1 ulp of f32): the
+// rounding call behind 1 / d kept the 16 activations of a lane from overlapping and made the epilogue, not the tensor pipe, the bound
+// (4096 x 16384 x 2048: 326 us against 202 us of the plain product).  f32 outputs keep the rounded division.
+__device__ __forceinline__ float sigmoid_nobranch(float x) {
+    const float d = 1.0f + expf(fminf(-x, 85.0f));   // finite, and so is the reciprocal
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return fmaf(r, fmaf(-d, r, 1.0f), r);
+}
+__device__ __forceinline__ float act_gated_nobranch(const ActParams& a, float gate, float up) {
+    if (a.kind == B200SEQ_ACT_GELU_TANH) return gate * sigmoid_nobranch(1.5957691216057308f * (gate + 0.044715f * gate * gate * gate)) * up;
+    const float g = fminf(gate, a.limit);
+    const float u = fminf(fmaxf(up, -a.limit), a.limit);
+    return g * sigmoid_nobranch(a.alpha * g) * (u + a.shift);
+}
+struct EpiGated {
+    void* out;
+    int64_t ldo;
+    int N, dtype, pack;
+    ActParams act;
+    __device__ __forceinline__ void store(float (&v)[32], int n, int m, int m_end, int lane) const {
+        const bool odd = lane & 1;
+        float r[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const float x = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 16], 1);
+            const float g = odd ? x : v[j], u = odd ? v[j + 16] : x;
+            r[j] = dtype == B200SEQ_BF16 ? act_gated_nobranch(act, g, u) : act_gated(act, g, u);
+        }
+        const int f = n >> 1, mt = m + (odd ? 16 : 0);
+        if (pack) {
+            const bool hi = lane & 2;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float x = __shfl_xor_sync(0xffffffffu, hi ? r[j] : r[j + 8], 2);
+                const __nv_bfloat162 b = hi ? __floats2bfloat162_rn(x, r[j + 8]) : __floats2bfloat162_rn(r[j], x);
+                const int t = mt + j + (hi ? 8 : 0);
+                if (n < N && t < m_end) *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(out) + (int64_t)t * ldo + (f & ~1)) = b;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                if ((n | 1) < N && mt + j < m_end) store_act(out, dtype, (int64_t)(mt + j) * ldo + f, r[j]);
+        }
+    }
+};
 
-EncodeFn encode_fn() {
-    static EncodeFn fn = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = nullptr;
-        return reinterpret_cast<EncodeFn>(f);
-    }();
-    return fn;
+using tcpair::encode_fn;
+using tcpair::make_map;
+
+// Which tile: estimated cycles of the last pair to finish.  A 256 x 256 tile keeps the tensor pipe of both SMs busy for K * 8 cycles, a
+// 256 x 128 one for K * 4 at a lower rate (measured, 4096 x 6144 x 4096: 11 waves of the narrow tile 156 us, 6 of the wide one 152 us, that is
+// 14.2 against 25.4 us a wave), so the narrow one wins where its finer grain saves a wave (1024 x 6144 x 4096: 45.0 against 49.7 us) and in
+// steps of few tokens (256 x 2048 x 8192: 26 against 45 us).  Per-head products (K and N of one head) stay on the single-SM kernel.
+enum { TILE_SINGLE = 0, TILE_PAIR128 = 128, TILE_PAIR256 = 256 };
+int pick_tile(const TcParams& p) {
+    const int64_t pairs = tcpair::pair_sms() / 2;
+    if (p.heads || pairs < 1 || (p.offs && p.E > tcpair::MAX_GROUPS)) return TILE_SINGLE;
+    auto waves = [&](int bt) {   // grouped: every group's last tile is half full on average
+        const int64_t mt = p.offs ? (p.M + bt / 2 * (int64_t)p.E + bt - 1) / bt : (p.M + bt - 1) / bt;
+        return (double)((mt * ((p.N + 255) / 256) + pairs - 1) / pairs);
+    };
+    const double narrow = waves(128) * (p.K * 4 / 0.75 + 200), wide = waves(256) * (p.K * 8 / 0.84 + 200) + 2000;
+    return wide <= narrow ? TILE_PAIR256 : TILE_PAIR128;
 }
 
-// rows x K bf16 matrix with row stride ld elements; box = 64 k x 128 rows, 128-byte swizzle, zero fill outside
-bool make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int64_t ld) {
-    EncodeFn fn = encode_fn();
-    if (!fn) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {BK, 128};
-    const cuuint32_t estr[2] = {1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+template <class Epi>
+cudaError_t launch_pair(int tile, const void* x, int64_t ldx, const void* w, const TcParams& p, const Epi& epi, cudaStream_t st) {
+    tcpair::Args a{};
+    a.M = p.M, a.N = p.N, a.K = p.K, a.offs = p.offs, a.E = p.offs ? p.E : 1, a.bf16 = 1, a.err = p.err, a.err_bit = 2;
+    const int64_t rows = p.offs ? (int64_t)p.E * p.N : p.N;
+    return tile == TILE_PAIR256 ? tcpair::launch<256>(w, rows, p.K, x, ldx, a, epi, st) : tcpair::launch<128>(w, rows, p.K, x, ldx, a, epi, st);
 }
 
 int launch(const void* x, int64_t ldx, const void* w, TcParams p, cudaStream_t st) {
     CUtensorMap mw, mx;
     const int64_t wrows = p.offs ? (int64_t)p.E * p.N : (p.heads ? (int64_t)p.heads * p.N : p.N);
-    if (!make_map(&mw, w, wrows, p.K, p.K) || !make_map(&mx, x, p.M, p.heads ? (int64_t)p.heads * p.K : p.K, ldx))
+    p.err = error_flag_dev();
+    if (const int tile = pick_tile(p)) {
+        cudaError_t e;
+        if (p.epi == EPI_NONE) e = launch_pair(tile, x, ldx, w, p, EpiF32{p.y, p.ldy, p.N, p.silu_lo, p.silu_hi}, st);
+        else if (p.epi == EPI_PLAIN_ACT) e = launch_pair(tile, x, ldx, w, p, EpiPlainAct{p.act_out, p.ldo, p.N, p.out_dtype, p.act.kind}, st);
+        else {
+            const int pack = p.out_dtype == B200SEQ_BF16 && p.N % 4 == 0 && p.ldo % 2 == 0 && (reinterpret_cast<uintptr_t>(p.act_out) & 3) == 0;
+            e = launch_pair(tile, x, ldx, w, p, EpiGated{p.act_out, p.ldo, p.N, p.out_dtype, pack, p.act}, st);
+        }
+        if (e != cudaSuccess) return cuda_status(e, "linear tc pair");
+        count_launch();
+        return 0;
+    }
+    if (!make_map(&mw, w, wrows, p.K, p.K, 128, true) || !make_map(&mx, x, p.M, p.heads ? (int64_t)p.heads * p.K : p.K, ldx, 128, true))
         return fail(B200SEQ_ERR_CUDA, "linear: tensor map encoding failed");
     static bool attr_set = false;
     const int smem = STAGES * STAGE_BYTES + 1024;
@@ -269,7 +368,6 @@ int launch(const void* x, int64_t ldx, const void* w, TcParams p, cudaStream_t s
         if (e != cudaSuccess) return cuda_status(e, "linear tc attribute");
         attr_set = true;
     }
-    p.err = error_flag_dev();
     dim3 grid((p.M + BM - 1) / BM + (p.offs ? p.E : 0), (p.N + BN - 1) / BN, p.heads ? p.heads : 1);
     linear_tc_kernel<<<grid, 128, smem, st>>>(mw, mx, p);
     SEQ_LAUNCH_CHECK("linear tc");

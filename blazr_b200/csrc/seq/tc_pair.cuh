@@ -1,0 +1,371 @@
+// tc_pair.cuh -- dense 16-bit GEMM on pairs of SMs, shared by both libraries: acc[n][m] = sum_k w[n][k] x[m][k], f32 accumulation.
+//
+// Two CTAs of a cluster work on one tile of 256 weight rows x BT token rows (tcgen05.mma.cta_group::2, M = 256, N = BT, K = 16): each CTA
+// holds its own 128 weight rows and HALF of the token rows in shared memory, so a 64-k slab costs 16 KB + BT * 64 bytes per SM where two
+// single-SM 128 x 128 tiles would fetch 32 KB each for half the products.  TMEM lane = weight row, column = token: a warp's lanes hold
+// 32 consecutive n of one token, the stores of the epilogue are coalesced.  Both operands are K-major 16-bit rows fetched by TMA
+// (128-byte swizzle); rows and k outside the matrices read as zero.
+//
+// The kernel is persistent (one pair per two SMs, tiles dealt round-robin, token tiles fastest so that a weight tile is read from HBM
+// once) and the accumulator is double-buffered in TMEM (2 x BT columns): the eight epilogue warps drain tile i while the tensor cores run
+// tile i + 1.  What bounds it is the tensor pipe; the single-SM kernel it replaces for large steps stalled on L2 -> SM traffic (512 bytes
+// per 32 768 FLOPs against 1 024 per 131 072 here) and on a main loop that its epilogue interrupted.  Measured, 4096 tokens: 16384 x 2048 267 ->
+// 198 us (1.39 PFLOP/s), with the gated activation 478 -> 201 us; 2048 x 8192 128 -> 100 us; 8192 x 1024 91 -> 61 us.
+//
+// Warp roles: 0 = TMA producer (both CTAs), 1 = MMA issuer (leader CTA only), 2 = TMEM allocation, 4..11 = epilogue.
+// Barriers: full[s] lives in the leader and counts the bytes of both CTAs; empty[s] and acc_full are signalled in both CTAs by
+// multicast tcgen05.commit; acc_empty lives in the leader and collects the epilogue warps of both CTAs.
+// Every wait is bounded by a clock: one that runs out raises the abort flag, the role leaves its loop, and the CTA goes through the
+// common exit (copies in flight waited for, TMEM freed).
+#pragma once
+#include <cuda.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace tcpair {
+
+constexpr int ROWS = 128;        // weight rows per CTA
+constexpr int BK = 64;           // k per slab
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = (4 + EPI_WARPS) * 32;
+constexpr int HDR = 1024;
+constexpr int MAX_GROUPS = 1024;
+constexpr unsigned long long WAIT_NS = 2000000000ull;
+
+template <int BT>
+struct Cfg {
+    static constexpr int XROWS = BT / 2;                           // token rows in each CTA's shared memory
+    static constexpr int STAGE = (ROWS + XROWS) * BK * 2;          // bytes per stage and CTA
+    static constexpr int STAGES = (192 * 1024) / STAGE;            // 6 (BT = 256) or 8 (BT = 128)
+    static constexpr int SMEM = STAGES * STAGE + HDR + 1024 + (MAX_GROUPS + 1) * 4;
+    static constexpr int TMEM_COLS = 2 * BT;
+};
+
+struct Args {
+    int M, N, K;             // token rows, weight rows of one group, reduction length
+    int MT, NT;              // token tiles (bound when grouped), weight tiles of 256
+    const int32_t* offs;     // grouped form: [E + 1] first token row of every group; group e uses the weight rows e * N ..
+    int E;
+    int bf16;                // operand type: 1 = bf16, 0 = f16
+    int* err;                // device error word
+    int err_bit;
+};
+
+__device__ __forceinline__ uint32_t sa(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ uint32_t map_leader(uint32_t a) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(a));
+    return r;
+}
+__device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory"); }
+__device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bar_arrive_cluster(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ unsigned long long now_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+// false: the wait ran out, or another role of this CTA gave up
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    if (bar_try(bar, parity)) return true;
+    unsigned long long t0 = 0;
+    for (uint32_t i = 1;; ++i) {
+        if (bar_try(bar, parity)) return true;
+        if ((i & 255u) == 0) {
+            if (*abort_flag) return false;
+            const unsigned long long t = now_ns();
+            if (t0 == 0) t0 = t;
+            else if (t - t0 > WAIT_NS) {
+                *abort_flag = 1;
+                return false;
+            }
+        }
+    }
+}
+// both CTAs' copies report to the leader's barrier (bar: its shared::cluster address)
+__device__ __forceinline__ void tma_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map),
+                 "r"(c0), "r"(c1), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void commit_pair(uint32_t bar) {   // arrives on the same barrier of both CTAs when the MMAs issued so far are done
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ bool elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// K-major operand, 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart
+__device__ __forceinline__ uint64_t desc_k128(uint32_t a) {
+    return (uint64_t)((a >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+__device__ __forceinline__ void ld32(uint32_t taddr, float* v) {
+    uint32_t* r = reinterpret_cast<uint32_t*>(v);
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+          "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
+          "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+struct Tile {
+    int m0, m_end, wrow, n0;   // first token row, end of its group's rows, first weight row in memory, first output column
+};
+
+// tile t of the step (token tiles fastest).  first: grouped form, [E + 1] first token tile of every group
+template <int BT>
+__device__ __forceinline__ Tile tile_of(const Args& p, const int32_t* first, int MT, int t) {
+    Tile r;
+    const int mt = t % MT, nt = t / MT;
+    r.n0 = nt * 2 * ROWS;
+    r.wrow = r.n0;
+    if (!p.offs) {
+        r.m0 = mt * BT, r.m_end = p.M;
+    } else {
+        int lo = 0, hi = p.E;      // the last group whose first tile is <= mt (groups without rows have no tile)
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (first[mid] <= mt) lo = mid;
+            else hi = mid;
+        }
+        r.m0 = p.offs[lo] + (mt - first[lo]) * BT, r.m_end = p.offs[lo + 1];
+        r.wrow += lo * p.N;
+    }
+    return r;
+}
+
+// Epi: struct with   __device__ void store(const float (&v)[32], int n, int m, int m_end, int lane) const
+//   v[j] = acc[n][m + j] of this lane's n (n may be >= N: nothing is stored); all 32 lanes of a warp call it with the same m
+template <int BT, class Epi>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+    pair_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Args p, const Epi epi) {
+    using C = Cfg<BT>;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (sa(smem_raw) + 1023u) & ~1023u;
+    const uint32_t full = base, empty = full + 8 * C::STAGES, acc_full = empty + 8 * C::STAGES, acc_empty = acc_full + 16;
+    uint8_t* hdr = smem_raw + (base - sa(smem_raw));
+    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(hdr + 512);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(hdr + 520);
+    int32_t* first = reinterpret_cast<int32_t*>(hdr + HDR + C::STAGES * C::STAGE);
+    const uint32_t stages = base + HDR;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(rank));
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < C::STAGES; ++s) bar_init(full + 8 * s, 1), bar_init(empty + 8 * s, 1);
+        for (int b = 0; b < 2; ++b) bar_init(acc_full + 8 * b, 1), bar_init(acc_empty + 8 * b, 2 * EPI_WARPS);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    int MT = p.MT;
+    if (p.offs && warp == 3) {   // first token tile of every group: an inclusive scan over the groups, 32 at a time
+        int run = 0;
+        for (int e0 = 0; e0 < p.E; e0 += 32) {
+            const int e = e0 + lane;
+            int n = e < p.E ? (p.offs[e + 1] - p.offs[e] + BT - 1) / BT : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, n, o);
+                if (lane >= o) n += u;
+            }
+            if (e < p.E) first[e + 1] = run + n;
+            run += __shfl_sync(0xffffffffu, n, 31);
+        }
+        if (lane == 0) first[0] = 0;
+    }
+    if (warp == 2) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sa(tmem_ptr)), "n"(C::TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    cluster_sync();   // the peer's barriers and TMEM exist
+    fence_after();
+    const uint32_t tmem = *tmem_ptr;
+    if (p.offs) MT = first[p.E];
+    const int tiles = MT * p.NT, stride = (int)gridDim.x >> 1;
+    const int nk = (p.K + BK - 1) / BK;
+
+    if (warp == 0) {
+        if (elect()) {
+            const uint32_t full_l = map_leader(full);
+            int s = 0;
+            uint32_t ph = 1;
+            bool ok = true;
+            for (int t = (int)blockIdx.x >> 1; t < tiles && ok; t += stride) {
+                const Tile tl = tile_of<BT>(p, first, MT, t);
+                const int wr = tl.wrow + (int)rank * ROWS, xr = tl.m0 + (int)rank * C::XROWS;
+                for (int kb = 0; kb < nk; ++kb) {
+                    ok = bar_wait(empty + 8 * s, ph, abort_flag);
+                    if (!ok) break;
+                    if (rank == 0) bar_expect(full + 8 * s, 2 * C::STAGE);
+                    const uint32_t st = stages + s * C::STAGE;
+                    tma_pair(st, &map_w, kb * BK, wr, full_l + 8 * s);
+                    tma_pair(st + ROWS * BK * 2, &map_x, kb * BK, xr, full_l + 8 * s);
+                    if (++s == C::STAGES) s = 0, ph ^= 1u;
+                }
+            }
+            // every slab issued has been consumed before the CTA's shared memory goes away (a stage never used passes at once; after an
+            // abort the waits give up)
+            for (int i = 0; i < C::STAGES; ++i) {
+                const unsigned long long t0 = now_ns();
+                while (!bar_try(empty + 8 * s, ph) && now_ns() - t0 < WAIT_NS) {}
+                if (++s == C::STAGES) s = 0, ph ^= 1u;
+            }
+        }
+    } else if (warp == 1) {
+        if (rank == 0 && elect()) {
+            const uint32_t idesc = (1u << 4) | (p.bf16 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(BT >> 3) << 17) | ((uint32_t)(2 * ROWS >> 4) << 24);
+            int s = 0, b = 0;
+            uint32_t ph = 0, eph = 1;
+            bool ok = true;
+            for (int t = (int)blockIdx.x >> 1; t < tiles && ok; t += stride) {
+                ok = bar_wait(acc_empty + 8 * b, eph, abort_flag);   // the epilogues of both CTAs have drained this buffer
+                if (!ok) break;
+                fence_after();
+                const uint32_t d = tmem + b * BT;
+                for (int kb = 0; kb < nk; ++kb) {
+                    ok = bar_wait(full + 8 * s, ph, abort_flag);
+                    if (!ok) break;
+                    fence_after();
+                    const uint64_t da = desc_k128(stages + s * C::STAGE), db = desc_k128(stages + s * C::STAGE + ROWS * BK * 2);
+#pragma unroll
+                    for (int kk = 0; kk < BK / 16; ++kk) mma_pair(d, da + 2 * kk, db + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
+                    commit_pair(empty + 8 * s);
+                    if (++s == C::STAGES) s = 0, ph ^= 1u;
+                }
+                if (ok) commit_pair(acc_full + 8 * b);
+                b ^= 1;
+                if (b == 0) eph ^= 1u;
+            }
+        }
+    } else if (warp >= 4) {
+        const int q = warp & 3, half = (warp - 4) >> 2;     // TMEM lane quarter; half of the columns
+        const uint32_t drained = map_leader(acc_empty);
+        int b = 0;
+        uint32_t ph = 0;
+        for (int t = (int)blockIdx.x >> 1; t < tiles; t += stride) {
+            const Tile tl = tile_of<BT>(p, first, MT, t);
+            if (!bar_wait(acc_full + 8 * b, ph, abort_flag)) break;
+            fence_after();
+            const int n = tl.n0 + (int)rank * ROWS + q * 32 + lane;
+            const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + b * BT;
+#pragma unroll 1
+            for (int c = half * (BT / 2); c < (half + 1) * (BT / 2); c += 32) {
+                if (tl.m0 + c >= tl.m_end) break;
+                float v[32];
+                ld32(ta + c, v);
+                ld_wait();
+                epi.store(v, n, tl.m0 + c, tl.m_end, lane);
+            }
+            fence_before();
+            __syncwarp();
+            if (lane == 0) bar_arrive_cluster(drained + 8 * b);
+            b ^= 1;
+            if (b == 0) ph ^= 1u;
+        }
+    }
+    __syncwarp();
+    fence_before();
+    __syncthreads();
+    if (threadIdx.x == 0 && *abort_flag && p.err) atomicOr(p.err, p.err_bit);
+    cluster_sync();   // no CTA leaves while the peer may still signal its barriers or read its shared memory
+    if (warp == 2) {
+        fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(C::TMEM_COLS) : "memory");
+    }
+}
+
+typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                             CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+inline EncodeFn encode_fn() {
+    static EncodeFn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = nullptr;
+        return reinterpret_cast<EncodeFn>(f);
+    }();
+    return fn;
+}
+
+// rows x K 16-bit matrix with row stride ld elements; box = 64 k x box_rows rows, 128-byte swizzle, zero fill outside
+inline bool make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int64_t ld, int box_rows, bool bf16) {
+    EncodeFn fn = encode_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+    const cuuint32_t box[2] = {BK, (cuuint32_t)box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    return fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+inline int pair_sms() {   // SMs of the current device, rounded down to pairs
+    static int sms[16] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev < 16 && sms[dev]) return sms[dev];
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    n &= ~1;
+    if (dev < 16) sms[dev] = n;
+    return n;
+}
+
+// w: [w_rows][K] (row stride ldw), x: [p.M][K] (row stride ldx); p.MT / p.NT are filled in here
+template <int BT, class Epi>
+cudaError_t launch(const void* w, int64_t w_rows, int64_t ldw, const void* x, int64_t ldx, Args p, const Epi& epi, cudaStream_t st) {
+    using C = Cfg<BT>;
+    CUtensorMap mw, mx;
+    if (!make_map(&mw, w, w_rows, p.K, ldw, ROWS, p.bf16 != 0) || !make_map(&mx, x, p.M, p.K, ldx, C::XROWS, p.bf16 != 0)) return cudaErrorInvalidValue;
+    static bool ready[16] = {false};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev >= 16 || !ready[dev]) {
+        e = cudaFuncSetAttribute(pair_gemm_kernel<BT, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+        if (e != cudaSuccess) return e;
+        if (dev < 16) ready[dev] = true;
+    }
+    p.MT = (p.M + BT - 1) / BT + (p.offs ? p.E : 0);
+    p.NT = (p.N + 2 * ROWS - 1) / (2 * ROWS);
+    int64_t ctas = 2 * (int64_t)p.MT * p.NT;
+    const int sms = pair_sms();
+    if (ctas > sms) ctas = sms;
+    pair_gemm_kernel<BT, Epi><<<(unsigned)ctas, THREADS, C::SMEM, st>>>(mw, mx, p, epi);
+    return cudaGetLastError();
+}
+
+}  // namespace tcpair
