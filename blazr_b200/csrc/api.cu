@@ -402,6 +402,8 @@ size_t b200q_workspace_bytes(const b200q_weight* w, int64_t M) {
     size_t mv = align256(matvec_ws_bytes(w, M));
     size_t act = align256(b200q_act_bytes(w->K, M <= 4 ? M : 4));
     size_t gm = align256(gemm_ws_bytes(w, M));
+    const size_t wide = align256(gemm_wide_ws_bytes(w, M));
+    if (wide > gm) gm = wide;
     size_t a = mv + act;
     return a > gm ? a : gm;
 }
@@ -553,6 +555,11 @@ int32_t b200q_matmul_path(const b200q_weight* w, int32_t path, const void* x, in
     if (path == 2) {
         size_t need = align256(gemm_ws_bytes(w, M));
         if (workspace_bytes < need) return fail(B200Q_ERR_WORKSPACE, "workspace too small: %zu < %zu", workspace_bytes, need);
+        const size_t wide = gemm_wide_ws_bytes(w, M);   // large steps; a workspace sized for less keeps the fused kernel
+        if (wide > 0 && workspace_bytes >= wide) {
+            CUDA_TRY(launch_gemm_wide(w, x, x_dtype, M, ldx, y, y_dtype, ldy, (uint8_t*)workspace, st));
+            return B200Q_OK;
+        }
         cudaError_t e = launch_gemm_tc(w, x, x_dtype, M, ldx, y, y_dtype, ldy, (uint8_t*)workspace, workspace_bytes, st);
         if (e == cudaErrorNotSupported) return fail(B200Q_ERR_UNSUPPORTED, "tcgen05 GEMM path not available for this weight/shape");
         if (e != cudaSuccess) return cuda_fail(e, "launch_gemm_tc");

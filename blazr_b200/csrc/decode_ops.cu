@@ -577,6 +577,11 @@ __global__ void embed_kernel(const __half* __restrict__ table, const int64_t* __
     if (k < H) h[(size_t)m * H + k] = __half2float(table[(size_t)ids[m] * H + k]);
 }
 
+int* decode_error_dev() {
+    void* p = nullptr;
+    return cudaGetSymbolAddress(&p, g_decode_error) == cudaSuccess ? (int*)p : nullptr;
+}
+
 }  // namespace b200q
 
 using namespace b200q;

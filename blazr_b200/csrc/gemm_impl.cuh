@@ -189,6 +189,65 @@ __device__ __forceinline__ void unit_to_f16(const Unit& u, uint32_t* out) {
     }
 }
 
+// ---- large steps: packed tiles -> f16 rows [rows][K_pad] in k order, the weight operand of the paired-SM GEMM (gemm_wide.cu) ----
+// Bound by memory: 0.56 - 1.06 bytes read and 2 written per weight (Q6_K, 4608 x 4096: 9.6 us = 5.5 TB/s).  A lane expands one unit (32 k of
+// one row) exactly as the fused kernel does (unit_to_f16: same roundings) and stores it as two whole 32-byte sectors; eight lanes write 512
+// consecutive bytes.  The grid is small enough to be resident beside the GEMM of the panel before (no shared memory), which this launch
+// overlaps: it waits for that GEMM only at its END, so that its own completion implies that the GEMM, whose operand buffer the panel after
+// the next one overwrites, is done.
+__device__ __forceinline__ void st_global_32b(void* p, const uint32_t* v) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+constexpr int DQ16_THREADS = 256;
+template <class F>
+__global__ void __launch_bounds__(DQ16_THREADS) dequant_f16_kernel(const uint8_t* __restrict__ data, int64_t KC, int chunk_bytes, int tile0, int ntiles, __half* __restrict__ out,
+                                                                   int64_t K_pad, FmtMeta meta) {
+    pdl_launch_dependents();
+    const int64_t chunks = (int64_t)ntiles * KC;
+    const int i = threadIdx.x & 7, r0 = threadIdx.x >> 3;
+    for (int64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
+        const int64_t t = c / KC, kc = c - t * KC;
+        const uint8_t* chunk = data + ((tile0 + t) * KC + kc) * chunk_bytes;
+        __half* o = out + (t * TILE_ROWS) * K_pad + kc * CHUNK_K + 32 * i;
+#pragma unroll
+        for (int j = 0; j < TILE_ROWS / (DQ16_THREADS / 8); j++) {
+            const int r = r0 + j * (DQ16_THREADS / 8);
+            Unit u;
+            F::template load_unit<false>(chunk, r, i, u, meta);
+            uint32_t pk[16], nat[16];
+            unit_to_f16<F::SIGNED>(u, pk);
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                nat[2 * k] = __byte_perm(pk[2 * k], pk[2 * k + 1], 0x5410);
+                nat[2 * k + 1] = __byte_perm(pk[2 * k], pk[2 * k + 1], 0x7632);
+            }
+            __half* dst = o + (int64_t)r * K_pad;
+            st_global_32b(dst, nat);
+            st_global_32b(dst + 16, nat + 8);
+        }
+    }
+    pdl_wait();
+}
+template <int FAMILY>
+cudaError_t dequant_f16_launch(const b200q_weight* w, int tile0, int ntiles, __half* out, cudaStream_t st);
+template <class F>
+static cudaError_t launch_dequant_f16(const b200q_weight* w, int tile0, int ntiles, __half* out, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    const int64_t chunks = (int64_t)ntiles * w->KC, most = 2 * (int64_t)w->num_sms;   // two blocks are resident beside a GEMM CTA; more would queue behind blocks that wait
+    cfg.gridDim = dim3((unsigned)(chunks < most ? chunks : most));
+    cfg.blockDim = dim3(DQ16_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, dequant_f16_kernel<F>, (const uint8_t*)w->data, w->KC, w->chunk_bytes, tile0, ntiles, out, w->K_pad, FmtMeta{w->gpc});
+    count_launch();
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
 // EPI: four dedicated epilogue warps (one per TMEM lane quarter) and two accumulator buffers (Mt <= 128), so the
 // dequant warps start the next work item while the previous accumulator drains -- skinny launches are made of many
 // short items and the drain (MMA latency + tcgen05.ld + global stores) otherwise sits between every pair of them.

@@ -319,28 +319,21 @@ struct EpiGated {
 using tcpair::encode_fn;
 using tcpair::make_map;
 
-// Which tile: estimated cycles of the last pair to finish.  A 256 x 256 tile keeps the tensor pipe of both SMs busy for K * 8 cycles, a
-// 256 x 128 one for K * 4 at a lower rate (measured, 4096 x 6144 x 4096: 11 waves of the narrow tile 156 us, 6 of the wide one 152 us, that is
-// 14.2 against 25.4 us a wave), so the narrow one wins where its finer grain saves a wave (1024 x 6144 x 4096: 45.0 against 49.7 us) and in
-// steps of few tokens (256 x 2048 x 8192: 26 against 45 us).  Per-head products (K and N of one head) stay on the single-SM kernel.
-enum { TILE_SINGLE = 0, TILE_PAIR128 = 128, TILE_PAIR256 = 256 };
+// Token rows per tile of the paired-SM kernel; 0: the product stays on the single-SM kernel (per-head products: K and N of one head)
 int pick_tile(const TcParams& p) {
     const int64_t pairs = tcpair::pair_sms() / 2;
-    if (p.heads || pairs < 1 || (p.offs && p.E > tcpair::MAX_GROUPS)) return TILE_SINGLE;
-    auto waves = [&](int bt) {   // grouped: every group's last tile is half full on average
+    if (p.heads || pairs < 1 || (p.offs && p.E > tcpair::MAX_GROUPS)) return 0;
+    return tcpair::pick_bt(pairs, p.K, [&](int bt) {   // grouped: every group's last tile is half full on average
         const int64_t mt = p.offs ? (p.M + bt / 2 * (int64_t)p.E + bt - 1) / bt : (p.M + bt - 1) / bt;
-        return (double)((mt * ((p.N + 255) / 256) + pairs - 1) / pairs);
-    };
-    const double narrow = waves(128) * (p.K * 4 / 0.75 + 200), wide = waves(256) * (p.K * 8 / 0.84 + 200) + 2000;
-    return wide <= narrow ? TILE_PAIR256 : TILE_PAIR128;
+        return mt * ((p.N + 255) / 256);
+    });
 }
 
 template <class Epi>
-cudaError_t launch_pair(int tile, const void* x, int64_t ldx, const void* w, const TcParams& p, const Epi& epi, cudaStream_t st) {
+cudaError_t launch_pair(int bt, const void* x, int64_t ldx, const void* w, const TcParams& p, const Epi& epi, cudaStream_t st) {
     tcpair::Args a{};
-    a.M = p.M, a.N = p.N, a.K = p.K, a.offs = p.offs, a.E = p.offs ? p.E : 1, a.bf16 = 1, a.err = p.err, a.err_bit = 2;
-    const int64_t rows = p.offs ? (int64_t)p.E * p.N : p.N;
-    return tile == TILE_PAIR256 ? tcpair::launch<256>(w, rows, p.K, x, ldx, a, epi, st) : tcpair::launch<128>(w, rows, p.K, x, ldx, a, epi, st);
+    a.M = p.M, a.N = p.N, a.K = p.K, a.offs = p.offs, a.E = p.offs ? p.E : 1, a.bf16 = 1, a.bt = bt, a.err = p.err, a.err_bit = 2;
+    return tcpair::launch(w, p.offs ? (int64_t)p.E * p.N : p.N, p.K, x, ldx, a, epi, st);
 }
 
 int launch(const void* x, int64_t ldx, const void* w, TcParams p, cudaStream_t st) {

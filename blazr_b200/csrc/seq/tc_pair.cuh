@@ -7,7 +7,7 @@
 // (128-byte swizzle); rows and k outside the matrices read as zero.
 //
 // The kernel is persistent (one pair per two SMs, tiles dealt round-robin, token tiles fastest so that a weight tile is read from HBM
-// once) and the accumulator is double-buffered in TMEM (2 x BT columns): the eight epilogue warps drain tile i while the tensor cores run
+// once) and the accumulator is double-buffered in TMEM (2 x 256 columns): the eight epilogue warps drain tile i while the tensor cores run
 // tile i + 1.  What bounds it is the tensor pipe; the single-SM kernel it replaces for large steps stalled on L2 -> SM traffic (512 bytes
 // per 32 768 FLOPs against 1 024 per 131 072 here) and on a main loop that its epilogue interrupted.  Measured, 4096 tokens: 16384 x 2048 267 ->
 // 198 us (1.39 PFLOP/s), with the gated activation 478 -> 201 us; 2048 x 8192 128 -> 100 us; 8192 x 1024 91 -> 61 us.
@@ -32,17 +32,18 @@ constexpr int HDR = 1024;
 constexpr int MAX_GROUPS = 1024;
 constexpr unsigned long long WAIT_NS = 2000000000ull;
 
-template <int BT>
-struct Cfg {
-    static constexpr int XROWS = BT / 2;                           // token rows in each CTA's shared memory
-    static constexpr int STAGE = (ROWS + XROWS) * BK * 2;          // bytes per stage and CTA
-    static constexpr int STAGES = (192 * 1024) / STAGE;            // 6 (BT = 256) or 8 (BT = 128)
-    static constexpr int SMEM = STAGES * STAGE + HDR + 1024 + (MAX_GROUPS + 1) * 4;
-    static constexpr int TMEM_COLS = 2 * BT;
-};
+constexpr int MAX_BT = 256;
+constexpr int ACC_STRIDE = MAX_BT;       // TMEM columns between the two accumulator buffers
+constexpr int RING = 192 * 1024;         // bytes of operand stages
+constexpr int MAX_STAGES = 9;
+constexpr int SMEM = RING + HDR + 1024 + (MAX_GROUPS + 1) * 4;
+constexpr int TMEM_COLS = 2 * ACC_STRIDE;
+__host__ __device__ constexpr int stage_bytes(int bt) { return ROWS * BK * 2 + bt / 2 * BK * 2; }   // per CTA
+__host__ __device__ constexpr int stage_count(int bt) { return RING / stage_bytes(bt) < MAX_STAGES ? RING / stage_bytes(bt) : MAX_STAGES; }
 
 struct Args {
     int M, N, K;             // token rows, weight rows of one group, reduction length
+    int bt;                  // token rows per tile: a multiple of 32, at most 256
     int MT, NT;              // token tiles (bound when grouped), weight tiles of 256
     const int32_t* offs;     // grouped form: [E + 1] first token row of every group; group e uses the weight rows e * N ..
     int E;
@@ -144,9 +145,9 @@ struct Tile {
 };
 
 // tile t of the step (token tiles fastest).  first: grouped form, [E + 1] first token tile of every group
-template <int BT>
 __device__ __forceinline__ Tile tile_of(const Args& p, const int32_t* first, int MT, int t) {
     Tile r;
+    const int BT = p.bt;
     const int mt = t % MT, nt = t / MT;
     r.n0 = nt * 2 * ROWS;
     r.wrow = r.n0;
@@ -167,27 +168,31 @@ __device__ __forceinline__ Tile tile_of(const Args& p, const int32_t* first, int
 
 // Epi: struct with   __device__ void store(const float (&v)[32], int n, int m, int m_end, int lane) const
 //   v[j] = acc[n][m + j] of this lane's n (n may be >= N: nothing is stored); all 32 lanes of a warp call it with the same m
-template <int BT, class Epi>
+template <class Epi>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     pair_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Args p, const Epi epi) {
-    using C = Cfg<BT>;
     extern __shared__ uint8_t smem_raw[];
+    const int BT = p.bt, STAGE = stage_bytes(BT), STAGES = stage_count(BT);
     const uint32_t base = (sa(smem_raw) + 1023u) & ~1023u;
-    const uint32_t full = base, empty = full + 8 * C::STAGES, acc_full = empty + 8 * C::STAGES, acc_empty = acc_full + 16;
+    const uint32_t full = base, empty = full + 8 * MAX_STAGES, acc_full = empty + 8 * MAX_STAGES, acc_empty = acc_full + 16;
     uint8_t* hdr = smem_raw + (base - sa(smem_raw));
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(hdr + 512);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(hdr + 520);
-    int32_t* first = reinterpret_cast<int32_t*>(hdr + HDR + C::STAGES * C::STAGE);
+    int32_t* first = reinterpret_cast<int32_t*>(hdr + HDR + RING);
     const uint32_t stages = base + HDR;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t rank;
     asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(rank));
     if (threadIdx.x == 0) {
-        for (int s = 0; s < C::STAGES; ++s) bar_init(full + 8 * s, 1), bar_init(empty + 8 * s, 1);
+        for (int s = 0; s < STAGES; ++s) bar_init(full + 8 * s, 1), bar_init(empty + 8 * s, 1);
         for (int b = 0; b < 2; ++b) bar_init(acc_full + 8 * b, 1), bar_init(acc_empty + 8 * b, 2 * EPI_WARPS);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    // programmatic launch: the operands (and what they were made from) are complete beyond this line, and what follows in the stream may start
+    // (both are no-ops in a plain launch)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     int MT = p.MT;
     if (p.offs && warp == 3) {   // first token tile of every group: an inclusive scan over the groups, 32 at a time
         int run = 0;
@@ -205,7 +210,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         if (lane == 0) first[0] = 0;
     }
     if (warp == 2) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sa(tmem_ptr)), "n"(C::TMEM_COLS) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sa(tmem_ptr)), "n"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     fence_before();
@@ -224,24 +229,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             uint32_t ph = 1;
             bool ok = true;
             for (int t = (int)blockIdx.x >> 1; t < tiles && ok; t += stride) {
-                const Tile tl = tile_of<BT>(p, first, MT, t);
-                const int wr = tl.wrow + (int)rank * ROWS, xr = tl.m0 + (int)rank * C::XROWS;
+                const Tile tl = tile_of(p, first, MT, t);
+                const int wr = tl.wrow + (int)rank * ROWS, xr = tl.m0 + (int)rank * (BT / 2);
                 for (int kb = 0; kb < nk; ++kb) {
                     ok = bar_wait(empty + 8 * s, ph, abort_flag);
                     if (!ok) break;
-                    if (rank == 0) bar_expect(full + 8 * s, 2 * C::STAGE);
-                    const uint32_t st = stages + s * C::STAGE;
+                    if (rank == 0) bar_expect(full + 8 * s, 2 * STAGE);
+                    const uint32_t st = stages + s * STAGE;
                     tma_pair(st, &map_w, kb * BK, wr, full_l + 8 * s);
                     tma_pair(st + ROWS * BK * 2, &map_x, kb * BK, xr, full_l + 8 * s);
-                    if (++s == C::STAGES) s = 0, ph ^= 1u;
+                    if (++s == STAGES) s = 0, ph ^= 1u;
                 }
             }
             // every slab issued has been consumed before the CTA's shared memory goes away (a stage never used passes at once; after an
             // abort the waits give up)
-            for (int i = 0; i < C::STAGES; ++i) {
+            for (int i = 0; i < STAGES; ++i) {
                 const unsigned long long t0 = now_ns();
                 while (!bar_try(empty + 8 * s, ph) && now_ns() - t0 < WAIT_NS) {}
-                if (++s == C::STAGES) s = 0, ph ^= 1u;
+                if (++s == STAGES) s = 0, ph ^= 1u;
             }
         }
     } else if (warp == 1) {
@@ -254,16 +259,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                 ok = bar_wait(acc_empty + 8 * b, eph, abort_flag);   // the epilogues of both CTAs have drained this buffer
                 if (!ok) break;
                 fence_after();
-                const uint32_t d = tmem + b * BT;
+                const uint32_t d = tmem + b * ACC_STRIDE;
                 for (int kb = 0; kb < nk; ++kb) {
                     ok = bar_wait(full + 8 * s, ph, abort_flag);
                     if (!ok) break;
                     fence_after();
-                    const uint64_t da = desc_k128(stages + s * C::STAGE), db = desc_k128(stages + s * C::STAGE + ROWS * BK * 2);
+                    const uint64_t da = desc_k128(stages + s * STAGE), db = desc_k128(stages + s * STAGE + ROWS * BK * 2);
 #pragma unroll
                     for (int kk = 0; kk < BK / 16; ++kk) mma_pair(d, da + 2 * kk, db + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
                     commit_pair(empty + 8 * s);
-                    if (++s == C::STAGES) s = 0, ph ^= 1u;
+                    if (++s == STAGES) s = 0, ph ^= 1u;
                 }
                 if (ok) commit_pair(acc_full + 8 * b);
                 b ^= 1;
@@ -271,18 +276,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             }
         }
     } else if (warp >= 4) {
-        const int q = warp & 3, half = (warp - 4) >> 2;     // TMEM lane quarter; half of the columns
+        const int q = warp & 3, half = (warp - 4) >> 2;     // TMEM lane quarter; every other group of 32 columns
         const uint32_t drained = map_leader(acc_empty);
         int b = 0;
         uint32_t ph = 0;
         for (int t = (int)blockIdx.x >> 1; t < tiles; t += stride) {
-            const Tile tl = tile_of<BT>(p, first, MT, t);
+            const Tile tl = tile_of(p, first, MT, t);
             if (!bar_wait(acc_full + 8 * b, ph, abort_flag)) break;
             fence_after();
             const int n = tl.n0 + (int)rank * ROWS + q * 32 + lane;
-            const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + b * BT;
+            const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + b * ACC_STRIDE;
 #pragma unroll 1
-            for (int c = half * (BT / 2); c < (half + 1) * (BT / 2); c += 32) {
+            for (int c = half * 32; c < BT; c += 64) {
                 if (tl.m0 + c >= tl.m_end) break;
                 float v[32];
                 ld32(ta + c, v);
@@ -303,7 +308,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     cluster_sync();   // no CTA leaves while the peer may still signal its barriers or read its shared memory
     if (warp == 2) {
         fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(C::TMEM_COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TMEM_COLS) : "memory");
     }
 }
 
@@ -344,28 +349,49 @@ inline int pair_sms() {   // SMs of the current device, rounded down to pairs
     return n;
 }
 
-// w: [w_rows][K] (row stride ldw), x: [p.M][K] (row stride ldx); p.MT / p.NT are filled in here
-template <int BT, class Epi>
-cudaError_t launch(const void* w, int64_t w_rows, int64_t ldw, const void* x, int64_t ldx, Args p, const Epi& epi, cudaStream_t st) {
-    using C = Cfg<BT>;
+// Estimated time of one wave of tiles (us): per k a part for the weight rows and a part that grows with the token rows (measured at K = 4096:
+// 25.4 us for 256 token rows, 14.2 us for 128), and a fixed part that keeps short products on wide tiles (32 experts of 512 rows, K = 1024:
+// 236 us with 256 token rows, 249 us with 160).
+inline double wave_us(int bt, int64_t K) { return (3.0 + 0.0875 * bt) * (double)K / 4096.0 + 0.6; }
+
+// Token rows per tile: the size whose last wave is not nearly empty and whose rows are not padding.  tiles(bt): number of tiles of the step
+template <class Tiles>
+inline int pick_bt(int64_t pairs, int64_t K, Tiles tiles) {
+    int best = MAX_BT;
+    double best_t = 0;
+    for (int bt = MAX_BT; bt >= 32; bt -= 32) {
+        const double t = (double)((tiles(bt) + pairs - 1) / pairs) * wave_us(bt, K);
+        if (bt == MAX_BT || t < best_t) best = bt, best_t = t;
+    }
+    return best;
+}
+
+// w: [w_rows][K] (row stride ldw), x: [p.M][K] (row stride ldx); p.bt is set, p.MT / p.NT are filled in here
+template <class Epi>
+cudaError_t launch(const void* w, int64_t w_rows, int64_t ldw, const void* x, int64_t ldx, Args p, const Epi& epi, cudaStream_t st, bool pdl = false) {
     CUtensorMap mw, mx;
-    if (!make_map(&mw, w, w_rows, p.K, ldw, ROWS, p.bf16 != 0) || !make_map(&mx, x, p.M, p.K, ldx, C::XROWS, p.bf16 != 0)) return cudaErrorInvalidValue;
+    if (!make_map(&mw, w, w_rows, p.K, ldw, ROWS, p.bf16 != 0) || !make_map(&mx, x, p.M, p.K, ldx, p.bt / 2, p.bf16 != 0)) return cudaErrorInvalidValue;
     static bool ready[16] = {false};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev >= 16 || !ready[dev]) {
-        e = cudaFuncSetAttribute(pair_gemm_kernel<BT, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+        e = cudaFuncSetAttribute(pair_gemm_kernel<Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         if (e != cudaSuccess) return e;
         if (dev < 16) ready[dev] = true;
     }
-    p.MT = (p.M + BT - 1) / BT + (p.offs ? p.E : 0);
+    p.MT = (p.M + p.bt - 1) / p.bt + (p.offs ? p.E : 0);
     p.NT = (p.N + 2 * ROWS - 1) / (2 * ROWS);
     int64_t ctas = 2 * (int64_t)p.MT * p.NT;
     const int sms = pair_sms();
     if (ctas > sms) ctas = sms;
-    pair_gemm_kernel<BT, Epi><<<(unsigned)ctas, THREADS, C::SMEM, st>>>(mw, mx, p, epi);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = SMEM, cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization, attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr, cfg.numAttrs = pdl ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, pair_gemm_kernel<Epi>, mw, mx, p, epi);
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace tcpair
