@@ -8,26 +8,9 @@
 //           in the same soft-max); scores, soft-max and the weighted sum in f32; optional per-head sigmoid gate.
 // A row's result depends on the token's position and on its sequence's pages only; the rest of the batch changes at most how the
 // keys are split among blocks (rounding).
-#include "seq_common.cuh"
+#include "seq_attn.cuh"
 
 namespace b200seq {
-
-__device__ __forceinline__ int64_t kv_row(const b200seq_step& st, int e, int pos, int* err) {
-    const int b = pos / st.block_size;
-    if (b >= st.max_blocks || pos < 0) {
-        atomicOr(err, 1);
-        return -1;
-    }
-    return (int64_t)st.block_table[(int64_t)e * st.max_blocks + b] * st.block_size + pos % st.block_size;
-}
-
-// pooled entry of block b (positions b * P .. b * P + P - 1) of a sequence: it lives in the page of the block's first position, at
-// the block's rank among the blocks that start in that page
-__device__ __forceinline__ int64_t pooled_row(const int32_t* bt, int bs, int P, int ppp, int b) {
-    const int pg = (b * P) / bs;
-    const int first = (pg * bs + P - 1) / P;
-    return (int64_t)bt[pg] * ppp + (b - first);
-}
 
 // mean key and mean value of block b (positions b * P .. b * P + P - 1) from the pool's rows, summed in position order
 // (columns c0, c0 + cstep, ... of the G * D key columns followed by the G * V value columns)
@@ -368,51 +351,6 @@ __global__ void latent_gather_kernel(const float* __restrict__ kpool, int64_t kl
 // the GPU (decode); the partial (maximum, sum, weighted values) of each split is merged by attn_merge_kernel.
 constexpr int AT_KT = 64;
 constexpr int AT_NT = 256;
-
-struct AttnArgs {
-    const float* qkvg;
-    int64_t ld;
-    const float *kpool, *vpool;
-    const float *kpp, *vpp;   // pooled keys / values, pool > 0
-    int pool, ppp;            // positions per pooled block; pooled entries per page
-    int q_col, gate_col;
-    int H, G, D, V, Rb, HB, QT, nsplit, share_kv;   // share_kv: V tiles reuse the K tile's shared memory (large heads: more blocks per SM)
-    float scale;
-    int chunk, window, gated;
-    void* out;
-    int out_dtype;
-    float* part;   // [T][H][nsplit][V + 2] when nsplit > 1
-    int* err;
-    const float* sink;   // [H] or null: exp(sink[h]) joins the soft-max denominator of head h once; it has no key and no value
-    const float* gate;   // gate logits [T][gld] (+ h)
-    int64_t gld;
-    int64_t kld, vld;    // floats per position in kpool / vpool (G * D and G * V, or the key row's width when the values lie inside the key rows)
-    int ctx_rows;        // 1: kpool / vpool rows are the step's gathered context, entry after entry, position after position (no pages)
-    int kd;              // floats of a key head that lie in kpool (at g * kd); the remaining D - kd come from krot, one part for all heads
-    const float* krot;   // paged rows of krld floats (pointer already at the part's first column), or null
-    int64_t krld;
-    const float* head_scale;   // [H] or null: one more factor of head h's scores
-    float softcap;             // > 0: score <- softcap * tanh(score / softcap)
-    int keep_first;            // with a window: positions below this stay visible to all later positions
-    int vdiv;                  // key head g reads value head g / vdiv
-    int gate_elem;             // the gate has one logit per output element: gate[t * gld + h * V + c]
-};
-
-__device__ __forceinline__ bool attn_find_tile(const b200seq_step& st, int idx, int QT, int& e, int& t0, int& nq) {
-    int acc = 0;
-    for (e = 0; e < st.B; ++e) {
-        const int s0 = st.ent_start[e], n = st.ent_start[e + 1] - s0;
-        const int nt = (n + QT - 1) / QT;
-        if (idx < acc + nt) {
-            const int local = idx - acc;
-            t0 = s0 + local * QT;
-            nq = min(QT, n - local * QT);
-            return true;
-        }
-        acc += nt;
-    }
-    return false;
-}
 
 __device__ __forceinline__ float dot4(const float4 a, const float4 b, float acc) {
     acc = fmaf(a.x, b.x, acc), acc = fmaf(a.y, b.y, acc), acc = fmaf(a.z, b.z, acc), acc = fmaf(a.w, b.w, acc);
@@ -817,6 +755,16 @@ int b200seq_attn_ex(const float* qkvg, int64_t ld, const b200seq_step* st, const
                d->kv_ld > 0 ? d->kv_ld : (d->latent_v ? (int64_t)G * D : (int64_t)(d->vg > 0 ? d->vg : G) * V), d->ctx_rows, (d->kd > 0 && d->kd < D) ? d->kd : D, d->krot, d->krot_ld,
                d->head_scale, d->softcap, d->keep_first, d->vg > 0 ? G / d->vg : 1, (gated && d->gate_elem) ? 1 : 0};
     if (d->latent_v) a.vpool = kpool;
+    cudaStream_t cs = (cudaStream_t)stream;
+    auto merge = [&]() -> int {
+        if (a.nsplit > 1) {
+            attn_merge_kernel<<<dim3(st->T, H), V <= 64 ? 64 : 128, 0, cs>>>(a);
+            SEQ_LAUNCH_CHECK("attn merge");
+        }
+        return 0;
+    };
+    int rc = 0;
+    if (launch_attn_tc(a, *st, max_keys, scratch ? scratch_floats : 0, cs, rc)) return rc ? rc : merge();
     const int VPT = V <= 64 ? 4 : (V <= 128 ? 8 : (V <= 256 ? 16 : 32));
     if (VPT == 32 && p.RT != 1) return fail(B200SEQ_ERR_UNSUPPORTED, "attn: value sizes above 256 only in steps of few tokens (one query row per thread)");
     const int RQ = 16 * p.RT, QS = ((D + 3) & ~3) + 4;
@@ -828,7 +776,6 @@ int b200seq_attn_ex(const float* qkvg, int64_t ld, const b200seq_step* st, const
     }
     if (smem > 220 * 1024) return fail(B200SEQ_ERR_UNSUPPORTED, "attn: head size too large");
     dim3 grid(p.tiles, G * p.HB, p.nsplit);
-    cudaStream_t cs = (cudaStream_t)stream;
     cudaError_t e = cudaSuccess;
 #define ATT_LAUNCH(RT_, VPT_)                                                                                                   \
     do {                                                                                                                        \
@@ -852,11 +799,7 @@ int b200seq_attn_ex(const float* qkvg, int64_t ld, const b200seq_step* st, const
 #undef ATT_LAUNCH
     if (e != cudaSuccess) return cuda_status(e, "attn attribute");
     SEQ_LAUNCH_CHECK("attn");
-    if (p.nsplit > 1) {
-        attn_merge_kernel<<<dim3(st->T, H), V <= 64 ? 64 : 128, 0, cs>>>(a);
-        SEQ_LAUNCH_CHECK("attn merge");
-    }
-    return 0;
+    return merge();
 }
 
 int b200seq_attn(const float* qkvg, int64_t ld, const b200seq_step* st, const float* kpool, const float* vpool, int H, int G, int D, int V, float scale,
