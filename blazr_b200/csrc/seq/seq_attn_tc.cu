@@ -10,10 +10,10 @@
 // One CTA works on MT tiles of 128 (token, query head) rows of one key head against tiles of 64 keys.  MT = 2 (heads up to 64): the two row
 // tiles alternate, one in the soft-max while the other is in the tensor pipe; MT = 1 (heads up to 128): consecutive key tiles alternate.
 //   warps 0 .. 4 MT - 1    soft-max: a thread owns a row -- its maximum, sum and value sums stay in registers, nothing is shuffled
-//   next 4 warps           loaders: K and V rows through the block table, split into bf16 planes, 128-byte swizzled (K: k-major, V: mn-major)
+//   next 8 warps           loaders: K and V rows through the block table, split into bf16 planes, 128-byte swizzled (K: k-major, V: mn-major)
 //   last 4 warps           the first of them issues the MMAs
-// Register split (setmaxnreg, per thread): launched with 128 (MT = 2) or 168 (MT = 1) for all; soft-max 184 / 240, loaders 104 / 120, issuer 40: the
-// sums (2 * 184 + 104 + 40 = 4 * 128, 240 + 120 + 40 < 3 * 168) stay within what the block was launched with.
+// Register split (setmaxnreg, per thread): launched with 96 (MT = 2) or 128 (MT = 1) for all; soft-max 160 / 240, loaders 64 / 104, issuer 32 / 64:
+// the sums (2 * 160 + 2 * 64 + 32 = 5 * 96, 240 + 2 * 104 + 64 = 4 * 128) are what the block was launched with.
 // TMEM: two slots of 96 columns (scores f32 [64], then the weights' three planes in the same columns), the value tile of every row tile,
 // and the queries' planes (the A operand of the scores comes from TMEM: from shared memory its reads alone would take longer than the MMA).
 // What bounds it: the tensor pipe, 6 x the products (D = V = 64: 1536 cycles per 128 x 64 scores), with the soft-max beside it at about 10
@@ -80,6 +80,39 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& p1, uint32_t&
     const float sa_ = ra - __uint_as_float(p2 << 16), sb_ = rb - __uint_as_float(p2 & 0xFFFF0000u);
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p3) : "f"(sb_), "f"(sa_));
 }
+// packed pairs of f32 (one instruction for both)
+__device__ __forceinline__ uint64_t pk(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void upk(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// a pair of weights (>= 0) -> three packed bf16 pairs by truncation: 8 + 8 + 8 significant bits, no conversion instruction
+__device__ __forceinline__ void cut2(float x, float y, uint64_t minus1, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
+    const float x1 = __uint_as_float(__float_as_uint(x) & 0xFFFF0000u), y1 = __uint_as_float(__float_as_uint(y) & 0xFFFF0000u);
+    float rx, ry, sx, sy;
+    upk(fma2(pk(x1, y1), minus1, pk(x, y)), rx, ry);
+    const float x2 = __uint_as_float(__float_as_uint(rx) & 0xFFFF0000u), y2 = __uint_as_float(__float_as_uint(ry) & 0xFFFF0000u);
+    upk(fma2(pk(x2, y2), minus1, pk(rx, ry)), sx, sy);
+    p1 = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+    p2 = __byte_perm(__float_as_uint(rx), __float_as_uint(ry), 0x7632);
+    p3 = __byte_perm(__float_as_uint(sx), __float_as_uint(sy), 0x7632);
+}
 __device__ __forceinline__ void sts8(uint32_t addr, uint32_t x, uint32_t y) { asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(x), "r"(y) : "memory"); }
 // mn-major operand, 128-byte swizzle: rows (k) of 128 bytes = 64 consecutive mn, 8-row groups 1024 bytes apart, the next 64 mn `lbo` bytes on
 __device__ __forceinline__ uint64_t desc_mn128(uint32_t a, uint32_t lbo) {
@@ -109,14 +142,17 @@ __device__ __forceinline__ int64_t pooled_slot(const int32_t* bt, int bs, int P,
     return (int64_t)bt[pg] * ppp + (b - (pg * bs + P - 1) / P);
 }
 
-template <int MT, int VM>
-__global__ void __launch_bounds__((4 * MT + 8) * 32, 1) attn_tc_kernel(const AttnArgs a, const b200seq_step st) {
+// DK: head size / 16, or 0 for a run-time one; CAP: scores are soft-capped.  The loops are kept short: with the soft-max in two unrolled passes,
+// two copies of the loader and the issuer unrolled over four steps the kernel waited for instructions (ncu: no_instruction the largest stall,
+// 0.21 instructions per cycle) and took 870 us where it now takes a fraction (4096 tokens, heads of 64).
+template <int MT, int VM, int DK, bool CAP>
+__global__ void __launch_bounds__((4 * MT + 12) * 32, 1) attn_tc_kernel(const AttnArgs a, const b200seq_step st) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint32_t tmem_base;
     __shared__ int abort_sh;
     __shared__ __align__(8) uint64_t bars[16];
     const uint32_t kv = (sa(smem_raw) + 1023u) & ~1023u;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // warp-uniform: the roles branch on it
     const int D = a.D, V = a.V, H = a.H, G = a.G;
     const int KB = (D + 63) >> 6, VB = (V + 63) >> 6;
     const uint32_t kbytes = KB * 3 * PLANE, vbytes = VB * 3 * PLANE, stage = kbytes + vbytes;
@@ -139,7 +175,7 @@ __global__ void __launch_bounds__((4 * MT + 8) * 32, 1) attn_tc_kernel(const Att
     const int ntile = kt.total > split ? (kt.total - split + a.nsplit - 1) / a.nsplit : 0;   // tiles split, split + nsplit, ...
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) {
-            bar_init(k_full + 8 * i, 4), bar_init(k_free + 8 * i, 1), bar_init(v_full + 8 * i, 4), bar_init(v_free + 8 * i, 1);
+            bar_init(k_full + 8 * i, 8), bar_init(k_free + 8 * i, 1), bar_init(v_full + 8 * i, 8), bar_init(v_free + 8 * i, 1);
             bar_init(s_full + 8 * i, 1), bar_init(p_ready + 8 * i, 4), bar_init(o_full + 8 * i, 1);
         }
         bar_init(B0 + 112, 1);
@@ -159,30 +195,13 @@ __global__ void __launch_bounds__((4 * MT + 8) * 32, 1) attn_tc_kernel(const Att
 
     if (warp < 4 * MT) {
         // ===================== soft-max: thread == row =====================
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(MT == 2 ? 184 : 240));
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(MT == 2 ? 160 : 240));
         const int m = warp >> 2, q = warp & 3;
         const uint32_t lanes = (uint32_t)(q * 32) << 16;
         const int r = m * 128 + q * 32 + lane;
         const int tq = r / a.Rb, hr = r - tq * a.Rb;
         const bool live = tq < nq && hr < nh;
-        {   // this row's query, split, to TMEM
-            const float* src = a.qkvg + (int64_t)(t0 + tq) * a.ld + a.q_col + (int64_t)(h0 + hr) * D;
-            const uint32_t qa = q0 + lanes + m * qtile;
-            for (int d = 0; d < D; d += 16) {
-                uint32_t p1[8], p2[8], p3[8];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float4 x = live ? ld4(src + d + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    split2(x.x, x.y, p1[2 * j], p2[2 * j], p3[2 * j]);
-                    split2(x.z, x.w, p1[2 * j + 1], p2[2 * j + 1], p3[2 * j + 1]);
-                }
-                st8(qa + (d >> 1), p1), st8(qa + qplane + (d >> 1), p2), st8(qa + 2 * qplane + (d >> 1), p3);
-            }
-            st_wait();
-            fence_before();
-        }
-        asm volatile("bar.sync 1, %0;" ::"n"((4 * MT + 1) * 32) : "memory");   // the queries are in place (with the MMA warp)
-        int rlo = 0, rhi = 0x7fffffff, rnb = 0x7fffffff;   // rows without a token see everything and are not stored
+        int rlo = 0, rhi = 0x3fffffff, rnb = 0x3fffffff;   // rows without a token see everything and are not stored
         float rsc = a.scale;
         const int keep = (a.window > 0 && a.keep_first > 0) ? a.keep_first : 0;
         if (live) {
@@ -193,95 +212,123 @@ __global__ void __launch_bounds__((4 * MT + 8) * 32, 1) attn_tc_kernel(const Att
             rnb = (a.pool > 0 && p - a.window + 1 > 0) ? (p - a.window + 1) / a.pool : 0;
             if (a.head_scale) rsc = a.scale * a.head_scale[h0 + hr];
         }
-        float mx = -INFINITY, l = 0.f, acc[VM];
+        // soft-max in base 2 over raw scores: weight = 2^(c s - mb), mb = c max(s); the sign of the scale goes into the query.  With a soft cap
+        // the scores are scaled and capped first (CAP) and c is log2 e alone.
+        const float sgn = rsc < 0.f ? -1.f : 1.f;
+        const float c = CAP ? LOG2E : fmaxf(fabsf(rsc) * LOG2E, 1e-37f);
+        {   // this row's query, split, to TMEM
+            const float* src = a.qkvg + (int64_t)(t0 + tq) * a.ld + a.q_col + (int64_t)(h0 + hr) * D;
+            const uint32_t qa = q0 + lanes + m * qtile;
+#pragma unroll 1
+            for (int d = 0; d < D; d += 16) {
+                float4 x[4];
 #pragma unroll
-        for (int c = 0; c < VM; ++c) acc[c] = 0.f;
+                for (int j = 0; j < 4; ++j) x[j] = live ? ld4(src + d + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                uint32_t p1[8], p2[8], p3[8];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    split2(x[j].x * sgn, x[j].y * sgn, p1[2 * j], p2[2 * j], p3[2 * j]);
+                    split2(x[j].z * sgn, x[j].w * sgn, p1[2 * j + 1], p2[2 * j + 1], p3[2 * j + 1]);
+                }
+                st8(qa + (d >> 1), p1), st8(qa + qplane + (d >> 1), p2), st8(qa + 2 * qplane + (d >> 1), p3);
+            }
+            st_wait();
+            fence_before();
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"((4 * MT + 1) * 32) : "memory");   // the queries are in place (with the MMA warp)
+        const uint64_t cc = pk(c, c), minus1 = pk(-1.f, -1.f);
+        float mx = -INFINITY, mb = -INFINITY, l = 0.f;
+        uint64_t acc[VM / 2];
+#pragma unroll
+        for (int i = 0; i < VM / 2; ++i) acc[i] = 0;
         bool ok = true;
+#pragma unroll 1
         for (int j = 0; j < ntile && ok; ++j) {
             const int step = j * MT + m, slot = step & 1;
             const int tile = split + j * a.nsplit;
             const bool pooled = tile < kt.npt, first = !pooled && tile < kt.npt + kt.nft;
             const int k0 = pooled ? tile * KT : (first ? (tile - kt.npt) * KT : kt.kbeg + (tile - kt.npt - kt.nft) * KT);
-            const bool whole = __all_sync(0xffffffffu, pooled ? k0 + KT <= rnb : (first ? k0 + KT <= kt.nfirst : (k0 >= rlo && k0 + KT - 1 <= rhi)));
-            auto seen = [&](int kp) { return pooled ? kp < rnb : (first ? kp < kt.nfirst : ((kp >= rlo || kp < keep) && kp <= rhi)); };
+            // visible keys of this row, relative to the tile: [lo, hi1) and, in the window's tiles, those below `kp`
+            const int lo = pooled || first ? 0 : rlo - k0, hi1 = (pooled ? rnb : (first ? kt.nfirst : rhi + 1)) - k0, kp = pooled || first ? 0 : keep - k0;
+            const bool whole = __all_sync(0xffffffffu, lo <= 0 && hi1 >= KT);
             const uint32_t S = slot0 + lanes + slot * SLOT_COLS + 32;   // scores: columns 32 .. 95 of the slot
-            ok = bar_wait(s_full + 8 * slot, (step >> 1) & 1, ab);
+            ok = bar_wait<false>(s_full + 8 * slot, (step >> 1) & 1, ab);
             if (!ok) break;
             fence_after();
-            float v[32];
-            // score of key c of this 32-key half, as the soft-max sees it
-            auto shape = [&](int half) {
+            float v[KT];
+            ld32(S, v);
+            ld32(S + 32, v + 32);
+            ld_wait();
+            if (CAP) {
 #pragma unroll
-                for (int c = 0; c < 32; ++c) v[c] *= rsc;
-                if (a.softcap > 0.f) {
-#pragma unroll
-                    for (int c = 0; c < 32; ++c) v[c] = a.softcap * tanhf(v[c] / a.softcap);
-                }
-                if (!whole) {
-#pragma unroll
-                    for (int c = 0; c < 32; ++c) v[c] = seen(k0 + 32 * half + c) ? v[c] : -INFINITY;
-                }
-            };
-            float mn = mx;
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                ld32(S + 32 * half, v);
-                ld_wait();
-                shape(half);
-                float m0 = v[0], m1 = v[1];
-#pragma unroll
-                for (int c = 2; c < 32; c += 2) m0 = fmaxf(m0, v[c]), m1 = fmaxf(m1, v[c + 1]);
-                mn = fmaxf(mn, fmaxf(m0, m1));
+                for (int i = 0; i < KT; ++i) v[i] = a.softcap * tanhf(v[i] * fabsf(rsc) / a.softcap);
             }
-            const float ms = mn == -INFINITY ? 0.f : mn;
-            const float mb = ms * LOG2E;
-            const float corr = ex2(fmaf(mx, LOG2E, -mb));   // 0 before the first visible key
-            mx = mn;
+            if (!whole) {
+                auto below = [](int n) { return n <= 0 ? 0u : (n >= 32 ? 0xffffffffu : (1u << n) - 1u); };
+                const uint32_t s0 = (below(hi1) & ~below(lo)) | (below(hi1) & below(kp)), s1 = (below(hi1 - 32) & ~below(lo - 32)) | (below(hi1 - 32) & below(kp - 32));
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    v[i] = (s0 >> i) & 1u ? v[i] : -INFINITY;
+                    v[32 + i] = (s1 >> i) & 1u ? v[32 + i] : -INFINITY;
+                }
+            }
+            float m0 = fmaxf(v[0], v[1]), m1 = fmaxf(v[2], v[3]);
+#pragma unroll
+            for (int i = 4; i < KT; i += 4) m0 = fmaxf(m0, fmaxf(v[i], v[i + 1])), m1 = fmaxf(m1, fmaxf(v[i + 2], v[i + 3]));
+            mx = fmaxf(mx, fmaxf(m0, m1));
+            const float mbn = mx * c;
+            const float corr = mx == -INFINITY ? 1.f : ex2(mb - mbn);   // 0 at the first visible key
+            mb = mbn;
+            const float off = mx == -INFINITY ? 0.f : -mbn;
+            const uint64_t off2 = pk(off, off);
+            uint64_t sum = 0;
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4) {   // the weights' planes: columns 48 half + 16 plane (over the scores, which are in registers)
+                uint32_t p1[8], p2[8], p3[8];
+#pragma unroll
+                for (int i = 0; i < 16; i += 2) {
+                    float x, y;
+                    upk(fma2(pk(v[16 * q4 + i], v[16 * q4 + i + 1]), cc, off2), x, y);
+                    x = ex2(x), y = ex2(y);
+                    sum = add2(sum, pk(x, y));
+                    cut2(x, y, minus1, p1[i >> 1], p2[i >> 1], p3[i >> 1]);
+                }
+                const uint32_t P = slot0 + lanes + slot * SLOT_COLS + 48 * (q4 >> 1) + 8 * (q4 & 1);
+                st8(P, p1), st8(P + 16, p2), st8(P + 32, p3);
+            }
+            float sx, sy;
+            upk(sum, sx, sy);
+            l = fmaf(l, corr, sx + sy);
             if (j > 0) {   // the value tile of the key tile before
                 const int ps = (step - MT) & 1;
-                ok = bar_wait(o_full + 8 * ps, ((step - MT) >> 1) & 1, ab);
+                ok = bar_wait<false>(o_full + 8 * ps, ((step - MT) >> 1) & 1, ab);
                 if (!ok) break;
                 fence_after();
+                const uint64_t corr2 = pk(corr, corr);
                 const bool same = __all_sync(0xffffffffu, corr == 1.f);
 #pragma unroll
-                for (int c = 0; c < VM; c += 16) {
-                    if (c >= V) break;
+                for (int i = 0; i < VM; i += 16) {
+                    if (i >= V) break;
                     float o[16];
-                    ld16(o0 + lanes + m * VM + c, o);
+                    ld16(o0 + lanes + m * VM + i, o);
                     ld_wait();
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) acc[c + i] += o[i];
-                    if (!same) {
+                    for (int u = 0; u < 16; u += 2) acc[(i + u) >> 1] = add2(acc[(i + u) >> 1], pk(o[u], o[u + 1]));
+                }
+                if (!same) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) acc[c + i] *= corr;
-                    }
+                    for (int i = 0; i < VM / 2; ++i) acc[i] = mul2(acc[i], corr2);
                 }
             }
-            float sum0 = 0.f, sum1 = 0.f;
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {   // the weights' planes: columns 48 half + 16 plane (over scores that are no longer needed)
-                ld32(S + 32 * half, v);
-                ld_wait();
-                shape(half);
-                uint32_t p1[16], p2[16], p3[16];
-#pragma unroll
-                for (int c = 0; c < 32; c += 2) {
-                    const float x = ex2(fmaf(v[c], LOG2E, -mb)), y = ex2(fmaf(v[c + 1], LOG2E, -mb));
-                    sum0 += x, sum1 += y;
-                    split2(x, y, p1[c >> 1], p2[c >> 1], p3[c >> 1]);
-                }
-                const uint32_t P = slot0 + lanes + slot * SLOT_COLS + 48 * half;
-                st16(P, p1), st16(P + 16, p2), st16(P + 32, p3);
-            }
-            l = fmaf(l, corr, sum0 + sum1);
             st_wait();
             fence_before();
             __syncwarp();
             if (lane == 0) bar_arrive(p_ready + 8 * slot);
         }
+        if (!CAP && mx != -INFINITY) mx = mb / LOG2E;   // in the units of the scores, for the sink and the merge of key splits
         if (ok && ntile > 0) {
             const int step = (ntile - 1) * MT + m;
-            ok = bar_wait(o_full + 8 * (step & 1), (step >> 1) & 1, ab);
+            ok = bar_wait<false>(o_full + 8 * (step & 1), (step >> 1) & 1, ab);
             fence_after();
         }
         if (ok) {
@@ -302,142 +349,191 @@ __global__ void __launch_bounds__((4 * MT + 8) * 32, 1) attn_tc_kernel(const Att
                 if (live) pp[0] = mx, pp[1] = l;
             }
 #pragma unroll
-            for (int c = 0; c < VM; c += 16) {
-                if (c >= V) break;
+            for (int cb = 0; cb < VM; cb += 16) {
+                if (cb >= V) break;
                 float o[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) o[i] = 0.f;
                 if (ntile > 0) {
-                    ld16(o0 + lanes + m * VM + c, o);
+                    ld16(o0 + lanes + m * VM + cb, o);
                     ld_wait();
                 }
                 if (!live) continue;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const float x = acc[c + i] + o[i];
-                    if (pp) pp[2 + c + i] = x;
-                    else o[i] = x * f * (a.gate_elem ? sigmoidf_acc(a.gate[(int64_t)t * a.gld + (int64_t)h * V + c + i]) : 1.f);
+                    float x, x1;
+                    upk(acc[(cb + i) >> 1], x, x1);
+                    x = ((i & 1) ? x1 : x) + o[i];
+                    if (pp) pp[2 + cb + i] = x;
+                    else o[i] = x * f * (a.gate_elem ? sigmoidf_acc(a.gate[(int64_t)t * a.gld + (int64_t)h * V + cb + i]) : 1.f);
                 }
                 if (!pp) {
 #pragma unroll
-                    for (int i = 0; i < 16; i += 4) store_act4(a.out, a.out_dtype, ((int64_t)t * H + h) * V + c + i, make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]));
+                    for (int i = 0; i < 16; i += 4) store_act4(a.out, a.out_dtype, ((int64_t)t * H + h) * V + cb + i, make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]));
                 }
             }
         }
-    } else if (warp < 4 * MT + 4) {
-        // ===================== loaders: 128 threads =====================
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(MT == 2 ? 104 : 120));
-        const int lw = warp - 4 * MT;
+    } else if (warp < 4 * MT + 8) {
+        // ===================== loaders: 256 threads =====================
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(MT == 2 ? 64 : 104));
+        // A unit is one operand's 64-wide block of a tile, or (two blocks wide) half of its keys: four 16-byte pieces per thread, 16 lanes to a
+        // key's 64 floats.  The next unit's loads are in flight while this one is split and stored, and the page lookups run a tile ahead
+        // (one key per lane, handed round by shuffles).
+        const int lw = warp - 4 * MT, nu = KB + VB;
+        const int hw = lw * 2 + (lane >> 4), c4 = lane & 15;
+        const int shift = (bs & (bs - 1)) == 0 ? 31 - __clz(bs) : -1;
+        struct TileAt {
+            int k0, klim;
+            bool pooled;
+        };
+        auto tile_at = [&](int j) {
+            const int tile = split + j * a.nsplit;
+            TileAt t;
+            t.pooled = tile < kt.npt;
+            const bool first = !t.pooled && tile < kt.npt + kt.nft;
+            t.k0 = t.pooled ? tile * KT : (first ? (tile - kt.npt) * KT : kt.kbeg + (tile - kt.npt - kt.nft) * KT);
+            t.klim = t.pooled ? kt.nbmax - 1 : (first ? kt.nfirst - 1 : hi);
+            return t;
+        };
+        auto lookup = [&](const TileAt& t, int key) {       // pool row of a key of the tile (keys beyond the last one: a valid row, its values become zero)
+            const int kp = min(t.k0 + key, t.klim);
+            if (t.pooled) return (int)pooled_slot(bt, bs, a.pool, a.ppp, kp);
+            return shift >= 0 ? bt[kp >> shift] * bs + (kp & (bs - 1)) : bt[kp / bs] * bs + kp % bs;
+        };
+        struct Piece {
+            int row0, per, d;
+            bool is_v;
+        };
+        auto piece = [&](int u) {
+            Piece p;
+            p.is_v = u >= KB;
+            const int wide = p.is_v ? VB : KB, pu = p.is_v ? u - KB : u;
+            p.per = wide == 2 ? 8 : 16;                      // keys per pass of the sixteen half-warps
+            p.row0 = pu * 32 + (wide == 2 ? hw >> 1 : hw);
+            p.d = (wide == 2 ? (hw & 1) * 64 : 0) + c4 * 4;
+            return p;
+        };
+        auto fetch = [&](const TileAt& t, int u, int ra, int rb, float4 (&x)[4]) {
+            const Piece p = piece(u);
+            const int width = p.is_v ? V : D;
+            const float* base = t.pooled ? (p.is_v ? a.vpp + (int64_t)g * V : a.kpp + (int64_t)g * D) : (p.is_v ? a.vpool + (int64_t)(g / a.vdiv) * V : a.kpool + (int64_t)g * D);
+            const int64_t ld = t.pooled ? (int64_t)G * width : (p.is_v ? a.vld : a.kld);
+            base += p.d < width ? p.d : 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int key = p.row0 + i * p.per;          // all keys of a warp in one pass lie in the same half
+                const int row = __shfl_sync(0xffffffffu, key < 32 ? ra : rb, key & 31);
+                x[i] = ld4(base + row * ld);
+            }
+        };
+        TileAt t = tile_at(0), tn = t;
+        int ra = 0, rb = 0, na = 0, nb = 0;
+        float4 cur[4], nxt[4];
+        if (ntile > 0) {
+            ra = lookup(t, lane), rb = lookup(t, lane + 32);
+            fetch(t, 0, ra, rb, nxt);
+        }
         bool ok = true;
+#pragma unroll 1
         for (int j = 0; j < ntile && ok; ++j) {
             const int s = j & 1;
-            const uint32_t ph = ((j >> 1) & 1) ^ 1;
-            const int tile = split + j * a.nsplit;
-            const bool pooled = tile < kt.npt, first = !pooled && tile < kt.npt + kt.nft;
-            const int k0 = pooled ? tile * KT : (first ? (tile - kt.npt) * KT : kt.kbeg + (tile - kt.npt - kt.nft) * KT);
-            const int klim = pooled ? kt.nbmax - 1 : (first ? kt.nfirst - 1 : hi);
-            // one operand: 16 lanes cover 64 floats of a key's row; `wide` blocks of 64
-            auto bring = [&](bool is_v, int width, int wide, uint32_t dst, uint32_t bfull, uint32_t bfree) {
-                const int per = 4 / wide * 2;                              // (rows per 8 half-warps) / blocks: 8 keys per pass (one block) or 4 (two)
-                const int hw = lw * 2 + (lane >> 4), blk = wide == 2 ? hw & 1 : 0, rowi = wide == 2 ? hw >> 1 : hw;
-                const int d = blk * 64 + (lane & 15) * 4;
+            const bool more = j + 1 < ntile;
+            if (more) tn = tile_at(j + 1), na = lookup(tn, lane), nb = lookup(tn, lane + 32);
 #pragma unroll 1
-                for (int part = 0; part < KT; part += 8 * per) {           // eight rows in flight per thread
-                    float4 x[8];
+            for (int u = 0; u < nu; ++u) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const int kp = k0 + part + i * per + rowi;
-                        x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (kp <= klim && d < width) {
-                            const float* p;
-                            if (pooled) p = is_v ? a.vpp + (pooled_slot(bt, bs, a.pool, a.ppp, kp) * G + g) * V : a.kpp + (pooled_slot(bt, bs, a.pool, a.ppp, kp) * G + g) * D;
-                            else {
-                                const int64_t prow = (int64_t)bt[kp / bs] * bs + kp % bs;
-                                if (is_v) p = a.vpool + prow * a.vld + (int64_t)(g / a.vdiv) * V;
-                                else p = a.kpool + prow * a.kld + (int64_t)g * D;
-                            }
-                            x[i] = ld4(p + d);
-                        }
-                    }
-                    if (part == 0) ok = bar_wait(bfree + 8 * s, ph, ab);
-                    if (!ok) return;
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const int row = part + i * per + rowi;
-                        uint32_t a1, a2, a3, b1, b2, b3;
-                        split2(x[i].x, x[i].y, a1, a2, a3);
-                        split2(x[i].z, x[i].w, b1, b2, b3);
-                        const uint32_t at = dst + blk * (3 * PLANE) + row * 128 + ((((lane & 15) >> 1) ^ (row & 7)) << 4) + ((lane & 1) << 3);
-                        sts8(at, a1, b1), sts8(at + PLANE, a2, b2), sts8(at + 2 * PLANE, a3, b3);
-                    }
+                for (int i = 0; i < 4; ++i) cur[i] = nxt[i];
+                const bool here = u + 1 < nu;
+                if (here || more) fetch(here ? t : tn, here ? u + 1 : 0, here ? ra : na, here ? rb : nb, nxt);
+                const Piece p = piece(u);
+                const int width = p.is_v ? V : D;
+                if (u == 0 || u == KB) {
+                    ok = bar_wait<false>((p.is_v ? v_free : k_free) + 8 * s, ((j >> 1) & 1) ^ 1, ab);
+                    if (!ok) break;
                 }
-                async_fence();
-                __syncwarp();
-                if (lane == 0) bar_arrive(bfull + 8 * s);
-            };
-            const uint32_t base = kv + s * stage;
-            bring(false, D, KB, base, k_full, k_free);
-            if (ok) bring(true, V, VB, base + kbytes, v_full, v_free);
+                const uint32_t dst = kv + s * stage + (p.is_v ? kbytes : 0) + (p.d >> 6) * (3 * PLANE) + ((c4 & 1) << 3);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int row = p.row0 + i * p.per;
+                    const bool in = t.k0 + row <= t.klim && p.d < width;
+                    uint32_t a1, a2, a3, b1, b2, b3;
+                    split2(in ? cur[i].x : 0.f, in ? cur[i].y : 0.f, a1, a2, a3);
+                    split2(in ? cur[i].z : 0.f, in ? cur[i].w : 0.f, b1, b2, b3);
+                    const uint32_t at = dst + row * 128 + (((c4 >> 1) ^ (row & 7)) << 4);
+                    sts8(at, a1, b1), sts8(at + PLANE, a2, b2), sts8(at + 2 * PLANE, a3, b3);
+                }
+                if (u == KB - 1 || u == nu - 1) {
+                    async_fence();
+                    __syncwarp();
+                    if (lane == 0) bar_arrive((p.is_v ? v_full : k_full) + 8 * s);
+                }
+            }
+            t = tn, ra = na, rb = nb;
         }
     } else {
         // ===================== MMA issuer =====================
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-        if (warp == 4 * MT + 4) asm volatile("bar.sync 1, %0;" ::"n"((4 * MT + 1) * 32) : "memory");
-        if (warp == 4 * MT + 4 && elect()) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(MT == 2 ? 32 : 64));
+        if (warp == 4 * MT + 8) asm volatile("bar.sync 1, %0;" ::"n"((4 * MT + 1) * 32) : "memory");
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        if (warp == 4 * MT + 8 && elect()) {
             fence_after();
-            const uint32_t ids = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(KT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+            constexpr uint32_t ids = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(KT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
             const uint32_t ido = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(V >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // B is mn-major
-            const int PX[6] = {0, 2, 1, 0, 1, 0}, PY[6] = {2, 0, 1, 1, 0, 0};   // smallest products first
-            const int steps = ntile * MT;
+            constexpr uint32_t O0 = 2 * SLOT_COLS, Q0 = O0 + MT * VM;
+            const int steps = ntile * MT, nkk = DK ? DK : D / 16;
+            const uint32_t qp = DK ? DK * 8 : (uint32_t)qplane;
             bool ok = true;
             auto scores = [&](int step) {
-                const int j = step / MT, m = step - j * MT, s = j & 1, slot = step & 1;
-                ok = bar_wait(k_full + 8 * s, (j >> 1) & 1, ab);
+                const int j = step / MT, s = j & 1, slot = step & 1, m = MT == 2 ? slot : 0;
+                ok = bar_wait<false>(k_full + 8 * s, (j >> 1) & 1, ab);
                 if (!ok) return;
                 fence_after();
-                const uint32_t kb = kv + s * stage, d = slot0 + slot * SLOT_COLS + 32;
-                uint32_t acc_ = 0;
+                const uint64_t kb = desc_k128(kv + s * stage);
+                const uint32_t d = tm + slot * SLOT_COLS + 32, qa = tm + Q0 + m * 3 * qp;
 #pragma unroll
-                for (int pr = 0; pr < 6; ++pr)
-                    for (int kk = 0; kk < D / 16; ++kk) {
-                        const uint64_t b = desc_k128(kb + (kk >> 2) * (3 * PLANE) + PY[pr] * PLANE) + 2 * (kk & 3);
-                        mma_ts(d, q0 + m * qtile + PX[pr] * qplane + kk * 8, b, ids, acc_);
-                        acc_ = 1;
+                for (int pr = 0; pr < 6; ++pr) {
+                    constexpr int PX[6] = {0, 2, 1, 0, 1, 0}, PY[6] = {2, 0, 1, 1, 0, 0};   // smallest products first
+                    if (DK) {
+#pragma unroll
+                        for (int kk = 0; kk < DK; ++kk)
+                            mma_ts(d, qa + PX[pr] * qp + kk * 8, kb + (uint64_t)(((kk >> 2) * (3 * PLANE) + PY[pr] * PLANE) / 16 + 2 * (kk & 3)), ids, (pr | kk) != 0 ? 1u : 0u);
+                    } else {
+#pragma unroll 1
+                        for (int kk = 0; kk < nkk; ++kk)
+                            mma_ts(d, qa + PX[pr] * qp + kk * 8, kb + (uint64_t)(((kk >> 2) * (3 * PLANE) + PY[pr] * PLANE) / 16 + 2 * (kk & 3)), ids, (pr | kk) != 0 ? 1u : 0u);
                     }
+                }
                 commit_one(s_full + 8 * slot);
-                if (m == MT - 1 && j + 2 < ntile) commit_one(k_free + 8 * s);   // (nobody waits for the last ones)
+                if ((MT == 1 || slot == 1) && j + 2 < ntile) commit_one(k_free + 8 * s);   // (nobody waits for the last ones)
             };
             if (steps > 0) scores(0);
+#pragma unroll 1
             for (int step = 0; step < steps && ok; ++step) {
                 if (step + 1 < steps) {
-                    if (step >= 1) {   // the other slot's weights have been read
-                        ok = bar_wait(o_full + 8 * ((step - 1) & 1), ((step - 1) >> 1) & 1, ab);
-                        if (!ok) break;
-                    }
-                    scores(step + 1);
+                    if (step >= 1) ok = bar_wait<false>(o_full + 8 * ((step + 1) & 1), ((step - 1) >> 1) & 1, ab);   // the other slot's weights have been read
+                    if (ok) scores(step + 1);
                     if (!ok) break;
                 }
-                const int j = step / MT, m = step - j * MT, s = j & 1, slot = step & 1;
-                ok = bar_wait(v_full + 8 * s, (j >> 1) & 1, ab) && bar_wait(p_ready + 8 * slot, (step >> 1) & 1, ab);
+                const int j = step / MT, s = j & 1, slot = step & 1, m = MT == 2 ? slot : 0;
+                ok = bar_wait<false>(v_full + 8 * s, (j >> 1) & 1, ab) && bar_wait<false>(p_ready + 8 * slot, (step >> 1) & 1, ab);
                 if (!ok) break;
                 fence_after();
-                const uint32_t vb = kv + s * stage + kbytes, d = o0 + m * VM;
-                uint32_t acc_ = 0;
+                const uint64_t vb = desc_mn128(kv + s * stage + kbytes, 3 * PLANE);
+                const uint32_t d = tm + O0 + m * VM, pa = tm + slot * SLOT_COLS;
 #pragma unroll
-                for (int pr = 0; pr < 6; ++pr)
+                for (int pr = 0; pr < 6; ++pr) {
+                    constexpr int PX[6] = {0, 2, 1, 0, 1, 0}, PY[6] = {2, 0, 1, 1, 0, 0};
 #pragma unroll
-                    for (int kk = 0; kk < KT / 16; ++kk) {
-                        const uint64_t b = desc_mn128(vb + PY[pr] * PLANE + kk * 2048, 3 * PLANE);
-                        mma_ts(d, slot0 + slot * SLOT_COLS + 48 * (kk >> 1) + 16 * PX[pr] + 8 * (kk & 1), b, ido, acc_);
-                        acc_ = 1;
-                    }
+                    for (int kk = 0; kk < KT / 16; ++kk)
+                        mma_ts(d, pa + 48 * (kk >> 1) + 16 * PX[pr] + 8 * (kk & 1), vb + (uint64_t)((PY[pr] * PLANE + kk * 2048) / 16), ido, (pr | kk) != 0 ? 1u : 0u);
+                }
                 commit_one(o_full + 8 * slot);
-                if (m == MT - 1 && j + 2 < ntile) commit_one(v_free + 8 * s);
+                if ((MT == 1 || slot == 1) && j + 2 < ntile) commit_one(v_free + 8 * s);
             }
             if (!ok) {   // what was issued reads shared memory and TMEM: wait for it (bounded) before the CTA goes
                 commit_one(B0 + 112);
                 const unsigned long long t0_ = now_ns();
-                while (!bar_try(B0 + 112, 0) && now_ns() - t0_ < WAIT_NS) {}
+                while (!bar_try<false>(B0 + 112, 0) && now_ns() - t0_ < WAIT_NS) {}
             }
         }
         __syncwarp();
@@ -451,8 +547,8 @@ __global__ void __launch_bounds__((4 * MT + 8) * 32, 1) attn_tc_kernel(const Att
     }
 }
 
-template <int MT, int VM>
-cudaError_t run(const AttnArgs& a, const b200seq_step& st, dim3 grid, cudaStream_t cs) {
+template <int MT, int VM, int DK, bool CAP>
+cudaError_t run_cap(const AttnArgs& a, const b200seq_step& st, dim3 grid, cudaStream_t cs) {
     const int KB = (a.D + 63) / 64, VB = (a.V + 63) / 64;
     int smem = 2 * (KB + VB) * 3 * PLANE + 1024;
     if (smem < 120 * 1024) smem = 120 * 1024;   // one CTA per SM: it takes all of TMEM
@@ -461,12 +557,17 @@ cudaError_t run(const AttnArgs& a, const b200seq_step& st, dim3 grid, cudaStream
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev >= 16 || ready[dev] < smem) {
-        e = cudaFuncSetAttribute(attn_tc_kernel<MT, VM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = cudaFuncSetAttribute(attn_tc_kernel<MT, VM, DK, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
         if (dev < 16) ready[dev] = smem;
     }
-    attn_tc_kernel<MT, VM><<<grid, (4 * MT + 8) * 32, smem, cs>>>(a, st);
+    attn_tc_kernel<MT, VM, DK, CAP><<<grid, (4 * MT + 12) * 32, smem, cs>>>(a, st);
     return cudaGetLastError();
+}
+
+template <int MT, int VM, int DK>
+cudaError_t run(const AttnArgs& a, const b200seq_step& st, dim3 grid, cudaStream_t cs) {
+    return a.softcap > 0.f ? run_cap<MT, VM, 0, true>(a, st, grid, cs) : run_cap<MT, VM, DK, false>(a, st, grid, cs);
 }
 
 }  // namespace
@@ -501,9 +602,9 @@ bool launch_attn_tc(AttnArgs& a, const b200seq_step& st, int max_keys, size_t pa
     a.nsplit = (int)ns;
     const dim3 grid(tiles, a.G * a.HB, (unsigned)ns);
     cudaError_t e;
-    if (mt == 2) e = run<2, 64>(a, st, grid, cs);
-    else if (a.V <= 64) e = run<1, 64>(a, st, grid, cs);
-    else e = run<1, 128>(a, st, grid, cs);
+    if (mt == 2) e = a.D == 64 ? run<2, 64, 4>(a, st, grid, cs) : run<2, 64, 0>(a, st, grid, cs);
+    else if (a.V <= 64) e = a.D == 64 ? run<1, 64, 4>(a, st, grid, cs) : run<1, 64, 0>(a, st, grid, cs);
+    else e = a.D == 128 ? run<1, 128, 8>(a, st, grid, cs) : run<1, 128, 0>(a, st, grid, cs);
     if (e != cudaSuccess) {
         rc = cuda_status(e, "attn tc");
         return true;

@@ -63,15 +63,26 @@ __device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void bar_arrive_cluster(uint32_t bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
+// CLUSTER: the arrivals may come from the other CTA of the pair (acquire at cluster scope; the CTA scope is the cheaper one)
+template <bool CLUSTER = true>
 __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
+    if (CLUSTER)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
     return ok != 0;
 }
 __device__ __forceinline__ unsigned long long now_ns() {
@@ -80,11 +91,12 @@ __device__ __forceinline__ unsigned long long now_ns() {
     return t;
 }
 // false: the wait ran out, or another role of this CTA gave up
+template <bool CLUSTER = true>
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    if (bar_try(bar, parity)) return true;
+    if (bar_try<CLUSTER>(bar, parity)) return true;
     unsigned long long t0 = 0;
     for (uint32_t i = 1;; ++i) {
-        if (bar_try(bar, parity)) return true;
+        if (bar_try<CLUSTER>(bar, parity)) return true;
         if ((i & 255u) == 0) {
             if (*abort_flag) return false;
             const unsigned long long t = now_ns();
