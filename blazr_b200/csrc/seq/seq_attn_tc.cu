@@ -4,8 +4,7 @@
 // a product runs as the six tcgen05.mma products that matter (x1y3, x3y1, x2y2, x1y2, x2y1, x1y1 -- smallest first, so that the tensor core's
 // truncating f32 accumulation costs what the last product's few steps cost).  What is left out is below 2^-24 of the product.  The values of
 // 64 keys at a time leave the tensor core and are summed over the key tiles by f32 adds in registers.  Error against 64 bits, 4096 tokens,
-// heads of 64, chunks of 2048: see the test; no larger than that of the f32 multiply-add tiles (seq_attn.cu) that this replaces for steps
-// of more than 16 tokens.
+// heads of 64, chunks of 2048: 2.0e-7, that of the f32 multiply-add tiles (seq_attn.cu) that this replaces for steps of more than 16 tokens 3.9e-7.
 //
 // One CTA works on MT tiles of 128 (token, query head) rows of one key head against tiles of 64 keys.  MT = 2 (heads up to 64): the two row
 // tiles alternate, one in the soft-max while the other is in the tensor pipe; MT = 1 (heads up to 128): consecutive key tiles alternate.
@@ -16,8 +15,8 @@
 // the sums (2 * 160 + 2 * 64 + 32 = 5 * 96, 240 + 2 * 104 + 64 = 4 * 128) are what the block was launched with.
 // TMEM: two slots of 96 columns (scores f32 [64], then the weights' three planes in the same columns), the value tile of every row tile,
 // and the queries' planes (the A operand of the scores comes from TMEM: from shared memory its reads alone would take longer than the MMA).
-// What bounds it: the tensor pipe, 6 x the products (D = V = 64: 1536 cycles per 128 x 64 scores), with the soft-max beside it at about 10
-// instructions per score.
+// What bounds it: the tensor pipe, 6 x the products (D = V = 64: 1536 cycles per 128 x 64 scores; a step takes 2 400, the difference being the
+// hand-overs between a value product and the next scores of the same slot), with the soft-max beside it at about 9 instructions per score.
 //
 // Values that are not finite: an infinite key or value part makes the row NaN (inf - inf in the split), where a plain f32 product could still be inf.
 // Every wait is bounded (tc_pair.cuh): one that runs out sets bit 1 of the library's error flags and the CTA leaves through the common exit.
@@ -52,33 +51,12 @@ __device__ __forceinline__ void st8(uint32_t taddr, const uint32_t* r) {
                  "r"(r[6]), "r"(r[7])
                  : "memory");
 }
-__device__ __forceinline__ void st16(uint32_t taddr, const uint32_t* r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
-                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-                 : "memory");
-}
-__device__ __forceinline__ void ld16(uint32_t taddr, float* v) {
-    uint32_t* r = reinterpret_cast<uint32_t*>(v);
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-                   "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr)
-                 : "memory");
-}
 __device__ __forceinline__ void st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void async_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-// two values -> three packed bf16 pairs (low half = a)
-__device__ __forceinline__ void split2(float a, float b, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p1) : "f"(b), "f"(a));
-    const float ra = a - __uint_as_float(p1 << 16), rb = b - __uint_as_float(p1 & 0xFFFF0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p2) : "f"(rb), "f"(ra));
-    const float sa_ = ra - __uint_as_float(p2 << 16), sb_ = rb - __uint_as_float(p2 & 0xFFFF0000u);
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p3) : "f"(sb_), "f"(sa_));
 }
 // packed pairs of f32 (one instruction for both)
 __device__ __forceinline__ uint64_t pk(float a, float b) {
@@ -101,6 +79,16 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     uint64_t r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
+}
+// two values -> three packed bf16 pairs (low half = a)
+__device__ __forceinline__ void split2(float a, float b, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p1) : "f"(b), "f"(a));
+    float ra, rb, sa_, sb_;
+    const uint64_t minus1 = pk(-1.f, -1.f);
+    upk(fma2(pk(__uint_as_float(p1 << 16), __uint_as_float(p1 & 0xFFFF0000u)), minus1, pk(a, b)), ra, rb);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p2) : "f"(rb), "f"(ra));
+    upk(fma2(pk(__uint_as_float(p2 << 16), __uint_as_float(p2 & 0xFFFF0000u)), minus1, pk(ra, rb)), sa_, sb_);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p3) : "f"(sb_), "f"(sa_));
 }
 // a pair of weights (>= 0) -> three packed bf16 pairs by truncation: 8 + 8 + 8 significant bits, no conversion instruction
 __device__ __forceinline__ void cut2(float x, float y, uint64_t minus1, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
@@ -144,7 +132,7 @@ __device__ __forceinline__ int64_t pooled_slot(const int32_t* bt, int bs, int P,
 
 // DK: head size / 16, or 0 for a run-time one; CAP: scores are soft-capped.  The loops are kept short: with the soft-max in two unrolled passes,
 // two copies of the loader and the issuer unrolled over four steps the kernel waited for instructions (ncu: no_instruction the largest stall,
-// 0.21 instructions per cycle) and took 870 us where it now takes a fraction (4096 tokens, heads of 64).
+// 0.21 instructions per cycle) and took 860 us where it now takes 206 (4096 tokens, 32 heads of 64, chunks of 2048; the f32 tiles: 1 656).
 template <int MT, int VM, int DK, bool CAP>
 __global__ void __launch_bounds__((4 * MT + 12) * 32, 1) attn_tc_kernel(const AttnArgs a, const b200seq_step st) {
     extern __shared__ uint8_t smem_raw[];
@@ -160,9 +148,16 @@ __global__ void __launch_bounds__((4 * MT + 12) * 32, 1) attn_tc_kernel(const At
     const uint32_t k_full = B0, k_free = B0 + 16, v_full = B0 + 32, v_free = B0 + 48, s_full = B0 + 64, p_ready = B0 + 80, o_full = B0 + 96;
     volatile int* ab = &abort_sh;
     int e, t0, nq;
-    // the tiles with the most keys first: a causal step's last tiles see the most
-    if (!attn_find_tile(st, (int)gridDim.x - 1 - (int)blockIdx.x, a.QT, e, t0, nq)) return;
-    const int g = blockIdx.y / a.HB, hb = blockIdx.y - g * a.HB, R = H / G;
+    // The tiles with the most keys first, for all heads at once, so that the last CTAs to start are short: a causal step's last tiles see the
+    // most, in a step of chunks the last ones of every chunk.
+    int tile_no = (int)gridDim.y - 1 - (int)blockIdx.y;
+    if (a.chunk > 0 && a.chunk % a.QT == 0 && a.chunk / a.QT < (int)gridDim.y) {
+        const int per = a.chunk / a.QT, n = gridDim.y, nc = (n + per - 1) / per, rem = n - (nc - 1) * per, r = blockIdx.y, longer = (per - rem) * (nc - 1);
+        if (r < longer) tile_no = (r % (nc - 1)) * per + per - 1 - r / (nc - 1);
+        else tile_no = ((r - longer) % nc) * per + rem - 1 - (r - longer) / nc;
+    }
+    if (!attn_find_tile(st, tile_no, a.QT, e, t0, nq)) return;
+    const int g = blockIdx.x / a.HB, hb = blockIdx.x - g * a.HB, R = H / G;
     const int h0 = g * R + hb * a.Rb, nh = min(a.Rb, R - hb * a.Rb);
     const int split = blockIdx.z;
     const int p0 = st.tok_pos[t0], hi = p0 + nq - 1, bs = st.block_size;
@@ -242,6 +237,22 @@ __global__ void __launch_bounds__((4 * MT + 12) * 32, 1) attn_tc_kernel(const At
 #pragma unroll
         for (int i = 0; i < VM / 2; ++i) acc[i] = 0;
         bool ok = true;
+        auto add_values = [&](int step) {   // acc += the value tile of a step
+            ok = bar_wait<false>(o_full + 8 * (step & 1), (step >> 1) & 1, ab);
+            if (!ok) return false;
+            fence_after();
+#pragma unroll
+            for (int i = 0; i < VM; i += 32) {
+                if (i >= V) break;
+                float o[32];
+                ld32(o0 + lanes + m * VM + i, o);     // (V = 16 or 48: the columns beyond are not used)
+                ld_wait();
+#pragma unroll
+                for (int u = 0; u < 32; u += 2) acc[(i + u) >> 1] = add2(acc[(i + u) >> 1], pk(o[u], o[u + 1]));
+            }
+            fence_before();
+            return true;
+        };
 #pragma unroll 1
         for (int j = 0; j < ntile && ok; ++j) {
             const int step = j * MT + m, slot = step & 1;
@@ -299,38 +310,23 @@ __global__ void __launch_bounds__((4 * MT + 12) * 32, 1) attn_tc_kernel(const At
             float sx, sy;
             upk(sum, sx, sy);
             l = fmaf(l, corr, sx + sy);
-            if (j > 0) {   // the value tile of the key tile before
-                const int ps = (step - MT) & 1;
-                ok = bar_wait<false>(o_full + 8 * ps, ((step - MT) >> 1) & 1, ab);
-                if (!ok) break;
-                fence_after();
-                const uint64_t corr2 = pk(corr, corr);
-                const bool same = __all_sync(0xffffffffu, corr == 1.f);
+            const uint64_t corr2 = pk(corr, corr);
+            const bool same = __all_sync(0xffffffffu, corr == 1.f);
+            // MT = 1: the value tile of the key tile before, whose product ran beside this soft-max
+            if (MT == 1 && j > 0 && !add_values(step - 1)) break;
+            if (!same) {
 #pragma unroll
-                for (int i = 0; i < VM; i += 16) {
-                    if (i >= V) break;
-                    float o[16];
-                    ld16(o0 + lanes + m * VM + i, o);
-                    ld_wait();
-#pragma unroll
-                    for (int u = 0; u < 16; u += 2) acc[(i + u) >> 1] = add2(acc[(i + u) >> 1], pk(o[u], o[u + 1]));
-                }
-                if (!same) {
-#pragma unroll
-                    for (int i = 0; i < VM / 2; ++i) acc[i] = mul2(acc[i], corr2);
-                }
+                for (int i = 0; i < VM / 2; ++i) acc[i] = mul2(acc[i], corr2);
             }
             st_wait();
             fence_before();
             __syncwarp();
             if (lane == 0) bar_arrive(p_ready + 8 * slot);
+            // MT = 2: this key tile's, while the next scores are made (the other row tile keeps the tensor pipe busy)
+            if (MT == 2 && !add_values(step)) break;
         }
         if (!CAP && mx != -INFINITY) mx = mb / LOG2E;   // in the units of the scores, for the sink and the merge of key splits
-        if (ok && ntile > 0) {
-            const int step = (ntile - 1) * MT + m;
-            ok = bar_wait<false>(o_full + 8 * (step & 1), (step >> 1) & 1, ab);
-            fence_after();
-        }
+        if (MT == 1 && ok && ntile > 0) add_values(ntile - 1);
         if (ok) {
             const int t = t0 + tq, h = h0 + hr;
             float f = 1.f;
@@ -352,18 +348,12 @@ __global__ void __launch_bounds__((4 * MT + 12) * 32, 1) attn_tc_kernel(const At
             for (int cb = 0; cb < VM; cb += 16) {
                 if (cb >= V) break;
                 float o[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) o[i] = 0.f;
-                if (ntile > 0) {
-                    ld16(o0 + lanes + m * VM + cb, o);
-                    ld_wait();
-                }
                 if (!live) continue;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     float x, x1;
                     upk(acc[(cb + i) >> 1], x, x1);
-                    x = ((i & 1) ? x1 : x) + o[i];
+                    x = (i & 1) ? x1 : x;
                     if (pp) pp[2 + cb + i] = x;
                     else o[i] = x * f * (a.gate_elem ? sigmoidf_acc(a.gate[(int64_t)t * a.gld + (int64_t)h * V + cb + i]) : 1.f);
                 }
@@ -451,16 +441,19 @@ __global__ void __launch_bounds__((4 * MT + 12) * 32, 1) attn_tc_kernel(const At
                     ok = bar_wait<false>((p.is_v ? v_free : k_free) + 8 * s, ((j >> 1) & 1) ^ 1, ab);
                     if (!ok) break;
                 }
-                const uint32_t dst = kv + s * stage + (p.is_v ? kbytes : 0) + (p.d >> 6) * (3 * PLANE) + ((c4 & 1) << 3);
+                uint32_t at = kv + s * stage + (p.is_v ? kbytes : 0) + (p.d >> 6) * (3 * PLANE) + p.row0 * 128 + (((c4 >> 1) ^ (p.row0 & 7)) << 4) + ((c4 & 1) << 3);
+                if (t.k0 + KT - 1 > t.klim || p.d >= width) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int row = p.row0 + i * p.per;
-                    const bool in = t.k0 + row <= t.klim && p.d < width;
+                    for (int i = 0; i < 4; ++i)
+                        if (t.k0 + p.row0 + i * p.per > t.klim || p.d >= width) cur[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {              // (the row's place in the swizzle is the same in every pass)
                     uint32_t a1, a2, a3, b1, b2, b3;
-                    split2(in ? cur[i].x : 0.f, in ? cur[i].y : 0.f, a1, a2, a3);
-                    split2(in ? cur[i].z : 0.f, in ? cur[i].w : 0.f, b1, b2, b3);
-                    const uint32_t at = dst + row * 128 + (((c4 >> 1) ^ (row & 7)) << 4);
+                    split2(cur[i].x, cur[i].y, a1, a2, a3);
+                    split2(cur[i].z, cur[i].w, b1, b2, b3);
                     sts8(at, a1, b1), sts8(at + PLANE, a2, b2), sts8(at + 2 * PLANE, a3, b3);
+                    at += p.per * 128;
                 }
                 if (u == KB - 1 || u == nu - 1) {
                     async_fence();
@@ -600,7 +593,7 @@ bool launch_attn_tc(AttnArgs& a, const b200seq_step& st, int max_keys, size_t pa
         ns = ns > 32 ? 32 : (ns < 1 ? 1 : ns);
     }
     a.nsplit = (int)ns;
-    const dim3 grid(tiles, a.G * a.HB, (unsigned)ns);
+    const dim3 grid(a.G * a.HB, tiles, (unsigned)ns);
     cudaError_t e;
     if (mt == 2) e = a.D == 64 ? run<2, 64, 4>(a, st, grid, cs) : run<2, 64, 0>(a, st, grid, cs);
     else if (a.V <= 64) e = a.D == 64 ? run<1, 64, 4>(a, st, grid, cs) : run<1, 64, 0>(a, st, grid, cs);

@@ -1,0 +1,98 @@
+"""Prompt attention on the tensor cores (csrc/seq/seq_attn_tc.cu) against float64 at the sizes where it can go wrong: head sizes that are not a
+power of two and differ between keys and values, row tiles that end inside a token's heads, several entries behind their own pasts, key tiles
+that end inside a page, windows, chunks, kept first positions, soft caps, sinks, negative head scales, gates, key splits.
+
+Bound: operands enter as 24-bit splits, products are summed by the tensor core in f32 over at most 128 terms (its truncation: 2^-23 of the sum
+a step, 8 steps) and the value tiles by f32 adds; the f32 tiles it stands beside are tested at 2e-5 of the largest value, this one at 4e-6."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    from blazr_b200 import seqops
+    seqops.lib()
+    return seqops
+
+
+CASES = [
+    # (tokens, past) per entry, H, G, D, V, options
+    ([(17, 0)], 4, 4, 16, 16, {}),
+    ([(64, 0), (33, 100)], 8, 2, 64, 64, dict(chunk=48)),
+    ([(130, 5)], 6, 2, 48, 80, dict(window=37)),
+    ([(40, 300), (1, 64), (20, 0)], 8, 1, 128, 128, dict(window=64, keep_first=3)),
+    ([(200, 0)], 3, 3, 96, 32, dict(softcap=5.0)),
+    ([(70, 10)], 10, 2, 64, 48, dict(sink=True, head_scale=True)),
+    ([(129, 63)], 4, 2, 112, 64, dict(gated=True, gate_elem=True)),
+    ([(300, 0)], 64, 8, 64, 64, dict(gated=True, chunk=128)),       # two row tiles per CTA
+    ([(1300, 0)], 32, 8, 64, 64, dict(window=200)),
+    ([(20, 1500)], 2, 1, 64, 64, dict(split=True)),
+    ([(18, 2000)], 4, 1, 128, 128, dict(split=True, sink=True, gated=True)),
+    ([(50, 0)], 300, 2, 32, 32, {}),                                # more heads of one key head than a tile has rows
+]
+
+
+@pytest.mark.parametrize("entries,H,G,D,V,o", CASES)
+@pytest.mark.parametrize("odt", [torch.float32, torch.bfloat16])
+def test_against_float64(ops, entries, H, G, D, V, o, odt):
+    from blazr_b200.batch import StepEntry, build_step
+    bs, gen = 16, torch.Generator().manual_seed(H * D + V)
+    rnd = lambda *s: torch.randn(*s, generator=gen)
+    need = [-(-(n + p) // bs) for n, p in entries]
+    perm = torch.randperm(sum(need), generator=gen).tolist()
+    tables, at = [], 0
+    for n in need:
+        tables.append(perm[at:at + n])
+        at += n
+    sa = build_step([StepEntry([0] * n, p, i, tables[i]) for i, (n, p) in enumerate(entries)], bs)
+    t = {k: torch.from_numpy(np.ascontiguousarray(getattr(sa, k))).to(DEV) for k in ("tok_ent", "tok_pos", "ent_start", "ent_slot", "ent_pos0", "block_table")}
+    st = ops.StepDesc(t["tok_ent"].data_ptr(), t["tok_pos"].data_ptr(), t["ent_start"].data_ptr(), t["ent_slot"].data_ptr(), t["ent_pos0"].data_ptr(),
+                      t["block_table"].data_ptr(), sa.T, sa.B, sa.block_table.shape[1], bs)
+    gated, elem = o.get("gated", False), o.get("gate_elem", False)
+    sink = rnd(H) if o.get("sink") else None
+    hs = rnd(H) if o.get("head_scale") else None
+    desc = ops.attn_desc(H, G, D, V, 2.0 * D ** -0.5, gated=gated, chunk=o.get("chunk", 0), window=o.get("window", 0), keep_first=o.get("keep_first", 0),
+                         softcap=o.get("softcap", 0.0), sink=sink.to(DEV) if sink is not None else None, head_scale=hs.to(DEV) if hs is not None else None, gate_elem=elem)
+    keep = (desc, sink, hs)
+    sink_d, hs_d = (x.to(DEV) if x is not None else None for x in (sink, hs))
+    desc.sink, desc.head_scale = (x.data_ptr() if x is not None else None for x in (sink_d, hs_d))
+    width = -(-desc.width // 4) * 4
+    rows = rnd(sa.T, width)
+    kp, vp = rnd(sum(need) * bs, G, D), rnd(sum(need) * bs, G, V)
+    kp[tables[0][-1] * bs + bs - 1] = float("nan") if (entries[0][0] + entries[0][1]) % bs else kp[tables[0][-1] * bs + bs - 1]   # a slot no position uses
+    ref = torch.zeros(sa.T, H, V, dtype=torch.float64)
+    r0 = 0
+    for (n, past), tab in zip(entries, tables):
+        slots = (torch.tensor(tab)[:, None] * bs + torch.arange(bs)).reshape(-1)[:n + past]
+        q, k, v = rows[r0:r0 + n, :H * D].double().reshape(n, H, D), kp[slots].double(), vp[slots].double()
+        qp, kpos = torch.arange(past, past + n)[:, None], torch.arange(n + past)[None]
+        see = kpos <= qp
+        if o.get("chunk"):
+            see = see & (kpos // o["chunk"] == qp // o["chunk"])
+        if o.get("window"):
+            see = see & ((qp - kpos < o["window"]) | (kpos < o.get("keep_first", 0)))
+        for h in range(H):
+            s = (q[:, h] @ k[:, h // (H // G)].T) * 2.0 * D ** -0.5 * (hs[h].double() if hs is not None else 1.0)
+            if o.get("softcap"):
+                s = o["softcap"] * torch.tanh(s / o["softcap"])
+            s = s.masked_fill(~see, float("-inf"))
+            if sink is not None:
+                s = torch.cat([s, sink[h].double().expand(n, 1)], 1)
+            p = torch.softmax(s, 1)[:, :n + past]
+            ref[r0:r0 + n, h] = p @ v[:, h // (H // G)]
+        if gated:
+            gl = rows[r0:r0 + n, desc.gate_col:].double()
+            ref[r0:r0 + n] *= torch.sigmoid(gl[:, :H * V].reshape(n, H, V) if elem else gl[:, :H, None])
+        r0 += n
+    out = torch.full((sa.T + 1, H * V), 3.0, device=DEV, dtype=odt)
+    scratch = torch.empty(1 << 22, device=DEV) if o.get("split") else None
+    ops.attn_ex(rows.to(DEV), st, desc, kp.to(DEV), vp.to(DEV), out[:sa.T], scratch)
+    err = (out[:sa.T].double().cpu() - ref.reshape(sa.T, -1)).abs().max().item() / ref.abs().max().item()
+    assert err < (4e-6 if odt == torch.float32 else 2 ** -8), err
+    assert bool((out[sa.T] == 3.0).all()) and ops.error_flags() == 0 and keep is not None
