@@ -262,6 +262,110 @@ __global__ void __launch_bounds__(256) swiglu_quant_kernel(const float* __restri
 }
 
 // ------------------------------------------------------------------------------------------------
+// The same operators for the rows of a prompt: each is one pass over memory, 16 bytes per access, and may leave its result as the f16 rows
+// (clamped, rounded once) that the dequant-GEMM's staging would round to anyway.  Same arithmetic as above, element by element.
+// ------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(__half* p, float4 v) {
+    auto c = [](float x) { return fminf(fmaxf(x, -65504.0f), 65504.0f); };
+    const __half2 a = __floats2half2_rn(c(v.x), c(v.y)), b = __floats2half2_rn(c(v.z), c(v.w));
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+
+// One block per row, the row in registers (NV float4 per thread): read once, where the decode form's H / 256 blocks per row each read all of
+// it and keep 1024 threads for 256 outputs (2048 rows of 2048: 105 us, now 15).  The f64 sum of squares does not depend on its order.
+constexpr int NORMR_NT = 256;
+template <int NV, typename T>
+__global__ void __launch_bounds__(NORMR_NT) add_rmsnorm_rows_kernel(const float* __restrict__ h_in, const float* __restrict__ delta, float* __restrict__ h_out,
+                                                                    const float* __restrict__ w, float eps, int H, T* __restrict__ out) {
+    pdl_launch_dependents();
+    const size_t row = (size_t)blockIdx.x * H;
+    const int t = threadIdx.x, n4 = H / 4;
+    __shared__ double red[NORMR_NT / 32];
+    pdl_wait();
+    float4 v[NV];
+    double ss = 0.0;
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        const int k4 = t + i * NORMR_NT;
+        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (k4 < n4) {
+            v[i] = reinterpret_cast<const float4*>(h_in + row)[k4];
+            if (delta) {
+                const float4 d = reinterpret_cast<const float4*>(delta + row)[k4];
+                v[i].x = __fadd_rn(v[i].x, d.x); v[i].y = __fadd_rn(v[i].y, d.y); v[i].z = __fadd_rn(v[i].z, d.z); v[i].w = __fadd_rn(v[i].w, d.w);
+            }
+            reinterpret_cast<float4*>(h_out + row)[k4] = v[i];
+        }
+        ss += fma((double)v[i].x, (double)v[i].x, (double)v[i].y * (double)v[i].y) + fma((double)v[i].z, (double)v[i].z, (double)v[i].w * (double)v[i].w);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if ((t & 31) == 0) red[t >> 5] = ss;
+    __syncthreads();
+    double tot = 0.0;
+#pragma unroll
+    for (int i = 0; i < NORMR_NT / 32; i++) tot += red[i];
+    const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn((float)tot, (float)H), eps)));
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        const int k4 = t + i * NORMR_NT;
+        if (k4 >= n4) break;
+        const float4 wk = reinterpret_cast<const float4*>(w)[k4];
+        store4(out + row + 4 * k4, make_float4(__fmul_rn(__fmul_rn(v[i].x, inv), wk.x), __fmul_rn(__fmul_rn(v[i].y, inv), wk.y), __fmul_rn(__fmul_rn(v[i].z, inv), wk.z),
+                                               __fmul_rn(__fmul_rn(v[i].w, inv), wk.w)));
+    }
+}
+
+// four outputs per thread (the decode form, one per thread: 2048 x 8192 70 us, now 33 us = 6 TB/s)
+template <typename T>
+__global__ void __launch_bounds__(256) swiglu_rows_kernel(const float* __restrict__ gu, int F, int64_t total4, T* __restrict__ act, int il) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= total4) return;
+    const int64_t m = idx / (F / 4);
+    const int k = (int)(idx - m * (F / 4)) * 4;
+    const size_t cg = il ? (size_t)(k >> 6) * 128 + 2 * (k & 63) : (size_t)k;
+    const float* p = gu + (size_t)m * 2 * F;
+    const float4 g = *reinterpret_cast<const float4*>(p + cg), u = *reinterpret_cast<const float4*>(p + (il ? cg + 4 : (size_t)F + k));
+    auto f = [](float a, float b) { return __fmul_rn(__fdiv_rn(a, __fadd_rn(1.0f, det_expf(-a))), b); };
+    store4(act + (size_t)m * F + k, make_float4(f(g.x, u.x), f(g.y, u.y), f(g.z, u.z), f(g.w, u.w)));
+}
+
+// RoPE of a prompt's q and k rows (positions 0 .. S - 1, products and sums rounded one by one), K / V into the cache (contiguous, or block pools
+// through the sequence's block table) in f32, and q, k, v as f16 rows [S][heads][hd] for the prompt attention.  One block per token, four columns
+// per thread.
+__global__ void __launch_bounds__(256) rope_kv_rows_kernel(const float* __restrict__ qkv, const float* __restrict__ rope, int nh, int nkv, int hd, __half* __restrict__ q16,
+                                                           __half* __restrict__ k16, __half* __restrict__ v16, float* __restrict__ ck, float* __restrict__ cv,
+                                                           const int* __restrict__ block_table, int block_size) {
+    pdl_launch_dependents();
+    const int s = blockIdx.x, nq = nh * hd, nk = nkv * hd;
+    pdl_wait();
+    const float* src = qkv + (size_t)s * (nq + 2 * nk);
+    const size_t slot = block_table ? (size_t)block_table[s / block_size] * block_size + s % block_size : (size_t)s;
+    for (int c = 4 * (int)threadIdx.x; c < nq + 2 * nk; c += 4 * (int)blockDim.x) {
+        float4 x = *reinterpret_cast<const float4*>(src + c);
+        const bool is_v = c >= nq + nk;
+        if (!is_v) {
+            const int e = c < nq ? c % hd : (c - nq) % hd;
+            const float4 r = *reinterpret_cast<const float4*>(rope + (size_t)s * hd + e);   // (cos, sin) of two pairs
+            x = make_float4(__fsub_rn(__fmul_rn(x.x, r.x), __fmul_rn(x.y, r.y)), __fadd_rn(__fmul_rn(x.x, r.y), __fmul_rn(x.y, r.x)),
+                            __fsub_rn(__fmul_rn(x.z, r.z), __fmul_rn(x.w, r.w)), __fadd_rn(__fmul_rn(x.z, r.w), __fmul_rn(x.w, r.z)));
+        }
+        const __half2 a = __floats2half2_rn(x.x, x.y), b = __floats2half2_rn(x.z, x.w);
+        const uint2 h = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        if (c < nq) {
+            *reinterpret_cast<uint2*>(q16 + (size_t)s * nq + c) = h;
+        } else {
+            const int d = c - nq - (is_v ? nk : 0);
+            *reinterpret_cast<float4*>((is_v ? cv : ck) + slot * nk + d) = x;
+            *reinterpret_cast<uint2*>((is_v ? v16 : k16) + (size_t)s * nk + d) = h;
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
 // RoPE (adjacent pairs, cos/sin from a host-built table) + KV append + single-query attention + output quant.
 // Two passes with f64 reductions and the deterministic exp, so the result is bit-reproducible against the
 // oracle:  s_j = f32(sum_e q_e k_je) * scale;  p_j = det_exp(s_j - max);  o_e = f32(sum_j p_j v_je) / f32(sum_j p_j).
@@ -586,6 +690,23 @@ int* decode_error_dev() {
 
 using namespace b200q;
 
+static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+template <typename T>
+static cudaError_t launch_norm_rows(const float* h_in, const float* delta, float* h_out, const float* w, float eps, int64_t H, int64_t M, T* out, cudaStream_t st) {
+    const dim3 grid((unsigned)M), block(NORMR_NT);
+    const int nv = (int)((H / 4 + NORMR_NT - 1) / NORMR_NT);
+    if (nv <= 2) return launch_pdl(add_rmsnorm_rows_kernel<2, T>, grid, block, 0, st, h_in, delta, h_out, w, eps, (int)H, out);
+    if (nv <= 4) return launch_pdl(add_rmsnorm_rows_kernel<4, T>, grid, block, 0, st, h_in, delta, h_out, w, eps, (int)H, out);
+    return launch_pdl(add_rmsnorm_rows_kernel<8, T>, grid, block, 0, st, h_in, delta, h_out, w, eps, (int)H, out);
+}
+
+template <typename T>
+static int32_t swiglu_rows(const float* gate_up, int64_t F, int64_t M, T* act, int il, void* stream) {
+    const int64_t total4 = M * (F / 4);
+    cudaError_t e = launch_pdl(swiglu_rows_kernel<T>, dim3((unsigned)((total4 + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, gate_up, (int)F, total4, act, il);
+    return e == cudaSuccess ? B200Q_OK : B200Q_ERR_CUDA;
+}
+
 extern "C" {
 
 static cudaError_t launch_norm_cluster(const CommDev& c, const float* h_in, const float* delta, float* h_out, const float* w, float eps, int64_t H, int64_t M,
@@ -609,6 +730,34 @@ static cudaError_t launch_norm_cluster(const CommDev& c, const float* h_in, cons
     return e;
 }
 
+/* Rows of a prompt: h_out = h_in (+ delta), x16 = f16(rmsnorm(h_out) * w).  H % 256 == 0, H <= 8192, 16-byte aligned rows */
+int32_t b200q_add_rmsnorm_f16(const float* h_in, const float* delta, float* h_out, const float* w, float eps, int64_t H, int64_t M, void* x16, void* stream) {
+    if (!h_in || !h_out || !w || !x16 || H <= 0 || H % CHUNK_K || M <= 0) return set_error(B200Q_ERR_INVALID_ARG, "add_rmsnorm_f16: bad arguments");
+    if (H > 4 * 8 * NORMR_NT || M > INT32_MAX || !aligned16(h_in) || !aligned16(delta) || !aligned16(h_out) || !aligned16(w) || !aligned16(x16))
+        return set_error(B200Q_ERR_UNSUPPORTED, "add_rmsnorm_f16: H <= 8192 and 16-byte aligned rows");
+    return launch_norm_rows(h_in, delta, h_out, w, eps, H, M, (__half*)x16, (cudaStream_t)stream) == cudaSuccess ? B200Q_OK : B200Q_ERR_CUDA;
+}
+
+/* Rows of a prompt: act16[M, F] = f16(silu(gate) * up); interleaved: gate_up columns in the row order of b200q_gate_up_row (F % 64 == 0) */
+int32_t b200q_swiglu_f16(const float* gate_up, int64_t F, int64_t M, int32_t interleaved, void* act16, void* stream) {
+    if (!gate_up || !act16 || F <= 0 || F % (interleaved ? 64 : 32) || M <= 0) return set_error(B200Q_ERR_INVALID_ARG, "swiglu_f16: bad arguments");
+    if (!aligned16(gate_up) || !aligned16(act16) || M * (F / 4) > (int64_t)INT32_MAX * 256) return set_error(B200Q_ERR_UNSUPPORTED, "swiglu_f16: 16-byte aligned rows");
+    return swiglu_rows(gate_up, F, M, (__half*)act16, interleaved ? 1 : 0, stream);
+}
+
+/* Rows of a prompt: RoPE on q and k (positions 0 .. S - 1 of rope_table), K / V rows into the sequence's cache -- k_cache / v_cache [positions][nkv][hd],
+ * or with block_table (int32, of this sequence) pools of blocks of block_size positions -- and f16 copies q16 [S][nh][hd], k16, v16 [S][nkv][hd] */
+int32_t b200q_rope_kv_prefill(const float* qkv, const float* rope_table, int32_t n_heads, int32_t n_kv_heads, int32_t head_dim, int64_t S, void* q16, void* k16, void* v16,
+                              float* k_cache, float* v_cache, const int32_t* block_table, int32_t block_size, void* stream) {
+    if (!qkv || !rope_table || !q16 || !k16 || !v16 || !k_cache || !v_cache || n_heads <= 0 || n_kv_heads <= 0 || head_dim <= 0 || S <= 0 || (block_table && block_size <= 0))
+        return set_error(B200Q_ERR_INVALID_ARG, "rope_kv_prefill: bad arguments");
+    if (head_dim % 4 || S > INT32_MAX || !aligned16(qkv) || !aligned16(rope_table) || !aligned16(q16) || !aligned16(k16) || !aligned16(v16) || !aligned16(k_cache) || !aligned16(v_cache))
+        return set_error(B200Q_ERR_UNSUPPORTED, "rope_kv_prefill: head_dim a multiple of 4 and 16-byte aligned rows");
+    cudaError_t e = launch_pdl(rope_kv_rows_kernel, dim3((unsigned)S), dim3(256), 0, (cudaStream_t)stream, qkv, rope_table, (int)n_heads, (int)n_kv_heads, (int)head_dim,
+                               (__half*)q16, (__half*)k16, (__half*)v16, k_cache, v_cache, (const int*)block_table, (int)block_size);
+    return e == cudaSuccess ? B200Q_OK : B200Q_ERR_CUDA;
+}
+
 int32_t b200q_add_rmsnorm_quant(const float* h_in, const float* delta, float* h_out, const float* w, float eps, int64_t H, int64_t M, void* xq,
                                 float* xnorm, void* stream) {
     if (!h_in || !h_out || !w || (!xq && !xnorm) || H <= 0 || H % CHUNK_K || M <= 0) return B200Q_ERR_INVALID_ARG;
@@ -622,6 +771,9 @@ int32_t b200q_add_rmsnorm_quant(const float* h_in, const float* delta, float* h_
         cudaError_t e = launch_norm_cluster(CommDev{}, h_in, delta, h_out, w, eps, H, M, xq, xnorm, (cudaStream_t)stream);
         return e == cudaSuccess ? B200Q_OK : B200Q_ERR_CUDA;
     }
+    // many rows: the one that reads a row once (fewer rows leave SMs idle in that form)
+    if (!xq && M >= 128 && H <= 4 * 8 * NORMR_NT && aligned16(h_in) && aligned16(delta) && aligned16(h_out) && aligned16(w) && aligned16(xnorm))
+        return launch_norm_rows(h_in, delta, h_out, w, eps, H, M, xnorm, (cudaStream_t)stream) == cudaSuccess ? B200Q_OK : B200Q_ERR_CUDA;
     cudaError_t e = launch_pdl(add_rmsnorm_quant_kernel, dim3((unsigned)(H / CHUNK_K), (unsigned)M), dim3(NORM_NT), 0, (cudaStream_t)stream, h_in, delta,
                                h_out, w, eps, (int)H, (int)M, (uint8_t*)xq, xnorm);
     return e == cudaSuccess ? B200Q_OK : B200Q_ERR_CUDA;
@@ -659,6 +811,7 @@ int32_t b200q_swiglu_quant(const float* gate_up, int64_t F, int64_t M, void* xq,
 /* batched decode (M > 4: the projections run on the tcgen05 path and take f32 activations): act[M, F] = silu(gate) * up */
 int32_t b200q_swiglu_f32(const float* gate_up, int64_t F, int64_t M, float* act, void* stream) {
     if (!gate_up || !act || F <= 0 || F % 32 || M <= 0 || M > 65535) return B200Q_ERR_INVALID_ARG;
+    if (aligned16(gate_up) && aligned16(act)) return swiglu_rows(gate_up, F, M, act, 0, stream);
     cudaError_t e = launch_pdl(swiglu_quant_kernel, dim3((unsigned)((F + CHUNK_K - 1) / CHUNK_K), (unsigned)M), dim3(256), 0, (cudaStream_t)stream, gate_up, (int)F,
                                (int)M, (uint8_t*)nullptr, act, 0);
     return e == cudaSuccess ? B200Q_OK : B200Q_ERR_CUDA;
@@ -668,6 +821,7 @@ int32_t b200q_swiglu_f32(const float* gate_up, int64_t F, int64_t M, float* act,
  * paths (prefill, batched decode) of a model whose gate|up weight is uploaded interleaved for the fused decode epilogue */
 int32_t b200q_swiglu_f32_interleaved(const float* gate_up, int64_t F, int64_t M, float* act, void* stream) {
     if (!gate_up || !act || F <= 0 || F % 64 || M <= 0 || M > 65535) return B200Q_ERR_INVALID_ARG;
+    if (aligned16(gate_up) && aligned16(act)) return swiglu_rows(gate_up, F, M, act, 1, stream);
     cudaError_t e = launch_pdl(swiglu_quant_kernel, dim3((unsigned)((F + CHUNK_K - 1) / CHUNK_K), (unsigned)M), dim3(256), 0, (cudaStream_t)stream, gate_up, (int)F,
                                (int)M, (uint8_t*)nullptr, act, 1);
     return e == cudaSuccess ? B200Q_OK : B200Q_ERR_CUDA;

@@ -552,19 +552,6 @@ class Decoder:
         nkv, hd = self.nkv, self.cfg.head_dim
         return lay["ck"].view(-1, nkv, hd)[idx], lay["cv"].view(-1, nkv, hd)[idx]
 
-    def _kv_write(self, lay, seq: int, k: torch.Tensor, v: torch.Tensor):
-        """prefill: store K (rotated) / V rows [S, nkv, hd] of sequence `seq`"""
-        S = k.shape[0]
-        if not self.paged:
-            lay["ck"][seq, :S].copy_(k)
-            lay["cv"][seq, :S].copy_(v)
-            return
-        j = torch.arange(S, device=self.dev)
-        idx = self.block_table[seq, j // self.block_size].long() * self.block_size + j % self.block_size
-        nkv, hd = self.nkv, self.cfg.head_dim
-        lay["ck"].view(-1, nkv, hd)[idx] = k
-        lay["cv"].view(-1, nkv, hd)[idx] = v
-
     def _advance(self):
         """host-side mirror of the device position counter: every step (eager or replayed) passes through here, so a
         sequence can never run past the KV cache / RoPE table (the kernel guards too: b200q_decode_error)"""
@@ -725,10 +712,9 @@ class Decoder:
     # ---- prefill: one M = S pass over the prompt (reference src/engine/executor_generate.rs:357, batch_engine.rs:172-272) ----
     def prefill(self, prompt, seq: int = 0) -> torch.Tensor:
         """prompt: int64 [S] token ids of sequence `seq`.  Runs every projection ONCE at M = S on the tcgen05 dequant-GEMM
-        (b200q_matmul, f32 activations -> f16 tiles, f32 accumulate), fills the KV cache rows [0, S) of that sequence, leaves
-        pos[seq] = S and ids[seq] = the greedy next token, and returns the f32 logits [vocab] of the last position.  RoPE and
-        the causal attention of the prompt run in torch (SDPA, f16) -- they are not the graded path; norms,
-        SwiGLU and all 7L+1 projections are libb200q kernels.  Tolerance contract: 1e-2 relative on the logits against the f32
+        (b200q_matmul, f16 activations written by the operators ahead, f32 accumulate), fills the KV cache rows [0, S) of that sequence, leaves
+        pos[seq] = S and ids[seq] = the greedy next token, and returns the f32 logits [vocab] of the last position.  The causal
+        attention of the prompt runs in torch (SDPA, f16); norms, RoPE and the cache rows, SwiGLU and all 7L+1 projections are libb200q kernels.  Tolerance contract: 1e-2 relative on the logits against the f32
         CPU path (the GEMM path quantises weights and activations to f16 tiles)."""
         import torch.nn.functional as Fnn
         cfg, L = self.cfg, ops.lib()
@@ -741,13 +727,14 @@ class Decoder:
         dev = self.dev
         st = ops._stream_ptr(dev)
         P = lambda t: C.c_void_p(t.data_ptr())
-        f32 = dict(dtype=torch.float32, device=dev)
+        f32, f16 = dict(dtype=torch.float32, device=dev), dict(dtype=torch.float16, device=dev)
         b = getattr(self, "_pf", None)
         if b is None or b["S"] != S:
             ws_bytes = max(ln.w.workspace_bytes(S) for lay in self.layers for key in ("qkv", "o", "gu", "down") for ln in lay[key])
-            b = dict(S=S, h=torch.empty((S, H), **f32), h2=torch.empty((S, H), **f32), xn=torch.empty((S, H), **f32),
-                     qkv=torch.empty((S, self.qd + 2 * self.kvd), **f32), attn=torch.empty((S, self.qd), **f32), delta=torch.empty((S, H), **f32),
-                     delta2=torch.empty((S, H), **f32), gu=torch.empty((S, 2 * ff), **f32), act=torch.empty((S, ff), **f32),
+            b = dict(S=S, h=torch.empty((S, H), **f32), h2=torch.empty((S, H), **f32), xn=torch.empty((S, H), **f16),
+                     qkv=torch.empty((S, self.qd + 2 * self.kvd), **f32), delta=torch.empty((S, H), **f32),
+                     delta2=torch.empty((S, H), **f32), gu=torch.empty((S, 2 * ff), **f32), act=torch.empty((S, ff), **f16),
+                     q16=torch.empty((S, nh, hd), **f16), k16=torch.empty((S, nkv, hd), **f16), v16=torch.empty((S, nkv, hd), **f16),
                      ws=torch.zeros(max(256, ws_bytes), dtype=torch.uint8, device=dev))
             b["xq1"] = torch.zeros(int(L.b200q_act_bytes(C.c_int64(H), C.c_int64(1))), dtype=torch.uint8, device=dev)
             b["h1"] = torch.empty((1, H), **f32)
@@ -757,44 +744,42 @@ class Decoder:
         ops._check(L.b200q_embed(P(self.embed), P(ids_d), C.c_int64(H), C.c_int64(S), P(b["h"]), st))
         hin, hout = b["h"], b["h2"]
         delta = None
-        rope = self.rope[:S]                                   # [S, hd/2, 2]
-        cos, sin = rope[:, None, :, 0], rope[:, None, :, 1]    # [S, 1, hd/2]
-
         def gemm(lins, x, out):
             for ln in lins:
-                ops._check(L.b200q_matmul(ln.w.handle, P(x), C.c_int32(ops.F32), C.c_int64(S), C.c_int64(x.stride(0)),
+                ops._check(L.b200q_matmul(ln.w.handle, P(x), C.c_int32(ops.F16), C.c_int64(S), C.c_int64(x.stride(0)),
                                           C.c_void_p(out.data_ptr() + 4 * ln.col0), C.c_int32(ops.F32), C.c_int64(out.stride(0)), P(b["ws"]),
                                           C.c_size_t(b["ws"].numel()), st))
 
         def norm(w):
             nonlocal hin, hout
-            ops._check(L.b200q_add_rmsnorm_quant(P(hin), P(delta) if delta is not None else None, P(hout), P(w), C.c_float(cfg.eps), C.c_int64(H),
-                                                 C.c_int64(S), None, P(b["xn"]), st))
+            if H <= 8192:
+                ops._check(L.b200q_add_rmsnorm_f16(P(hin), P(delta) if delta is not None else None, P(hout), P(w), C.c_float(cfg.eps), C.c_int64(H), C.c_int64(S), P(b["xn"]), st))
+            else:
+                x32 = torch.empty((S, H), **f32)
+                ops._check(L.b200q_add_rmsnorm_quant(P(hin), P(delta) if delta is not None else None, P(hout), P(w), C.c_float(cfg.eps), C.c_int64(H),
+                                                     C.c_int64(S), None, P(x32), st))
+                b["xn"].copy_(x32.clamp_(-65504.0, 65504.0))
             hin, hout = hout, hin
-
-        def rot(x):  # adjacent-pair RoPE, same table as the decode kernel
-            x2 = x.reshape(S, -1, hd // 2, 2)
-            x0, x1 = x2[..., 0], x2[..., 1]
-            return torch.stack((x0 * cos - x1 * sin, x0 * sin + x1 * cos), dim=-1).reshape(S, -1, hd)
 
         for lay in self.layers:
             norm(lay["attn_norm"])
             gemm(lay["qkv"], b["xn"], b["qkv"])
-            q = rot(b["qkv"][:, :self.qd])
-            k = rot(b["qkv"][:, self.qd:self.qd + self.kvd])
-            v = b["qkv"][:, self.qd + self.kvd:].reshape(S, nkv, hd)
-            self._kv_write(lay, seq, k, v)
-            o = Fnn.scaled_dot_product_attention(q.permute(1, 0, 2)[None].half(), k.permute(1, 0, 2)[None].half(), v.permute(1, 0, 2)[None].half(),
-                                                 is_causal=True, enable_gqa=(nh != nkv))
-            b["attn"].copy_(o[0].permute(1, 0, 2).reshape(S, self.qd))
-            gemm(lay["o"], b["attn"], b["delta"])
+            if self.paged:
+                ck, cv, table = lay["ck"], lay["cv"], self.block_table[seq]
+            else:
+                ck, cv, table = lay["ck"][seq], lay["cv"][seq], None
+            ops._check(L.b200q_rope_kv_prefill(P(b["qkv"]), P(self.rope), C.c_int32(nh), C.c_int32(nkv), C.c_int32(hd), C.c_int64(S), P(b["q16"]), P(b["k16"]), P(b["v16"]),
+                                               P(ck), P(cv), P(table) if table is not None else None, C.c_int32(self.block_size), st))
+            o = Fnn.scaled_dot_product_attention(b["q16"].transpose(0, 1)[None], b["k16"].transpose(0, 1)[None], b["v16"].transpose(0, 1)[None], is_causal=True,
+                                                 enable_gqa=(nh != nkv))
+            attn = o[0].transpose(0, 1).reshape(S, self.qd)
+            gemm(lay["o"], attn, b["delta"])
             if self.world > 1:
                 torch.distributed.all_reduce(b["delta"], group=self.group)   # prefill-size message: NCCL over NVLink
             delta = b["delta"]
             norm(lay["mlp_norm"])
             gemm(lay["gu"], b["xn"], b["gu"])
-            sw = L.b200q_swiglu_f32_interleaved if lay["swiglu_epi"] else L.b200q_swiglu_f32
-            ops._check(sw(P(b["gu"]), C.c_int64(ff), C.c_int64(S), P(b["act"]), st))
+            ops._check(L.b200q_swiglu_f16(P(b["gu"]), C.c_int64(ff), C.c_int64(S), C.c_int32(1 if lay["swiglu_epi"] else 0), P(b["act"]), st))
             gemm(lay["down"], b["act"], b["delta2"])
             if self.world > 1:
                 torch.distributed.all_reduce(b["delta2"], group=self.group)

@@ -288,6 +288,16 @@ int32_t b200q_swiglu_quant(const float* gate_up, int64_t F, int64_t M, void* xq,
 int32_t b200q_swiglu_f32(const float* gate_up, int64_t F, int64_t M, float* act, void* stream);
 /* same, for gate_up columns in the SwiGLU-epilogue row order of an interleaved gate|up weight (b200q_gate_up_row) */
 int32_t b200q_swiglu_f32_interleaved(const float* gate_up, int64_t F, int64_t M, float* act, void* stream);
+/* Rows of a prompt, results as f16 rows (clamped to the f16 range) for b200q_matmul:
+ *   h_out = h_in (+ delta), x16 = f16(rmsnorm(h_out) * w)      H % 256 == 0, H <= 8192
+ *   act16 = f16(silu(gate) * up)                               interleaved: columns as in b200q_swiglu_f32_interleaved
+ *   RoPE of q and k at positions 0 .. S - 1, K / V rows into the sequence's cache (contiguous [positions][nkv][hd], or block pools through
+ *   its block table), f16 copies q16 [S][nh][hd], k16, v16 [S][nkv][hd]
+ * All rows 16-byte aligned (B200Q_ERR_UNSUPPORTED otherwise). */
+int32_t b200q_add_rmsnorm_f16(const float* h_in, const float* delta, float* h_out, const float* w, float eps, int64_t H, int64_t M, void* x16, void* stream);
+int32_t b200q_swiglu_f16(const float* gate_up, int64_t F, int64_t M, int32_t interleaved, void* act16, void* stream);
+int32_t b200q_rope_kv_prefill(const float* qkv, const float* rope_table, int32_t n_heads, int32_t n_kv_heads, int32_t head_dim, int64_t S, void* q16, void* k16,
+                              void* v16, float* k_cache, float* v_cache, const int32_t* block_table, int32_t block_size, void* stream);
 /* RoPE (adjacent pairs; cos/sin from rope_table [max_ctx][hd/2][2] f32) on q and the new k, KV append at pos[m],
  * single-query attention (f64 reductions, deterministic exp), quantised output.
  * qkv[M,(nh+2nkv)*hd] f32; caches [M][max_ctx][nkv][hd] f32; attn_out (nullable) receives the f32 result */
