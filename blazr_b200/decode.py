@@ -817,11 +817,12 @@ class Decoder:
             self.capture()
         self.reset(prompt[:, 0])
         run = self.replay if use_graph else self.step
+        fed = torch.from_numpy(np.ascontiguousarray(prompt.T)).to(self.dev)   # one upload: a copy per step made the host wait for every step
         out = []
         for s_ in range(S + n_new - 1):
             run()
             if s_ + 1 < S:
-                self.ids.copy_(torch.from_numpy(prompt[:, s_ + 1]).to(self.dev))  # teacher-force the prompt
+                self.ids.copy_(fed[s_ + 1])  # teacher-force the prompt
             else:
                 out.append(self.ids.clone())
         torch.cuda.synchronize(self.dev)

@@ -83,6 +83,8 @@ def lib() -> C.CDLL:
         L.b200q_weight_set_next.argtypes = [C.c_void_p, C.c_void_p]
         L.b200q_gate_up_row.restype = C.c_int64
         L.b200q_gate_up_row.argtypes = [C.c_int64, C.c_int64]
+        p, i32, i64, sz = C.c_void_p, C.c_int32, C.c_int64, C.c_size_t      # the call of every projection: plain numbers, converted once by ctypes
+        L.b200q_matmul_path.argtypes = [p, i32, p, i32, i64, i64, p, i32, i64, p, sz, p]
         _lib = L
     return _lib
 
@@ -245,22 +247,23 @@ class B200Client:
     def quant_matmul(self, x: torch.Tensor, w: QuantWeight, out: Optional[torch.Tensor] = None, out_dtype=None,
                      path: int = PATH_AUTO, workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Y[..., N] = X[..., K] @ dequant(W)[N, K]^T (+bias).  x: f32 / f16 / bf16 on this device."""
-        assert x.is_cuda and x.shape[-1] == w.K, (x.shape, w.K)
-        lead = x.shape[:-1]
-        x2 = x.reshape(-1, w.K)
-        if x2.stride(-1) != 1:
+        shape = x.shape
+        assert x.is_cuda and shape[-1] == w.K, (shape, w.K)
+        x2 = x if len(shape) == 2 else x.reshape(-1, w.K)
+        M, K = x2.shape
+        ldx, one = x2.stride()
+        if one != 1:
             x2 = x2.contiguous()
-        M = x2.shape[0]
-        ydt = out_dtype or x.dtype
+            ldx = K
         if out is None:
-            out = torch.empty((M, w.N), dtype=ydt, device=x.device)
-        y2 = out.reshape(M, w.N)
+            out = torch.empty((M, w.N), dtype=out_dtype or x.dtype, device=x.device)
+        y2 = out if len(out.shape) == 2 and out.shape[0] == M and out.shape[1] == w.N else out.reshape(M, w.N)
         ws = workspace if workspace is not None else w.workspace(M)
-        _check(lib().b200q_matmul_path(w.handle, C.c_int32(path), C.c_void_p(x2.data_ptr()), C.c_int32(_TORCH2DT[x2.dtype]),
-                                       C.c_int64(M), C.c_int64(x2.stride(0)), C.c_void_p(y2.data_ptr()),
-                                       C.c_int32(_TORCH2DT[y2.dtype]), C.c_int64(y2.stride(0)), C.c_void_p(ws.data_ptr()),
-                                       C.c_size_t(ws.numel()), _stream_ptr(x.device)))
-        return out.reshape(*lead, w.N)
+        rc = lib().b200q_matmul_path(w._h, path, x2.data_ptr(), _TORCH2DT[x2.dtype], M, ldx, y2.data_ptr(), _TORCH2DT[y2.dtype], y2.stride(0), ws.data_ptr(), ws.numel(),
+                                     torch._C._cuda_getCurrentRawStream(x.device.index))
+        if rc != 0:
+            _check(rc)
+        return out if len(shape) == 2 and y2 is out else out.reshape(*shape[:-1], w.N)
 
     def quantize_act(self, x: torch.Tensor, perm: Optional[torch.Tensor] = None) -> torch.Tensor:
         x2 = x.reshape(-1, x.shape[-1])
