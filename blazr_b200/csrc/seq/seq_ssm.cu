@@ -12,6 +12,8 @@
 //   B  per entry, in order: start[s] = S;  S = exp(sum log-decay of s) * S + E[s]   (elementwise; the last S goes to the slot)
 //   C  each segment runs again from start[s] and writes the outputs
 // which costs twice the arithmetic of the plain recurrence and removes the dependence on the portion's length.
+// States of up to 128 x any multiple of 4 columns take passes A and C as products of tiles instead (below): the recurrence spends a multiply on the
+// decay and one on the input for every multiply-add that counts, and walks its tokens one after another; pass B runs eight segments ahead.
 #include "seq_common.cuh"
 
 namespace b200seq {
@@ -169,25 +171,347 @@ __global__ void __launch_bounds__(SSM_WARPS * 32) ssm_kernel(const SsmArgs a, co
     if (MODE == SSM_LOCAL && tid == 0 && blockIdx.x == 0) a.seg_logdec[(int64_t)blockIdx.z * H + h] = logdec;
 }
 
-// pass B: one thread per (entry, head, n, v); walks the entry's segments in order
+// pass B: VW values (one thread) of an (entry, head, n, v); walks the entry's segments in order.  The loads of eight segments do not depend on one
+// another and are issued together (one at a time, each behind the store before it: 791 us for 33 segments of 64 x 128 x 64, now bound by memory).
+template <int VW>
 __global__ void ssm_combine_kernel(const SsmArgs a, const b200seq_step st) {
     const int64_t per = (int64_t)a.H * a.N * a.V;
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t idx = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * VW;
     const int e = blockIdx.y;
     if (idx >= per) return;
     const int h = (int)(idx / ((int64_t)a.N * a.V));
     int seg0 = 0;
     for (int i = 0; i < e; ++i) seg0 += (st.ent_start[i + 1] - st.ent_start[i] + a.seg_len - 1) / a.seg_len;
     const int ns = (st.ent_start[e + 1] - st.ent_start[e] + a.seg_len - 1) / a.seg_len;
-    float* slot = a.state + (int64_t)st.ent_slot[e] * per + idx;
-    float S = st.ent_pos0[e] == 0 ? 0.f : *slot;
-    for (int s = 0; s < ns; ++s) {
-        float* p = a.seg_state + (int64_t)(seg0 + s) * per + idx;
-        const float E = *p;
-        *p = S;
-        S = fmaf(expf(a.seg_logdec[(int64_t)(seg0 + s) * a.H + h]), S, E);
+    struct alignas(4 * VW) Vec {
+        float f[VW];
+    };
+    Vec* slot = reinterpret_cast<Vec*>(a.state + (int64_t)st.ent_slot[e] * per + idx);
+    Vec S{};
+    if (st.ent_pos0[e] != 0) S = *slot;
+    constexpr int AHEAD = 8;
+    for (int s0 = 0; s0 < ns; s0 += AHEAD) {
+        Vec E[AHEAD];
+        float d[AHEAD];
+        Vec* p = reinterpret_cast<Vec*>(a.seg_state + (int64_t)(seg0 + s0) * per + idx);
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i)
+            if (s0 + i < ns) E[i] = *reinterpret_cast<const Vec*>(reinterpret_cast<const float*>(p) + i * per), d[i] = expf(a.seg_logdec[(int64_t)(seg0 + s0 + i) * a.H + h]);
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i)
+            if (s0 + i < ns) {
+                *reinterpret_cast<Vec*>(reinterpret_cast<float*>(p) + i * per) = S;
+#pragma unroll
+                for (int u = 0; u < VW; ++u) S.f[u] = fmaf(d[i], S.f[u], E[i].f[u]);
+            }
     }
     *slot = S;
+}
+
+// ---- passes A and C as tile products -----------------------------------------------------------------------------------------------
+// Over a segment of up to SSM_SEG tokens with step sizes dt and L_t the sum of the log-decays up to and including t:
+//     E        = sum_s (dt_s exp(L_end - L_s)) B_s x_s^T                                                   [N x V]
+//     y_t      = exp(L_t) C_t^T S_start + sum_(s <= t) (C_t . B_s) exp(L_t - L_s) dt_s x_s                  [V]
+// f32 multiply-adds (packed pairs) on register tiles of 8 x 4 of a 128 x 64 result, operands staged in shared memory 32 deep.  Decays are
+// exponentials of differences of the sums (never above 1), the sums kept as a float pair of the f64 running sum, so that a difference late in
+// the segment is as exact as an early one.  C_t . B_s does not depend on the head: a block of pass C makes the 128 x 128 of them once and
+// serves SSM_HB heads of the group; earlier tokens enter blockwise -- after 32 tokens the running rows are scaled to the new reference point -- and
+// the tokens of a row's own 32 through a masked 32 x 32 block with exact decays.
+// Bound by the f32 pipe (4096 tokens, 64 heads of 64, state 128: 13 GFLOP).
+constexpr int ST_NT = 256, ST_K = 32, ST_V = 64, ST_P = SSM_SEG + 4;
+constexpr int SSM_HB = 4;
+
+__device__ __forceinline__ uint64_t ss_pk(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void ss_fma2(uint64_t& c, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
+__device__ __forceinline__ float2 ss_upk(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+
+// dt and the running log-decay of the segment's tokens for head h (threads 0 .. 127); tokens beyond the segment: dt 0, the last sum
+struct SegDecay {
+    float dt[SSM_SEG], hi[SSM_SEG], lo[SSM_SEG];
+    double part[4];
+};
+__device__ __forceinline__ void seg_decay(SegDecay& d, const SsmArgs& a, int h, int row0, int len) {
+    const int t = threadIdx.x, lane = t & 31;
+    double L = 0.0;
+    if (t < SSM_SEG) {
+        const float dt = t < len ? softplusf_acc(a.proj[(int64_t)(row0 + t) * a.ldp + a.dt0 + h] + a.dt_bias[h]) : 0.f;
+        d.dt[t] = dt;
+        L = (double)(-expf(a.A_log[h]) * dt);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double u = __shfl_up_sync(0xffffffffu, L, o);
+            if (lane >= o) L += u;
+        }
+        if (lane == 31) d.part[t >> 5] = L;
+    }
+    __syncthreads();
+    if (t < SSM_SEG) {
+        for (int w = 0; w < (t >> 5); ++w) L += d.part[w];
+        const float hi = (float)L;
+        d.hi[t] = hi, d.lo[t] = (float)(L - (double)hi);
+    }
+    __syncthreads();
+}
+// exp(L_t - L_s), t >= s (s = -1: from the segment's start)
+__device__ __forceinline__ float seg_exp(const SegDecay& d, int t, int s) {
+    return s < 0 ? expf(d.hi[t] + d.lo[t]) : expf((d.hi[t] - d.hi[s]) + (d.lo[t] - d.lo[s]));
+}
+
+// pass A: grid (V / 64, H, segments); thread (ty, tx) owns the state rows 4 ty + {0..3} (+ 64) and the columns 4 tx + {0..3}
+template <int NR>   // state rows / 64: 1 or 2
+__global__ void __launch_bounds__(ST_NT) ssm_tile_local_kernel(const SsmArgs a, const b200seq_step st) {
+    __shared__ __align__(16) float Bs[ST_K][64 * NR], Xs[ST_K][ST_V];
+    __shared__ SegDecay dec;
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int h = blockIdx.y, v0 = blockIdx.x * ST_V, N = a.N, V = a.V, inner = a.H * V, g = h / (a.H / a.G);
+    int e, row0, len;
+    if (!ssm_find_segment(st, blockIdx.z, a.seg_len, e, row0, len)) return;
+    seg_decay(dec, a, h, row0, len);
+    uint64_t acc[2 * NR][4];
+#pragma unroll
+    for (int i = 0; i < 2 * NR; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+    const float* xb = a.xbc + (int64_t)h * V + v0;
+    const float* bb = a.xbc + inner + (int64_t)g * N;
+    float4 rb[2 * NR], rx[2];
+    auto fetch = [&](int t0) {
+#pragma unroll
+        for (int i = 0; i < 2 * NR; ++i) {
+            const int idx = tid + i * ST_NT, tt = idx / (16 * NR), c = idx % (16 * NR) * 4;
+            rb[i] = t0 + tt < len && c < N ? ld4(bb + (int64_t)(row0 + t0 + tt) * a.ldx + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int idx = tid + i * ST_NT, tt = idx / 16, c = idx % 16 * 4;
+            rx[i] = t0 + tt < len && v0 + c < V ? ld4(xb + (int64_t)(row0 + t0 + tt) * a.ldx + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    fetch(0);
+    for (int t0 = 0; t0 < len; t0 += ST_K) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 2 * NR; ++i) {
+            const int idx = tid + i * ST_NT;
+            *reinterpret_cast<float4*>(&Bs[idx / (16 * NR)][idx % (16 * NR) * 4]) = rb[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int idx = tid + i * ST_NT, tt = idx / 16;
+            const float w = dec.dt[t0 + tt] * seg_exp(dec, SSM_SEG - 1, t0 + tt);
+            *reinterpret_cast<float4*>(&Xs[tt][idx % 16 * 4]) = make_float4(rx[i].x * w, rx[i].y * w, rx[i].z * w, rx[i].w * w);
+        }
+        __syncthreads();
+        if (t0 + ST_K < len) fetch(t0 + ST_K);
+#pragma unroll 8
+        for (int k = 0; k < ST_K; ++k) {
+            const float4 x = *reinterpret_cast<const float4*>(&Xs[k][4 * tx]);
+            const uint64_t xx[4] = {ss_pk(x.x, x.x), ss_pk(x.y, x.y), ss_pk(x.z, x.z), ss_pk(x.w, x.w)};
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(&Bs[k][64 * r + 4 * ty]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) ss_fma2(acc[2 * r][j], b.x, xx[j]), ss_fma2(acc[2 * r + 1][j], b.y, xx[j]);
+            }
+        }
+    }
+    float* dst = a.seg_state + ((int64_t)blockIdx.z * a.H + h) * N * V + v0 + 4 * tx;
+    if (v0 + 4 * tx < V) {
+#pragma unroll
+        for (int i = 0; i < 2 * NR; ++i) {
+            const int n = 64 * (i >> 1) + 4 * ty + 2 * (i & 1);
+            const float2 p0 = ss_upk(acc[i][0]), p1 = ss_upk(acc[i][1]), p2 = ss_upk(acc[i][2]), p3 = ss_upk(acc[i][3]);
+            if (n < N) *reinterpret_cast<float4*>(dst + (int64_t)n * V) = make_float4(p0.x, p1.x, p2.x, p3.x);
+            if (n + 1 < N) *reinterpret_cast<float4*>(dst + (int64_t)(n + 1) * V) = make_float4(p0.y, p1.y, p2.y, p3.y);
+        }
+    }
+    if (tid == 0 && blockIdx.x == 0) a.seg_logdec[(int64_t)blockIdx.z * a.H + h] = dec.hi[SSM_SEG - 1] + dec.lo[SSM_SEG - 1];
+}
+
+// pass C: grid (V / 64, group x head blocks, segments).  Token t of the segment sits at place 8 (t % 16) + t / 16 of a shared-memory row, so that
+// the eight tokens ty + 16 i of a thread are two 16-byte loads, and the first 2 c of them belong to the first c blocks of 32 tokens.
+struct TileOut {
+    float Ct[128][ST_P];            // [n][token place]
+    float Gt[SSM_SEG][ST_P];        // [s][token place]: C_t . B_s
+    float K[ST_K][ST_P];            // 32-deep tile of B (transposed), or of S / x ([.][64])
+    float M[ST_K][ST_K + 4];        // the own block's masked weights [s][t]
+    SegDecay dec;
+};
+__device__ __forceinline__ int tok_place(int t) { return 8 * (t & 15) + (t >> 4); }
+
+__global__ void __launch_bounds__(ST_NT) ssm_tile_out_kernel(const SsmArgs a, const b200seq_step st) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    TileOut& sm = *reinterpret_cast<TileOut*>(raw);
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int N = a.N, V = a.V, H = a.H, v0 = blockIdx.x * ST_V, per = H / a.G, nb = (per + SSM_HB - 1) / SSM_HB;
+    const int g = blockIdx.y / nb, h_first = g * per + (blockIdx.y % nb) * SSM_HB, h_end = min(h_first + SSM_HB, (g + 1) * per);
+    const int inner = H * V;
+    int e, row0, len;
+    if (!ssm_find_segment(st, blockIdx.z, a.seg_len, e, row0, len)) return;
+    const float* bb = a.xbc + inner + (int64_t)g * N;
+    const float* cb = bb + (int64_t)a.G * N;
+    // C, transposed (rows beyond the segment and n beyond the state are zero)
+    for (int idx = tid; idx < SSM_SEG * 32; idx += ST_NT) {
+        const int t = idx >> 5, n = (idx & 31) * 4, at = tok_place(t);
+        const float4 c = t < len && n < N ? ld4(cb + (int64_t)(row0 + t) * a.ldx + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+        sm.Ct[n][at] = c.x, sm.Ct[n + 1][at] = c.y, sm.Ct[n + 2][at] = c.z, sm.Ct[n + 3][at] = c.w;
+    }
+    {   // C_t . B_s: a thread's 8 tokens x 8 columns (s = 4 tx + {0..3}, + 64); the tokens of the first half see none of the second
+        uint64_t acc[4][8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[i][j] = 0;
+        for (int n0 = 0; n0 < N; n0 += ST_K) {
+            __syncthreads();
+            for (int idx = tid; idx < SSM_SEG * 8; idx += ST_NT) {
+                const int s = idx >> 3, n = (idx & 7) * 4;
+                const float4 b = s < len && n0 + n < N ? ld4(bb + (int64_t)(row0 + s) * a.ldx + n0 + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+                sm.K[n][s] = b.x, sm.K[n + 1][s] = b.y, sm.K[n + 2][s] = b.z, sm.K[n + 3][s] = b.w;
+            }
+            __syncthreads();
+#pragma unroll 4
+            for (int k = 0; k < ST_K; ++k) {
+                const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(&sm.Ct[n0 + k][8 * ty]), c1 = *reinterpret_cast<const ulonglong2*>(&sm.Ct[n0 + k][8 * ty + 4]);
+                const float4 x = *reinterpret_cast<const float4*>(&sm.K[k][4 * tx]), y = *reinterpret_cast<const float4*>(&sm.K[k][64 + 4 * tx]);
+                const uint64_t xx[4] = {ss_pk(x.x, x.x), ss_pk(x.y, x.y), ss_pk(x.z, x.z), ss_pk(x.w, x.w)};
+                const uint64_t yy[4] = {ss_pk(y.x, y.x), ss_pk(y.y, y.y), ss_pk(y.z, y.z), ss_pk(y.w, y.w)};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    ss_fma2(acc[0][j], c0.x, xx[j]), ss_fma2(acc[1][j], c0.y, xx[j]), ss_fma2(acc[2][j], c1.x, xx[j]), ss_fma2(acc[3][j], c1.y, xx[j]);
+                    ss_fma2(acc[2][4 + j], c1.x, yy[j]), ss_fma2(acc[3][4 + j], c1.y, yy[j]);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int s = (j >> 2) * 64 + 4 * tx + (j & 3);
+            *reinterpret_cast<ulonglong2*>(&sm.Gt[s][8 * ty]) = make_ulonglong2(acc[0][j], acc[1][j]);
+            *reinterpret_cast<ulonglong2*>(&sm.Gt[s][8 * ty + 4]) = make_ulonglong2(acc[2][j], acc[3][j]);
+        }
+    }
+    for (int h = h_first; h < h_end; ++h) {
+        __syncthreads();   // Gt is complete, and the head before is done with K, M and dec
+        seg_decay(sm.dec, a, h, row0, len);
+        uint64_t acc[4][4];   // tokens ty + 16 (2 i, 2 i + 1), columns 4 tx + j
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+        const float* sb = a.seg_state + ((int64_t)blockIdx.z * H + h) * N * V + v0;
+        const float* xb = a.xbc + (int64_t)h * V + v0;
+        for (int n0 = 0; n0 < N; n0 += ST_K) {   // C_t^T S_start
+            __syncthreads();
+            for (int idx = tid; idx < ST_K * 16; idx += ST_NT) {
+                const int n = idx >> 4, c = (idx & 15) * 4;
+                *reinterpret_cast<float4*>(&sm.K[n][c]) = n0 + n < N && v0 + c < V ? ld4(sb + (int64_t)(n0 + n) * V + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            __syncthreads();
+#pragma unroll 8
+            for (int k = 0; k < ST_K; ++k) {
+                const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(&sm.Ct[n0 + k][8 * ty]), c1 = *reinterpret_cast<const ulonglong2*>(&sm.Ct[n0 + k][8 * ty + 4]);
+                const float4 x = *reinterpret_cast<const float4*>(&sm.K[k][4 * tx]);
+                const uint64_t xx[4] = {ss_pk(x.x, x.x), ss_pk(x.y, x.y), ss_pk(x.z, x.z), ss_pk(x.w, x.w)};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) ss_fma2(acc[0][j], c0.x, xx[j]), ss_fma2(acc[1][j], c0.y, xx[j]), ss_fma2(acc[2][j], c1.x, xx[j]), ss_fma2(acc[3][j], c1.y, xx[j]);
+            }
+        }
+        // rows are relative to the reference point r = 32 c - 1 (the segment's start for c = 0)
+#pragma unroll
+        for (int c = 0; c < SSM_SEG / ST_K; ++c) {
+            const int s0 = c * ST_K;
+            if (s0 < len) {
+                __syncthreads();
+                for (int idx = tid; idx < ST_K * 16; idx += ST_NT) {   // x of the block's tokens times dt
+                    const int s = idx >> 4, col = (idx & 15) * 4;
+                    const float w = sm.dec.dt[s0 + s];
+                    float4 x = s0 + s < len && v0 + col < V ? ld4(xb + (int64_t)(row0 + s0 + s) * a.ldx + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    x.x *= w, x.y *= w, x.z *= w, x.w *= w;
+                    *reinterpret_cast<float4*>(&sm.K[s][col]) = x;
+                }
+                for (int idx = tid; idx < ST_K * ST_K; idx += ST_NT) {   // own block: [s][t], place 16 * (t / 16) + t % 16
+                    const int s = idx >> 5, t = idx & 31;
+                    sm.M[s][t] = t >= s ? sm.Gt[s0 + s][tok_place(s0 + t)] * seg_exp(sm.dec, s0 + t, s0 + s) : 0.f;
+                }
+                __syncthreads();
+                {   // the block's own rows (tokens s0 + ty, s0 + 16 + ty) are finished: scale to the token, add the block's own part
+                    const float f0 = seg_exp(sm.dec, s0 + ty, s0 - 1), f1 = seg_exp(sm.dec, s0 + 16 + ty, s0 - 1);
+                    const uint64_t ff = ss_pk(f0, f1);
+                    uint64_t own[4] = {0, 0, 0, 0};
+#pragma unroll 8
+                    for (int k = 0; k < ST_K; ++k) {
+                        const uint64_t m = ss_pk(sm.M[k][ty], sm.M[k][16 + ty]);
+                        const float4 x = *reinterpret_cast<const float4*>(&sm.K[k][4 * tx]);
+                        ss_fma2(own[0], m, ss_pk(x.x, x.x)), ss_fma2(own[1], m, ss_pk(x.y, x.y)), ss_fma2(own[2], m, ss_pk(x.z, x.z)), ss_fma2(own[3], m, ss_pk(x.w, x.w));
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        uint64_t r = own[j];
+                        ss_fma2(r, acc[c][j], ff);
+                        acc[c][j] = r;
+                    }
+                }
+                if (s0 + ST_K < len) {   // later rows: to the reference point at the block's end
+                    __syncthreads();
+                    for (int idx = tid; idx < ST_K * 16; idx += ST_NT) {
+                        const int s = idx >> 4, col = (idx & 15) * 4;
+                        const float w = seg_exp(sm.dec, s0 + ST_K - 1, s0 + s);
+                        float4 x = *reinterpret_cast<float4*>(&sm.K[s][col]);
+                        x.x *= w, x.y *= w, x.z *= w, x.w *= w;
+                        *reinterpret_cast<float4*>(&sm.K[s][col]) = x;
+                    }
+                    __syncthreads();
+                    const float f = seg_exp(sm.dec, s0 + ST_K - 1, s0 - 1);
+                    const uint64_t ff = ss_pk(f, f);
+#pragma unroll
+                    for (int i = c + 1; i < 4; ++i)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            uint64_t r = 0;
+                            ss_fma2(r, acc[i][j], ff);
+                            acc[i][j] = r;
+                        }
+#pragma unroll 8
+                    for (int k = 0; k < ST_K; ++k) {
+                        const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(&sm.Gt[s0 + k][8 * ty]), c1 = *reinterpret_cast<const ulonglong2*>(&sm.Gt[s0 + k][8 * ty + 4]);
+                        const uint64_t cc[4] = {c0.x, c0.y, c1.x, c1.y};
+                        const float4 x = *reinterpret_cast<const float4*>(&sm.K[k][4 * tx]);
+                        const uint64_t xx[4] = {ss_pk(x.x, x.x), ss_pk(x.y, x.y), ss_pk(x.z, x.z), ss_pk(x.w, x.w)};
+#pragma unroll
+                        for (int i = c + 1; i < 4; ++i)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) ss_fma2(acc[i][j], cc[i], xx[j]);
+                    }
+                }
+            }
+        }
+        // + D x, times silu(z)
+        const float Dh = a.Dp[h];
+        const float* zb = a.proj + a.z0 + (int64_t)h * V + v0;
+        float* ob = a.out + (int64_t)h * V + v0;
+        const int col = 4 * tx;
+        if (v0 + col < V) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int t = ty + 16 * i;
+                if (t >= len) break;
+                const int64_t row = row0 + t;
+                const float2 p0 = ss_upk(acc[i >> 1][0]), p1 = ss_upk(acc[i >> 1][1]), p2 = ss_upk(acc[i >> 1][2]), p3 = ss_upk(acc[i >> 1][3]);
+                const float4 y = (i & 1) ? make_float4(p0.y, p1.y, p2.y, p3.y) : make_float4(p0.x, p1.x, p2.x, p3.x);
+                const float4 x = ld4(xb + row * a.ldx + col), z = ld4(zb + row * a.ldp + col);
+                *reinterpret_cast<float4*>(ob + row * inner + col) =
+                    make_float4(fmaf(Dh, x.x, y.x) * siluf_acc(z.x), fmaf(Dh, x.y, y.y) * siluf_acc(z.y), fmaf(Dh, x.z, y.z) * siluf_acc(z.z), fmaf(Dh, x.w, y.w) * siluf_acc(z.w));
+            }
+        }
+    }
 }
 
 template <int NPL, int MODE>
@@ -232,12 +556,37 @@ extern "C" int b200seq_ssm_scan(const float* proj, int64_t ldp, int z0, int dt0,
     const int segs = (st->T + SSM_SEG - 1) / SSM_SEG + st->B;   // upper bound of the step's segment count
     a.seg_state = scratch;
     a.seg_logdec = scratch + (size_t)segs * H * N * V;
-    e = small ? ssm_launch<16, SSM_LOCAL>(a, *st, segs, cs) : ssm_launch<32, SSM_LOCAL>(a, *st, segs, cs);
+    // tile products: 16-byte rows everywhere and a state of 33 .. 128 rows (smaller ones leave the 64-row tiles mostly empty)
+    auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    const bool tiles = N > 32 && N <= 128 && N % 4 == 0 && V % 4 == 0 && ((ldp | ldx | z0) & 3) == 0 && al(proj) && al(xbc) && al(state) && al(out) && al(scratch);
+    const int vt = (V + ST_V - 1) / ST_V;
+    if (tiles) {
+        if (N <= 64) ssm_tile_local_kernel<1><<<dim3(vt, H, segs), ST_NT, 0, cs>>>(a, *st);
+        else ssm_tile_local_kernel<2><<<dim3(vt, H, segs), ST_NT, 0, cs>>>(a, *st);
+        e = cudaGetLastError();
+    } else {
+        e = small ? ssm_launch<16, SSM_LOCAL>(a, *st, segs, cs) : ssm_launch<32, SSM_LOCAL>(a, *st, segs, cs);
+    }
     if (e != cudaSuccess) return cuda_status(e, "ssm_scan local pass");
     const int64_t per = (int64_t)H * N * V;
-    ssm_combine_kernel<<<dim3((unsigned)((per + 255) / 256), st->B), 256, 0, cs>>>(a, *st);
+    if (tiles) ssm_combine_kernel<4><<<dim3((unsigned)((per / 4 + 255) / 256), st->B), 256, 0, cs>>>(a, *st);
+    else ssm_combine_kernel<1><<<dim3((unsigned)((per + 255) / 256), st->B), 256, 0, cs>>>(a, *st);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e, "ssm_scan combine pass");
-    e = small ? ssm_launch<16, SSM_FINAL>(a, *st, segs, cs) : ssm_launch<32, SSM_FINAL>(a, *st, segs, cs);
+    if (tiles) {
+        static bool ready[16] = {false};
+        int dev = 0;
+        e = cudaGetDevice(&dev);
+        if (e == cudaSuccess && (dev >= 16 || !ready[dev])) {
+            e = cudaFuncSetAttribute(ssm_tile_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileOut));
+            if (e == cudaSuccess && dev < 16) ready[dev] = true;
+        }
+        if (e == cudaSuccess) {
+            ssm_tile_out_kernel<<<dim3(vt, G * ((H / G + SSM_HB - 1) / SSM_HB), segs), ST_NT, sizeof(TileOut), cs>>>(a, *st);
+            e = cudaGetLastError();
+        }
+    } else {
+        e = small ? ssm_launch<16, SSM_FINAL>(a, *st, segs, cs) : ssm_launch<32, SSM_FINAL>(a, *st, segs, cs);
+    }
     if (e != cudaSuccess) return cuda_status(e, "ssm_scan final pass");
     count_launch(3);
     return 0;

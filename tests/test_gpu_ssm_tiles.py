@@ -1,0 +1,58 @@
+"""The state-space scan of long steps as tile products (csrc/seq/seq_ssm.cu) against the recurrence in float64: portions that end inside a segment and
+inside a block of 32, state and column counts that end inside a tile, one to many heads per group, carried states, fast and slow decays.
+
+Bound: f32 products and sums in another order than the recurrence's; the recurrence is tested at 2e-5 of the largest value, this at 3e-6."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    from blazr_b200 import seqops
+    seqops.lib()
+    return seqops
+
+
+@pytest.mark.parametrize("lens,H,V,N,G", [([129], 2, 64, 128, 1), ([300, 31], 6, 68, 36, 2), ([257, 1, 130], 5, 4, 64, 5), ([700], 9, 64, 100, 1), ([128, 128], 4, 132, 48, 4)])
+@pytest.mark.parametrize("speed", [-8.0, 0.0, 3.0])
+def test_against_the_recurrence(ops, lens, H, V, N, G, speed):
+    from blazr_b200.batch import StepEntry, build_step
+    g = torch.Generator(device=DEV)
+    g.manual_seed(H * V + N)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    T, inner, B = sum(lens), H * V, len(lens)
+    pos0 = [0 if i % 2 == 0 else 64 for i in range(B)]
+    sa = build_step([StepEntry([0] * n, p, B - 1 - i, list(range(-(-(p + n) // 16)))) for i, (n, p) in enumerate(zip(lens, pos0))], 16)
+    t = {k: torch.from_numpy(getattr(sa, k)).to(DEV) for k in ("tok_ent", "tok_pos", "ent_start", "ent_slot", "ent_pos0", "block_table")}
+    st = ops.StepDesc(*(t[k].data_ptr() for k in ("tok_ent", "tok_pos", "ent_start", "ent_slot", "ent_pos0", "block_table")), sa.T, sa.B, sa.block_table.shape[1], 16)
+    ld, ldx = -(-(2 * inner + 2 * G * N + H) // 4) * 4, -(-(inner + 2 * G * N) // 4) * 4
+    proj, xbc, A_log, Dp, dtb = rnd(T, ld), rnd(T, ldx), 0.7 * rnd(H) + speed, rnd(H), rnd(H) - 1.0
+    dt0 = 2 * inner + 2 * G * N
+    state = rnd(B, H, N, V)
+    ref_state, ref = state.double().clone(), torch.empty(T, inner, dtype=torch.float64, device=DEV)
+    x = xbc[:, :inner].double().reshape(T, H, V)
+    Bm, Cm = (xbc[:, inner + i * G * N:inner + (i + 1) * G * N].double().reshape(T, G, N).repeat_interleave(H // G, 1) for i in (0, 1))
+    dt = torch.nn.functional.softplus(proj[:, dt0:dt0 + H].double() + dtb.double())
+    dec = torch.exp(-torch.exp(A_log.double()) * dt)
+    r = 0
+    for i, n in enumerate(lens):
+        S = ref_state[B - 1 - i]
+        if pos0[i] == 0:
+            S.zero_()
+        for k in range(r, r + n):
+            S.mul_(dec[k][:, None, None]).add_(Bm[k][:, :, None] * (dt[k][:, None] * x[k])[:, None, :])
+            y = torch.einsum("hn,hnv->hv", Cm[k], S) + Dp.double()[:, None] * x[k]
+            ref[k] = (y.reshape(-1) * torch.nn.functional.silu(proj[k, :inner].double()))
+        r += n
+    out = torch.empty(T, inner, device=DEV)
+    scratch = torch.empty(ops.ssm_scratch_floats(T, B, H, V, N), device=DEV)
+    assert scratch.numel() > 0
+    ops.ssm_scan(proj, 0, dt0, xbc, A_log, Dp, dtb, state, st, H, V, N, G, out, scratch)
+    for got, want in ((out, ref), (state, ref_state)):
+        err = (got.double() - want).abs().max().item() / want.abs().max().item()
+        assert err < 3e-6, err
