@@ -217,6 +217,7 @@ __global__ void ssm_combine_kernel(const SsmArgs a, const b200seq_step st) {
 // the segment is as exact as an early one.  C_t . B_s does not depend on the head: a block of pass C makes the 128 x 128 of them once and
 // serves SSM_HB heads of the group; earlier tokens enter blockwise -- after 32 tokens the running rows are scaled to the new reference point -- and
 // the tokens of a row's own 32 through a masked 32 x 32 block with exact decays.
+// Every 32 terms are summed by themselves and then added: the rounding of a chain grows with its length.
 // Bound by the f32 pipe (4096 tokens, 64 heads of 64, state 128: 13 GFLOP).
 constexpr int ST_NT = 256, ST_K = 32, ST_V = 64, ST_P = SSM_SEG + 4;
 constexpr int SSM_HB = 4;
@@ -227,6 +228,11 @@ __device__ __forceinline__ uint64_t ss_pk(float a, float b) {
     return r;
 }
 __device__ __forceinline__ void ss_fma2(uint64_t& c, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
+__device__ __forceinline__ uint64_t ss_add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 __device__ __forceinline__ float2 ss_upk(uint64_t v) {
     float2 r;
     asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
@@ -238,8 +244,9 @@ struct SegDecay {
     float dt[SSM_SEG], hi[SSM_SEG], lo[SSM_SEG];
     double part[4];
 };
-__device__ __forceinline__ void seg_decay(SegDecay& d, const SsmArgs& a, int h, int row0, int len) {
-    const int t = threadIdx.x, lane = t & 31;
+__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 256;" ::"r"(1 + group) : "memory"); }   // ST_NT threads each
+__device__ __forceinline__ void seg_decay(SegDecay& d, const SsmArgs& a, int h, int row0, int len, int t, int group) {
+    const int lane = t & 31;
     double L = 0.0;
     if (t < SSM_SEG) {
         const float dt = t < len ? softplusf_acc(a.proj[(int64_t)(row0 + t) * a.ldp + a.dt0 + h] + a.dt_bias[h]) : 0.f;
@@ -252,13 +259,13 @@ __device__ __forceinline__ void seg_decay(SegDecay& d, const SsmArgs& a, int h, 
         }
         if (lane == 31) d.part[t >> 5] = L;
     }
-    __syncthreads();
+    group_sync(group);
     if (t < SSM_SEG) {
         for (int w = 0; w < (t >> 5); ++w) L += d.part[w];
         const float hi = (float)L;
         d.hi[t] = hi, d.lo[t] = (float)(L - (double)hi);
     }
-    __syncthreads();
+    group_sync(group);
 }
 // exp(L_t - L_s), t >= s (s = -1: from the segment's start)
 __device__ __forceinline__ float seg_exp(const SegDecay& d, int t, int s) {
@@ -274,7 +281,7 @@ __global__ void __launch_bounds__(ST_NT) ssm_tile_local_kernel(const SsmArgs a, 
     const int h = blockIdx.y, v0 = blockIdx.x * ST_V, N = a.N, V = a.V, inner = a.H * V, g = h / (a.H / a.G);
     int e, row0, len;
     if (!ssm_find_segment(st, blockIdx.z, a.seg_len, e, row0, len)) return;
-    seg_decay(dec, a, h, row0, len);
+    seg_decay(dec, a, h, row0, len, tid, 0);
     uint64_t acc[2 * NR][4];
 #pragma unroll
     for (int i = 0; i < 2 * NR; ++i)
@@ -311,6 +318,11 @@ __global__ void __launch_bounds__(ST_NT) ssm_tile_local_kernel(const SsmArgs a, 
         }
         __syncthreads();
         if (t0 + ST_K < len) fetch(t0 + ST_K);
+        uint64_t sum[2 * NR][4];
+#pragma unroll
+        for (int i = 0; i < 2 * NR; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sum[i][j] = 0;
 #pragma unroll 8
         for (int k = 0; k < ST_K; ++k) {
             const float4 x = *reinterpret_cast<const float4*>(&Xs[k][4 * tx]);
@@ -319,9 +331,13 @@ __global__ void __launch_bounds__(ST_NT) ssm_tile_local_kernel(const SsmArgs a, 
             for (int r = 0; r < NR; ++r) {
                 const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(&Bs[k][64 * r + 4 * ty]);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) ss_fma2(acc[2 * r][j], b.x, xx[j]), ss_fma2(acc[2 * r + 1][j], b.y, xx[j]);
+                for (int j = 0; j < 4; ++j) ss_fma2(sum[2 * r][j], b.x, xx[j]), ss_fma2(sum[2 * r + 1][j], b.y, xx[j]);
             }
         }
+#pragma unroll
+        for (int i = 0; i < 2 * NR; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = ss_add2(acc[i][j], sum[i][j]);
     }
     float* dst = a.seg_state + ((int64_t)blockIdx.z * a.H + h) * N * V + v0 + 4 * tx;
     if (v0 + 4 * tx < V) {
@@ -336,120 +352,164 @@ __global__ void __launch_bounds__(ST_NT) ssm_tile_local_kernel(const SsmArgs a, 
     if (tid == 0 && blockIdx.x == 0) a.seg_logdec[(int64_t)blockIdx.z * a.H + h] = dec.hi[SSM_SEG - 1] + dec.lo[SSM_SEG - 1];
 }
 
-// pass C: grid (V / 64, group x head blocks, segments).  Token t of the segment sits at place 8 (t % 16) + t / 16 of a shared-memory row, so that
-// the eight tokens ty + 16 i of a thread are two 16-byte loads, and the first 2 c of them belong to the first c blocks of 32 tokens.
-struct TileOut {
-    float Ct[128][ST_P];            // [n][token place]
-    float Gt[SSM_SEG][ST_P];        // [s][token place]: C_t . B_s
-    float K[ST_K][ST_P];            // 32-deep tile of B (transposed), or of S / x ([.][64])
+// pass C: grid (V / 64, group x head blocks, segments), two groups of 256 threads that take every other head.  Token t of the segment sits at
+// place 8 (t % 16) + t / 16 of a shared-memory row, so that the eight tokens ty + 16 i of a thread are two 16-byte loads, and the first 2 c of
+// them belong to the first c blocks of 32 tokens.  With one group of 256 threads and each tile fetched when it was needed the pass took 649 us
+// (4096 tokens, 64 heads of 64, state 128): two warps per scheduler waiting for loads and barriers.
+struct TileGroup {
+    float K[ST_K][ST_P];            // 32-deep tile of S, or of the block's dt x (columns 0 .. 63) beside the same decayed to the block's end (64 .. 127)
     float M[ST_K][ST_K + 4];        // the own block's masked weights [s][t]
     SegDecay dec;
 };
+struct TileOut {
+    float Ct[128][ST_P];            // [n][token place]
+    float Gt[SSM_SEG][ST_P];        // [s][token place]: C_t . B_s
+    TileGroup grp[2];
+};
 __device__ __forceinline__ int tok_place(int t) { return 8 * (t & 15) + (t >> 4); }
 
-__global__ void __launch_bounds__(ST_NT) ssm_tile_out_kernel(const SsmArgs a, const b200seq_step st) {
+__global__ void __launch_bounds__(2 * ST_NT) ssm_tile_out_kernel(const SsmArgs a, const b200seq_step st) {
     extern __shared__ __align__(16) unsigned char raw[];
     TileOut& sm = *reinterpret_cast<TileOut*>(raw);
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int gi = threadIdx.x / ST_NT, tid = threadIdx.x % ST_NT, tx = tid & 15, ty = tid >> 4;
+    TileGroup& sg = sm.grp[gi];
     const int N = a.N, V = a.V, H = a.H, v0 = blockIdx.x * ST_V, per = H / a.G, nb = (per + SSM_HB - 1) / SSM_HB;
     const int g = blockIdx.y / nb, h_first = g * per + (blockIdx.y % nb) * SSM_HB, h_end = min(h_first + SSM_HB, (g + 1) * per);
-    const int inner = H * V;
+    const int inner = H * V, nq = (N + ST_K - 1) / ST_K;
     int e, row0, len;
     if (!ssm_find_segment(st, blockIdx.z, a.seg_len, e, row0, len)) return;
+    const int nblk = (len + ST_K - 1) / ST_K;
     const float* bb = a.xbc + inner + (int64_t)g * N;
     const float* cb = bb + (int64_t)a.G * N;
-    // C, transposed (rows beyond the segment and n beyond the state are zero)
-    for (int idx = tid; idx < SSM_SEG * 32; idx += ST_NT) {
-        const int t = idx >> 5, n = (idx & 31) * 4, at = tok_place(t);
-        const float4 c = t < len && n < N ? ld4(cb + (int64_t)(row0 + t) * a.ldx + n) : make_float4(0.f, 0.f, 0.f, 0.f);
-        sm.Ct[n][at] = c.x, sm.Ct[n + 1][at] = c.y, sm.Ct[n + 2][at] = c.z, sm.Ct[n + 3][at] = c.w;
-    }
-    {   // C_t . B_s: a thread's 8 tokens x 8 columns (s = 4 tx + {0..3}, + 64); the tokens of the first half see none of the second
-        uint64_t acc[4][8];
+    // tile i of head h: rows 32 i .. of the start state (i < nq), then the x rows of block i - nq
+    float4 nx[2];
+    auto fetch = [&](int h, int i) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[i][j] = 0;
-        for (int n0 = 0; n0 < N; n0 += ST_K) {
-            __syncthreads();
-            for (int idx = tid; idx < SSM_SEG * 8; idx += ST_NT) {
-                const int s = idx >> 3, n = (idx & 7) * 4;
-                const float4 b = s < len && n0 + n < N ? ld4(bb + (int64_t)(row0 + s) * a.ldx + n0 + n) : make_float4(0.f, 0.f, 0.f, 0.f);
-                sm.K[n][s] = b.x, sm.K[n + 1][s] = b.y, sm.K[n + 2][s] = b.z, sm.K[n + 3][s] = b.w;
-            }
-            __syncthreads();
-#pragma unroll 4
-            for (int k = 0; k < ST_K; ++k) {
-                const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(&sm.Ct[n0 + k][8 * ty]), c1 = *reinterpret_cast<const ulonglong2*>(&sm.Ct[n0 + k][8 * ty + 4]);
-                const float4 x = *reinterpret_cast<const float4*>(&sm.K[k][4 * tx]), y = *reinterpret_cast<const float4*>(&sm.K[k][64 + 4 * tx]);
-                const uint64_t xx[4] = {ss_pk(x.x, x.x), ss_pk(x.y, x.y), ss_pk(x.z, x.z), ss_pk(x.w, x.w)};
-                const uint64_t yy[4] = {ss_pk(y.x, y.x), ss_pk(y.y, y.y), ss_pk(y.z, y.z), ss_pk(y.w, y.w)};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    ss_fma2(acc[0][j], c0.x, xx[j]), ss_fma2(acc[1][j], c0.y, xx[j]), ss_fma2(acc[2][j], c1.x, xx[j]), ss_fma2(acc[3][j], c1.y, xx[j]);
-                    ss_fma2(acc[2][4 + j], c1.x, yy[j]), ss_fma2(acc[3][4 + j], c1.y, yy[j]);
+        for (int u = 0; u < 2; ++u) {
+            const int idx = tid + u * ST_NT, r = idx >> 4, c = (idx & 15) * 4;
+            nx[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (h < h_end && v0 + c < V) {
+                if (i < nq) {
+                    if (i * ST_K + r < N) nx[u] = ld4(a.seg_state + (((int64_t)blockIdx.z * H + h) * N + i * ST_K + r) * V + v0 + c);
+                } else if ((i - nq) * ST_K + r < len) {
+                    nx[u] = ld4(a.xbc + (int64_t)(row0 + (i - nq) * ST_K + r) * a.ldx + (int64_t)h * V + v0 + c);
                 }
             }
         }
+    };
+    fetch(h_first + gi, 0);
+    // C, transposed (rows beyond the segment and n beyond the state are zero)
+    for (int idx = threadIdx.x; idx < SSM_SEG * 32; idx += 2 * ST_NT) {
+        const int t = (idx & 7) + 8 * (idx >> 8), n = ((idx >> 3) & 31) * 4, at = tok_place(t);
+        const float4 c = t < len && n < N ? ld4(cb + (int64_t)(row0 + t) * a.ldx + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+        sm.Ct[n][at] = c.x, sm.Ct[n + 1][at] = c.y, sm.Ct[n + 2][at] = c.z, sm.Ct[n + 3][at] = c.w;
+    }
+    {   // C_t . B_s: a thread's 8 tokens x 4 columns s = 64 gi + 4 tx + {0..3}; the tokens of the first half see none of the second
+        uint64_t acc[4][4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int s = (j >> 2) * 64 + 4 * tx + (j & 3);
-            *reinterpret_cast<ulonglong2*>(&sm.Gt[s][8 * ty]) = make_ulonglong2(acc[0][j], acc[1][j]);
-            *reinterpret_cast<ulonglong2*>(&sm.Gt[s][8 * ty + 4]) = make_ulonglong2(acc[2][j], acc[3][j]);
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+        for (int n0 = 0; n0 < N; n0 += ST_K) {
+            __syncthreads();
+            for (int idx = threadIdx.x; idx < SSM_SEG * 8; idx += 2 * ST_NT) {   // B's tile, transposed, in group 0's buffer
+                const int s_ = idx >> 3, n = (idx & 7) * 4;
+                const float4 b = s_ < len && n0 + n < N ? ld4(bb + (int64_t)(row0 + s_) * a.ldx + n0 + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+                sm.grp[0].K[n][s_] = b.x, sm.grp[0].K[n + 1][s_] = b.y, sm.grp[0].K[n + 2][s_] = b.z, sm.grp[0].K[n + 3][s_] = b.w;
+            }
+            __syncthreads();
+            uint64_t sum[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) sum[i][j] = 0;
+#pragma unroll 8
+            for (int k = 0; k < ST_K; ++k) {
+                const float4 x = *reinterpret_cast<const float4*>(&sm.grp[0].K[k][64 * gi + 4 * tx]);
+                const uint64_t xx[4] = {ss_pk(x.x, x.x), ss_pk(x.y, x.y), ss_pk(x.z, x.z), ss_pk(x.w, x.w)};
+                const ulonglong2 c1 = *reinterpret_cast<const ulonglong2*>(&sm.Ct[n0 + k][8 * ty + 4]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) ss_fma2(sum[2][j], c1.x, xx[j]), ss_fma2(sum[3][j], c1.y, xx[j]);
+                if (gi == 0) {
+                    const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(&sm.Ct[n0 + k][8 * ty]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) ss_fma2(sum[0][j], c0.x, xx[j]), ss_fma2(sum[1][j], c0.y, xx[j]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = ss_add2(acc[i][j], sum[i][j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            *reinterpret_cast<ulonglong2*>(&sm.Gt[64 * gi + 4 * tx + j][8 * ty]) = make_ulonglong2(acc[0][j], acc[1][j]);
+            *reinterpret_cast<ulonglong2*>(&sm.Gt[64 * gi + 4 * tx + j][8 * ty + 4]) = make_ulonglong2(acc[2][j], acc[3][j]);
         }
     }
-    for (int h = h_first; h < h_end; ++h) {
-        __syncthreads();   // Gt is complete, and the head before is done with K, M and dec
-        seg_decay(sm.dec, a, h, row0, len);
+    __syncthreads();   // Gt is complete, B's tile has been read
+    for (int h = h_first + gi; h < h_end; h += 2) {
+        seg_decay(sg.dec, a, h, row0, len, tid, gi);   // (its first barrier lies behind the head before's last use of dec: see the barrier at the loop's end)
         uint64_t acc[4][4];   // tokens ty + 16 (2 i, 2 i + 1), columns 4 tx + j
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j] = 0;
-        const float* sb = a.seg_state + ((int64_t)blockIdx.z * H + h) * N * V + v0;
-        const float* xb = a.xbc + (int64_t)h * V + v0;
-        for (int n0 = 0; n0 < N; n0 += ST_K) {   // C_t^T S_start
-            __syncthreads();
-            for (int idx = tid; idx < ST_K * 16; idx += ST_NT) {
-                const int n = idx >> 4, c = (idx & 15) * 4;
-                *reinterpret_cast<float4*>(&sm.K[n][c]) = n0 + n < N && v0 + c < V ? ld4(sb + (int64_t)(n0 + n) * V + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int q = 0; q < nq; ++q) {   // C_t^T S_start
+            if (q > 0) group_sync(gi);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int idx = tid + u * ST_NT;
+                *reinterpret_cast<float4*>(&sg.K[idx >> 4][(idx & 15) * 4]) = nx[u];
             }
-            __syncthreads();
+            group_sync(gi);
+            fetch(h, q + 1);
+            uint64_t sum[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) sum[i][j] = 0;
 #pragma unroll 8
             for (int k = 0; k < ST_K; ++k) {
-                const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(&sm.Ct[n0 + k][8 * ty]), c1 = *reinterpret_cast<const ulonglong2*>(&sm.Ct[n0 + k][8 * ty + 4]);
-                const float4 x = *reinterpret_cast<const float4*>(&sm.K[k][4 * tx]);
+                const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(&sm.Ct[q * ST_K + k][8 * ty]), c1 = *reinterpret_cast<const ulonglong2*>(&sm.Ct[q * ST_K + k][8 * ty + 4]);
+                const float4 x = *reinterpret_cast<const float4*>(&sg.K[k][4 * tx]);
                 const uint64_t xx[4] = {ss_pk(x.x, x.x), ss_pk(x.y, x.y), ss_pk(x.z, x.z), ss_pk(x.w, x.w)};
 #pragma unroll
-                for (int j = 0; j < 4; ++j) ss_fma2(acc[0][j], c0.x, xx[j]), ss_fma2(acc[1][j], c0.y, xx[j]), ss_fma2(acc[2][j], c1.x, xx[j]), ss_fma2(acc[3][j], c1.y, xx[j]);
+                for (int j = 0; j < 4; ++j) ss_fma2(sum[0][j], c0.x, xx[j]), ss_fma2(sum[1][j], c0.y, xx[j]), ss_fma2(sum[2][j], c1.x, xx[j]), ss_fma2(sum[3][j], c1.y, xx[j]);
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = ss_add2(acc[i][j], sum[i][j]);
         }
         // rows are relative to the reference point r = 32 c - 1 (the segment's start for c = 0)
 #pragma unroll
         for (int c = 0; c < SSM_SEG / ST_K; ++c) {
             const int s0 = c * ST_K;
-            if (s0 < len) {
-                __syncthreads();
-                for (int idx = tid; idx < ST_K * 16; idx += ST_NT) {   // x of the block's tokens times dt
-                    const int s = idx >> 4, col = (idx & 15) * 4;
-                    const float w = sm.dec.dt[s0 + s];
-                    float4 x = s0 + s < len && v0 + col < V ? ld4(xb + (int64_t)(row0 + s0 + s) * a.ldx + col) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    x.x *= w, x.y *= w, x.z *= w, x.w *= w;
-                    *reinterpret_cast<float4*>(&sm.K[s][col]) = x;
+            if (c < nblk) {
+                group_sync(gi);
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int idx = tid + u * ST_NT, r = idx >> 4, col = (idx & 15) * 4;
+                    const float w = sg.dec.dt[s0 + r], w2 = w * seg_exp(sg.dec, s0 + ST_K - 1, s0 + r);
+                    *reinterpret_cast<float4*>(&sg.K[r][col]) = make_float4(nx[u].x * w, nx[u].y * w, nx[u].z * w, nx[u].w * w);
+                    *reinterpret_cast<float4*>(&sg.K[r][64 + col]) = make_float4(nx[u].x * w2, nx[u].y * w2, nx[u].z * w2, nx[u].w * w2);
                 }
-                for (int idx = tid; idx < ST_K * ST_K; idx += ST_NT) {   // own block: [s][t], place 16 * (t / 16) + t % 16
-                    const int s = idx >> 5, t = idx & 31;
-                    sm.M[s][t] = t >= s ? sm.Gt[s0 + s][tok_place(s0 + t)] * seg_exp(sm.dec, s0 + t, s0 + s) : 0.f;
+#pragma unroll
+                for (int u = 0; u < ST_K * ST_K / ST_NT; ++u) {
+                    const int idx = tid + u * ST_NT, s_ = idx >> 5, t = idx & 31;
+                    sg.M[s_][t] = t >= s_ ? sm.Gt[s0 + s_][tok_place(s0 + t)] * seg_exp(sg.dec, s0 + t, s0 + s_) : 0.f;
                 }
-                __syncthreads();
+                group_sync(gi);
+                if (c + 1 < nblk) fetch(h, nq + c + 1);
+                else fetch(h + 2, 0);
                 {   // the block's own rows (tokens s0 + ty, s0 + 16 + ty) are finished: scale to the token, add the block's own part
-                    const float f0 = seg_exp(sm.dec, s0 + ty, s0 - 1), f1 = seg_exp(sm.dec, s0 + 16 + ty, s0 - 1);
-                    const uint64_t ff = ss_pk(f0, f1);
+                    const uint64_t ff = ss_pk(seg_exp(sg.dec, s0 + ty, s0 - 1), seg_exp(sg.dec, s0 + 16 + ty, s0 - 1));
                     uint64_t own[4] = {0, 0, 0, 0};
 #pragma unroll 8
                     for (int k = 0; k < ST_K; ++k) {
-                        const uint64_t m = ss_pk(sm.M[k][ty], sm.M[k][16 + ty]);
-                        const float4 x = *reinterpret_cast<const float4*>(&sm.K[k][4 * tx]);
+                        const uint64_t m = ss_pk(sg.M[k][ty], sg.M[k][16 + ty]);
+                        const float4 x = *reinterpret_cast<const float4*>(&sg.K[k][4 * tx]);
                         ss_fma2(own[0], m, ss_pk(x.x, x.x)), ss_fma2(own[1], m, ss_pk(x.y, x.y)), ss_fma2(own[2], m, ss_pk(x.z, x.z)), ss_fma2(own[3], m, ss_pk(x.w, x.w));
                     }
 #pragma unroll
@@ -459,42 +519,38 @@ __global__ void __launch_bounds__(ST_NT) ssm_tile_out_kernel(const SsmArgs a, co
                         acc[c][j] = r;
                     }
                 }
-                if (s0 + ST_K < len) {   // later rows: to the reference point at the block's end
-                    __syncthreads();
-                    for (int idx = tid; idx < ST_K * 16; idx += ST_NT) {
-                        const int s = idx >> 4, col = (idx & 15) * 4;
-                        const float w = seg_exp(sm.dec, s0 + ST_K - 1, s0 + s);
-                        float4 x = *reinterpret_cast<float4*>(&sm.K[s][col]);
-                        x.x *= w, x.y *= w, x.z *= w, x.w *= w;
-                        *reinterpret_cast<float4*>(&sm.K[s][col]) = x;
-                    }
-                    __syncthreads();
-                    const float f = seg_exp(sm.dec, s0 + ST_K - 1, s0 - 1);
+                if (c + 1 < nblk) {   // later rows: to the reference point at the block's end
+                    const float f = seg_exp(sg.dec, s0 + ST_K - 1, s0 - 1);
                     const uint64_t ff = ss_pk(f, f);
+                    uint64_t sum[4][4];
 #pragma unroll
                     for (int i = c + 1; i < 4; ++i)
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            uint64_t r = 0;
-                            ss_fma2(r, acc[i][j], ff);
-                            acc[i][j] = r;
-                        }
+                        for (int j = 0; j < 4; ++j) sum[i][j] = 0;
 #pragma unroll 8
                     for (int k = 0; k < ST_K; ++k) {
                         const ulonglong2 c0 = *reinterpret_cast<const ulonglong2*>(&sm.Gt[s0 + k][8 * ty]), c1 = *reinterpret_cast<const ulonglong2*>(&sm.Gt[s0 + k][8 * ty + 4]);
                         const uint64_t cc[4] = {c0.x, c0.y, c1.x, c1.y};
-                        const float4 x = *reinterpret_cast<const float4*>(&sm.K[k][4 * tx]);
+                        const float4 x = *reinterpret_cast<const float4*>(&sg.K[k][64 + 4 * tx]);
                         const uint64_t xx[4] = {ss_pk(x.x, x.x), ss_pk(x.y, x.y), ss_pk(x.z, x.z), ss_pk(x.w, x.w)};
 #pragma unroll
                         for (int i = c + 1; i < 4; ++i)
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) ss_fma2(acc[i][j], cc[i], xx[j]);
+                            for (int j = 0; j < 4; ++j) ss_fma2(sum[i][j], cc[i], xx[j]);
                     }
+#pragma unroll
+                    for (int i = c + 1; i < 4; ++i)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            ss_fma2(sum[i][j], acc[i][j], ff);
+                            acc[i][j] = sum[i][j];
+                        }
                 }
             }
         }
         // + D x, times silu(z)
         const float Dh = a.Dp[h];
+        const float* xb = a.xbc + (int64_t)h * V + v0;
         const float* zb = a.proj + a.z0 + (int64_t)h * V + v0;
         float* ob = a.out + (int64_t)h * V + v0;
         const int col = 4 * tx;
@@ -511,6 +567,7 @@ __global__ void __launch_bounds__(ST_NT) ssm_tile_out_kernel(const SsmArgs a, co
                     make_float4(fmaf(Dh, x.x, y.x) * siluf_acc(z.x), fmaf(Dh, x.y, y.y) * siluf_acc(z.y), fmaf(Dh, x.z, y.z) * siluf_acc(z.z), fmaf(Dh, x.w, y.w) * siluf_acc(z.w));
             }
         }
+        group_sync(gi);   // the group is done with this head's K, M and dec
     }
 }
 
@@ -581,7 +638,7 @@ extern "C" int b200seq_ssm_scan(const float* proj, int64_t ldp, int z0, int dt0,
             if (e == cudaSuccess && dev < 16) ready[dev] = true;
         }
         if (e == cudaSuccess) {
-            ssm_tile_out_kernel<<<dim3(vt, G * ((H / G + SSM_HB - 1) / SSM_HB), segs), ST_NT, sizeof(TileOut), cs>>>(a, *st);
+            ssm_tile_out_kernel<<<dim3(vt, G * ((H / G + SSM_HB - 1) / SSM_HB), segs), 2 * ST_NT, sizeof(TileOut), cs>>>(a, *st);
             e = cudaGetLastError();
         }
     } else {
