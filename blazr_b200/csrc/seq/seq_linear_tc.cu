@@ -17,6 +17,8 @@
 // exit (its copies in flight are waited for, again bounded, and its tensor memory is freed).
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "seq_common.cuh"
 #include "tc_pair.cuh"
 
@@ -234,13 +236,16 @@ __global__ void __launch_bounds__(128) linear_tc_kernel(const __grid_constant__ 
 }
 
 // ---- epilogues of the paired-SM kernel (tc_pair.cuh): v[j] = acc[n][m + j] ----
+// One instantiation per activation kind and output type: with the kind tested per value, every kind's code (divisions, erfc, tanh) was inlined for
+// each of the 16 or 32 values and the epilogue warps waited for instructions.
+template <bool SILU>
 struct EpiF32 {
     float* y;
     int64_t ldy;
     int N, silu_lo, silu_hi;
     __device__ __forceinline__ void store(float (&v)[32], int n, int m, int m_end, int) const {
         if (n >= N) return;
-        if (n >= silu_lo && n < silu_hi) {
+        if (SILU && n >= silu_lo && n < silu_hi) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = siluf_acc(v[j]);
         }
@@ -255,20 +260,23 @@ struct EpiF32 {
         }
     }
 };
+template <int KIND, typename T>
 struct EpiPlainAct {
-    void* out;
+    T* out;
     int64_t ldo;
-    int N, dtype, kind;
+    int N;
     __device__ __forceinline__ void store(float (&v)[32], int n, int m, int m_end, int) const {
         if (n >= N) return;
+        T* o = out + (int64_t)m * ldo + n;
 #pragma unroll
         for (int j = 0; j < 32; ++j)
-            if (m + j < m_end) store_act(out, dtype, (int64_t)(m + j) * ldo + n, act_plain(kind, v[j]));
+            if (m + j < m_end) {
+                const float r = act_plain(KIND, v[j]);
+                if constexpr (sizeof(T) == 4) o[(int64_t)j * ldo] = r;
+                else o[(int64_t)j * ldo] = __float2bfloat16_rn(r);
+            }
     }
 };
-// rows alternate (gate j, up j): an even lane holds the gates, the odd lane beside it the ups of the same 32 tokens.  They trade halves, so
-// that the even lane computes tokens 0 .. 15 and the odd one 16 .. 31 (one activation per lane and token instead of one per lane pair).
-// pack: bf16 output with 4-byte aligned pairs of columns -- lanes two apart trade again and store two columns at once
 // Activations that leave as bf16 take the division without its branches (reciprocal approximation and one Newton step, 1 ulp of f32): the
 // rounding call behind 1 / d kept the 16 activations of a lane from overlapping and made the epilogue, not the tensor pipe, the bound
 // (4096 x 16384 x 2048: 326 us against 202 us of the plain product).  f32 outputs keep the rounded division.
@@ -278,41 +286,56 @@ __device__ __forceinline__ float sigmoid_nobranch(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(r, fmaf(-d, r, 1.0f), r);
 }
+template <int KIND>
 __device__ __forceinline__ float act_gated_nobranch(const ActParams& a, float gate, float up) {
-    if (a.kind == B200SEQ_ACT_GELU_TANH) return gate * sigmoid_nobranch(1.5957691216057308f * (gate + 0.044715f * gate * gate * gate)) * up;
+    if (KIND == B200SEQ_ACT_GELU_TANH) return gate * sigmoid_nobranch(1.5957691216057308f * (gate + 0.044715f * gate * gate * gate)) * up;
     const float g = fminf(gate, a.limit);
     const float u = fminf(fmaxf(up, -a.limit), a.limit);
     return g * sigmoid_nobranch(a.alpha * g) * (u + a.shift);
 }
+// rows alternate (gate j, up j): an even lane holds the gates, the odd lane beside it the ups of the same 32 tokens.  They trade halves, so
+// that the even lane computes tokens 0 .. 15 and the odd one 16 .. 31 (one activation per lane and token instead of one per lane pair).
+// pack: bf16 output with 4-byte aligned pairs of columns -- lanes two apart trade again and store two columns at once
+template <int KIND, typename T>
 struct EpiGated {
-    void* out;
+    T* out;
     int64_t ldo;
-    int N, dtype, pack;
+    int N, pack;
     ActParams act;
     __device__ __forceinline__ void store(float (&v)[32], int n, int m, int m_end, int lane) const {
+        constexpr bool BF16 = sizeof(T) == 2;
         const bool odd = lane & 1;
+        ActParams a = act;
+        a.kind = KIND;
         float r[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
             const float x = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 16], 1);
             const float g = odd ? x : v[j], u = odd ? v[j + 16] : x;
-            r[j] = dtype == B200SEQ_BF16 ? act_gated_nobranch(act, g, u) : act_gated(act, g, u);
+            r[j] = BF16 ? act_gated_nobranch<KIND>(a, g, u) : act_gated(a, g, u);
         }
         const int f = n >> 1, mt = m + (odd ? 16 : 0);
-        if (pack) {
-            const bool hi = lane & 2;
+        if constexpr (BF16) {
+            if (pack) {
+                const bool hi = lane & 2;
+                const int t0 = mt + (hi ? 8 : 0);
+                T* o = out + (int64_t)t0 * ldo + (f & ~1);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float x = __shfl_xor_sync(0xffffffffu, hi ? r[j] : r[j + 8], 2);
-                const __nv_bfloat162 b = hi ? __floats2bfloat162_rn(x, r[j + 8]) : __floats2bfloat162_rn(r[j], x);
-                const int t = mt + j + (hi ? 8 : 0);
-                if (n < N && t < m_end) *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(out) + (int64_t)t * ldo + (f & ~1)) = b;
+                for (int j = 0; j < 8; ++j) {
+                    const float x = __shfl_xor_sync(0xffffffffu, hi ? r[j] : r[j + 8], 2);
+                    const __nv_bfloat162 b = hi ? __floats2bfloat162_rn(x, r[j + 8]) : __floats2bfloat162_rn(r[j], x);
+                    if (n < N && t0 + j < m_end) *reinterpret_cast<__nv_bfloat162*>(o + (int64_t)j * ldo) = b;
+                }
+                return;
             }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-                if ((n | 1) < N && mt + j < m_end) store_act(out, dtype, (int64_t)(mt + j) * ldo + f, r[j]);
         }
+        T* o = out + (int64_t)mt * ldo + f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            if ((n | 1) < N && mt + j < m_end) {
+                if constexpr (BF16) o[(int64_t)j * ldo] = __float2bfloat16_rn(r[j]);
+                else o[(int64_t)j * ldo] = r[j];
+            }
     }
 };
 
@@ -341,12 +364,26 @@ int launch(const void* x, int64_t ldx, const void* w, TcParams p, cudaStream_t s
     const int64_t wrows = p.offs ? (int64_t)p.E * p.N : (p.heads ? (int64_t)p.heads * p.N : p.N);
     p.err = error_flag_dev();
     if (const int tile = pick_tile(p)) {
-        cudaError_t e;
-        if (p.epi == EPI_NONE) e = launch_pair(tile, x, ldx, w, p, EpiF32{p.y, p.ldy, p.N, p.silu_lo, p.silu_hi}, st);
-        else if (p.epi == EPI_PLAIN_ACT) e = launch_pair(tile, x, ldx, w, p, EpiPlainAct{p.act_out, p.ldo, p.N, p.out_dtype, p.act.kind}, st);
-        else {
-            const int pack = p.out_dtype == B200SEQ_BF16 && p.N % 4 == 0 && p.ldo % 2 == 0 && (reinterpret_cast<uintptr_t>(p.act_out) & 3) == 0;
-            e = launch_pair(tile, x, ldx, w, p, EpiGated{p.act_out, p.ldo, p.N, p.out_dtype, pack, p.act}, st);
+        cudaError_t e = cudaErrorInvalidValue;
+        auto typed = [&](auto* out) {
+            using T = std::remove_pointer_t<decltype(out)>;
+            const int pack = sizeof(T) == 2 && p.N % 4 == 0 && p.ldo % 2 == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0;
+            switch (p.act.kind) {
+                case B200SEQ_ACT_SWISH_CLAMP: return launch_pair(tile, x, ldx, w, p, EpiGated<B200SEQ_ACT_SWISH_CLAMP, T>{out, p.ldo, p.N, pack, p.act}, st);
+                case B200SEQ_ACT_GELU_TANH: return launch_pair(tile, x, ldx, w, p, EpiGated<B200SEQ_ACT_GELU_TANH, T>{out, p.ldo, p.N, pack, p.act}, st);
+                case B200SEQ_ACT_RELU2: return launch_pair(tile, x, ldx, w, p, EpiPlainAct<B200SEQ_ACT_RELU2, T>{out, p.ldo, p.N}, st);
+                case B200SEQ_ACT_GELU_ERF: return launch_pair(tile, x, ldx, w, p, EpiPlainAct<B200SEQ_ACT_GELU_ERF, T>{out, p.ldo, p.N}, st);
+                case B200SEQ_ACT_TANH: return launch_pair(tile, x, ldx, w, p, EpiPlainAct<B200SEQ_ACT_TANH, T>{out, p.ldo, p.N}, st);
+                default: return launch_pair(tile, x, ldx, w, p, EpiPlainAct<B200SEQ_ACT_IDENT, T>{out, p.ldo, p.N}, st);
+            }
+        };
+        if (p.epi == EPI_NONE) {
+            if (p.silu_hi > p.silu_lo) e = launch_pair(tile, x, ldx, w, p, EpiF32<true>{p.y, p.ldy, p.N, p.silu_lo, p.silu_hi}, st);
+            else e = launch_pair(tile, x, ldx, w, p, EpiF32<false>{p.y, p.ldy, p.N, 0, 0}, st);
+        } else if (p.out_dtype == B200SEQ_F32) {
+            e = typed(reinterpret_cast<float*>(p.act_out));
+        } else {
+            e = typed(reinterpret_cast<__nv_bfloat16*>(p.act_out));
         }
         if (e != cudaSuccess) return cuda_status(e, "linear tc pair");
         count_launch();

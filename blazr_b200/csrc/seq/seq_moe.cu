@@ -217,48 +217,56 @@ __global__ void __launch_bounds__(256) moe_router_rows_kernel(const XT* __restri
     if (cr == 0 && wid == 0) route_token(sm, sm + NR, t, lane, rule, ids, wts, nullptr);
 }
 
-// grid (E), 256 threads: block e places the pairs of expert e behind those of the experts before it, in pair order
-__global__ void moe_sort_kernel(const int32_t* __restrict__ ids, int pairs, int E, const int32_t* __restrict__ counts, int32_t* __restrict__ offs,
-                                int32_t* __restrict__ sorted, int32_t* __restrict__ slot_of) {
-    __shared__ int seg[9];
-    __shared__ int red[8];
+// grid (E), SORT_NT threads: block e places the pairs of expert e behind those of the experts before it, in pair order.  Bound by latency (a few
+// hundred KB in all): eight ids per lane are requested together and 32 warps share the pairs (eight warps with one id at a time: 18 us for
+// 16 384 pairs, now 6).
+constexpr int SORT_NT = 1024, SORT_W = SORT_NT / 32, SORT_U = 8;
+__global__ void __launch_bounds__(SORT_NT) moe_sort_kernel(const int32_t* __restrict__ ids, int pairs, int E, const int32_t* __restrict__ counts, int32_t* __restrict__ offs,
+                                                           int32_t* __restrict__ sorted, int32_t* __restrict__ slot_of) {
+    __shared__ int seg[SORT_W], red[SORT_W];
     const int e = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int per = ((pairs + SORT_W - 1) / SORT_W + 31) & ~31;   // a warp's contiguous share of the pairs
+    const int lo = min(pairs, wid * per), hi = min(pairs, lo + per);
+    int n = 0;
+    for (int p0 = lo; p0 < hi; p0 += 32 * SORT_U) {
+        bool mine[SORT_U];
+#pragma unroll
+        for (int i = 0; i < SORT_U; ++i) {
+            const int p = p0 + 32 * i + lane;
+            mine[i] = p < hi && ids[p] == e;
+        }
+#pragma unroll
+        for (int i = 0; i < SORT_U; ++i) n += __popc(__ballot_sync(0xffffffffu, mine[i]));
+    }
     int before = 0;
     for (int i = threadIdx.x; i < e; i += blockDim.x) before += counts[i];
     for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
-    if (lane == 0) red[wid] = before;
+    if (lane == 0) red[wid] = before, seg[wid] = n;
     __syncthreads();
-    int off = 0;
-    for (int w = 0; w < 8; ++w) off += red[w];
+    int off = __reduce_add_sync(0xffffffffu, red[lane]);
+    const int at0 = __reduce_add_sync(0xffffffffu, lane < wid ? seg[lane] : 0);
     if (threadIdx.x == 0) {
         offs[e] = off;
         if (e == E - 1) offs[E] = off + counts[e];
     }
-    const int per = ((pairs + 7) / 8 + 31) & ~31;   // a warp's contiguous share of the pairs
-    const int lo = wid * per, hi = min(pairs, lo + per);
-    int n = 0;
-    for (int p0 = lo; p0 < hi; p0 += 32) {
-        const int p = p0 + lane;
-        n += __popc(__ballot_sync(0xffffffffu, p < hi && ids[p] == e));
-    }
-    if (lane == 0) seg[wid + 1] = n;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        seg[0] = 0;
-        for (int w = 1; w <= 8; ++w) seg[w] += seg[w - 1];
-    }
-    __syncthreads();
-    int at = off + seg[wid];
-    for (int p0 = lo; p0 < hi; p0 += 32) {
-        const int p = p0 + lane;
-        const bool mine = p < hi && ids[p] == e;
-        const uint32_t bal = __ballot_sync(0xffffffffu, mine);
-        if (mine) {
-            const int slot = at + __popc(bal & ((1u << lane) - 1));
-            sorted[slot] = p;
-            slot_of[p] = slot;
+    int at = off + at0;
+    for (int p0 = lo; p0 < hi; p0 += 32 * SORT_U) {
+        bool mine[SORT_U];
+#pragma unroll
+        for (int i = 0; i < SORT_U; ++i) {
+            const int p = p0 + 32 * i + lane;
+            mine[i] = p < hi && ids[p] == e;
         }
-        at += __popc(bal);
+#pragma unroll
+        for (int i = 0; i < SORT_U; ++i) {
+            const uint32_t bal = __ballot_sync(0xffffffffu, mine[i]);
+            if (mine[i]) {
+                const int p = p0 + 32 * i + lane, slot = at + __popc(bal & ((1u << lane) - 1));
+                sorted[slot] = p;
+                slot_of[p] = slot;
+            }
+            at += __popc(bal);
+        }
     }
 }
 
@@ -530,10 +538,36 @@ __global__ void __launch_bounds__(256) head_tiled_kernel(const HeadLin a) {
 // grid (T)
 __global__ void moe_combine_kernel(const float* __restrict__ ys, const float* __restrict__ wts, const int32_t* __restrict__ slot_of, int top, int W,
                                    const float* __restrict__ shared, const float* __restrict__ gate_z, int64_t ldg, float* __restrict__ y,
-                                   const int32_t* __restrict__ ids, int E_real, const float* __restrict__ x_id) {
+                                   const int32_t* __restrict__ ids, int E_real, const float* __restrict__ x_id, int vec) {
     const int64_t t = blockIdx.x;
     float gate = 1.f;
     if (shared && gate_z) gate = sigmoidf_acc(gate_z[t * ldg]);
+    if (vec) {   // four columns per thread, four choices' rows requested together (one column and one row at a time: 20 us for 4096 x 4 rows of 1024)
+        for (int c = 4 * threadIdx.x; c < W; c += 4 * blockDim.x) {
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int j0 = 0; j0 < top; j0 += 4) {
+                float4 v[4];
+                float w[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int64_t p = t * top + j0 + u;
+                    if (j0 + u < top) {
+                        w[u] = wts[p];
+                        v[u] = ld4((ids && ids[p] >= E_real) ? x_id + t * W + c : ys + (slot_of ? (int64_t)slot_of[p] : p) * W + c);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (j0 + u < top) acc.x = fmaf(w[u], v[u].x, acc.x), acc.y = fmaf(w[u], v[u].y, acc.y), acc.z = fmaf(w[u], v[u].z, acc.z), acc.w = fmaf(w[u], v[u].w, acc.w);
+            }
+            if (shared) {
+                const float4 s = ld4(shared + t * W + c);
+                acc.x = fmaf(gate, s.x, acc.x), acc.y = fmaf(gate, s.y, acc.y), acc.z = fmaf(gate, s.z, acc.z), acc.w = fmaf(gate, s.w, acc.w);
+            }
+            *reinterpret_cast<float4*>(y + t * W + c) = acc;
+        }
+        return;
+    }
     for (int c = threadIdx.x; c < W; c += blockDim.x) {
         float acc = 0.f;
         for (int j = 0; j < top; ++j) {
@@ -649,7 +683,7 @@ int b200seq_moe_router_rule(const void* x, int x_dtype, int64_t ldx_, const void
 
 int b200seq_moe_sort(const int32_t* ids, int pairs, int E, const int32_t* counts, int32_t* offs, int32_t* sorted, int32_t* slot_of, void* stream) {
     if (!ids || !counts || !offs || !sorted || !slot_of || pairs < 0 || E < 1) return fail(B200SEQ_ERR_INVALID_ARG, "moe_sort: bad arguments");
-    moe_sort_kernel<<<E, 256, 0, (cudaStream_t)stream>>>(ids, pairs, E, counts, offs, sorted, slot_of);
+    moe_sort_kernel<<<E, SORT_NT, 0, (cudaStream_t)stream>>>(ids, pairs, E, counts, offs, sorted, slot_of);
     SEQ_LAUNCH_CHECK("moe_sort");
     return 0;
 }
@@ -766,7 +800,9 @@ int b200seq_moe_combine_ex(const float* ys, const float* wts, const int32_t* slo
                            const float* shared, const float* gate_z, int64_t ldg, float* y, void* stream) {
     if (!ys || !wts || !y || T < 0 || top < 1 || W < 1 || (ids && !x_id)) return fail(B200SEQ_ERR_INVALID_ARG, "moe_combine: bad arguments");
     if (T == 0) return 0;
-    moe_combine_kernel<<<T, W >= 1024 ? 256 : 128, 0, (cudaStream_t)stream>>>(ys, wts, slot_of, top, W, shared, gate_z, ldg, y, ids, E_real, x_id);
+    auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    moe_combine_kernel<<<T, W >= 1024 ? 256 : 128, 0, (cudaStream_t)stream>>>(ys, wts, slot_of, top, W, shared, gate_z, ldg, y, ids, E_real, x_id,
+        W % 4 == 0 && al(ys) && al(shared) && al(y) && al(x_id));
     SEQ_LAUNCH_CHECK("moe_combine");
     return 0;
 }
