@@ -143,8 +143,10 @@ static WidePlan wide_plan(const b200q_weight* w, int64_t M) {
 }
 
 // The fused kernel is the better one for fewer rows: it has no expansion pass, and up to 256 rows it expands a weight once too.  Its time is
-// about (12 + 0.1 rows) us per wave of 128-row weight tiles at K = 4096 plus 4 us of staging and launch (measured from 64 to 4096 rows; it
-// cuts K when there are fewer tiles than SMs, which costs it a pass over the partial sums).
+// about (12 + 0.1 rows) us per wave of 128-row weight tiles at K = 4096 plus 4 us of staging and launch (measured from 136 to 4096 rows over the
+// projections of hidden sizes 2048, 4096 and 8192; it cuts K when there are fewer tiles than SMs, which costs it a pass over the partial
+// sums).  Lines drawn from the same measurements: never below 512 rows; weights of several panels from 768 rows and with 14 % in hand (8192 x 8192,
+// 800 rows: estimated 12 % faster, measured 3 % slower; 10240 x 8192, 300 to 640 rows: 10 to 25 % slower, 800: 8 to 14 % faster).
 static bool wide_wins(const b200q_weight* w, int64_t M, const WidePlan& p) {
     const int64_t mt = (M + 255) / 256, rows = ((M + mt - 1) / mt + 31) / 32 * 32, items = w->T * mt;
     const double wave = (12.0 + 0.1 * (double)rows) * (double)w->K_pad / 4096.0;
@@ -154,7 +156,7 @@ static bool wide_wins(const b200q_weight* w, int64_t M, const WidePlan& p) {
         const int64_t cut = w->num_sms / items < 8 ? w->num_sms / items : 8;
         fused += wave / cut + (cut > 1 ? 4.0 + (double)(cut + 1) * M * w->N * 4.0 / 4.0e6 : 0.0);
     }
-    return p.us < fused;
+    return p.panels == 1 ? p.us < fused : M >= 768 && p.us * 1.14 < fused;
 }
 
 size_t gemm_wide_ws_bytes(const b200q_weight* w, int64_t M) {
