@@ -59,7 +59,9 @@ cudaError_t matvec_plan(const b200q_weight* w, int64_t M, MatvecPlan* plan, int 
     int mb = M == 1 ? 1 : (M == 2 ? 2 : 4);
     const b200q_weight* w2 = dual_partner(w);
     const int cbmax = (w2 && w2->chunk_bytes > w->chunk_bytes) ? w2->chunk_bytes : w->chunk_bytes;
-    int stage = cbmax + (pro ? 0 : (int)M * ACT_REC_BYTES);
+    // room for mb records, not M: three rows run the four-row kernel, whose loads of the (unused) fourth record would otherwise
+    // pass the end of the CTA's shared memory in the ring's last stage.  The copies and the record stride stay those of M rows.
+    int stage = cbmax + (pro ? 0 : mb * ACT_REC_BYTES);
     stage = (stage + 127) & ~127;
     int xhat = pro ? (int)(((size_t)w->KC * M * ACT_REC_BYTES + 127) & ~(size_t)127) : 0;
     // > half an SM on purpose: two CTAs of one launch must never share an SM (measured: after glue kernels perturb

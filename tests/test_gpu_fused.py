@@ -170,3 +170,15 @@ def test_decode_default_fusions_reproduce_the_separate_operators(client, scheme,
     prompt = np.asarray([[3, 1, 4, 1, 5]])
     assert np.array_equal(ref.generate(prompt, 16, use_graph=True), fus.generate(prompt, 16, use_graph=True))
     assert fus.launches_per_step() <= ref.launches_per_step() - 3 * cfg.n_layers
+
+
+@pytest.mark.parametrize("fmt,N,K", [("Q6_K", 28672, 4096), ("Q4_K", 28672, 4096), ("Q8_0", 16384, 4096), ("Q6_K", 4096, 4096)])
+def test_three_rows_run_the_whole_ring(client, fmt, N, K):
+    """Three rows take the four-row kernel with three activation records a stage.  Weights large enough that every CTA reaches the last stage of
+    its ring: the result is that of the first three of four rows, bit for bit (f64 sums of exact products)."""
+    from blazr_b200 import synth
+    t = synth.GGML[fmt]
+    w = client.weight_from_ggml(t, synth.random_ggml(t, N, K, seed=3), N, K)
+    x = torch.randn((4, K), device="cuda:0")
+    for dt in (torch.float32, torch.float16):
+        assert torch.equal(client.quant_matmul(x[:3].contiguous(), w, out_dtype=dt), client.quant_matmul(x, w, out_dtype=dt)[:3])
