@@ -566,11 +566,13 @@ cudaError_t run(const AttnArgs& a, const b200seq_step& st, dim3 grid, cudaStream
 }  // namespace
 
 // Steps of more than 16 tokens with whole 16-byte rows and head sizes up to 128 in steps of 16.  What stays on the f32 tiles of seq_attn.cu:
-// decode steps (too few rows for a 128-row tile), keys that come in two parts or from gathered rows, odd head sizes, unaligned rows.
+// decode steps (too few rows for a 128-row tile), keys that come in two parts or from gathered rows, odd head sizes, unaligned rows -- and up to
+// 64 tokens that see no more than 128 keys, where one or two key tiles do not repay this kernel's set-up (whole call, 32 heads of 128, f32 tiles
+// against this kernel: 48 tokens 41 / 45 us, 64 tokens 39 / 58; beyond the line 100 tokens 50 / 46, and 64 tokens behind 1000 earlier ones 95 / 60).
 bool launch_attn_tc(AttnArgs& a, const b200seq_step& st, int max_keys, size_t part_floats, cudaStream_t cs, int& rc) {
     auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     const int R = a.H / a.G;
-    if (st.T <= 16 || a.D % 16 || a.V % 16 || a.D > 128 || a.V > 128 || a.ctx_rows || a.krot || a.kd != a.D || ((a.ld | a.kld | a.vld | a.q_col) & 3) || !al(a.qkvg) ||
+    if (st.T <= 16 || (st.T <= 64 && max_keys <= 128) || a.D % 16 || a.V % 16 || a.D > 128 || a.V > 128 || a.ctx_rows || a.krot || a.kd != a.D || ((a.ld | a.kld | a.vld | a.q_col) & 3) || !al(a.qkvg) ||
         !al(a.kpool) || !al(a.vpool) || (a.pool > 0 && (!al(a.kpp) || !al(a.vpp))) || !al(a.out))
         return false;
     const int sms = tcpair::pair_sms();

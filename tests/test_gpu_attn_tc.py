@@ -23,7 +23,11 @@ def ops():
 
 CASES = [
     # (tokens, past) per entry, H, G, D, V, options
-    ([(17, 0)], 4, 4, 16, 16, {}),
+    ([(17, 0)], 4, 4, 16, 16, {}),                                  # few tokens with few keys: the f32 tiles
+    ([(64, 64)], 4, 2, 32, 32, {}),                                 # the last such step, and the first ones beside it
+    ([(64, 65)], 4, 2, 32, 32, {}),
+    ([(65, 0)], 4, 4, 16, 16, {}),
+    ([(66, 0)], 300, 2, 32, 32, {}),
     ([(64, 0), (33, 100)], 8, 2, 64, 64, dict(chunk=48)),
     ([(130, 5)], 6, 2, 48, 80, dict(window=37)),
     ([(40, 300), (1, 64), (20, 0)], 8, 1, 128, 128, dict(window=64, keep_first=3)),
