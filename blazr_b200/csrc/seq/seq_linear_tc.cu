@@ -1,6 +1,10 @@
 // seq_linear_tc.cu -- tensor-core path of the dense linear layer: y[M,N] (f32) = x[M,K] (bf16) . w[N,K]^T (bf16), f32 accumulation
 // on the 5th-generation tensor cores (tcgen05.mma, accumulator in tensor memory).
 //
+// Ordinary and grouped products of 32 rows and more run on the paired-SM kernel of tc_pair.cuh (one tile of 256 weight rows per CTA pair,
+// persistent; the epilogue functors and the choice of the token tile are below).  What follows describes the kernel that is kept for products of
+// one weight per head and for banks of more experts than the paired kernel's shared memory lists.
+//
 // One CTA per 128 (n) x 128 (m) output tile.  The weight tile is the MMA's A operand (TMEM lane = n), the activation tile its B
 // operand (TMEM column = m), so that in the epilogue the 32 threads of a warp hold 32 consecutive n of one token: coalesced stores.
 // Both operands are K-major bf16 rows in global memory; TMA (cp.async.bulk.tensor.2d, 128-byte swizzle) brings 64-k slabs of both
