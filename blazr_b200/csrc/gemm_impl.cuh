@@ -163,7 +163,7 @@ __device__ __forceinline__ uint64_t make_b_desc(uint32_t saddr) {
 
 // 32 integer weights of a unit (one byte each) -> 16 packed f16 pairs  w = a*(v-off) - b,  rounded once to f16.
 // Bytes become f16 with the 0x6400 trick (0x6400 | v == 1024 + v exactly), the integer offset is removed with an
-// exact HSUB2 and the scale/min applied with one HFMA2: one PRMT + HSUB2 + HFMA2 per pair of weights, no I2F.
+// exact __hsub2 and the scale/min applied with one __hfma2: a byte permutation, a subtraction and a multiply-add per pair of weights.
 // Pair order: word k yields (e0,e2) then (e1,e3) -- the activation staging kernel applies the same [0,2,1,3]
 // permutation inside every group of 4 k, so the contraction is unchanged.
 template <bool SIGNED>

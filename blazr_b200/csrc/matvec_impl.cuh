@@ -201,16 +201,15 @@ __device__ __forceinline__ void fused_prologue(const MatvecParams& p, uint8_t* x
 }
 
 // int32 -> f64.  -DB200Q_MV_MAGIC_I2D: without the conversion unit -- the double with high word 0x43300000 and low word
-// (s ^ 0x80000000) is 2^52 + 2^31 + s exactly, one DADD (FP64 pipe) removes the bias -- instead of I2F.F64 (XU pipe, 8 issue
-// cycles per warp instruction, 3-4 per chunk).  Measured in round 2: NEUTRAL (Q4_K gate|up 15.69 vs 15.59 us, 70B step 108.7 vs
-// 109.7 tok/s): the XU pipe (24-26 % busy) is not what paces the consumer loop.  Kept as a compile-time experiment.
+// (s ^ 0x80000000) is 2^52 + 2^31 + s exactly, one f64 subtraction removes the bias.  Measured NEUTRAL (Q4_K gate|up 15.69 vs 15.59 us,
+// 70B step 108.7 vs 109.7 tok/s): the conversion unit (24-26 % busy) is not what paces the consumer loop.  Kept as a compile-time experiment.
 #ifdef B200Q_MV_MAGIC_I2D
 __device__ __forceinline__ double i2d(int s) { return __hiloint2double(0x43300000, (int)((unsigned)s ^ 0x80000000u)) - 4503601774854144.0; }
 #else
 __device__ __forceinline__ double i2d(int s) { return (double)s; }
 #endif
 
-// Per-CTA globaltimer trace and the "skip the math" debug flag cost ~6 instructions per chunk in the consumer loop: they are
+// Per-CTA globaltimer trace and the "skip the math" debug flag cost 3-12 % in the consumer loop: they are
 // compiled in only with -DB200Q_MV_TRACE (make TRACE=1; tools/trace_matvec.py, tools/trace_step.py need that build).
 #ifdef B200Q_MV_TRACE
 #define MV_TRACE_ON(p) ((p).trace != nullptr)
@@ -600,7 +599,7 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_kernel(const MatvecParam
     int n_full_done = 0;  // OUT_SWIGLU: full tiles flushed so far (selects the s_y buffer)
     // Everything the hot loop addresses is a 32-bit shared-window address built from values computed ONCE here: the ring /
     // barrier bases and, per lane, the byte offsets of its (row, unit) inside a chunk and of its unit inside an activation
-    // record.  (Left to the compiler, these were re-derived from threadIdx every chunk: ~25 of ~120 instructions per chunk.)
+    // record.  (They would otherwise be derived from threadIdx again for every chunk.)
     constexpr int NOFF = FmtNoff<F>::value;
     const uint32_t stages_sa = smem_u32(stages), full_sa = keep_in_reg(smem_u32(full)), xhat_sa = smem_u32(xhat);
     constexpr uint32_t EMPTY_OFF = MV_MAX_STAGES * 8;                     // empty[] follows full[]

@@ -16,7 +16,7 @@
 // TMEM: two slots of 96 columns (scores f32 [64], then the weights' three planes in the same columns), the value tile of every row tile,
 // and the queries' planes (the A operand of the scores comes from TMEM: from shared memory its reads alone would take longer than the MMA).
 // What bounds it: the tensor pipe, 6 x the products (D = V = 64: 1536 cycles per 128 x 64 scores; a step takes 2 400, the difference being the
-// hand-overs between a value product and the next scores of the same slot), with the soft-max beside it at about 9 instructions per score.
+// hand-overs between a value product and the next scores of the same slot), with the soft-max beside it on the same schedulers.
 //
 // Values that are not finite: an infinite key or value part makes the row NaN (inf - inf in the split), where a plain f32 product could still be inf.
 // Every wait is bounded (tc_pair.cuh): one that runs out sets bit 1 of the library's error flags and the CTA leaves through the common exit.

@@ -43,7 +43,7 @@ __device__ __forceinline__ SkPlan sk_plan(int64_t c0, int64_t c1, int64_t KC) {
     return s;
 }
 
-// 32-bit forms (the host guarantees (C + 1) * G < 2^32): a 64-bit division is a ~150-instruction subroutine on the GPU and
+// 32-bit forms (the host guarantees (C + 1) * G < 2^32): a 64-bit division is a long serial sequence on the GPU and
 // the plan sits on the critical path of every launch's prologue
 __device__ __forceinline__ uint32_t sk_begin32(uint32_t g, uint32_t C, uint32_t G) { return g * C / G; }
 __device__ __forceinline__ SkPlan sk_plan32(uint32_t c0, uint32_t c1, uint32_t KC) {

@@ -33,7 +33,7 @@ def main():
     raw = subprocess.run(["ncu", "-i", rep, "--page", "raw", "--csv"], capture_output=True, text=True, check=True).stdout
     rows = list(csv.reader(io.StringIO(raw)))
     hdr, units = rows[0], rows[1]
-    lines = [f"# {header}", f"# source: {os.path.basename(rep)} -- ncu --set full --clock-control none --import-source on (gpurun, one B200, cold cache, serialised); per launch", ""]
+    lines = [f"# {header}", f"# source: {os.path.basename(rep)} -- ncu --set full --clock-control none (one B200, cold cache, serialised); per launch", ""]
     traffic = None
     for vals in rows[2:]:
         d = {h: (v, u) for h, u, v in zip(hdr, units, vals)}
