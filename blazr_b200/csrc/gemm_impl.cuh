@@ -51,29 +51,22 @@ struct GemmParams {
     // their partial accumulators go to partial_tail [tail_n][tail_splits][128][Mt] f32 and splitk_tail_reduce_kernel sums them
     int tail_first, tail_n, tail_splits;
     float* partial_tail;
-    int xmc;           // 1: launched as clusters of two CTAs that work on ADJACENT weight tiles of the same activation tile; each
-                       // CTA fetches half of every activation stage and TMA-multicasts it to both (halves the L2 -> SM traffic
-                       // that bounds the wide-M kernel: 128 KB of X per 27 KB chunk of W)
 };
 
-// work item -> (weight tile t, activation tile mt, K split sp).  Plain: items = tiles, one CTA each.  xmc: items are tile
-// PAIRS (2 tp, 2 tp + 1) walked by a cluster; the odd CTA of a trailing pair recomputes tile T-1 and stores nothing.
+// work item -> (weight tile t, activation tile mt, K split sp), one CTA each
 struct GemmItem {
     int t, mt, sp, nsp;   // weight tile, activation tile, K split index / count of this item
     int kc0, kc1;         // k-chunk range
     int tail;             // >= 0: index of this tile among the tail tiles (partials go to partial_tail); -1 otherwise
-    bool valid;
 };
-__device__ __forceinline__ int gemm_first(const GemmParams& p) { return p.xmc ? (int)(blockIdx.x >> 1) : (int)blockIdx.x; }
-__device__ __forceinline__ int gemm_stride(const GemmParams& p) { return p.xmc ? (int)(gridDim.x >> 1) : (int)gridDim.x; }
 __device__ __forceinline__ int gemm_total(const GemmParams& p) {
     if (p.tail_splits > 1) return p.tail_first + p.tail_n * p.tail_splits;
-    return (p.xmc ? (p.T + 1) / 2 : p.T) * p.MT * p.splits;
+    return p.T * p.MT * p.splits;
 }
 __device__ __forceinline__ GemmItem gemm_item(const GemmParams& p, int it) {
     GemmItem g;
     int rest;
-    if (p.tail_splits > 1) {   // (splits == 1, no clusters)
+    if (p.tail_splits > 1) {   // (splits == 1)
         if (it >= p.tail_first) {
             const int r = it - p.tail_first;
             g.tail = r / p.tail_splits;
@@ -91,10 +84,7 @@ __device__ __forceinline__ GemmItem gemm_item(const GemmParams& p, int it) {
         rest = it / p.splits;
     }
     g.mt = rest % p.MT;
-    int t = rest / p.MT;
-    if (p.xmc) t = 2 * t + (int)(blockIdx.x & 1);
-    g.valid = t < p.T;
-    g.t = g.valid ? t : p.T - 1;
+    g.t = rest / p.MT;
     g.kc0 = g.sp * p.KC / g.nsp;
     g.kc1 = (g.sp + 1) * p.KC / g.nsp;
     return g;
@@ -110,19 +100,6 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_commit_mc(uint64_t* bar, uint16_t cta_mask) {  // arrive on the same barrier of every CTA in the mask
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"(cta_mask)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_g2s_mc(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar, uint16_t cta_mask) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1], %2, [%3], %4;" ::"r"(smem_u32(smem_dst)),
-                 "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar)), "h"(cta_mask)
-                 : "memory");
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -271,7 +248,7 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         for (int s = 0; s < p.nw; s++) { mbar_init(&full_w[s], 1); mbar_init(&empty_w[s], GT_DQ_WARPS); }
-        for (int s = 0; s < p.nx; s++) { mbar_init(&full_x[s], 1); mbar_init(&empty_x[s], p.xmc ? 2 : 1); }  // xmc: both CTAs' MMAs release a stage
+        for (int s = 0; s < p.nx; s++) { mbar_init(&full_x[s], 1); mbar_init(&empty_x[s], 1); }
         for (int s = 0; s < p.nslots; s++) { mbar_init(&a_full[s], GT_DQ_WARPS); mbar_init(&a_empty[s], 1); }
         for (int s = 0; s < 2; s++) { mbar_init(&d_full[s], 1); mbar_init(&d_empty[s], 4); }
         fence_mbar_init();
@@ -283,7 +260,6 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
     }
     tc_fence_before();
     __syncthreads();
-    if (p.xmc) cluster_sync_all();  // the peer's barriers exist before anything is multicast into this CTA
     tc_fence_after();
     const uint32_t tmem = *tmem_ptr;
     // PDL: the weight stream (static data) starts right away and overlaps the predecessor's tail; only the activation
@@ -291,7 +267,7 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
     pdl_launch_dependents();
 
     const int total_tiles = gemm_total(p);
-    const int it0 = gemm_first(p), its = gemm_stride(p);
+    const int it0 = (int)blockIdx.x, its = (int)gridDim.x;
     const int KS = p.KC * 4;  // 64-k sub-stages along K
 
     if (warp == 0) {
@@ -321,7 +297,6 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
             pdl_wait();
             int s = 0;
             uint32_t ph = 1;
-            const uint32_t half = (uint32_t)p.x_stage_bytes >> 1, hoff = (uint32_t)(blockIdx.x & 1) * half;
             for (int tile = it0; tile < total_tiles; tile += its) {
                 const GemmItem gi = gemm_item(p, tile);
                 const int mt = gi.mt;
@@ -330,10 +305,9 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
                 // 4 (a whole chunk) for skinny ones, where per-stage handshakes would otherwise pace the MMA issuer
                 const uint8_t* src = p.xs + ((size_t)mt * KS + 4 * kc0) * (size_t)(p.Mt * 128);
                 for (int ks = 4 * kc0; ks < 4 * kc1; ks += p.xsub) {
-                    mbar_wait(&empty_x[s], ph);   // xmc: BOTH CTAs have consumed this stage (their commits are multicast)
+                    mbar_wait(&empty_x[s], ph);
                     mbar_arrive_expect_tx(&full_x[s], (uint32_t)p.x_stage_bytes);
-                    if (p.xmc) bulk_g2s_mc(xst + (size_t)s * p.x_stage_bytes + hoff, src + hoff, half, &full_x[s], (uint16_t)3);  // my half -> both CTAs
-                    else bulk_g2s(xst + (size_t)s * p.x_stage_bytes, src, (uint32_t)p.x_stage_bytes, &full_x[s]);
+                    bulk_g2s(xst + (size_t)s * p.x_stage_bytes, src, (uint32_t)p.x_stage_bytes, &full_x[s]);
                     src += p.x_stage_bytes;
                     if (++s == p.nx) { s = 0; ph ^= 1u; }
                 }
@@ -366,7 +340,7 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
 #pragma unroll
                             for (int kk = 0; kk < 4; kk++)
                                 tc_mma_ts(tmem + d_col, a_chunk + j * 32 + kk * 8, bdesc0 + j * sub + (uint64_t)(kk * 2), p.idesc, ((kc - kc0) | j | kk) != 0 ? 1u : 0u);
-                        if (p.xmc) tc_commit_mc(&empty_x[xs], (uint16_t)3); else tc_commit(&empty_x[xs]);
+                        tc_commit(&empty_x[xs]);
                         if (++xs == p.nx) { xs = 0; xph ^= 1u; }
                     } else {
 #pragma unroll 1
@@ -377,7 +351,7 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
 #pragma unroll
                             for (int kk = 0; kk < 4; kk++)
                                 tc_mma_ts(tmem + d_col, a_chunk + j * 32 + kk * 8, bdesc + (uint64_t)(kk * 2), p.idesc, ((kc - kc0) | j | kk) != 0 ? 1u : 0u);
-                            if (p.xmc) tc_commit_mc(&empty_x[xs], (uint16_t)3); else tc_commit(&empty_x[xs]);
+                            tc_commit(&empty_x[xs]);
                             if (++xs == p.nx) { xs = 0; xph ^= 1u; }
                         }
                     }
@@ -413,7 +387,7 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&d_empty[acc]);
                 }
-                if (n < p.N && gi.valid) {
+                if (n < p.N) {
 #pragma unroll
                     for (int c = 0; c < 16; c++) {
                         const int64_t m = (int64_t)mt * p.Mt + cb + c;
@@ -473,7 +447,7 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
                 uint32_t v[16];
                 tc_ld16(lane_base + GT_D_COL + h * half_cols + cb, v);
                 tc_wait_ld();
-                if (n < p.N && gi.valid) {
+                if (n < p.N) {
 #pragma unroll
                     for (int c = 0; c < 16; c++) {
                         const int64_t m = (int64_t)mt * p.Mt + h * half_cols + cb + c;
@@ -490,7 +464,6 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
 
     tc_fence_before();
     __syncthreads();
-    if (p.xmc) cluster_sync_all();  // the peer may still multicast into this CTA's stages / arrive on its barriers until it is done too
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
@@ -512,17 +485,10 @@ static cudaError_t launch_gemm_dq(const GemmParams& p, int grid, int smem, cudaS
     cfg.blockDim = dim3((4 + DQW + (EPI ? 4 : 0)) * 32);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // PDL: see the kernel's griddepcontrol placement
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.numAttrs = 1;
-    if (p.xmc) {  // clusters of two CTAs (adjacent weight tiles, shared activation stages)
-        attr[1].id = cudaLaunchAttributeClusterDimension;
-        attr[1].val.clusterDim.x = 2;
-        attr[1].val.clusterDim.y = 1;
-        attr[1].val.clusterDim.z = 1;
-        cfg.numAttrs = 2;
-    }
     cfg.attrs = attr;
     cudaError_t le = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<F, DQW, EPI>, p);
     count_launch();

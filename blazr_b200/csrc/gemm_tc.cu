@@ -80,7 +80,7 @@ static cudaError_t launch_pdl_g(void (*kern)(KArgs...), dim3 grid, dim3 block, s
 // tail plan of a wide-M launch: (first tail tile, tail tiles, splits); splits == 1 means "no tail split"
 static void tail_plan(const b200q_weight* w, int MT, int64_t M, int grid, int* first, int* n, int* S) {
     *first = 0; *n = 0; *S = 1;
-    // Measured in round 2 (B200Q_GEMM_TAIL=1): correct, and 3-6 % SLOWER (14336x4096xM2048: 814 vs 864 TFLOP/s; 28672: 943 vs 992)
+    // Measured (B200Q_GEMM_TAIL=1): correct, and 3-6 % SLOWER (14336x4096xM2048: 814 vs 864 TFLOP/s; 28672: 943 vs 992)
     // although it removes a 7th wave that is 95 % empty -- the 8 CTAs of that wave run alone at a much higher rate, i.e. the kernel
     // is bounded by a chip-wide resource (power / L2), not per-SM time, and the extra registers + partial traffic cost more than
     // the idle SMs.  Kept as an opt-in experiment.
@@ -218,19 +218,12 @@ cudaError_t launch_gemm_tc(const b200q_weight* w, const void* x, int x_dtype, in
     p.splits = pick_splits(w, MT, M);
     p.dq_warps = Mt <= 128 ? 16 : 8;
     p.partial = reinterpret_cast<float*>(ws + (((size_t)MT * Mt * (size_t)w->K_pad * 2 + 255) & ~(size_t)255));
-    // wide M tiles (prefill): pairs of CTAs on adjacent weight tiles can share every activation stage by TMA multicast
-    // (B200Q_GEMM_XMC=1).  Measured in round 2: correct (all GEMM parity tests, odd tile counts included) and NEUTRAL -- 862 vs 863
-    // TFLOP/s on 14336x4096xM2048, 986 vs 979 on 28672x4096 -- so the activation tile's L2 -> SM traffic is not what bounds the
-    // kernel (round 1's hypothesis); the 14336-row shape loses 14 % to wave quantisation (896 tiles on 148 SMs = 6.05 waves).  Off by default.
-    static const bool xmc_on = [] { const char* e_ = getenv("B200Q_GEMM_XMC"); return e_ && atoi(e_) != 0; }();
-    p.xmc = (xmc_on && Mt > 128 && p.xsub == 1 && w->T >= 2) ? 1 : 0;
-    int64_t tiles = (int64_t)(p.xmc ? (p.T + 1) / 2 * 2 : p.T) * MT * p.splits;
+    int64_t tiles = (int64_t)p.T * MT * p.splits;
     int grid = (int)(tiles < w->num_sms ? tiles : w->num_sms);
-    if (p.xmc) grid &= ~1;
     p.tail_first = p.tail_n = 0;
     p.tail_splits = 1;
     p.partial_tail = nullptr;
-    if (!p.xmc && p.splits == 1 && grid == w->num_sms) {
+    if (p.splits == 1 && grid == w->num_sms) {
         tail_plan(w, MT, M, grid, &p.tail_first, &p.tail_n, &p.tail_splits);
         if (p.tail_splits > 1) p.partial_tail = p.partial;   // (splits == 1: the uniform split-K buffer is empty, the tail buffer starts there)
     }
