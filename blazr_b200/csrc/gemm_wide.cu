@@ -7,7 +7,7 @@
 //     stage x -> f16 rows;   [expand panel p -> buffer p % 2;   GEMM of panel p]  for all p
 // as one chain of programmatic launches.  The GEMM of panel p lets the expansion of panel p + 1 start as soon as its own operands are
 // complete; the expansion waits for that GEMM at its end, so buffer p % 2 is free again when panel p + 2 is expanded.
-// Same operands (f16 roundings of weights and activations) and the same order of k as the fused kernel.
+// Same operands (f16 roundings of weights and activations), the same order of k and the same cuts of it as the fused kernel: the same results, bit for bit.
 #include "gemm_impl.cuh"
 #include "seq/tc_pair.cuh"
 
@@ -109,9 +109,10 @@ struct WidePlan {
     int bt;            // token rows per tile
     int per, panels;   // weight tiles of 256 rows per panel (the last one has the rest)
     size_t x_bytes, buf_bytes;
-    int nbuf;
+    int nbuf, parts;   // parts: runs that K is cut into (one panel), as the fused kernel would
+    size_t part_bytes; // their sums, f32 [parts][M][N]
     double us;         // estimated time
-    size_t bytes() const { return x_bytes + nbuf * buf_bytes; }
+    size_t bytes() const { return x_bytes + nbuf * buf_bytes + part_bytes; }
 };
 
 // Panels of at most 64 MB of f16 weights, which L2 keeps; tile and panel sizes together are those with the least waves of tiles.  Nothing hides
@@ -119,6 +120,7 @@ struct WidePlan {
 // is best up to that size.  A wave of tiles: tcpair::pick_bt.
 static WidePlan wide_plan(const b200q_weight* w, int64_t M) {
     WidePlan p{};
+    p.parts = gemm_k_splits(w, M);
     const int64_t pairs = w->num_sms / 2, NT = (w->T + 1) / 2, row_bytes = w->K_pad * 2;
     int64_t cap = (64ll << 20) / (256 * row_bytes);
     if (cap < 1) cap = 1;
@@ -126,16 +128,17 @@ static WidePlan wide_plan(const b200q_weight* w, int64_t M) {
     const int64_t least = panels > 1 ? (NT - 1) / panels + 1 : NT, most = panels > 1 ? cap : NT;
     for (int bt = tcpair::MAX_BT; bt >= 32; bt -= 32) {
         const int64_t MT = (M + bt - 1) / bt;
-        const double wave = tcpair::wave_us(bt, w->K_pad);
+        const double wave = tcpair::wave_us(bt, w->K_pad / p.parts);
         for (int64_t per = most; per >= least; per--) {
             const int64_t full = NT / per, rest = NT - full * per;
-            const double expand = (double)per * 256.0 * row_bytes * 1.5 / 5.0e6, gemm = (double)((per * MT + pairs - 1) / pairs) * wave;
+            const double expand = (double)per * 256.0 * row_bytes * 1.5 / 5.0e6, gemm = (double)((per * MT * p.parts + pairs - 1) / pairs) * wave;
             const double last = (double)((rest * MT + pairs - 1) / pairs) * wave;
             const double us = expand + (double)(full - 1) * (gemm > expand ? gemm : expand) + gemm + last + 9.0 * (full + (rest > 0));
             if (p.bt == 0 || us < p.us) p.bt = bt, p.per = (int)per, p.panels = (int)(full + (rest > 0)), p.us = us;
         }
     }
-    p.us += (double)M * w->K_pad * 6.0 / 5.0e6;
+    p.us += (double)M * w->K_pad * 6.0 / 5.0e6 + (p.parts > 1 ? 4.0 + (double)(p.parts + 1) * M * w->N * 4.0 / 4.0e6 : 0.0);
+    p.part_bytes = p.parts > 1 ? (size_t)p.parts * M * w->N * sizeof(float) : 0;
     p.x_bytes = ((size_t)M * row_bytes + 1023) & ~(size_t)1023;
     p.buf_bytes = (size_t)p.per * 256 * row_bytes;
     p.nbuf = p.panels > 1 ? 2 : 1;
@@ -144,18 +147,18 @@ static WidePlan wide_plan(const b200q_weight* w, int64_t M) {
 
 // The fused kernel is the better one for fewer rows: it has no expansion pass, and up to 256 rows it expands a weight once too.  Its time is
 // about (12 + 0.1 rows) us per wave of 128-row weight tiles at K = 4096 plus 4 us of staging and launch (measured from 136 to 4096 rows over the
-// projections of hidden sizes 2048, 4096 and 8192; it cuts K when there are fewer tiles than SMs, which costs it a pass over the partial
-// sums).  Lines drawn from the same measurements: never below 512 rows; weights of several panels from 768 rows and with 14 % in hand (8192 x 8192,
-// 800 rows: estimated 12 % faster, measured 3 % slower; 10240 x 8192, 300 to 640 rows: 10 to 25 % slower, 800: 8 to 14 % faster).
+// projections of hidden sizes 2048, 4096 and 8192; it cuts K when there are at most half as many tiles as SMs, which costs a pass over the partial
+// sums, here as there).  Lines drawn from the same measurements: never below 512 rows; weights of several panels from 768 rows, with 14 % in hand
+// (8192 x 8192, 800 rows: estimated 12 % faster, measured 3 % slower; 10240 x 8192, 300 to 640 rows: 10 to 25 % slower, 800: 8 to 14 % faster) and
+// not where K is cut.
 static bool wide_wins(const b200q_weight* w, int64_t M, const WidePlan& p) {
     const int64_t mt = (M + 255) / 256, rows = ((M + mt - 1) / mt + 31) / 32 * 32, items = w->T * mt;
     const double wave = (12.0 + 0.1 * (double)rows) * (double)w->K_pad / 4096.0;
-    double fused = 4.0 + (double)M * w->K_pad * 6.0 / 3.0e6;
-    if (items >= w->num_sms) fused += (double)((items + w->num_sms - 1) / w->num_sms) * wave;
-    else {
-        const int64_t cut = w->num_sms / items < 8 ? w->num_sms / items : 8;
-        fused += wave / cut + (cut > 1 ? 4.0 + (double)(cut + 1) * M * w->N * 4.0 / 4.0e6 : 0.0);
+    if (p.parts > 1) {
+        if (p.panels > 1 || (int64_t)p.parts * M > INT32_MAX / 2) return false;
+        return p.us < 16.0 + (double)M * w->K_pad * 6.0 / 1.36e6 + wave / p.parts + (double)(p.parts + 1) * M * w->N * 4.0 / 4.0e6;
     }
+    const double fused = 4.0 + (double)M * w->K_pad * 6.0 / 3.0e6 + (double)((items + w->num_sms - 1) / w->num_sms) * wave;
     return p.panels == 1 ? p.us < fused : M >= 768 && p.us * 1.14 < fused;
 }
 
@@ -196,8 +199,15 @@ cudaError_t launch_gemm_wide(const b200q_weight* w, const void* x, int x_dtype, 
         if (e != cudaSuccess) break;
         tcpair::Args a{};
         a.M = (int)M, a.N = ntiles * TILE_ROWS, a.K = (int)w->K_pad, a.E = 1, a.bt = p.bt, a.err = decode_error_dev(), a.err_bit = 2;
+        a.parts = p.parts;
         auto run = [&](const auto& epi) { return tcpair::launch(buf, a.N, w->K_pad, xr, w->K_pad, a, epi, st, true); };
         const int n0 = nt0 * 256;
+        if (p.parts > 1) {
+            float* part = reinterpret_cast<float*>(ws + p.x_bytes + p.buf_bytes);
+            e = tcpair::launch<true>(buf, a.N, w->K_pad, xr, w->K_pad, a, EpiOut<float>{part, w->N, nullptr, (int)w->N, 0}, st, true);
+            count_launch();
+            return e != cudaSuccess ? e : launch_splitk_reduce(part, p.parts, M, w, y, y_dtype, ldy, st);
+        }
         if (y_dtype == 0) e = run(EpiOut<float>{(float*)y, ldy, w->bias, (int)w->N, n0});
         else if (y_dtype == 1) e = run(EpiOut<__half>{(__half*)y, ldy, w->bias, (int)w->N, n0});
         else e = run(EpiOut<__nv_bfloat16>{(__nv_bfloat16*)y, ldy, w->bias, (int)w->N, n0});

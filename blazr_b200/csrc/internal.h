@@ -88,6 +88,8 @@ int* decode_error_dev();   // the device error word of b200q_decode_error (decod
 
 // ---- gemm_tc.cu ----
 size_t gemm_ws_bytes(const b200q_weight* w, int64_t M);
+int gemm_k_splits(const b200q_weight* w, int64_t M);   // parts that the fused kernel cuts K into
+cudaError_t launch_splitk_reduce(const float* partial, int splits, int64_t M, const b200q_weight* w, void* y, int y_dtype, int64_t ldy, cudaStream_t st);   // their sums, f32 [splits][M][N]
 cudaError_t launch_gemm_tc(const b200q_weight* w, const void* x, int x_dtype, int64_t M, int64_t ldx, void* y, int y_dtype, int64_t ldy,
                            uint8_t* ws, size_t ws_bytes, cudaStream_t st);
 

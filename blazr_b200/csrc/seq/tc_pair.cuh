@@ -45,6 +45,7 @@ struct Args {
     int M, N, K;             // token rows, weight rows of one group, reduction length
     int bt;                  // token rows per tile: a multiple of 32, at most 256
     int MT, NT;              // token tiles (bound when grouped), weight tiles of 256
+    int parts;               // PARTS (not grouped): K cut into this many runs of whole 256-k chunks, run i to the result rows i * M ..
     const int32_t* offs;     // grouped form: [E + 1] first token row of every group; group e uses the weight rows e * N ..
     int E;
     int bf16;                // operand type: 1 = bf16, 0 = f16
@@ -154,13 +155,32 @@ __device__ __forceinline__ void ld_wait() { asm volatile("tcgen05.wait::ld.sync.
 
 struct Tile {
     int m0, m_end, wrow, n0;   // first token row, end of its group's rows, first weight row in memory, first output column
+    int kb0, kb1, out;         // slabs of k; result row of token row 0
 };
 
+// slabs of k of tile t (PARTS: K is cut)
+template <bool PARTS>
+__device__ __forceinline__ void slabs_of(const Args& p, int MT, int t, int& kb0, int& kb1) {
+    kb0 = 0, kb1 = (p.K + BK - 1) / BK;
+    if (PARTS) {
+        const int part = t / (MT * p.NT), chunks = p.K / (4 * BK);
+        kb0 = 4 * (part * chunks / p.parts), kb1 = 4 * ((part + 1) * chunks / p.parts);
+    }
+}
+
 // tile t of the step (token tiles fastest).  first: grouped form, [E + 1] first token tile of every group
+template <bool PARTS>
 __device__ __forceinline__ Tile tile_of(const Args& p, const int32_t* first, int MT, int t) {
     Tile r;
     const int BT = p.bt;
-    const int mt = t % MT, nt = t / MT;
+    const int mt = t % MT;
+    int nt = t / MT;
+    r.out = 0;
+    if (PARTS) {
+        const int part = nt / p.NT;
+        nt -= part * p.NT, r.out = part * p.M;
+    }
+    slabs_of<PARTS>(p, MT, t, r.kb0, r.kb1);
     r.n0 = nt * 2 * ROWS;
     r.wrow = r.n0;
     if (!p.offs) {
@@ -180,7 +200,7 @@ __device__ __forceinline__ Tile tile_of(const Args& p, const int32_t* first, int
 
 // Epi: struct with   __device__ void store(const float (&v)[32], int n, int m, int m_end, int lane) const
 //   v[j] = acc[n][m + j] of this lane's n (n may be >= N: nothing is stored); all 32 lanes of a warp call it with the same m
-template <class Epi>
+template <class Epi, bool PARTS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     pair_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Args p, const Epi epi) {
     extern __shared__ uint8_t smem_raw[];
@@ -231,8 +251,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     fence_after();
     const uint32_t tmem = *tmem_ptr;
     if (p.offs) MT = first[p.E];
-    const int tiles = MT * p.NT, stride = (int)gridDim.x >> 1;
-    const int nk = (p.K + BK - 1) / BK;
+    const int tiles = MT * p.NT * (PARTS ? p.parts : 1), stride = (int)gridDim.x >> 1;
 
     if (warp == 0) {
         if (elect()) {
@@ -241,9 +260,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             uint32_t ph = 1;
             bool ok = true;
             for (int t = (int)blockIdx.x >> 1; t < tiles && ok; t += stride) {
-                const Tile tl = tile_of(p, first, MT, t);
+                const Tile tl = tile_of<PARTS>(p, first, MT, t);
                 const int wr = tl.wrow + (int)rank * ROWS, xr = tl.m0 + (int)rank * (BT / 2);
-                for (int kb = 0; kb < nk; ++kb) {
+                for (int kb = tl.kb0; kb < tl.kb1; ++kb) {
                     ok = bar_wait(empty + 8 * s, ph, abort_flag);
                     if (!ok) break;
                     if (rank == 0) bar_expect(full + 8 * s, 2 * STAGE);
@@ -272,6 +291,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                 if (!ok) break;
                 fence_after();
                 const uint32_t d = tmem + b * ACC_STRIDE;
+                int kb0, kb1;
+                slabs_of<PARTS>(p, MT, t, kb0, kb1);
+                const int nk = kb1 - kb0;
                 for (int kb = 0; kb < nk; ++kb) {
                     ok = bar_wait(full + 8 * s, ph, abort_flag);
                     if (!ok) break;
@@ -293,7 +315,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         int b = 0;
         uint32_t ph = 0;
         for (int t = (int)blockIdx.x >> 1; t < tiles; t += stride) {
-            const Tile tl = tile_of(p, first, MT, t);
+            const Tile tl = tile_of<PARTS>(p, first, MT, t);
             if (!bar_wait(acc_full + 8 * b, ph, abort_flag)) break;
             fence_after();
             const int n = tl.n0 + (int)rank * ROWS + q * 32 + lane;
@@ -304,7 +326,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                 float v[32];
                 ld32(ta + c, v);
                 ld_wait();
-                epi.store(v, n, tl.m0 + c, tl.m_end, lane);
+                epi.store(v, n, tl.out + tl.m0 + c, tl.out + tl.m_end, lane);
             }
             fence_before();
             __syncwarp();
@@ -378,8 +400,8 @@ inline int pick_bt(int64_t pairs, int64_t K, Tiles tiles) {
     return best;
 }
 
-// w: [w_rows][K] (row stride ldw), x: [p.M][K] (row stride ldx); p.bt is set, p.MT / p.NT are filled in here
-template <class Epi>
+// w: [w_rows][K] (row stride ldw), x: [p.M][K] (row stride ldx); p.bt is set, p.MT / p.NT are filled in here; PARTS: K cut into p.parts runs
+template <bool PARTS = false, class Epi>
 cudaError_t launch(const void* w, int64_t w_rows, int64_t ldw, const void* x, int64_t ldx, Args p, const Epi& epi, cudaStream_t st, bool pdl = false) {
     CUtensorMap mw, mx;
     if (!make_map(&mw, w, w_rows, p.K, ldw, ROWS, p.bf16 != 0) || !make_map(&mx, x, p.M, p.K, ldx, p.bt / 2, p.bf16 != 0)) return cudaErrorInvalidValue;
@@ -388,13 +410,13 @@ cudaError_t launch(const void* w, int64_t w_rows, int64_t ldw, const void* x, in
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev >= 16 || !ready[dev]) {
-        e = cudaFuncSetAttribute(pair_gemm_kernel<Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        e = cudaFuncSetAttribute(pair_gemm_kernel<Epi, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         if (e != cudaSuccess) return e;
         if (dev < 16) ready[dev] = true;
     }
     p.MT = (p.M + p.bt - 1) / p.bt + (p.offs ? p.E : 0);
     p.NT = (p.N + 2 * ROWS - 1) / (2 * ROWS);
-    int64_t ctas = 2 * (int64_t)p.MT * p.NT;
+    int64_t ctas = 2 * (int64_t)p.MT * p.NT * (PARTS ? p.parts : 1);
     const int sms = pair_sms();
     if (ctas > sms) ctas = sms;
     cudaLaunchConfig_t cfg = {};
@@ -402,7 +424,7 @@ cudaError_t launch(const void* w, int64_t w_rows, int64_t ldw, const void* x, in
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization, attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr, cfg.numAttrs = pdl ? 1 : 0;
-    e = cudaLaunchKernelEx(&cfg, pair_gemm_kernel<Epi>, mw, mx, p, epi);
+    e = cudaLaunchKernelEx(&cfg, pair_gemm_kernel<Epi, PARTS>, mw, mx, p, epi);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 

@@ -85,3 +85,57 @@ def test_extreme_activations_are_clamped_as_before(client):
     y = client.quant_matmul(x, w)
     small = client.quant_matmul(x[:16].contiguous(), w)          # the fused kernel's staging
     assert torch.isfinite(y).all() and ((y[:16] - small).abs().max() / small.abs().max()).item() < 1e-5
+
+
+@pytest.mark.parametrize("N,K,M", [(512, 2048, 512), (512, 2048, 2048), (1024, 4096, 2048), (4096, 1024, 512)])
+def test_products_that_are_cut_along_k_stay_cut(client, N, K, M):
+    """Weights of one, 65504 in the first half of K, 1 / 64 in the second.  A single chain of f32 sums loses the small terms (16 of them make 1 / 4, half a
+    unit of the large sum is 4 and more); cut along K, they are summed by themselves first and arrive whole."""
+    blk = np.zeros((N, K // 32, 34), np.uint8)
+    blk[:, :, :2] = np.frombuffer(np.float16(1.0).tobytes(), np.uint8)
+    blk[:, :, 2:] = 1
+    w = client.weight_from_ggml(8, blk.reshape(N, -1), N, K)
+    x = torch.full((M, K), 65504.0, device="cuda:0")
+    x[:, K // 2:] = 2.0 ** -6
+    y = client.quant_matmul(x, w)
+    big, small = K // 2 * 65504.0, K // 2 * 2.0 ** -6
+    want = torch.tensor(big + small, dtype=torch.float64).float().item()
+    assert want > big and (y == want).all()
+
+
+def fused_need(w, N, K, M):
+    """bytes of scratch that the fused kernel asks for: staged rows, and partial sums where it cuts K (csrc/gemm_tc.cu)"""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    mt, tiles = -(-M // 256), -(-N // 128)
+    rows = -(-(-(-M // mt)) // 32) * 32
+    cut = max(1, min(sms // (tiles * mt), 8, max(1, w.K_pad // 256 // 2)))
+    return -(-(mt * rows * w.K_pad * 2) // 256) * 256 + (cut * M * N * 4 if cut > 1 else 0)
+
+
+@pytest.mark.parametrize("fmt,N,K,M,launches", [
+    ("Q4_K", 512, 2048, 520, 4),            # K in four parts: rows staged, weight expanded, one GEMM, sums of the parts
+    ("Q6_K", 1000, 4096, 1500, 4),          # K in three parts that are not equal, rows of a weight that end inside a tile
+    ("AWQ", 6144, 4096, 1531, 3),
+    ("Q6_K", 14400, 4096, 2048, 5),         # two panels
+    ("Q4_K", 24700, 8192, 800, 15),         # seven panels, odd tile counts and a short last one: both buffers are used again
+    ("Q8_0", 12300, 4128, 2000, 5),         # K that ends inside a chunk
+])
+def test_the_expanded_weight_is_used_and_gives_the_fused_kernels_bits(client, fmt, N, K, M, launches):
+    """Same operands, same order of k, same cuts of it: equal bits.  Several calls run back to back over one workspace, each on rows of its own."""
+    from blazr_b200 import ops
+    w = weight(client, fmt, N, K)
+    full, least = w.workspace_bytes(M), -(-fused_need(w, N, K, M) // 256) * 256
+    assert full > least
+    ws = torch.zeros(full, dtype=torch.uint8, device="cuda:0")
+    g = torch.Generator(device="cuda:0")
+    g.manual_seed(2)
+    xs = [torch.randn((M, K), device="cuda:0", generator=g).half() for _ in range(3)]
+    ys = [torch.empty((M, N), device="cuda:0") for _ in xs]
+    n0 = ops.launch_count()
+    for x, y in zip(xs, ys):
+        client.quant_matmul(x, w, out=y, workspace=ws)
+    assert ops.launch_count() - n0 == 3 * launches
+    y2 = torch.empty_like(ys[0])
+    for x, y in zip(xs, ys):
+        client.quant_matmul(x, w, out=y2, workspace=ws[:least])
+        assert torch.equal(y, y2)
