@@ -712,7 +712,8 @@ class Decoder:
     # ---- prefill: one M = S pass over the prompt (reference src/engine/executor_generate.rs:357, batch_engine.rs:172-272) ----
     def prefill(self, prompt, seq: int = 0) -> torch.Tensor:
         """prompt: int64 [S] token ids of sequence `seq`.  Runs every projection ONCE at M = S on the tcgen05 dequant-GEMM
-        (b200q_matmul, f16 activations written by the operators ahead, f32 accumulate), fills the KV cache rows [0, S) of that sequence, leaves
+        (b200q_matmul, f16 activations written by the operators ahead, f32 accumulate; up to four tokens take the integer matvec of a decode
+        step instead, which quantises f32 rows), fills the KV cache rows [0, S) of that sequence, leaves
         pos[seq] = S and ids[seq] = the greedy next token, and returns the f32 logits [vocab] of the last position.  The causal
         attention of the prompt runs in torch (SDPA, f16); norms, RoPE and the cache rows, SwiGLU and all 7L+1 projections are libb200q kernels.  Tolerance contract: 1e-2 relative on the logits against the f32
         CPU path (the GEMM path quantises weights and activations to f16 tiles)."""
@@ -728,12 +729,13 @@ class Decoder:
         st = ops._stream_ptr(dev)
         P = lambda t: C.c_void_p(t.data_ptr())
         f32, f16 = dict(dtype=torch.float32, device=dev), dict(dtype=torch.float16, device=dev)
+        rows = f32 if S <= 4 else f16    # what the products read: the GEMM rounds its activations to f16 anyway, the matvec quantises f32 rows
         b = getattr(self, "_pf", None)
         if b is None or b["S"] != S:
             ws_bytes = max(ln.w.workspace_bytes(S) for lay in self.layers for key in ("qkv", "o", "gu", "down") for ln in lay[key])
-            b = dict(S=S, h=torch.empty((S, H), **f32), h2=torch.empty((S, H), **f32), xn=torch.empty((S, H), **f16),
+            b = dict(S=S, h=torch.empty((S, H), **f32), h2=torch.empty((S, H), **f32), xn=torch.empty((S, H), **rows),
                      qkv=torch.empty((S, self.qd + 2 * self.kvd), **f32), delta=torch.empty((S, H), **f32),
-                     delta2=torch.empty((S, H), **f32), gu=torch.empty((S, 2 * ff), **f32), act=torch.empty((S, ff), **f16),
+                     delta2=torch.empty((S, H), **f32), gu=torch.empty((S, 2 * ff), **f32), act=torch.empty((S, ff), **rows),
                      q16=torch.empty((S, nh, hd), **f16), k16=torch.empty((S, nkv, hd), **f16), v16=torch.empty((S, nkv, hd), **f16),
                      ws=torch.zeros(max(256, ws_bytes), dtype=torch.uint8, device=dev))
             b["xq1"] = torch.zeros(int(L.b200q_act_bytes(C.c_int64(H), C.c_int64(1))), dtype=torch.uint8, device=dev)
@@ -746,19 +748,20 @@ class Decoder:
         delta = None
         def gemm(lins, x, out):
             for ln in lins:
-                ops._check(L.b200q_matmul(ln.w.handle, P(x), C.c_int32(ops.F16), C.c_int64(S), C.c_int64(x.stride(0)),
+                ops._check(L.b200q_matmul(ln.w.handle, P(x), C.c_int32(ops._TORCH2DT[x.dtype]), C.c_int64(S), C.c_int64(x.stride(0)),
                                           C.c_void_p(out.data_ptr() + 4 * ln.col0), C.c_int32(ops.F32), C.c_int64(out.stride(0)), P(b["ws"]),
                                           C.c_size_t(b["ws"].numel()), st))
 
         def norm(w):
             nonlocal hin, hout
-            if H <= 8192:
+            if rows is f16 and H <= 8192:
                 ops._check(L.b200q_add_rmsnorm_f16(P(hin), P(delta) if delta is not None else None, P(hout), P(w), C.c_float(cfg.eps), C.c_int64(H), C.c_int64(S), P(b["xn"]), st))
             else:
-                x32 = torch.empty((S, H), **f32)
+                x32 = b["xn"] if rows is f32 else torch.empty((S, H), **f32)
                 ops._check(L.b200q_add_rmsnorm_quant(P(hin), P(delta) if delta is not None else None, P(hout), P(w), C.c_float(cfg.eps), C.c_int64(H),
                                                      C.c_int64(S), None, P(x32), st))
-                b["xn"].copy_(x32.clamp_(-65504.0, 65504.0))
+                if rows is f16:
+                    b["xn"].copy_(x32.clamp_(-65504.0, 65504.0))
             hin, hout = hout, hin
 
         for lay in self.layers:
@@ -779,7 +782,11 @@ class Decoder:
             delta = b["delta"]
             norm(lay["mlp_norm"])
             gemm(lay["gu"], b["xn"], b["gu"])
-            ops._check(L.b200q_swiglu_f16(P(b["gu"]), C.c_int64(ff), C.c_int64(S), C.c_int32(1 if lay["swiglu_epi"] else 0), P(b["act"]), st))
+            if rows is f16:
+                ops._check(L.b200q_swiglu_f16(P(b["gu"]), C.c_int64(ff), C.c_int64(S), C.c_int32(1 if lay["swiglu_epi"] else 0), P(b["act"]), st))
+            else:
+                sw = L.b200q_swiglu_f32_interleaved if lay["swiglu_epi"] else L.b200q_swiglu_f32
+                ops._check(sw(P(b["gu"]), C.c_int64(ff), C.c_int64(S), P(b["act"]), st))
             gemm(lay["down"], b["act"], b["delta2"])
             if self.world > 1:
                 torch.distributed.all_reduce(b["delta2"], group=self.group)

@@ -77,3 +77,46 @@ def test_rope_and_cache_rows(L, S, nh, nkv, hd, bs):
     rest = torch.ones(64, dtype=torch.bool, device=DEV)
     rest[at] = False
     assert bool((ck[rest] == 9.0).all()) and bool((cv[rest] == 9.0).all())
+
+
+def _decoders(cfg, scheme, change=None):
+    from blazr_b200 import decode, ops
+    hm = decode.build_host_model(cfg, scheme, seed=4)
+    for lay in hm.layers:
+        if change is not None:
+            change(lay)
+    client = ops.B200Client(0)
+    return [decode.Decoder(client, cfg, scheme, batch=1, max_ctx=16, host=hm) for _ in range(2)]
+
+
+def _token_by_token(dec, prompt):
+    dec.reset([int(prompt[0])])
+    for t in prompt:
+        dec.ids.fill_(int(t))
+        dec.step()
+    torch.cuda.synchronize()
+    return dec.full_logits().reshape(-1)
+
+
+@pytest.mark.parametrize("scheme", ["Q4_K_M", "Q6_K", "Q8_0"])
+@pytest.mark.parametrize("S", [1, 2, 3, 4])
+def test_prompts_of_up_to_four_tokens_quantize_their_f32_rows(scheme, S):
+    """Up to four rows take the integer matvec, as a decode step does: the first layer's keys and values are those of token-by-token decoding, bit for
+    bit, and rows beyond the f16 range are not clamped (norm weights of 1e5: the activations reach 1e10, and clamped at 65504 little but their signs
+    would be left).  Bound of that part: the attention of a prompt is rounded to f16, which moves int8 roundings (half a unit of 1 / 127 of a block of 32's
+    largest value, 0.3 % of the block's size each) in four products of each of the two layers and the head: below 3e-2."""
+    from blazr_b200 import decode
+    cfg = decode.PRESETS["tiny"]
+    prompt = torch.arange(7, 7 + S).numpy() * 31
+    a, b = _decoders(cfg, scheme)
+    a.prefill(prompt)
+    _token_by_token(b, prompt)
+    for name in ("ck", "cv"):
+        assert torch.equal(a.layers[0][name][0, :S], b.layers[0][name][0, :S])
+
+    def loud(lay):
+        lay["mlp_norm"] = (lay["mlp_norm"] * 1e5).astype("float32")
+
+    a, b = _decoders(cfg, scheme, loud)
+    got, want = a.prefill(prompt).double(), _token_by_token(b, prompt).double()
+    assert ((got - want).norm() / want.norm()).item() < 3e-2
