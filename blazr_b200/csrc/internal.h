@@ -81,7 +81,7 @@ int comm_device(const b200q_comm* c);
 int32_t set_error(int32_t code, const char* fmt, ...);  // api.cu: thread-local b200q_last_error message
 
 // ---- gemm_wide.cu ----
-constexpr int64_t GEMM_WIDE_MIN_M = 512;
+constexpr int64_t GEMM_WIDE_MIN_M = 512;   // ops.py: LARGE_STEP
 size_t gemm_wide_ws_bytes(const b200q_weight* w, int64_t M);   // 0: this M stays on the fused kernel
 cudaError_t launch_gemm_wide(const b200q_weight* w, const void* x, int x_dtype, int64_t M, int64_t ldx, void* y, int y_dtype, int64_t ldy, uint8_t* ws, cudaStream_t st);
 int* decode_error_dev();   // the device error word of b200q_decode_error (decode_ops.cu)

@@ -137,6 +137,9 @@ class DecomposedQuantTensor:
     zero_plus_one: int = 1
 
 
+LARGE_STEP = 512   # rows from which a weight may be expanded into its scratch (csrc/gemm_wide.cu)
+
+
 class QuantWeight:
     """Owning wrapper of an opaque b200q_weight handle (immutable once built)."""
 
@@ -149,7 +152,7 @@ class QuantWeight:
         self.N, self.K = int(info.N), int(info.K)
         self.K_pad = int(info.K_pad)
         self.canonical_bytes = int(info.canonical_bytes)
-        self._ws = {}
+        self._ws, self._ws_bytes = {}, {}
 
     @property
     def handle(self):
@@ -159,12 +162,22 @@ class QuantWeight:
         return int(lib().b200q_workspace_bytes(self._h, C.c_int64(M)))
 
     def workspace(self, M: int) -> torch.Tensor:
-        """Zero-filled scratch for calls with this M (cached per M; one in-flight call per workspace)."""
+        """Zero-filled scratch for calls with this M (cached per M as long as the weight lives; one in-flight call per workspace)."""
         ws = self._ws.get(M)
         if ws is None:
             ws = torch.zeros(max(256, self.workspace_bytes(M)), dtype=torch.uint8, device=self.device)
             self._ws[M] = ws
         return ws
+
+    def _scratch(self, M: int) -> torch.Tensor:
+        """Scratch of a call that brings none.  That of a large step is tens of megabytes (the expanded weight) and holds nothing from call to call: it
+        comes from the stream-ordered allocator and returns there."""
+        if M < LARGE_STEP:
+            return self.workspace(M)
+        n = self._ws_bytes.get(M)
+        if n is None:
+            n = self._ws_bytes[M] = max(256, self.workspace_bytes(M))
+        return torch.empty(n, dtype=torch.uint8, device=self.device)
 
     def set_next(self, nxt: Optional["QuantWeight"]):
         """streaming-order hint (include/b200q.h b200q_weight_set_next): the decode matvec on this weight prefetches the head
@@ -258,7 +271,7 @@ class B200Client:
         if out is None:
             out = torch.empty((M, w.N), dtype=out_dtype or x.dtype, device=x.device)
         y2 = out if len(out.shape) == 2 and out.shape[0] == M and out.shape[1] == w.N else out.reshape(M, w.N)
-        ws = workspace if workspace is not None else w.workspace(M)
+        ws = workspace if workspace is not None else w._scratch(M)
         rc = lib().b200q_matmul_path(w._h, path, x2.data_ptr(), _TORCH2DT[x2.dtype], M, ldx, y2.data_ptr(), _TORCH2DT[y2.dtype], y2.stride(0), ws.data_ptr(), ws.numel(),
                                      torch._C._cuda_getCurrentRawStream(x.device.index))
         if rc != 0:

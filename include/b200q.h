@@ -144,6 +144,8 @@ int32_t b200q_shard_range(int64_t total, int64_t rank, int64_t world, int64_t* s
 int32_t b200q_shard_range_blocks(int64_t total, int64_t granule, int64_t rank, int64_t world, int64_t* start, int64_t* end);
 
 /* ---- compute ---- */
+/* M >= 512: may include the expanded weight (2 bytes per element, up to 2 x 64 MB); the scratch of such a call holds nothing afterwards and need not be
+ * zero-filled, and b200q_matmul also accepts that of the GEMM that expands its weight tile by tile */
 size_t b200q_workspace_bytes(const b200q_weight* w, int64_t M);
 /* Y[M,N] (ldy elements between rows) = X[M,K] (ldx) . dequant(W)^T (+bias).  x,y,workspace: device memory.
  * M == 1..4 : dp4a stream-K matvec on int8-quantised activations (decode);

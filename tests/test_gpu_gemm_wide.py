@@ -139,3 +139,17 @@ def test_the_expanded_weight_is_used_and_gives_the_fused_kernels_bits(client, fm
     for x, y in zip(xs, ys):
         client.quant_matmul(x, w, out=y2, workspace=ws[:least])
         assert torch.equal(y, y2)
+
+
+def test_large_steps_leave_no_scratch_behind(client):
+    """Scratch of a large step is tens of megabytes (the expanded weight): it goes back to the allocator with the call, whatever lengths a program runs."""
+    w = weight(client, "Q4_K", 4096, 2048)
+    x = torch.randn((1500, 2048), device="cuda:0")
+    y = torch.empty((1500, 4096), device="cuda:0")
+    client.quant_matmul(x[:1024], w, out=y[:1024])
+    torch.cuda.synchronize()
+    held = torch.cuda.memory_allocated()
+    for M in (1500, 1400, 1300, 1200, 1100, 600):
+        client.quant_matmul(x[:M], w, out=y[:M])
+    torch.cuda.synchronize()
+    assert torch.cuda.memory_allocated() == held
