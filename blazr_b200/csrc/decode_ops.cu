@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(256) swiglu_quant_kernel(const float* __restri
 
 // ------------------------------------------------------------------------------------------------
 // The same operators for the rows of a prompt: each is one pass over memory, 16 bytes per access, and may leave its result as the f16 rows
-// (clamped, rounded once) that the dequant-GEMM's staging would round to anyway.  Same arithmetic as above, element by element.
+// (clamped, rounded once) that the dequant-GEMM's staging (five rows and more) would round to anyway.  Same arithmetic as above, element by element.
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 __device__ __forceinline__ void store4(__half* p, float4 v) {
@@ -334,8 +334,9 @@ __global__ void __launch_bounds__(256) swiglu_rows_kernel(const float* __restric
 }
 
 // RoPE of a prompt's q and k rows (positions 0 .. S - 1, products and sums rounded one by one), K / V into the cache (contiguous, or block pools
-// through the sequence's block table) in f32, and q, k, v as f16 rows [S][heads][hd] for the prompt attention.  One block per token, four columns
-// per thread.
+// through the sequence's block table) in f32, and q, k, v as f16 rows [S][heads][hd] for the prompt attention.  One block per token, W columns per
+// thread: two pairs, or one where a head is not a multiple of four.
+template <int W>
 __global__ void __launch_bounds__(256) rope_kv_rows_kernel(const float* __restrict__ qkv, const float* __restrict__ rope, int nh, int nkv, int hd, __half* __restrict__ q16,
                                                            __half* __restrict__ k16, __half* __restrict__ v16, float* __restrict__ ck, float* __restrict__ cv,
                                                            const int* __restrict__ block_table, int block_size) {
@@ -344,23 +345,31 @@ __global__ void __launch_bounds__(256) rope_kv_rows_kernel(const float* __restri
     pdl_wait();
     const float* src = qkv + (size_t)s * (nq + 2 * nk);
     const size_t slot = block_table ? (size_t)block_table[s / block_size] * block_size + s % block_size : (size_t)s;
-    for (int c = 4 * (int)threadIdx.x; c < nq + 2 * nk; c += 4 * (int)blockDim.x) {
-        float4 x = *reinterpret_cast<const float4*>(src + c);
+    struct alignas(4 * W) Cols {
+        float2 p[W / 2];
+    };
+    struct alignas(2 * W) Halves {
+        __half2 p[W / 2];
+    };
+    for (int c = W * (int)threadIdx.x; c < nq + 2 * nk; c += W * (int)blockDim.x) {
+        Cols x = *reinterpret_cast<const Cols*>(src + c);
         const bool is_v = c >= nq + nk;
         if (!is_v) {
             const int e = c < nq ? c % hd : (c - nq) % hd;
-            const float4 r = *reinterpret_cast<const float4*>(rope + (size_t)s * hd + e);   // (cos, sin) of two pairs
-            x = make_float4(__fsub_rn(__fmul_rn(x.x, r.x), __fmul_rn(x.y, r.y)), __fadd_rn(__fmul_rn(x.x, r.y), __fmul_rn(x.y, r.x)),
-                            __fsub_rn(__fmul_rn(x.z, r.z), __fmul_rn(x.w, r.w)), __fadd_rn(__fmul_rn(x.z, r.w), __fmul_rn(x.w, r.z)));
+            const Cols r = *reinterpret_cast<const Cols*>(rope + (size_t)s * hd + e);   // (cos, sin) of the pairs
+#pragma unroll
+            for (int i = 0; i < W / 2; i++)
+                x.p[i] = make_float2(__fsub_rn(__fmul_rn(x.p[i].x, r.p[i].x), __fmul_rn(x.p[i].y, r.p[i].y)), __fadd_rn(__fmul_rn(x.p[i].x, r.p[i].y), __fmul_rn(x.p[i].y, r.p[i].x)));
         }
-        const __half2 a = __floats2half2_rn(x.x, x.y), b = __floats2half2_rn(x.z, x.w);
-        const uint2 h = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        Halves h;
+#pragma unroll
+        for (int i = 0; i < W / 2; i++) h.p[i] = __floats2half2_rn(x.p[i].x, x.p[i].y);
         if (c < nq) {
-            *reinterpret_cast<uint2*>(q16 + (size_t)s * nq + c) = h;
+            *reinterpret_cast<Halves*>(q16 + (size_t)s * nq + c) = h;
         } else {
             const int d = c - nq - (is_v ? nk : 0);
-            *reinterpret_cast<float4*>((is_v ? cv : ck) + slot * nk + d) = x;
-            *reinterpret_cast<uint2*>((is_v ? v16 : k16) + (size_t)s * nk + d) = h;
+            *reinterpret_cast<Cols*>((is_v ? cv : ck) + slot * nk + d) = x;
+            *reinterpret_cast<Halves*>((is_v ? v16 : k16) + (size_t)s * nk + d) = h;
         }
     }
 }
@@ -751,9 +760,11 @@ int32_t b200q_rope_kv_prefill(const float* qkv, const float* rope_table, int32_t
                               float* k_cache, float* v_cache, const int32_t* block_table, int32_t block_size, void* stream) {
     if (!qkv || !rope_table || !q16 || !k16 || !v16 || !k_cache || !v_cache || n_heads <= 0 || n_kv_heads <= 0 || head_dim <= 0 || S <= 0 || (block_table && block_size <= 0))
         return set_error(B200Q_ERR_INVALID_ARG, "rope_kv_prefill: bad arguments");
-    if (head_dim % 4 || S > INT32_MAX || !aligned16(qkv) || !aligned16(rope_table) || !aligned16(q16) || !aligned16(k16) || !aligned16(v16) || !aligned16(k_cache) || !aligned16(v_cache))
-        return set_error(B200Q_ERR_UNSUPPORTED, "rope_kv_prefill: head_dim a multiple of 4 and 16-byte aligned rows");
-    cudaError_t e = launch_pdl(rope_kv_rows_kernel, dim3((unsigned)S), dim3(256), 0, (cudaStream_t)stream, qkv, rope_table, (int)n_heads, (int)n_kv_heads, (int)head_dim,
+    const uintptr_t at = head_dim % 4 ? 7 : 15;   // columns of a thread: 8 or 16 bytes of f32
+    auto aligned = [at](const void* p) { return ((uintptr_t)p & at) == 0; };
+    if (head_dim % 2 || S > INT32_MAX || !aligned(qkv) || !aligned(rope_table) || !aligned(q16) || !aligned(k16) || !aligned(v16) || !aligned(k_cache) || !aligned(v_cache))
+        return set_error(B200Q_ERR_UNSUPPORTED, "rope_kv_prefill: an even head_dim and 16-byte aligned buffers (8-byte where it is not a multiple of 4)");
+    cudaError_t e = launch_pdl(head_dim % 4 ? rope_kv_rows_kernel<2> : rope_kv_rows_kernel<4>, dim3((unsigned)S), dim3(256), 0, (cudaStream_t)stream, qkv, rope_table, (int)n_heads, (int)n_kv_heads, (int)head_dim,
                                (__half*)q16, (__half*)k16, (__half*)v16, k_cache, v_cache, (const int*)block_table, (int)block_size);
     return e == cudaSuccess ? B200Q_OK : B200Q_ERR_CUDA;
 }

@@ -120,3 +120,17 @@ def test_prompts_of_up_to_four_tokens_quantize_their_f32_rows(scheme, S):
     a, b = _decoders(cfg, scheme, loud)
     got, want = a.prefill(prompt).double(), _token_by_token(b, prompt).double()
     assert ((got - want).norm() / want.norm()).item() < 3e-2
+
+
+def test_prompts_of_heads_that_are_not_a_multiple_of_four():
+    from blazr_b200 import decode
+    from oracle.model import OracleModel
+    cfg = decode.ModelConfig("odd", 512, 2, 16, 4, 66, 1024, 512)
+    a, _ = _decoders(cfg, "Q8_0")
+    prompt = torch.arange(3, 12).numpy() * 17
+    got = a.prefill(prompt).double().cpu()
+    oracle = OracleModel(decode.build_host_model(cfg, "Q8_0", seed=4), flavour="A")
+    for t in prompt:
+        want = oracle.step(int(t))
+    want = torch.as_tensor(want).double().reshape(-1)
+    assert ((got - want).norm() / want.norm()).item() < 1e-2
