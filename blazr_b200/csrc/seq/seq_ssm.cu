@@ -245,6 +245,11 @@ struct SegDecay {
     double part[4];
 };
 __device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 256;" ::"r"(1 + group) : "memory"); }   // ST_NT threads each
+__device__ __forceinline__ bool group_any(int group, bool mine) {   // the same barrier; true for all when it is for one
+    uint32_t any;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbar.red.or.pred q, %2, 256, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(any) : "r"((int)mine), "r"(1 + group) : "memory");
+    return any != 0;
+}
 __device__ __forceinline__ void seg_decay(SegDecay& d, const SsmArgs& a, int h, int row0, int len, int t, int group) {
     const int lane = t & 31;
     double L = 0.0;
@@ -488,11 +493,14 @@ __global__ void __launch_bounds__(2 * ST_NT) ssm_tile_out_kernel(const SsmArgs a
             const int s0 = c * ST_K;
             if (c < nblk) {
                 group_sync(gi);
+                bool odd = false;
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     const int idx = tid + u * ST_NT, r = idx >> 4, col = (idx & 15) * 4;
                     const float w = sg.dec.dt[s0 + r], w2 = w * seg_exp(sg.dec, s0 + ST_K - 1, s0 + r);
-                    *reinterpret_cast<float4*>(&sg.K[r][col]) = make_float4(nx[u].x * w, nx[u].y * w, nx[u].z * w, nx[u].w * w);
+                    const float4 k = make_float4(nx[u].x * w, nx[u].y * w, nx[u].z * w, nx[u].w * w);
+                    odd |= !(isfinite(k.x) && isfinite(k.y) && isfinite(k.z) && isfinite(k.w));
+                    *reinterpret_cast<float4*>(&sg.K[r][col]) = k;
                     *reinterpret_cast<float4*>(&sg.K[r][64 + col]) = make_float4(nx[u].x * w2, nx[u].y * w2, nx[u].z * w2, nx[u].w * w2);
                 }
 #pragma unroll
@@ -500,17 +508,30 @@ __global__ void __launch_bounds__(2 * ST_NT) ssm_tile_out_kernel(const SsmArgs a
                     const int idx = tid + u * ST_NT, s_ = idx >> 5, t = idx & 31;
                     sg.M[s_][t] = t >= s_ ? sm.Gt[s0 + s_][tok_place(s0 + t)] * seg_exp(sg.dec, s0 + t, s0 + s_) : 0.f;
                 }
-                group_sync(gi);
+                odd = group_any(gi, odd);
                 if (c + 1 < nblk) fetch(h, nq + c + 1);
                 else fetch(h + 2, 0);
                 {   // the block's own rows (tokens s0 + ty, s0 + 16 + ty) are finished: scale to the token, add the block's own part
                     const uint64_t ff = ss_pk(seg_exp(sg.dec, s0 + ty, s0 - 1), seg_exp(sg.dec, s0 + 16 + ty, s0 - 1));
                     uint64_t own[4] = {0, 0, 0, 0};
+                    if (!odd) {
 #pragma unroll 8
-                    for (int k = 0; k < ST_K; ++k) {
-                        const uint64_t m = ss_pk(sg.M[k][ty], sg.M[k][16 + ty]);
-                        const float4 x = *reinterpret_cast<const float4*>(&sg.K[k][4 * tx]);
-                        ss_fma2(own[0], m, ss_pk(x.x, x.x)), ss_fma2(own[1], m, ss_pk(x.y, x.y)), ss_fma2(own[2], m, ss_pk(x.z, x.z)), ss_fma2(own[3], m, ss_pk(x.w, x.w));
+                        for (int k = 0; k < ST_K; ++k) {
+                            const uint64_t m = ss_pk(sg.M[k][ty], sg.M[k][16 + ty]);
+                            const float4 x = *reinterpret_cast<const float4*>(&sg.K[k][4 * tx]);
+                            ss_fma2(own[0], m, ss_pk(x.x, x.x)), ss_fma2(own[1], m, ss_pk(x.y, x.y)), ss_fma2(own[2], m, ss_pk(x.z, x.z)), ss_fma2(own[3], m, ss_pk(x.w, x.w));
+                        }
+                    } else {   // a value that is not finite: a masked weight of zero does not keep it from earlier tokens, so each token's sum ends at its own
+#pragma unroll 1
+                        for (int k = 0; k <= 16 + ty; ++k) {
+                            const float m0 = sg.M[k][ty], m1 = sg.M[k][16 + ty];
+                            const float x[4] = {sg.K[k][4 * tx], sg.K[k][4 * tx + 1], sg.K[k][4 * tx + 2], sg.K[k][4 * tx + 3]};
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const float2 o = ss_upk(own[j]);
+                                own[j] = ss_pk(k <= ty ? fmaf(m0, x[j], o.x) : o.x, fmaf(m1, x[j], o.y));
+                            }
+                        }
                     }
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {

@@ -18,9 +18,8 @@ def ops():
     return seqops
 
 
-@pytest.mark.parametrize("lens,H,V,N,G", [([129], 2, 64, 128, 1), ([300, 31], 6, 68, 36, 2), ([257, 1, 130], 5, 4, 64, 5), ([700], 9, 64, 100, 1), ([128, 128], 4, 132, 48, 4)])
-@pytest.mark.parametrize("speed", [-8.0, 0.0, 3.0])
-def test_against_the_recurrence(ops, lens, H, V, N, G, speed):
+def scan(ops, lens, H, V, N, G, speed, plant=None):
+    """(outputs, states) of the kernel and of the recurrence in float64; plant(xbc, A_log, Dp) changes the inputs first"""
     from blazr_b200.batch import StepEntry, build_step
     g = torch.Generator(device=DEV)
     g.manual_seed(H * V + N)
@@ -33,6 +32,8 @@ def test_against_the_recurrence(ops, lens, H, V, N, G, speed):
     ld, ldx = -(-(2 * inner + 2 * G * N + H) // 4) * 4, -(-(inner + 2 * G * N) // 4) * 4
     proj, xbc, A_log, Dp, dtb = rnd(T, ld), rnd(T, ldx), 0.7 * rnd(H) + speed, rnd(H), rnd(H) - 1.0
     dt0 = 2 * inner + 2 * G * N
+    if plant is not None:
+        plant(xbc, A_log, Dp)
     state = rnd(B, H, N, V)
     ref_state, ref = state.double().clone(), torch.empty(T, inner, dtype=torch.float64, device=DEV)
     x = xbc[:, :inner].double().reshape(T, H, V)
@@ -53,6 +54,27 @@ def test_against_the_recurrence(ops, lens, H, V, N, G, speed):
     scratch = torch.empty(ops.ssm_scratch_floats(T, B, H, V, N), device=DEV)
     assert scratch.numel() > 0
     ops.ssm_scan(proj, 0, dt0, xbc, A_log, Dp, dtb, state, st, H, V, N, G, out, scratch)
-    for got, want in ((out, ref), (state, ref_state)):
+    return (out, ref), (state, ref_state)
+
+
+@pytest.mark.parametrize("lens,H,V,N,G", [([129], 2, 64, 128, 1), ([300, 31], 6, 68, 36, 2), ([257, 1, 130], 5, 4, 64, 5), ([700], 9, 64, 100, 1), ([128, 128], 4, 132, 48, 4)])
+@pytest.mark.parametrize("speed", [-8.0, 0.0, 3.0])
+def test_against_the_recurrence(ops, lens, H, V, N, G, speed):
+    for got, want in scan(ops, lens, H, V, N, G, speed):
         err = (got.double() - want).abs().max().item() / want.abs().max().item()
         assert err < 3e-6, err
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("token", [0, 17, 31, 32, 200, 255])
+def test_a_value_that_is_not_finite_reaches_no_earlier_token(ops, value, token):
+    """Head 1, column 5 of one token: the outputs of the tokens before it, of the other columns and of the other heads stay what they are."""
+    def plant(xbc, A_log, Dp):
+        xbc[token, 64 + 5] = value
+    (out, ref), (state, ref_state) = scan(ops, [256], 4, 64, 64, 2, 0.0, plant)
+    top = ref[torch.isfinite(ref)].abs().max().item()
+    fine = torch.isfinite(ref)
+    assert bool(fine[:token].all()) and not bool(fine[token, 64 + 5]) and torch.equal(torch.isfinite(out), fine)
+    assert ((out.double() - ref)[fine].abs().max().item()) / top < 3e-6
+    fine = torch.isfinite(ref_state)
+    assert torch.equal(torch.isfinite(state), fine) and ((state.double() - ref_state)[fine].abs().max().item()) / ref_state[fine].abs().max().item() < 3e-6
