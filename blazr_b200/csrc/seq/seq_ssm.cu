@@ -256,7 +256,8 @@ __device__ __forceinline__ void seg_decay(SegDecay& d, const SsmArgs& a, int h, 
     if (t < SSM_SEG) {
         const float dt = t < len ? softplusf_acc(a.proj[(int64_t)(row0 + t) * a.ldp + a.dt0 + h] + a.dt_bias[h]) : 0.f;
         d.dt[t] = dt;
-        L = (double)(-expf(a.A_log[h]) * dt);
+        const float ld = t < len ? -expf(a.A_log[h]) * dt : 0.f;
+        L = ld < -200.f ? -200.0 : (double)ld;   // exp of either is 0 in f32; a sum of infinite terms would have no differences
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const double u = __shfl_up_sync(0xffffffffu, L, o);

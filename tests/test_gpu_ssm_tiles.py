@@ -78,3 +78,12 @@ def test_a_value_that_is_not_finite_reaches_no_earlier_token(ops, value, token):
     assert ((out.double() - ref)[fine].abs().max().item()) / top < 3e-6
     fine = torch.isfinite(ref_state)
     assert torch.equal(torch.isfinite(state), fine) and ((state.double() - ref_state)[fine].abs().max().item()) / ref_state[fine].abs().max().item() < 3e-6
+
+
+def test_decays_that_forget_at_once(ops):
+    """A head whose rate overflows f32 (exp(100)) keeps nothing of the token before, as the recurrence has it; the heads beside it are what they are."""
+    def plant(xbc, A_log, Dp):
+        A_log[1], A_log[2] = 100.0, 12.0
+    for got, want in scan(ops, [300, 40], 4, 64, 64, 2, 0.0, plant):
+        assert bool(torch.isfinite(got).all())
+        assert (got.double() - want).abs().max().item() / want.abs().max().item() < 3e-6
