@@ -283,12 +283,14 @@ struct EpiPlainAct {
 };
 // Activations that leave as bf16 take the division without its branches (reciprocal approximation and one Newton step, 1 ulp of f32): the
 // rounding call behind 1 / d kept the 16 activations of a lane from overlapping and made the epilogue, not the tensor pipe, the bound
-// (4096 x 16384 x 2048: 326 us against 202 us of the plain product).  f32 outputs keep the rounded division.
+// (4096 x 16384 x 2048: 326 us against 202 us of the plain product).  f32 outputs keep the rounded division.  A quarter of 1 + exp(-x) is formed,
+// so that its reciprocal is a normal number as far as the exponential is finite; beyond, the sigmoid is 0.
 __device__ __forceinline__ float sigmoid_nobranch(float x) {
-    const float d = 1.0f + expf(fminf(-x, 85.0f));   // finite, and so is the reciprocal
+    const float d = fmaf(0.25f, expf(fminf(-x, 88.7f)), 0.25f);
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    return fmaf(r, fmaf(-d, r, 1.0f), r);
+    r = 0.25f * fmaf(r, fmaf(-d, r, 1.0f), r);
+    return x < -88.7f ? 0.0f : r;
 }
 template <int KIND>
 __device__ __forceinline__ float act_gated_nobranch(const ActParams& a, float gate, float up) {

@@ -81,3 +81,27 @@ def test_grouped_rows(ops, sizes, act):
     ops.moe_linear(x.to(DEV), 0, w.to(DEV), ids.to(DEV), order, offs.to(DEV), rows, kind, out, 7.0, 1.702, 1.0)
     close(out[:rows].float(), ref, 5e-6 if act == "none" else 2 ** -8)
     assert bool((out[rows] == 3.0).all()) and ops.error_flags() == 0
+
+
+@pytest.mark.parametrize("kind", ["swish_clamp", "gelu_tanh"])
+def test_gates_far_below_zero(ops, kind):
+    """The sigmoid of a gate falls to zero, so that nothing is left of a product whose gate is large: gates of -50 to -1e36 and one that is -inf."""
+    M, F, K = 300, 64, 64
+    x, w = torch.zeros(M, K).bfloat16(), torch.zeros(2 * F, K).bfloat16()
+    gates = [-50.0, -80.0, -86.0, -87.5, -90.0, -1e3, -1e9, -1e18, -1e30, -1e36, float("-inf")]
+    for i, v in enumerate(gates):
+        x[i, 0] = v
+    x[:, 1] = 1.0
+    w[0::2, 0] = 1.0
+    w[1::2, 1] = 2.0
+    g, u = x[:, :1].double(), torch.full((M, F), 2.0, dtype=torch.float64)
+    if kind == "swish_clamp":
+        ref = g * torch.sigmoid(g) * (u + 1.0)
+    else:
+        ref = g * torch.sigmoid(1.5957691216057308 * (g + 0.044715 * g ** 3)) * u
+    out = torch.full((M, F), 3.0, device=DEV, dtype=torch.bfloat16)
+    ops.linear_act(x.to(DEV), w.to(DEV), ops.ACT_KINDS[kind], out, 3e38, 1.0, 1.0)
+    got = out.double().cpu()
+    n = len(gates)
+    assert torch.isnan(got[n - 1]).all() and torch.isnan(ref[n - 1]).all()
+    assert ((got[:n - 1] - ref[:n - 1]).abs() <= ref[:n - 1].abs() * 2 ** -8 + 1e-36).all() and (got[n:] == 0).all()
