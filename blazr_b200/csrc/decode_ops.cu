@@ -44,7 +44,7 @@ struct GlueTrace {
     __device__ __forceinline__ void mark(int) {}
 };
 #endif
-constexpr int B200Q_DECODE_ERR_POSITION = 1;  // attention: pos[m] outside [0, max_ctx)
+constexpr int B200Q_DECODE_ERR_POSITION = 1;  // attention: pos[m] outside [0, max_ctx); 2: B200Q_DECODE_ERR_GEMM_WAIT (internal.h)
 
 // ---- shared: quantise 256 values held one per thread (thread t <-> k = kc*256 + t) into a record ----
 __device__ __forceinline__ void quant_store_record(float v, uint8_t* rec, int t) {

@@ -198,7 +198,7 @@ cudaError_t launch_gemm_wide(const b200q_weight* w, const void* x, int x_dtype, 
         e = dequant_f16_family(w, tile0, ntiles, buf, st);
         if (e != cudaSuccess) break;
         tcpair::Args a{};
-        a.M = (int)M, a.N = ntiles * TILE_ROWS, a.K = (int)w->K_pad, a.E = 1, a.bt = p.bt, a.err = decode_error_dev(), a.err_bit = 2;
+        a.M = (int)M, a.N = ntiles * TILE_ROWS, a.K = (int)w->K_pad, a.E = 1, a.bt = p.bt, a.err = decode_error_dev(), a.err_bit = B200Q_DECODE_ERR_GEMM_WAIT;
         a.parts = p.parts;
         auto run = [&](const auto& epi) { return tcpair::launch(buf, a.N, w->K_pad, xr, w->K_pad, a, epi, st, true); };
         const int n0 = nt0 * 256;

@@ -566,11 +566,8 @@ class Decoder:
         self.graph.replay()
 
     def check_device_errors(self):
-        """raises if a kernel refused an out-of-range position since the last check (synchronises the device)"""
-        flags = C.c_int32(0)
-        ops._check(ops.lib().b200q_decode_error(C.byref(flags)))
-        if flags.value:
-            raise RuntimeError(f"decode kernels reported error flags 0x{flags.value:x} (bit 0: position outside [0, max_ctx))")
+        """raises if a kernel refused an out-of-range position, or a prompt's GEMM gave up waiting, since the last check (synchronises the device)"""
+        ops.check_device_errors()
 
     def step(self):
         """ids (device) -> next ids (device); positions advance on the device: graph-replayable."""
@@ -716,7 +713,8 @@ class Decoder:
         step instead, which quantises f32 rows), fills the KV cache rows [0, S) of that sequence, leaves
         pos[seq] = S and ids[seq] = the greedy next token, and returns the f32 logits [vocab] of the last position.  The causal
         attention of the prompt runs in torch (SDPA, f16); norms, RoPE and the cache rows, SwiGLU and all 7L+1 projections are libb200q kernels.  Tolerance contract: 1e-2 relative on the logits against the f32
-        CPU path (the GEMM path quantises weights and activations to f16 tiles)."""
+        CPU path (the GEMM path quantises weights and activations to f16 tiles).  The call does not wait for the device: check_device_errors() does, and
+        raises what the kernels reported."""
         import torch.nn.functional as Fnn
         cfg, L = self.cfg, ops.lib()
         ids_h = np.asarray(prompt, dtype=np.int64).reshape(-1)

@@ -107,6 +107,18 @@ def _src(a):
     return C.c_void_p(a.ctypes.data), 0, a
 
 
+DEVICE_ERRORS = {1: "bit 0: position outside [0, max_ctx)", 2: "bit 1: a wait of the large-step GEMM ran out, rows of its result are unwritten"}
+
+
+def check_device_errors():
+    """Raises when a kernel of the current device reported an error since the last check (include/b200q.h b200q_decode_error); waits for the device."""
+    flags = C.c_int32(0)
+    _check(lib().b200q_decode_error(C.byref(flags)))
+    if flags.value:
+        what = [text for bit, text in DEVICE_ERRORS.items() if flags.value & bit]
+        raise RuntimeError(f"kernels reported error flags 0x{flags.value:x} ({'; '.join(what) or 'unknown'})")
+
+
 def shard_range(total: int, rank: int, world: int, granule: int = 1):
     """reference src/engine/tensor_parallel.rs:61-67 (at `granule` granularity)"""
     s, e = C.c_int64(), C.c_int64()
@@ -259,7 +271,8 @@ class B200Client:
     # ---- QuantMatmulOps ----------------------------------------------------------------------------
     def quant_matmul(self, x: torch.Tensor, w: QuantWeight, out: Optional[torch.Tensor] = None, out_dtype=None,
                      path: int = PATH_AUTO, workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """Y[..., N] = X[..., K] @ dequant(W)[N, K]^T (+bias).  x: f32 / f16 / bf16 on this device."""
+        """Y[..., N] = X[..., K] @ dequant(W)[N, K]^T (+bias).  x: f32 / f16 / bf16 on this device.  The call does not wait for the device: what its
+        kernels report (a wait that ran out in a step of 512 rows and more) is raised by check_device_errors()."""
         shape = x.shape
         assert x.is_cuda and shape[-1] == w.K, (shape, w.K)
         x2 = x if len(shape) == 2 else x.reshape(-1, w.K)

@@ -162,3 +162,24 @@ def test_stream_k_segment_plan():
             slot_gf = 0 if _sk_begin(gf, C_, G) == t * KC else 1
             assert lst[0][1] == slot_gf and all(sl == 0 for _, sl in lst[1:])
             assert len(lst) >= 2  # a tile with a single contributor is never "partial"
+
+
+@pytest.mark.parametrize("flags,text", [(1, "position outside"), (2, "large-step GEMM"), (3, "position.*GEMM"), (0, None)])
+def test_device_errors_are_named(monkeypatch, flags, text):
+    """b200q_decode_error gives a word of bits; the header says what each means and so does what Decoder.check_device_errors raises."""
+    from blazr_b200 import decode
+
+    class Lib:
+        @staticmethod
+        def b200q_decode_error(p):
+            p._obj.value = flags
+            return 0
+
+    monkeypatch.setattr(ops, "lib", lambda: Lib)
+    if text is None:
+        decode.Decoder.check_device_errors(None)
+    else:
+        with pytest.raises(RuntimeError, match=text):
+            decode.Decoder.check_device_errors(None)
+    doc = open(HEADER).read().split("b200q_decode_error reads and clears")[1].split("*/")[0]
+    assert "bit 0 =" in doc and "bit 1 =" in doc
