@@ -105,3 +105,22 @@ def test_gates_far_below_zero(ops, kind):
     n = len(gates)
     assert torch.isnan(got[n - 1]).all() and torch.isnan(ref[n - 1]).all()
     assert ((got[:n - 1] - ref[:n - 1]).abs() <= ref[:n - 1].abs() * 2 ** -8 + 1e-36).all() and (got[n:] == 0).all()
+
+
+def test_more_experts_than_the_pair_kernel_lists(ops):
+    """A bank of more than 1024 experts keeps the one-SM kernel, with its grouped and gated epilogues."""
+    E, N, K = 1030, 64, 40
+    sizes = [(3 * e) % 5 if e % 7 else 0 for e in range(E)]
+    rows = sum(sizes)
+    x, w = rnd(rows, K, seed=8).bfloat16(), rnd(E, N, K, seed=9, scale=K ** -0.5).bfloat16()
+    offs = torch.zeros(E + 1, dtype=torch.int32)
+    offs[1:] = torch.tensor(sizes).cumsum(0)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(sizes)).to(torch.int32)
+    z = torch.einsum("rk,rnk->rn", x.double(), w.double()[ids.long()])
+    g, u = z[:, 0::2].clamp(max=7.0), z[:, 1::2].clamp(-7.0, 7.0)
+    order = torch.arange(rows, dtype=torch.int32, device=DEV)
+    for kind, ref, dt, tol in ((ops.ACT_NONE, z, torch.float32, 5e-6), (ops.ACT_SWISH_CLAMP, g * torch.sigmoid(1.702 * g) * (u + 1.0), torch.bfloat16, 2 ** -8)):
+        out = torch.full((rows + 1, ref.shape[1]), 3.0, device=DEV, dtype=dt)
+        ops.moe_linear(x.to(DEV), 0, w.to(DEV), ids.to(DEV), order, offs.to(DEV), rows, kind, out, 7.0, 1.702, 1.0)
+        close(out[:rows].float(), ref, tol)
+        assert bool((out[rows] == 3.0).all()) and ops.error_flags() == 0
