@@ -18,7 +18,9 @@
 // What bounds it: the tensor pipe, 6 x the products (D = V = 64: 1536 cycles per 128 x 64 scores; a step takes 2 400, the difference being the
 // hand-overs between a value product and the next scores of the same slot), with the soft-max beside it on the same schedulers.
 //
-// Values that are not finite: an infinite key or value part makes the row NaN (inf - inf in the split), where a plain f32 product could still be inf.
+// Values without such parts (infinities, NaN, beyond the bf16 range): a part that is not finite would reach rows that do not see its key (0 x inf)
+// and make infinities NaN.  Any such part leaves a NaN in every row that meets it -- a key's in its scores, a value's in its column, whatever the weight --
+// so a row that ends with a sum that is not finite is made again, by plain f32 sums over the keys it sees (plain_row).
 // Every wait is bounded (tc_pair.cuh): one that runs out sets bit 1 of the library's error flags and the CTA leaves through the common exit.
 #include "seq_attn.cuh"
 #include "tc_pair.cuh"
@@ -80,7 +82,7 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
-// two values -> three packed bf16 pairs (low half = a)
+// two values -> three packed bf16 pairs (low half = a); a value without finite parts has a NaN among them
 __device__ __forceinline__ void split2(float a, float b, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p1) : "f"(b), "f"(a));
     float ra, rb, sa_, sb_;
@@ -130,11 +132,79 @@ __device__ __forceinline__ int64_t pooled_slot(const int32_t* bt, int bs, int P,
     return (int64_t)bt[pg] * ppp + (b - (pg * bs + P - 1) / P);
 }
 
+// One (token, query head) row by plain f32 sums over the keys it sees in the tiles of a split, maximum first, then weights and sums, as the f32 tiles have
+// it (seq_attn.cu).  Called after the row's results are stored; out of line, so that nothing it needs is kept through the loops.
+__device__ __noinline__ void plain_row(const AttnArgs& a, const b200seq_step& st, int e, int p0, int hi, int t, int h, int split) {
+    const int D = a.D, V = a.V, G = a.G, g = h / (a.H / G), bs = st.block_size, p = st.tok_pos[t];
+    const int32_t* bt = st.block_table + (int64_t)e * st.max_blocks;
+    const KeyTiles kt = key_tiles(a, p0, hi);
+    const int keep = (a.window > 0 && a.keep_first > 0) ? a.keep_first : 0;
+    int lo = a.chunk > 0 ? (p / a.chunk) * a.chunk : 0;
+    if (a.window > 0) lo = max(lo, p - a.window + 1);
+    const int nb = (a.pool > 0 && p - a.window + 1 > 0) ? (p - a.window + 1) / a.pool : 0;
+    const float sc = a.head_scale ? a.scale * a.head_scale[h] : a.scale;
+    const float* q = a.qkvg + (int64_t)t * a.ld + a.q_col + (int64_t)h * D;
+    float mx = -INFINITY, l = 0.f, f = 1.f;
+    float* pp = a.nsplit > 1 ? a.part + (((int64_t)t * a.H + h) * a.nsplit + split) * (V + 2) : nullptr;
+    for (int c = -16; c < V; c += 16) {   // first pass: the maximum; then 16 columns at a time (the first of them with the sum of the weights)
+        float acc[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+        for (int tile = split; tile < kt.total; tile += a.nsplit) {
+            const bool pooled = tile < kt.npt, first = !pooled && tile < kt.npt + kt.nft;
+            const int k0 = pooled ? tile * KT : (first ? (tile - kt.npt) * KT : kt.kbeg + (tile - kt.npt - kt.nft) * KT);
+            for (int kp = k0; kp < k0 + KT; ++kp) {
+                if (!(pooled ? kp < nb : (first ? kp < kt.nfirst : (kp >= lo || kp < keep) && kp <= p))) continue;
+                const int64_t row = pooled ? pooled_slot(bt, bs, a.pool, a.ppp, kp) : (int64_t)bt[kp / bs] * bs + kp % bs;
+                const float* k = pooled ? a.kpp + (row * G + g) * D : a.kpool + row * a.kld + (int64_t)g * D;
+                float s = 0.f;
+#pragma unroll 4
+                for (int d = 0; d < D; d += 4) {
+                    const float4 x = ld4(q + d), y = ld4(k + d);
+                    s = fmaf(x.x, y.x, s), s = fmaf(x.y, y.y, s), s = fmaf(x.z, y.z, s), s = fmaf(x.w, y.w, s);
+                }
+                s *= sc;
+                if (s != s) return;   // the row is NaN, and so is what has been stored
+                if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
+                if (s == -INFINITY) continue;
+                if (c < 0) {
+                    mx = fmaxf(mx, s);
+                    continue;
+                }
+                const float w = expf(s - mx), *v = (pooled ? a.vpp + (row * G + g) * V : a.vpool + row * a.vld + (int64_t)(g / a.vdiv) * V) + c;
+                if (c == 0) l += w;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) acc[i] = fmaf(w, v[i], acc[i]);
+            }
+        }
+        if (c < 0) continue;
+        if (c == 0) {
+            if (pp) {
+                pp[0] = mx, pp[1] = l;
+            } else {
+                float gate = 1.f, den = l, resc = 1.f;
+                if (a.gated && !a.gate_elem) gate = sigmoidf_acc(a.gate[(int64_t)t * a.gld + h]);
+                if (a.sink) {
+                    const float sk = a.sink[h], mn = fmaxf(mx, sk);
+                    resc = expf(mx - mn);
+                    den = fmaf(l, resc, expf(sk - mn));
+                }
+                f = gate * resc / den;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            if (pp) pp[2 + c + i] = acc[i];
+            else store_act(a.out, a.out_dtype, ((int64_t)t * a.H + h) * V + c + i, acc[i] * f * (a.gate_elem ? sigmoidf_acc(a.gate[(int64_t)t * a.gld + (int64_t)h * V + c + i]) : 1.f));
+        }
+    }
+}
+
 // DK: head size / 16, or 0 for a run-time one; CAP: scores are soft-capped.  The loops are kept short: with the soft-max in two unrolled passes,
 // two copies of the loader and the issuer unrolled over four steps the kernel waited for instructions (ncu: no_instruction the largest stall,
 // 0.21 instructions per cycle) and took 860 us where it now takes 206 (4096 tokens, 32 heads of 64, chunks of 2048; the f32 tiles: 1 656).
 template <int MT, int VM, int DK, bool CAP>
-__global__ void __launch_bounds__((4 * MT + 12) * 32, 1) attn_tc_kernel(const AttnArgs a, const b200seq_step st) {
+__global__ void __launch_bounds__((4 * MT + 12) * 32, 1) attn_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ b200seq_step st) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint32_t tmem_base;
     __shared__ int abort_sh;
@@ -344,6 +414,12 @@ __global__ void __launch_bounds__((4 * MT + 12) * 32, 1) attn_tc_kernel(const At
                 pp = a.part + (((int64_t)t * H + h) * a.nsplit + split) * (V + 2);
                 if (live) pp[0] = mx, pp[1] = l;
             }
+            uint64_t odd = pk(l * 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < VM / 2; ++i)
+                if (2 * i < V) odd = fma2(acc[i], 0, odd);
+            float odd0, odd1;
+            upk(odd, odd0, odd1);
 #pragma unroll
             for (int cb = 0; cb < VM; cb += 16) {
                 if (cb >= V) break;
@@ -362,6 +438,7 @@ __global__ void __launch_bounds__((4 * MT + 12) * 32, 1) attn_tc_kernel(const At
                     for (int i = 0; i < 16; i += 4) store_act4(a.out, a.out_dtype, ((int64_t)t * H + h) * V + cb + i, make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]));
                 }
             }
+            if (live && !(odd0 + odd1 == 0.f)) plain_row(a, st, e, p0, hi, t, h, split);   // a sum that is not finite
         }
     } else if (warp < 4 * MT + 8) {
         // ===================== loaders: 256 threads =====================

@@ -39,12 +39,13 @@ CASES = [
     ([(20, 1500)], 2, 1, 64, 64, dict(split=True)),
     ([(18, 2000)], 4, 1, 128, 128, dict(split=True, sink=True, gated=True)),
     ([(50, 0)], 300, 2, 32, 32, {}),                                # more heads of one key head than a tile has rows
+    ([(100, 0)], 300, 2, 32, 32, {}),
 ]
 
 
-@pytest.mark.parametrize("entries,H,G,D,V,o", CASES)
-@pytest.mark.parametrize("odt", [torch.float32, torch.bfloat16])
-def test_against_float64(ops, entries, H, G, D, V, o, odt):
+def attend(ops, entries, H, G, D, V, o, odt, plant=None):
+    """(outputs, float64 reference): a query row meets the keys it sees and no others.  plant(rows, kp, vp, slot) changes the inputs first; slot(entry,
+    position) is a position's row in the pools"""
     from blazr_b200.batch import StepEntry, build_step
     bs, gen = 16, torch.Generator().manual_seed(H * D + V)
     rnd = lambda *s: torch.randn(*s, generator=gen)
@@ -70,6 +71,8 @@ def test_against_float64(ops, entries, H, G, D, V, o, odt):
     rows = rnd(sa.T, width)
     kp, vp = rnd(sum(need) * bs, G, D), rnd(sum(need) * bs, G, V)
     kp[tables[0][-1] * bs + bs - 1] = float("nan") if (entries[0][0] + entries[0][1]) % bs else kp[tables[0][-1] * bs + bs - 1]   # a slot no position uses
+    if plant is not None:
+        plant(rows, kp, vp, lambda e, pos: tables[e][pos // bs] * bs + pos % bs)
     ref = torch.zeros(sa.T, H, V, dtype=torch.float64)
     r0 = 0
     for (n, past), tab in zip(entries, tables):
@@ -89,7 +92,10 @@ def test_against_float64(ops, entries, H, G, D, V, o, odt):
             if sink is not None:
                 s = torch.cat([s, sink[h].double().expand(n, 1)], 1)
             p = torch.softmax(s, 1)[:, :n + past]
-            ref[r0:r0 + n, h] = p @ v[:, h // (H // G)]
+            if plant is None:
+                ref[r0:r0 + n, h] = p @ v[:, h // (H // G)]
+            else:                                                   # (0 x inf: keys that are not seen stay out of the sum)
+                ref[r0:r0 + n, h] = (p[:, :, None] * v[None, :, h // (H // G)]).masked_fill(~see[:, :, None] | (s[:, :n + past, None] == float("-inf")), 0.0).sum(1)
         if gated:
             gl = rows[r0:r0 + n, desc.gate_col:].double()
             ref[r0:r0 + n] *= torch.sigmoid(gl[:, :H * V].reshape(n, H, V) if elem else gl[:, :H, None])
@@ -97,6 +103,43 @@ def test_against_float64(ops, entries, H, G, D, V, o, odt):
     out = torch.full((sa.T + 1, H * V), 3.0, device=DEV, dtype=odt)
     scratch = torch.empty(1 << 22, device=DEV) if o.get("split") else None
     ops.attn_ex(rows.to(DEV), st, desc, kp.to(DEV), vp.to(DEV), out[:sa.T], scratch)
-    err = (out[:sa.T].double().cpu() - ref.reshape(sa.T, -1)).abs().max().item() / ref.abs().max().item()
-    assert err < (4e-6 if odt == torch.float32 else 2 ** -8), err
     assert bool((out[sa.T] == 3.0).all()) and ops.error_flags() == 0 and keep is not None
+    return out[:sa.T].double().cpu(), ref.reshape(sa.T, -1)
+
+
+@pytest.mark.parametrize("entries,H,G,D,V,o", CASES)
+@pytest.mark.parametrize("odt", [torch.float32, torch.bfloat16])
+def test_against_float64(ops, entries, H, G, D, V, o, odt):
+    out, ref = attend(ops, entries, H, G, D, V, o, odt)
+    err = (out - ref).abs().max().item() / ref.abs().max().item()
+    assert err < (4e-6 if odt == torch.float32 else 2 ** -8), err
+
+
+INF, NAN = float("inf"), float("nan")
+PLANTS = {
+    # what is planted at position 70 of the first entry (key head 1, column 3): values, keys, the query of that position
+    "value inf": lambda rows, kp, vp, at, w: vp.__setitem__((at, 1, 3), INF),
+    "value -inf": lambda rows, kp, vp, at, w: vp.__setitem__((at, 1, 3), -INF),
+    "value nan": lambda rows, kp, vp, at, w: vp.__setitem__((at, 1, 3), NAN),
+    "value 3.4e38": lambda rows, kp, vp, at, w: vp.__setitem__((at, 1, 3), 3.4e38),
+    "key -inf": lambda rows, kp, vp, at, w: kp.__setitem__((at, 1, 3), -INF),
+    "key 3.4e38": lambda rows, kp, vp, at, w: (kp.__setitem__((at, 1, 3), 3.4e38), rows[:, 3::16].mul_(1e-37)),
+    "key nan": lambda rows, kp, vp, at, w: kp.__setitem__((at, 1, 3), NAN),
+    "query inf": lambda rows, kp, vp, at, w: rows.__setitem__((70, w), INF),
+}
+
+
+@pytest.mark.parametrize("what", sorted(PLANTS))
+@pytest.mark.parametrize("H,G,D,V,o", [(8, 2, 64, 64, {}), (4, 2, 128, 128, dict(window=100)), (64, 2, 32, 48, dict(softcap=5.0)), (64, 8, 16, 16, dict(tokens=600)), (6, 2, 64, 64, dict(split=True, sink=True, gated=True))])
+def test_values_that_are_not_finite(ops, what, H, G, D, V, o):
+    """They reach the rows that see them, as infinities or NaN where plain f32 sums give those, and no other row."""
+    R = H // G
+    out, ref = attend(ops, [(150, 700)] if o.get("split") else [(o.get("tokens", 150), 0), (90, 20)], H, G, D, V, o, torch.float32,
+                      lambda rows, kp, vp, slot: PLANTS[what](rows, kp, vp, slot(0, 70), R * D + 3))
+    ref32 = ref.float().double()                                    # a sum beyond the f32 range is infinite
+    fine = torch.isfinite(ref32)
+    assert fine.any() and ("key -inf" in what or "3.4e38" in what or (what == "query inf" and o.get("softcap")) or not fine.all())
+    seen_big = (out - ref).abs() > 1e30                             # (near the range's end a sum may overflow on the way)
+    assert bool(((torch.isnan(out) == torch.isnan(ref32)) | seen_big).all()) and bool(((torch.isposinf(out) == torch.isposinf(ref32)) | seen_big).all())
+    ok = fine & (ref32.abs() < 1e30)
+    assert ((out - ref)[ok].abs().max() / ref[ok].abs().max()).item() < 4e-6
