@@ -220,14 +220,15 @@ __global__ void __launch_bounds__((4 * MT + 12) * 32, 1) attn_tc_kernel(const __
     int e, t0, nq;
     // The tiles with the most keys first, for all heads at once, so that the last CTAs to start are short: a causal step's last tiles see the
     // most, in a step of chunks the last ones of every chunk.
-    int tile_no = (int)gridDim.y - 1 - (int)blockIdx.y;
-    if (a.chunk > 0 && a.chunk % a.QT == 0 && a.chunk / a.QT < (int)gridDim.y) {
-        const int per = a.chunk / a.QT, n = gridDim.y, nc = (n + per - 1) / per, rem = n - (nc - 1) * per, r = blockIdx.y, longer = (per - rem) * (nc - 1);
+    const int units = G * a.HB, n = (int)gridDim.x / units, r = (int)blockIdx.x / units, unit = (int)blockIdx.x - r * units;
+    int tile_no = n - 1 - r;
+    if (a.chunk > 0 && a.chunk % a.QT == 0 && a.chunk / a.QT < n) {
+        const int per = a.chunk / a.QT, nc = (n + per - 1) / per, rem = n - (nc - 1) * per, longer = (per - rem) * (nc - 1);
         if (r < longer) tile_no = (r % (nc - 1)) * per + per - 1 - r / (nc - 1);
         else tile_no = ((r - longer) % nc) * per + rem - 1 - (r - longer) / nc;
     }
     if (!attn_find_tile(st, tile_no, a.QT, e, t0, nq)) return;
-    const int g = blockIdx.x / a.HB, hb = blockIdx.x - g * a.HB, R = H / G;
+    const int g = unit / a.HB, hb = unit - g * a.HB, R = H / G;
     const int h0 = g * R + hb * a.Rb, nh = min(a.Rb, R - hb * a.Rb);
     const int split = blockIdx.z;
     const int p0 = st.tok_pos[t0], hi = p0 + nq - 1, bs = st.block_size;
@@ -672,7 +673,7 @@ bool launch_attn_tc(AttnArgs& a, const b200seq_step& st, int max_keys, size_t pa
         ns = ns > 32 ? 32 : (ns < 1 ? 1 : ns);
     }
     a.nsplit = (int)ns;
-    const dim3 grid(a.G * a.HB, tiles, (unsigned)ns);
+    const dim3 grid((unsigned)(a.G * a.HB * tiles), 1, (unsigned)ns);   // (head blocks fastest; the second dimension would end at 65 535 tiles)
     cudaError_t e;
     if (mt == 2) e = a.D == 64 ? run<2, 64, 4>(a, st, grid, cs) : run<2, 64, 0>(a, st, grid, cs);
     else if (a.V <= 64) e = a.D == 64 ? run<1, 64, 4>(a, st, grid, cs) : run<1, 64, 0>(a, st, grid, cs);

@@ -143,3 +143,24 @@ def test_values_that_are_not_finite(ops, what, H, G, D, V, o):
     assert bool(((torch.isnan(out) == torch.isnan(ref32)) | seen_big).all()) and bool(((torch.isposinf(out) == torch.isposinf(ref32)) | seen_big).all())
     ok = fine & (ref32.abs() < 1e30)
     assert ((out - ref)[ok].abs().max() / ref[ok].abs().max()).item() < 4e-6
+
+
+def test_more_tokens_than_a_grid_has_rows(ops):
+    """128 query heads of one key head: a tile holds one token, and a step has more tiles than the second dimension of a grid."""
+    T, H, D, bs = 65600, 128, 16, 16
+    g = torch.Generator(device=DEV)
+    g.manual_seed(5)
+    rows = torch.randn(T, H * D + 2 * D, device=DEV, generator=g)
+    kp, vp = (torch.randn(T, 1, D, device=DEV, generator=g) for _ in range(2))
+    i32 = dict(dtype=torch.int32, device=DEV)
+    t = [torch.zeros(T, **i32), torch.arange(T, **i32), torch.tensor([0, T], **i32), torch.zeros(1, **i32), torch.zeros(1, **i32), torch.arange(T // bs, **i32)[None].contiguous()]
+    st = ops.StepDesc(*(x.data_ptr() for x in t), T, 1, T // bs, bs)
+    desc = ops.attn_desc(H, 1, D, D, D ** -0.5, gated=False, window=8)
+    out = torch.empty(T, H * D, device=DEV)
+    ops.attn_ex(rows, st, desc, kp, vp, out, None)
+    for p in (0, 7, 40000, 65535, 65599):
+        lo = max(0, p - 7)
+        s = rows[p, :H * D].double().reshape(H, D) @ kp[lo:p + 1, 0].double().T * D ** -0.5
+        want = torch.softmax(s, 1) @ vp[lo:p + 1, 0].double()
+        assert ((out[p].double() - want.reshape(-1)).abs().max() / want.abs().max()).item() < 4e-6
+    assert ops.error_flags() == 0
