@@ -5,9 +5,9 @@
 //           completes (from the pool's rows, in position order: the result does not depend on how the prompt was cut).
 //   attend: tiles of (token, query head) rows against tiles of the keys they can see (the token's own chunk and / or window, read
 //           through the entry's block table, and with pooling the pooled entries of the blocks that lie wholly before the window,
-//           in the same soft-max); scores, soft-max and the weighted sum in f32; optional per-head sigmoid gate.  Prompt steps whose head
-//           sizes allow it go to the tensor-core kernel of seq_attn_tc.cu (rule at launch_attn_tc): the tiles here keep decode steps, short
-//           prompts and every other form.
+//           in the same soft-max); scores, soft-max and the weighted sum in f32; optional per-head sigmoid gate.  Steps of many tokens whose head
+//           sizes allow it go to the tensor-core kernel of seq_attn_tc.cu (rule at launch_attn_tc): the tiles here keep steps of up to 16 tokens,
+//           steps of few keys and every other form.
 // A row's result depends on the token's position and on its sequence's pages only; the rest of the batch changes at most how the
 // keys are split among blocks (rounding).
 #include "seq_attn.cuh"

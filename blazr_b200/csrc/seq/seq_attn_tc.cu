@@ -643,14 +643,29 @@ cudaError_t run(const AttnArgs& a, const b200seq_step& st, dim3 grid, cudaStream
 
 }  // namespace
 
+// Which of the two kernels is the faster one for a step, from its row tiles and the keys a token may see.  Here a CTA has an SM to itself: about 15 us
+// (33 with heads above 64) of set-up, load and store, whatever the rows it has, and 2.2 (3.3) us a key tile.  The f32 tiles (seq_attn.cu) are half or a
+// quarter of the rows, two or three to an SM: a wave of them takes about 33 (37) us, 22 (29) where each has an SM, and 18 (21) us more for every
+// further key tile of its share.  Merging key splits: 6 and 10 us.  Measured, us, f32 tiles / this kernel, 32 query heads of 8 key heads of 64 (of 128):
+//   65 sequences of one token, 10 earlier ones   57 /  66 ( 73 / 130)      128 of them    110 / 164 (153 / 282)      40 of two tokens  34 /  42 ( 56 /  89)
+//   65 of one token, 200 earlier ones           162 /  90 (263 / 177)      17, 1000       151 /  42 (256 /  97)      64, 2000         902 / 287 (1526 / 648)
+//   one sequence, 100 tokens                     21 /  16 ( 29 /  29)      600 tokens     168 /  29 (227 /  62)      4 of 300, 100    182 /  44 (281 / 109)
+bool tc_is_faster(const AttnArgs& f32, int64_t units, int64_t splits, int64_t f32_units, int key_tiles, int sms) {
+    const bool big = f32.D > 64 || f32.V > 64;
+    const auto up = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
+    const double tc = (double)up(units * splits, sms) * ((big ? 33.0 : 15.0) + (big ? 3.3 : 2.2) * (double)up(key_tiles, splits)) + (splits > 1 ? 6.0 : 0.0);
+    const int64_t blocks = f32_units * f32.nsplit, share = up(key_tiles, f32.nsplit), fit = (big ? 2 : 3) * (int64_t)sms;
+    const double wave = (blocks <= sms ? (big ? 29.0 : 22.0) : (big ? 37.0 : 33.0)) + (big ? 21.0 : 18.0) * (double)(share - 1);
+    return tc < (double)up(blocks, fit) * wave + (f32.nsplit > 1 ? 10.0 : 0.0);
+}
+
 // Steps of more than 16 tokens with whole 16-byte rows and head sizes up to 128 in steps of 16.  What stays on the f32 tiles of seq_attn.cu:
-// decode steps (too few rows for a 128-row tile), keys that come in two parts or from gathered rows, odd head sizes, unaligned rows -- and up to
-// 64 tokens that see no more than 128 keys, where one or two key tiles do not repay this kernel's set-up (whole call, 32 heads of 128, f32 tiles
-// against this kernel: 48 tokens 41 / 45 us, 64 tokens 39 / 58; beyond the line 100 tokens 50 / 46, and 64 tokens behind 1000 earlier ones 95 / 60).
+// steps of fewer tokens, keys that come in two parts or from gathered rows, odd head sizes, unaligned rows, up to 64 tokens that see no more than 128
+// keys (whole call, 32 heads of 128, f32 tiles against this kernel: 48 tokens 41 / 45 us, 64 tokens 39 / 58) -- and what tc_is_faster leaves there.
 bool launch_attn_tc(AttnArgs& a, const b200seq_step& st, int max_keys, size_t part_floats, cudaStream_t cs, int& rc) {
     auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     const int R = a.H / a.G;
-    if (st.T <= 16 || (st.T <= 64 && max_keys <= 128) || a.D % 16 || a.V % 16 || a.D > 128 || a.V > 128 || a.ctx_rows || a.krot || a.kd != a.D || ((a.ld | a.kld | a.vld | a.q_col) & 3) || !al(a.qkvg) ||
+    if (st.T <= 16 || st.B < 1 || (st.T <= 64 && max_keys <= 128) || a.D % 16 || a.V % 16 || a.D > 128 || a.V > 128 || a.ctx_rows || a.krot || a.kd != a.D || ((a.ld | a.kld | a.vld | a.q_col) & 3) || !al(a.qkvg) ||
         !al(a.kpool) || !al(a.vpool) || (a.pool > 0 && (!al(a.kpp) || !al(a.vpp))) || !al(a.out))
         return false;
     const int sms = tcpair::pair_sms();
@@ -659,11 +674,13 @@ bool launch_attn_tc(AttnArgs& a, const b200seq_step& st, int max_keys, size_t pa
     // two row tiles per CTA where the heads are small enough and there are rows for it
     const int mt = a.D <= 64 && a.V <= 64 && rows >= 256ll * sms ? 2 : 1;
     const int RQ = 128 * mt;
-    a.Rb = R < RQ ? R : RQ;
-    a.HB = (R + a.Rb - 1) / a.Rb;
-    a.QT = RQ / a.Rb;
-    const int tiles = (st.T + a.QT - 1) / a.QT + st.B - (st.B == 1);   // upper bound of the step's query tiles (exact for one entry)
-    const int64_t real = (int64_t)((st.T + a.QT - 1) / a.QT) * a.G * a.HB;
+    const int Rb = R < RQ ? R : RQ, HB = (R + Rb - 1) / Rb, QT = RQ / Rb;
+    const int tiles = (st.T + QT - 1) / QT + st.B - (st.B == 1);   // upper bound of the step's query tiles (exact for one entry)
+    // (Counted over full tiles, 32 sequences of one token were one tile a key head instead of 32, and their keys were dealt to 16 CTAs each: 17 sequences
+    // behind 1000 tokens 66 us, now 42; 64 behind 2000 579, now 287.)
+    const int each = (st.T + st.B - 1) / st.B;
+    auto units = [&](int qt, int hb) { return (int64_t)st.B * ((each + qt - 1) / qt) * a.G * hb; };   // row tiles, were all entries equally long: each has its own
+    const int64_t real = units(QT, HB);
     int64_t ns = 1;
     if (2 * real <= sms) {   // too few tiles: deal the key tiles to several CTAs, at least four each
         ns = sms / real;
@@ -672,7 +689,8 @@ bool launch_attn_tc(AttnArgs& a, const b200seq_step& st, int max_keys, size_t pa
         ns = ns < fits ? ns : fits;
         ns = ns > 32 ? 32 : (ns < 1 ? 1 : ns);
     }
-    a.nsplit = (int)ns;
+    if (!tc_is_faster(a, real, ns, units(a.QT, a.HB), (max_keys + KT - 1) / KT, sms)) return false;
+    a.Rb = Rb, a.HB = HB, a.QT = QT, a.nsplit = (int)ns;
     const dim3 grid((unsigned)(a.G * a.HB * tiles), 1, (unsigned)ns);   // (head blocks fastest; the second dimension would end at 65 535 tiles)
     cudaError_t e;
     if (mt == 2) e = a.D == 64 ? run<2, 64, 4>(a, st, grid, cs) : run<2, 64, 0>(a, st, grid, cs);

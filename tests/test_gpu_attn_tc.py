@@ -40,6 +40,11 @@ CASES = [
     ([(18, 2000)], 4, 1, 128, 128, dict(split=True, sink=True, gated=True)),
     ([(50, 0)], 300, 2, 32, 32, {}),                                # more heads of one key head than a tile has rows
     ([(100, 0)], 300, 2, 32, 32, {}),
+    # the same forms with enough keys for this kernel to be the one chosen (tc_is_faster)
+    ([(130, 5)], 6, 2, 48, 80, dict(window=100)),
+    ([(40, 300), (1, 64), (20, 0), (50, 7)], 8, 1, 128, 128, dict(window=128, keep_first=3)),
+    ([(20, 1500)], 16, 4, 64, 64, dict(split=True)),
+    ([(18, 2000)], 32, 4, 128, 128, dict(split=True, sink=True, gated=True)),
 ]
 
 
@@ -113,6 +118,16 @@ def test_against_float64(ops, entries, H, G, D, V, o, odt):
     out, ref = attend(ops, entries, H, G, D, V, o, odt)
     err = (out - ref).abs().max().item() / ref.abs().max().item()
     assert err < (4e-6 if odt == torch.float32 else 2 ** -8), err
+
+
+@pytest.mark.parametrize("H,G,D", [(16, 4, 64), (8, 1, 128)])
+@pytest.mark.parametrize("B,extra", [(17, 0), (40, 0), (65, 0), (24, 70)])
+@pytest.mark.parametrize("split", [False, True])
+def test_many_entries_of_one_token(ops, H, G, D, B, extra, split):
+    """Batched decoding: every entry has a tile of its own, some beside a longer portion of another sequence."""
+    entries = [(1, (37 * i) % 300) for i in range(B)] + ([(extra, 11)] if extra else [])
+    out, ref = attend(ops, entries, H, G, D, D, dict(split=split), torch.float32)
+    assert (out - ref).abs().max().item() / ref.abs().max().item() < 4e-6
 
 
 INF, NAN = float("inf"), float("nan")
