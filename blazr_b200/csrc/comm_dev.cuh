@@ -11,8 +11,8 @@
 //               in its own memory until all are non-zero, writes +0.0 back (slot free for the exchange after next), sums
 //               them in RANK ORDER in f64 from +0.0 and rounds once: identical bits on every rank and identical to the
 //               1-GPU sum (the partials are exact products accumulated in f64).  An exchange is consumed exactly once.
-//   Round 2 measured the flag form (per-CTA fence.acq_rel.sys + arrival atomic, last CTA raises `world` flags, consumer
-//   acquires them, then loads) at ~13 us per exchange at TP8 -- a system-scope fence waits for every outstanding NVLink store
+//   The flag form (per-CTA fence.acq_rel.sys + arrival atomic, last CTA raises `world` flags, consumer
+//   acquires them, then loads) measured ~13 us per exchange at TP8 -- a system-scope fence waits for every outstanding NVLink store
 //   of the CTA; with self-validating data the exchange costs one NVLink store latency.
 //
 // The same mechanism carries the lm_head all-gather (column-parallel over the vocabulary): f32 logits are stored into

@@ -18,7 +18,7 @@ namespace b200q {
 // memory (they write nothing and return); read and cleared by b200q_decode_error()
 __device__ int g_decode_error = 0;
 
-// TRACE builds only (make TRACE=1; tools/trace_step.py): globaltimer stamps of the glue kernels in launch order --
+// TRACE builds only (make TRACE=1): globaltimer stamps of the glue kernels in launch order --
 // record = {kind, entry, after griddepcontrol.wait, exit, 4 phase marks} written by thread 0 of block (0, 0)
 #ifdef B200Q_MV_TRACE
 __device__ long long* g_glue_trace = nullptr;
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(NORMC_NT) add_rmsnorm_quant_cluster_kernel(con
     gt.mark(2);
     if (warp == 0) {
         // lane r fetches CTA r's share (ONE distributed-shared-memory latency instead of ncta dependent ones: measured 1.4 us
-        // between the cluster barrier and the stores in round 2), then the shares are summed in CTA order: identical on every CTA
+        // between the cluster barrier and the stores), then the shares are summed in CTA order: identical on every CTA
         double mine_part = 0.0;
         if (lane < ncta) mine_part = *cluster.map_shared_rank(&cta_part, lane);
         double tot = 0.0;
@@ -773,7 +773,7 @@ int32_t b200q_add_rmsnorm_quant(const float* h_in, const float* delta, float* h_
                                 float* xnorm, void* stream) {
     if (!h_in || !h_out || !w || (!xq && !xnorm) || H <= 0 || H % CHUNK_K || M <= 0) return B200Q_ERR_INVALID_ARG;
     if (delta && h_in == h_out) return B200Q_ERR_INVALID_ARG;  // CTAs re-read the whole input row: no in-place update
-    // measured (round 2, Mistral-7B / Llama-3.2-1B steps): without an exchange to consume, the H/256-CTA kernel (every CTA
+    // measured (Mistral-7B / Llama-3.2-1B steps): without an exchange to consume, the H/256-CTA kernel (every CTA
     // re-reads the L2-resident row) beats the cluster form by ~1.3 us per call -- two cluster barriers cost more than the
     // redundant reads.  The cluster kernel is the tensor-parallel consumer (reading `world` slots per CTA would not scale);
     // B200Q_NORM_CLUSTER=1 forces it here for A/B runs.

@@ -24,7 +24,7 @@ namespace b200q {
 
 // dequant warps (template parameter DQW): DQW/4 per TMEM lane quarter, each 4/DQW of the chunk's k.  8 for wide M tiles
 // (the MMA is the bottleneck; 16 measured slower there), 16 for skinny M (<= 64), where every weight is expanded for a
-// handful of MMAs and the expansion's latency chains are what bounds the kernel (ncu r1: 2 warps/scheduler, IPC 0.4).
+// handful of MMAs and the expansion's latency chains are what bounds the kernel (ncu: 2 warps per scheduler, 0.4 instructions per cycle).
 constexpr int GT_NX = 16;      // max activation sub-stage ring depth (64 k each); runtime depth p.nx
 constexpr int GT_ASLOTS = 3;   // max TMEM A slots; one slot = one whole 256-k chunk of f16 (128 columns)
 constexpr int GT_MAX_NW = 4;   // weight chunk ring

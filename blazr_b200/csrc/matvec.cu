@@ -174,7 +174,7 @@ cudaError_t launch_matvec(const b200q_weight* w, const uint8_t* xq, int64_t M, v
     {
         // L2 prefetch budget: at most ~64 MB per launch so a huge weight (lm_head) cannot thrash the 126 MB L2
         int64_t per_cta = (64ll << 20) / ((int64_t)plan.grid * p.chunk_bytes);
-        p.l2_prefetch_chunks = 0;  // measured: prefetching into L2 from here delays the x copy and slows the predecessor (r1 notes)
+        p.l2_prefetch_chunks = 0;  // measured: prefetching into L2 from here delays the x copy and slows the predecessor
         (void)per_cta;
         if (const char* e = getenv("B200Q_MV_L2PF")) p.l2_prefetch_chunks = atoi(e);
     }

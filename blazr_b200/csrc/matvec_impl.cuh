@@ -210,7 +210,7 @@ __device__ __forceinline__ double i2d(int s) { return (double)s; }
 #endif
 
 // Per-CTA globaltimer trace and the "skip the math" debug flag cost 3-12 % in the consumer loop: they are
-// compiled in only with -DB200Q_MV_TRACE (make TRACE=1; tools/trace_matvec.py, tools/trace_step.py need that build).
+// compiled in only with -DB200Q_MV_TRACE (make TRACE=1).
 #ifdef B200Q_MV_TRACE
 #define MV_TRACE_ON(p) ((p).trace != nullptr)
 #define MV_DEBUG_SKIP(p) (((p).debug_flags & 1) != 0)
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_kernel(const MatvecParam
         // value has landed, sums them in CTA order (deterministic) and writes y.  The slots double as their own ready flags:
         // the workspace is zero-filled, contributors store -0.0 for an exact zero, so +0.0 bits mean "not written yet", and
         // the reducer restores +0.0 after reading.  One L2 visibility latency after the last partial store, instead of a
-        // release fence + atomic round trip + load round trip behind it (measured 2-3.8 us of tail per launch in round 2).
+        // release fence + atomic round trip + load round trip behind it (measured 2-3.8 us of tail per launch).
         int64_t tqs[2] = {sp.tH, sp.tT};
 #pragma unroll
         for (int seg = 0; seg < 2; seg++) {

@@ -299,7 +299,7 @@ class Decoder:
             self.xq_h, self.xq_attn, self.xq_ff = act(H), act(self.qd), act(self.ff)
         # streaming-order hints: every decode matvec prefetches the head of the next projection's weights into L2 while its own
         # tail drains (qkv -> o -> gate|up -> down -> next layer ... -> lm_head -> layer 0 of the next token)
-        if not self.wide and _os.environ.get("B200Q_CHAIN", "0") != "0":  # measured neutral on whole steps (round 2): opt-in
+        if not self.wide and _os.environ.get("B200Q_CHAIN", "0") != "0":  # measured neutral on whole steps: opt-in
             order = [ln.w for lay in self.layers for key in ("qkv", "o", "gu", "down") for ln in lay[key]] + [ln.w for ln in self.head]
             for a, b in zip(order, order[1:] + order[:1]):
                 if a is not b:
@@ -309,7 +309,7 @@ class Decoder:
         ept = H // 512
         # Tensor parallel: the exchange's consumer is the cluster add+norm+quant kernel and plain matvecs follow.  B200Q_TP_FINISH=1
         # (opt-in) makes the element-wise b200q_allreduce_finish the consumer (delta = f32(sum over ranks)) followed by the same fused
-        # norm-prologue / SwiGLU-epilogue matvecs as on one GPU.  Measured (round 2, 70B Q4_K_M): equal at TP2 (6.21 vs 6.17 ms/step),
+        # norm-prologue / SwiGLU-epilogue matvecs as on one GPU.  Measured (70B Q4_K_M): equal at TP2 (6.21 vs 6.17 ms/step),
         # SLOWER on the TP8 shard (3.81 vs 3.50 ms): the per-CTA norm prologue (3.6 us) costs more than the cluster kernel saves.
         self.tp_finish = tp_world > 1 and _os.environ.get("B200Q_TP_FINISH", "0") != "0" and _os.environ.get("B200Q_TP_NCCL", "0") == "0"
         self.fused = (_os.environ.get("B200Q_FUSED", "1") != "0" and not self.wide and (tp_world == 1 or self.tp_finish) and H % 512 == 0 and ept <= 16

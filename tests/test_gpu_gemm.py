@@ -95,8 +95,8 @@ def test_gemm_prefill_shape_property(client):
 
 @pytest.mark.parametrize("fmt,bias", [("Q6_K", False), ("Q4_K", False), ("GPTQ", True)])
 def test_gemm_tail_split_k_wave_quantisation(client, fmt, bias, monkeypatch):
-    """(opt-in path, B200Q_GEMM_TAIL=1 -- the switch is read once per process, so the driver's default suite exercises the plain
-    persistent loop on this shape and `B200Q_GEMM_TAIL=1 pytest -k tail_split` the split form; both were run green in round 2)
+    """(opt-in path, B200Q_GEMM_TAIL=1 -- the switch is read once per process, so the default suite exercises the plain
+    persistent loop on this shape and `B200Q_GEMM_TAIL=1 pytest -k tail_split` the split form; both have run green)
     wide-M launch whose tile count is not a multiple of the SM count: the tiles of the last, partial wave are split along K
     (tail split-K: 19 x 8 = 152 tiles on 148 SMs -> 4 tail tiles x 4 splits), partial accumulators reduced by a second kernel;
     ragged M so the last activation tile is partly empty"""

@@ -1,8 +1,8 @@
-"""Parity depth (VERDICT round 1, item 8):
-  (i)   BASELINE config 1 at FULL size: Llama-3.2-1B Q4_K_M (16 layers, vocab 128256), 32-token prompt + 128 greedy tokens, the GPU
+"""Parity depth:
+  (i)   Llama-3.2-1B at FULL size: Q4_K_M (16 layers, vocab 128256), 32-token prompt + 128 greedy tokens, the GPU
         stream equals the CPU oracle's (flavour B, exact integer / f64 arithmetic);
   (ii)  M = 1 decode logits against the f32 CPU path (flavour A: dequant(W) . x) within 1e-2 relative on a 32-layer stack,
-        where the per-32 int8 activation error compounds through every layer -- the north_star's logit contract;
+        where the per-32 int8 activation error compounds through every layer -- the contract on the logits;
   (iii) tensor-parallel shard uploads (b200q_weight_from_{ggml,awq,gptq}_shard) against the oracle on the sliced matrix;
   (iv)  the prefill pass (M = S through every projection on the tcgen05 GEMM) against the f32 CPU path, and decode continuing
         from the prefilled KV cache;
@@ -42,7 +42,7 @@ DEEP = decode.ModelConfig("deep-32", 512, 32, 8, 2, 64, 1024, 2048, 10000.0)
 
 @pytest.mark.parametrize("scheme", ["Q4_K_M", "Q8_0", "AWQ"])
 def test_m1_decode_logits_vs_f32_cpu_path_32_layers(client, scheme):
-    """MEASURED FINDING (round 2): through 32 random-init layers the int8-activation decode path is NOT within 1e-2 of the
+    """MEASURED FINDING: through 32 random-init layers the int8-activation decode path is NOT within 1e-2 of the
     f32-activation CPU path (flavour A): 3.3 % (Q4_K_M), 3.8 % (Q8_0), 5.9 % (AWQ) max-abs / max-abs on the logits -- the
     ~0.5 % rounding noise of per-32 int8 activations enters the residual stream twice per layer and random-init layers pass
     it on undamped (a random walk over 64 additions).  It is a property of quantising ACTIVATIONS to int8 (which ggml's and,

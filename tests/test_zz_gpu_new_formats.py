@@ -1,7 +1,6 @@
 """GPU parity of the remaining K / IQ / TQ formats: Q5_K, Q4_1, Q5_1, Q2_K, Q3_K, IQ4_XS, TQ2_0, TQ1_0, IQ2_XXS, IQ2_XS, IQ3_XXS,
 IQ2_S, IQ3_S, IQ1_S, IQ1_M -- the same contracts as the headline formats (#1 dequantized weights, #2 integer partials, #3 matvec,
-GEMM tolerance).  Round 1 shipped them xfail(strict=False) because they had never run on a B200; round 2's first GPU call ran all
-of them green (gpurun_out/r2_pytest_gpu_1.log: 271 xpassed), so the marks are gone: a failure now turns the suite red.
+GEMM tolerance).
 """
 import pytest
 
@@ -47,7 +46,7 @@ def test_gemm_vs_oracle(client, fmt, NKM):
     tg.test_gemm_vs_oracle(client, fmt, NKM)
 
 
-# ---- EXPERIMENTAL persistent op-list kernel (csrc/dstep_impl.cuh): green on hardware in round 2 (8 passed) and measured SLOWER
+# ---- EXPERIMENTAL persistent op-list kernel (csrc/dstep_impl.cuh): green on hardware (8 passed) and measured SLOWER
 # than the PDL-chained launches (407 vs 560 tok/s on Mistral-7B Q6_K), so it stays opt-in.  A persistent kernel with grid barriers
 # can hang if it is ever broken, and a hung kernel cannot be interrupted by pytest: the test only runs when asked for
 # (B200Q_TEST_EXPERIMENTAL=1, under `timeout`), never in the default -m gpu suite.

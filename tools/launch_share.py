@@ -1,6 +1,6 @@
 """Per-kernel share of a decode step from an `ncu --metrics gpu__time_duration.sum --csv` launch list (CPU only).
 
-    python tools/launch_share.py gpurun_out/r2_decode_step_launches.csv > profiles/r2_decode_step_share.txt
+    python tools/launch_share.py launches.csv > profiles/decode_step_share.txt
 ncu durations are cold-cache and serialised: the SHARE per kernel is what must agree with the bench, not the absolute time."""
 import collections, csv, re, sys
 

@@ -1,7 +1,7 @@
 """Summarise an .ncu-rep (read here with `ncu -i`, no GPU needed) into profiles/<name>.txt and update
 profiles/r2_traffic.json (per-launch DRAM bytes of the bench's roofline kernel, read by bench.py).
 
-    python tools/ncu_summary.py gpurun_out/prof_x.ncu-rep profiles/r1_x_ncu.txt "header text" [--traffic-key KEY]
+    python tools/ncu_summary.py prof_x.ncu-rep profiles/x_ncu.txt "header text" [--traffic-key KEY]
 """
 import csv
 import io
