@@ -150,7 +150,8 @@ static WidePlan wide_plan(const b200q_weight* w, int64_t M) {
 // projections of hidden sizes 2048, 4096 and 8192; it cuts K when there are at most half as many tiles as SMs, which costs a pass over the partial
 // sums, here as there).  Lines drawn from the same measurements: never below 512 rows; weights of several panels from 768 rows, with 14 % in hand
 // (8192 x 8192, 800 rows: estimated 12 % faster, measured 3 % slower; 10240 x 8192, 300 to 640 rows: 10 to 25 % slower, 800: 8 to 14 % faster) and
-// not where K is cut.
+// not where K is cut.  Cut products, fused / expanded, us: 512 x 2048, 2048 rows 45.8 / 24.1; 1024 x 4096, 1280 rows 55.9 / 30.8; 1024 x 8192, 2048 rows
+// 120 / 67; 4096 x 4096, 512 rows 49.0 / 47.0.
 static bool wide_wins(const b200q_weight* w, int64_t M, const WidePlan& p) {
     const int64_t mt = (M + 255) / 256, rows = ((M + mt - 1) / mt + 31) / 32 * 32, items = w->T * mt;
     const double wave = (12.0 + 0.1 * (double)rows) * (double)w->K_pad / 4096.0;

@@ -644,16 +644,18 @@ cudaError_t run(const AttnArgs& a, const b200seq_step& st, dim3 grid, cudaStream
 }  // namespace
 
 // Which of the two kernels is the faster one for a step, from its row tiles and the keys a token may see.  Here a CTA has an SM to itself: about 15 us
-// (33 with heads above 64) of set-up, load and store, whatever the rows it has, and 2.2 (3.3) us a key tile.  The f32 tiles (seq_attn.cu) are half or a
+// (33 with heads above 64) of set-up, load and store, whatever the rows it has, a little less where one wave is all, and 2.2 (3.3) us a key tile.  The f32 tiles (seq_attn.cu) are half or a
 // quarter of the rows, two or three to an SM: a wave of them takes about 33 (37) us, 22 (29) where each has an SM, and 18 (21) us more for every
-// further key tile of its share.  Merging key splits: 6 and 10 us.  Measured, us, f32 tiles / this kernel, 32 query heads of 8 key heads of 64 (of 128):
+// further key tile of its share.  Merging key splits: 3 and 10 us.  Measured, us, f32 tiles / this kernel, 32 query heads of 8 key heads of 64 (of 128):
 //   65 sequences of one token, 10 earlier ones   57 /  66 ( 73 / 130)      128 of them    110 / 164 (153 / 282)      40 of two tokens  34 /  42 ( 56 /  89)
 //   65 of one token, 200 earlier ones           162 /  90 (263 / 177)      17, 1000       151 /  42 (256 /  97)      64, 2000         902 / 287 (1526 / 648)
 //   one sequence, 100 tokens                     21 /  16 ( 29 /  29)      600 tokens     168 /  29 (227 /  62)      4 of 300, 100    182 /  44 (281 / 109)
 bool tc_is_faster(const AttnArgs& f32, int64_t units, int64_t splits, int64_t f32_units, int key_tiles, int sms) {
     const bool big = f32.D > 64 || f32.V > 64;
     const auto up = [](int64_t a, int64_t b) { return (a + b - 1) / b; };
-    const double tc = (double)up(units * splits, sms) * ((big ? 33.0 : 15.0) + (big ? 3.3 : 2.2) * (double)up(key_tiles, splits)) + (splits > 1 ? 6.0 : 0.0);
+    const int64_t waves = up(units * splits, sms);
+    const double set_up = waves == 1 ? (big ? 30.0 : 12.5) : (big ? 33.0 : 15.0);
+    const double tc = (double)waves * (set_up + (big ? 3.3 : 2.2) * (double)up(key_tiles, splits)) + (splits > 1 ? 3.0 : 0.0);
     const int64_t blocks = f32_units * f32.nsplit, share = up(key_tiles, f32.nsplit), fit = (big ? 2 : 3) * (int64_t)sms;
     const double wave = (blocks <= sms ? (big ? 29.0 : 22.0) : (big ? 37.0 : 33.0)) + (big ? 21.0 : 18.0) * (double)(share - 1);
     return tc < (double)up(blocks, fit) * wave + (f32.nsplit > 1 ? 10.0 : 0.0);
