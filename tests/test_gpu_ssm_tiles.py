@@ -1,4 +1,4 @@
-"""The state-space scan of long steps as tile products (csrc/seq/seq_ssm.cu) against the recurrence in float64: portions that end inside a segment and
+"""The state-space scan of long steps as tile products (csrc/seq/seq_ssm_tc.cu) against the recurrence in float64: portions that end inside a segment and
 inside a block of 32, state and column counts that end inside a tile, one to many heads per group, carried states, fast and slow decays.
 
 Bound: f32 products and sums in another order than the recurrence's; the recurrence is tested at 2e-5 of the largest value, this at 3e-6."""
@@ -52,7 +52,7 @@ def scan(ops, lens, H, V, N, G, speed, plant=None):
         r += n
     out = torch.empty(T, inner, device=DEV)
     scratch = torch.empty(ops.ssm_scratch_floats(T, B, H, V, N), device=DEV)
-    assert scratch.numel() > 0
+    assert (scratch.numel() > 0) == (T > 128)
     ops.ssm_scan(proj, 0, dt0, xbc, A_log, Dp, dtb, state, st, H, V, N, G, out, scratch)
     return (out, ref), (state, ref_state)
 
@@ -65,19 +65,32 @@ def test_against_the_recurrence(ops, lens, H, V, N, G, speed):
         assert err < 3e-6, err
 
 
+@pytest.mark.parametrize("lens,H,V,N,G", [([32], 2, 64, 128, 1), ([41], 9, 68, 36, 3), ([128], 4, 4, 100, 1), ([90, 1, 33], 3, 64, 64, 3), ([64, 64], 16, 132, 128, 2), ([31], 2, 64, 128, 1)])
+@pytest.mark.parametrize("speed", [-8.0, 0.0, 3.0])
+def test_entries_of_one_segment(ops, lens, H, V, N, G, speed):
+    """Steps of up to 128 tokens: outputs from the slots' states (new and carried), then the states; the last one stays on the recurrence."""
+    test_against_the_recurrence(ops, lens, H, V, N, G, speed)
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
 @pytest.mark.parametrize("token", [0, 17, 31, 32, 200, 255])
-def test_a_value_that_is_not_finite_reaches_no_earlier_token(ops, value, token):
+def test_a_value_that_is_not_finite_reaches_no_earlier_token(ops, value, token, T=256):
     """Head 1, column 5 of one token: the outputs of the tokens before it, of the other columns and of the other heads stay what they are."""
     def plant(xbc, A_log, Dp):
         xbc[token, 64 + 5] = value
-    (out, ref), (state, ref_state) = scan(ops, [256], 4, 64, 64, 2, 0.0, plant)
+    (out, ref), (state, ref_state) = scan(ops, [T], 4, 64, 64, 2, 0.0, plant)
     top = ref[torch.isfinite(ref)].abs().max().item()
     fine = torch.isfinite(ref)
     assert bool(fine[:token].all()) and not bool(fine[token, 64 + 5]) and torch.equal(torch.isfinite(out), fine)
     assert ((out.double() - ref)[fine].abs().max().item()) / top < 3e-6
     fine = torch.isfinite(ref_state)
     assert torch.equal(torch.isfinite(state), fine) and ((state.double() - ref_state)[fine].abs().max().item()) / ref_state[fine].abs().max().item() < 3e-6
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("token", [0, 17, 63])
+def test_a_value_that_is_not_finite_in_one_segment(ops, value, token):
+    test_a_value_that_is_not_finite_reaches_no_earlier_token(ops, value, token, 64)
 
 
 def test_decays_that_forget_at_once(ops):
