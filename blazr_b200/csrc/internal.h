@@ -53,13 +53,16 @@ struct MatvecPlan {
     int grid, nstages, stage_bytes, smem_bytes, mb, xhat_bytes;
 };
 struct FusedPrologue {
-    int mode;  // 1 = add + rmsnorm + quant, 2 = swiglu + quant
+    int mode;  // 1 = add + rmsnorm + quant, 2 = swiglu + quant, 3 = quant of x
     const float* h_in;
     const float* delta;
     float* h_out;
     const float* norm_w;
     float eps;
     const float* gate_up;
+    const void* x = nullptr;   // mode 3
+    int x_dtype = 0;
+    int64_t ldx = 0;
 };
 cudaError_t matvec_plan(const b200q_weight* w, int64_t M, MatvecPlan* plan, int pro = 0);
 size_t matvec_ws_bytes(const b200q_weight* w, int64_t M);  // counters + partials (excludes the activation buffer)

@@ -54,6 +54,10 @@ void set_matvec_trace(long long* p) { g_trace = p; g_trace_launch = 0; }
 // dual-format partner honoured by a launch: plain / norm-prologue matvecs only (not the SwiGLU, grouped or fused-exchange forms)
 static const b200q_weight* dual_partner(const b200q_weight* w) { return w->pair; }
 
+// Most records that a CTA makes in the quantising prologue: one pass of its 16 warps, two at a time.  More take longer than the ring covers (in a chain
+// of calls, us, a launch of its own / prologue: 4 records 6.2 / 5.6, 16: 14.4 / 13.4, 32: 57.9 / 56.5, but 49: 38.0 / 39.1, 52: 19.1 / 21.3, 196: 51.5 / 55.4).
+constexpr int MV_QUANT_RECORDS = 32;
+
 cudaError_t matvec_plan(const b200q_weight* w, int64_t M, MatvecPlan* plan, int pro) {
     if (M < 1 || M > 4) return cudaErrorInvalidValue;
     int mb = M == 1 ? 1 : (M == 2 ? 2 : 4);
@@ -63,21 +67,25 @@ cudaError_t matvec_plan(const b200q_weight* w, int64_t M, MatvecPlan* plan, int 
     // pass the end of the CTA's shared memory in the ring's last stage.  The copies and the record stride stay those of M rows.
     int stage = cbmax + (pro ? 0 : mb * ACT_REC_BYTES);
     stage = (stage + 127) & ~127;
-    int xhat = pro ? (int)(((size_t)w->KC * M * ACT_REC_BYTES + 127) & ~(size_t)127) : 0;
+    int64_t C = (w->T + (w2 ? w2->T : 0)) * w->KC;
+    int64_t G = (int64_t)w->num_sms;
+    if (const char* e = getenv("B200Q_MV_GRID")) { int v = atoi(e); if (v >= 1 && v <= w->num_sms) G = v; }  // ws_part holds num_sms slots
+    if (G > C) G = C;
+    int64_t recs = w->KC;   // records that the prologue makes: all, or (pro 3) those of the CTA's own chunks
+    if (pro == 3 && (C + G - 1) / G < recs) recs = (C + G - 1) / G;
+    int xhat = pro ? (int)(((size_t)recs * M * ACT_REC_BYTES + 127) & ~(size_t)127) : 0;
+    if (pro == 3 && recs * M > MV_QUANT_RECORDS) return cudaErrorInvalidValue;
     // > half an SM on purpose: two CTAs of one launch must never share an SM (measured: after glue kernels perturb
     // the placement, doubled-up CTAs run at half speed and the launch takes 2x); cross-launch overlap is done
     // with the L2 prefetch kernel instead
     int budget_kb = 150;
     if (const char* e = getenv("B200Q_MV_SMEM_KB")) { int v = atoi(e); if (v >= 64 && v <= 214) budget_kb = v; }
     int budget = budget_kb * 1024 - MV_HDR_BYTES - xhat;
+    if (pro == 3) budget = (budget_kb * 1024 < 216 * 1024 - xhat ? budget_kb * 1024 : 216 * 1024 - xhat) - MV_HDR_BYTES;   // the records beside a whole ring
     int nst = budget / stage;
     if (nst > MV_MAX_STAGES) nst = MV_MAX_STAGES;
     if (const char* e = getenv("B200Q_MV_STAGES")) { int v = atoi(e); if (v >= 2 && v < nst) nst = v; }
     if (nst < 2) return cudaErrorInvalidValue;
-    int64_t C = (w->T + (w2 ? w2->T : 0)) * w->KC;
-    int64_t G = (int64_t)w->num_sms;
-    if (const char* e = getenv("B200Q_MV_GRID")) { int v = atoi(e); if (v >= 1 && v <= w->num_sms) G = v; }  // ws_part holds num_sms slots
-    if (G > C) G = C;
     plan->grid = (int)G;
     plan->nstages = nst;
     plan->stage_bytes = stage;
@@ -135,6 +143,11 @@ cudaError_t launch_matvec(const b200q_weight* w, const uint8_t* xq, int64_t M, v
     p.norm_w = fp ? fp->norm_w : nullptr;
     p.eps = fp ? fp->eps : 0.0f;
     p.gate_up = fp ? fp->gate_up : nullptr;
+    p.x = fp ? fp->x : nullptr;
+    p.x_dtype = fp ? fp->x_dtype : 0;
+    p.ldx = fp ? fp->ldx : 0;
+    p.K = w->K;
+    p.perm = w->perm;
     p.w_table = nullptr;
     p.sel = nullptr;
     p.n_experts = 0;

@@ -32,6 +32,7 @@ struct MatvecParams {
     int l2_prefetch_chunks;  // per CTA: chunks beyond the smem ring to pull into L2 before griddepcontrol.wait
     // fused activation producers (prologue): 0 = records arrive by TMA from xq, 1 = quant(rmsnorm(h_in + delta) * nw),
     // 2 = quant(silu(gate) * up).  The whole quantised activation then lives in shared memory for the CTA's life.
+    // 3 = quant(x), only the records of the CTA's own chunks (record 0 = that of its first chunk, then on modulo KC).
     int pro;
     int xhat_bytes;
     const float* h_in;
@@ -40,6 +41,10 @@ struct MatvecParams {
     const float* norm_w;
     float eps;
     const float* gate_up;
+    const void* x;         // pro 3: x[M][ldx] (x_dtype) of K columns, gathered through perm if there is one
+    int x_dtype;
+    int64_t ldx, K;
+    const int32_t* perm;
     // grouped (expert bank) mode, w_table != null: the launch runs n_slots independent M = 1 matvecs; slot s uses the
     // weight w_table[sel[s]], the activation record row s / x_slot_div of xq (x_rows rows per k-chunk) and writes
     // y[s * y_slot_stride + n].  Tiles are numbered slot-major (tile t -> slot t / tpw), so the stream-K split, the

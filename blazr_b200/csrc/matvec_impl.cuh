@@ -14,7 +14,7 @@
 //     two contributors -> the first one's fix-up warp polls and sums beside the consumers; three or more ->
 //     all 16 consumer warps of contributor gf + 1 poll one contributor each (MV_WIDE_MIN); always CTA order,
 //     no float atomics;
-//   * compile-time variants: norm prologue (PRO), SwiGLU epilogue / fused tensor-parallel exchange (OUT),
+//   * compile-time variants: norm / quantising prologue (PRO), SwiGLU epilogue / fused tensor-parallel exchange (OUT),
 //     grouped expert-bank launch (GRP), dual-format launch (F2 != F: two weights of different formats, one grid).
 #pragma once
 #include <atomic>
@@ -180,6 +180,79 @@ __device__ __forceinline__ void norm_prologue(const MatvecParams& p, uint8_t* xh
     named_bar_sync(4, NT);  // records visible to every consumer warp
 }
 
+// ---- quantising prologue: the records of the CTA's own chunks from x itself.  A warp makes a record (256 elements of one row, eight consecutive ones
+// per lane, a 32-block is four lanes), the loads of two records in flight.  Arithmetic as act_quant_kernel: the same bits.  A launch of its own for these
+// records cost (one f32 row, Q4_K): 4096 x 4096 6.2 us in two launches, 5.6 in one; 28672 x 4096 16.1 and 14.2; from a caller that is not captured the
+// second launch itself is what counts (4096 x 4096: 8.95 and 6.8 a call). ----
+template <int DT>
+__device__ __forceinline__ void load_x8(const MatvecParams& p, int kc, int m, int lane, bool vec, float (&v)[8]) {
+    const int64_t k = (int64_t)kc * CHUNK_K + 8 * lane, at = (int64_t)m * p.ldx + k;
+    if (vec && k + 8 <= p.K) {
+        if (DT == 0) {
+            const float4* q = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.x) + at);
+            const float4 a = __ldcg(q), b = __ldcg(q + 1);
+            v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+        } else {
+            const uint4 u = __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(p.x) + at));
+            const uint32_t wd[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (DT == 1) {
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&wd[j]));
+                    v[2 * j] = f.x, v[2 * j + 1] = f.y;
+                } else {
+                    v[2 * j] = __uint_as_float(wd[j] << 16), v[2 * j + 1] = __uint_as_float(wd[j] & 0xFFFF0000u);
+                }
+            }
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = k + j < p.K ? load_in(p.x, DT, (int64_t)m * p.ldx + (p.perm ? p.perm[k + j] : k + j)) : 0.0f;
+    }
+}
+__device__ __forceinline__ void quant8_to_record(const float (&v)[8], uint8_t* rec, int lane) {
+    float amax = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(v[j]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    const float d = __fdiv_rn(amax, 127.0f);
+    const float id = (d != 0.0f) ? __fdiv_rn(1.0f, d) : 0.0f;
+    uint32_t w[2] = {0, 0};
+    int s = 0;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const int q = (int)roundf(__fmul_rn(v[j], id));
+        s += (int)(int8_t)q;
+        w[j >> 2] |= ((uint32_t)q & 0xFFu) << (8 * (j & 3));
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    const int s_hi = __shfl_xor_sync(0xffffffffu, s, 2);
+    *reinterpret_cast<uint2*>(rec + 8 * lane) = make_uint2(w[0], w[1]);
+    if ((lane & 3) == 0) {
+        reinterpret_cast<float*>(rec + 256)[lane >> 2] = d;
+        reinterpret_cast<uint32_t*>(rec + 288)[lane >> 2] = ((uint32_t)s & 0xFFFFu) | ((uint32_t)s_hi << 16);
+    }
+}
+template <int DT>
+__device__ __forceinline__ void quant_prologue_t(const MatvecParams& p, uint8_t* xhat, int n_rec, int kc_first, int warp, int lane) {
+    const int KC = (int)p.KC, M = p.M, total = n_rec * M;
+    const bool vec = !p.perm && (reinterpret_cast<uintptr_t>(p.x) & 15) == 0 && ((p.ldx * (DT == 0 ? 4 : 2)) & 15) == 0;
+    auto chunk_of = [&](int idx) {
+        const int kc = kc_first + idx / M;
+        return kc < KC ? kc : kc - KC;
+    };
+    for (int idx = warp; idx < total; idx += 2 * MV_CONSUMER_WARPS) {
+        const int idx2 = idx + MV_CONSUMER_WARPS;
+        float a[8], b[8];
+        load_x8<DT>(p, chunk_of(idx), idx % M, lane, vec, a);
+        if (idx2 < total) load_x8<DT>(p, chunk_of(idx2), idx2 % M, lane, vec, b);
+        quant8_to_record(a, xhat + (size_t)idx * ACT_REC_BYTES, lane);
+        if (idx2 < total) quant8_to_record(b, xhat + (size_t)idx2 * ACT_REC_BYTES, lane);
+    }
+    named_bar_sync(4, MV_CONSUMER_WARPS * 32);  // records visible to every consumer warp
+}
+
 template <int MB>
 __device__ __forceinline__ void fused_prologue(const MatvecParams& p, uint8_t* xhat, int tid, int warp, int lane, bool writer) {
     constexpr int NT = MV_CONSUMER_WARPS * 32;
@@ -254,6 +327,7 @@ constexpr int MV_BAR_EPI_FULL = 6;   // (+ buffer 0/1) consumers -> fix-up warp:
 constexpr int MV_BAR_EPI_FREE = 8;   // (+ buffer 0/1) fix-up warp -> consumers: s_y[buffer] may be overwritten
 
 // where finished row sums go (compile time, like GRP: the plain matvec carries none of the other forms)
+enum { PRO_NONE = 0, PRO_FUSED = 1, PRO_QUANT = 2 };
 enum { OUT_PLAIN = 0, OUT_REMOTE = 1 /* fused tensor-parallel exchange */, OUT_SWIGLU = 2 /* fused SwiGLU + quantise epilogue */ };
 
 // ---- OUT_SWIGLU: one finished 128-row tile (64 gate / 64 up rows interleaved, f32 in shared memory) -> 64 activations
@@ -288,7 +362,8 @@ __device__ __forceinline__ void sk_tile_span(const MatvecParams& p, int64_t tq, 
 // for up to 16 contributors instead of one per 4 in the single fix-up warp (measured 4.6 us of tail on 17-way split tiles)
 constexpr int MV_WIDE_MIN = 3;
 
-template <class F, int MB, bool PRO, bool GRP, int OUT, class F2 = F>
+// PRO: PRO_FUSED = norm / SwiGLU prologue (p.pro 1, 2), PRO_QUANT = quantising prologue (p.pro 3)
+template <class F, int MB, int PRO, bool GRP, int OUT, class F2 = F>
 __global__ void __launch_bounds__(MV_THREADS, 1) matvec_kernel(const MatvecParams p) {
     constexpr bool RP = OUT == OUT_REMOTE;
     constexpr bool EPI = OUT == OUT_SWIGLU;
@@ -565,7 +640,7 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_kernel(const MatvecParam
 #pragma unroll
         for (int m = 0; m < MB; m++) acc[s4][m] = 0.0;
 
-    if constexpr (PRO) {
+    if constexpr (PRO == PRO_FUSED) {
         if (p.pro == 1) {
             // norm prologue: K = EPT * 512 with EPT in {1, 2, 4, 8, 16} (checked by the host)
             __shared__ double s_red[MV_CONSUMER_WARPS];
@@ -581,6 +656,13 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_kernel(const MatvecParam
             fused_prologue<MB>(p, xhat, tid, warp, lane, g == 0);
         }
     }
+    if constexpr (PRO == PRO_QUANT) {
+        pdl_wait();
+        const int kc_first = sp.nH > 0 ? sp.kcH : 0, n_rec = n_chunks < KC ? n_chunks : KC;
+        if (p.x_dtype == 0) quant_prologue_t<0>(p, xhat, n_rec, kc_first, warp, lane);
+        else if (p.x_dtype == 1) quant_prologue_t<1>(p, xhat, n_rec, kc_first, warp, lane);
+        else quant_prologue_t<2>(p, xhat, n_rec, kc_first, warp, lane);
+    }
 
     // am I the wide reducer of my head tile?  (then that segment is my whole range: see MV_WIDE_MIN)
     bool wide_reducer = false;
@@ -591,6 +673,8 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_kernel(const MatvecParam
     }
     // segment walk: 0 = head (partial, slot 0), 1 = tail (partial, slot 1), 2 = full tiles
     int kcur = sp.nH > 0 ? sp.kcH : 0;  // k-chunk index of the chunk being processed (fused prologue addressing)
+    const int krec0 = PRO == PRO_QUANT && sp.nH > 0 ? KC - kcur : 0;   // where the record of k-chunk 0 lies (PRO_QUANT: record 0 is that of the first chunk)
+    if (PRO == PRO_QUANT && sp.nH > 0) kcur = 0;
     int seg = sp.nH > 0 ? 0 : (sp.nT > 0 ? 1 : 2);
     int seg_left = seg == 0 ? sp.nH : (seg == 1 ? sp.nT : KC);  // chunks until the next flush
     int t = seg == 0 ? sp.tH : (seg == 1 ? sp.tT : sp.tF);
@@ -827,8 +911,8 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_kernel(const MatvecParam
             for (int m = 0; m < MB; m++) acc[s4][m] = 0.0;
 
         // ---- next segment / tile ----
-        if (seg == 0 && sp.nT > 0) { seg = 1; seg_left = sp.nT; t = sp.tT; kcur = 0; xk_off = 0u; }
-        else if (seg != 2) { seg = 2; seg_left = KC; t = sp.tF; kcur = 0; xk_off = 0u; }
+        if (seg == 0 && sp.nT > 0) { seg = 1; seg_left = sp.nT; t = sp.tT; kcur = krec0; xk_off = (uint32_t)krec0 * xrec_step; }
+        else if (seg != 2) { seg = 2; seg_left = KC; t = sp.tF; kcur = krec0; xk_off = (uint32_t)krec0 * xrec_step; }
         else { seg_left = KC; t++; }
 
     }
@@ -856,7 +940,7 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_kernel(const MatvecParam
     if (MV_TRACE_ON(p) && tid == 0) p.trace[g * 8 + 3] = globaltimer_ns();
 }
 
-template <class F, int MB, bool PRO, bool GRP, int OUT = OUT_PLAIN, class F2 = F>
+template <class F, int MB, int PRO, bool GRP, int OUT = OUT_PLAIN, class F2 = F>
 static cudaError_t launch_t(const MatvecParams& p, int grid, int smem, cudaStream_t st) {
     static std::atomic<bool> configured[16];   // per device; racing first calls both set the attribute (idempotent): re-entrant
     int dev = 0;
@@ -887,9 +971,9 @@ template <class F, class F2>
 static cudaError_t launch_dual(const MatvecParams& p, int mb, int grid, int smem, cudaStream_t st) {
     if (p.w_table || p.rp_mode != RP_NONE || p.xq_out || !p.w2) return cudaErrorInvalidValue;
     switch (mb) {
-        case 1: return p.pro ? launch_t<F, 1, true, false, OUT_PLAIN, F2>(p, grid, smem, st) : launch_t<F, 1, false, false, OUT_PLAIN, F2>(p, grid, smem, st);
-        case 2: return p.pro ? launch_t<F, 2, true, false, OUT_PLAIN, F2>(p, grid, smem, st) : launch_t<F, 2, false, false, OUT_PLAIN, F2>(p, grid, smem, st);
-        case 4: return p.pro ? launch_t<F, 4, true, false, OUT_PLAIN, F2>(p, grid, smem, st) : launch_t<F, 4, false, false, OUT_PLAIN, F2>(p, grid, smem, st);
+        case 1: return p.pro ? launch_t<F, 1, PRO_FUSED, false, OUT_PLAIN, F2>(p, grid, smem, st) : launch_t<F, 1, PRO_NONE, false, OUT_PLAIN, F2>(p, grid, smem, st);
+        case 2: return p.pro ? launch_t<F, 2, PRO_FUSED, false, OUT_PLAIN, F2>(p, grid, smem, st) : launch_t<F, 2, PRO_NONE, false, OUT_PLAIN, F2>(p, grid, smem, st);
+        case 4: return p.pro ? launch_t<F, 4, PRO_FUSED, false, OUT_PLAIN, F2>(p, grid, smem, st) : launch_t<F, 4, PRO_NONE, false, OUT_PLAIN, F2>(p, grid, smem, st);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -898,29 +982,38 @@ template <class F>
 static cudaError_t launch_f(const MatvecParams& p, int mb, int grid, int smem, cudaStream_t st) {
     if (p.w_table) {
         if (mb != 1 || p.pro || p.rp_mode) return cudaErrorInvalidValue;
-        return p.xq_out ? launch_t<F, 1, false, true, OUT_SWIGLU>(p, grid, smem, st) : launch_t<F, 1, false, true>(p, grid, smem, st);
+        return p.xq_out ? launch_t<F, 1, PRO_NONE, true, OUT_SWIGLU>(p, grid, smem, st) : launch_t<F, 1, PRO_NONE, true>(p, grid, smem, st);
     }
     if (p.rp_mode != RP_NONE) {  // fused tensor-parallel exchange (row-parallel o / down, vocabulary-parallel lm_head)
         if (p.pro || p.xq_out) return cudaErrorInvalidValue;
         switch (mb) {
-            case 1: return launch_t<F, 1, false, false, OUT_REMOTE>(p, grid, smem, st);
-            case 2: return launch_t<F, 2, false, false, OUT_REMOTE>(p, grid, smem, st);
-            case 4: return launch_t<F, 4, false, false, OUT_REMOTE>(p, grid, smem, st);
+            case 1: return launch_t<F, 1, PRO_NONE, false, OUT_REMOTE>(p, grid, smem, st);
+            case 2: return launch_t<F, 2, PRO_NONE, false, OUT_REMOTE>(p, grid, smem, st);
+            case 4: return launch_t<F, 4, PRO_NONE, false, OUT_REMOTE>(p, grid, smem, st);
+            default: return cudaErrorInvalidValue;
+        }
+    }
+    if (p.pro == 3) {   // quantising prologue
+        if (p.xq_out) return cudaErrorInvalidValue;
+        switch (mb) {
+            case 1: return launch_t<F, 1, PRO_QUANT, false>(p, grid, smem, st);
+            case 2: return launch_t<F, 2, PRO_QUANT, false>(p, grid, smem, st);
+            case 4: return launch_t<F, 4, PRO_QUANT, false>(p, grid, smem, st);
             default: return cudaErrorInvalidValue;
         }
     }
     if (p.xq_out) {  // fused SwiGLU + quantise epilogue (interleaved gate|up weight)
         switch (mb) {
-            case 1: return p.pro ? launch_t<F, 1, true, false, OUT_SWIGLU>(p, grid, smem, st) : launch_t<F, 1, false, false, OUT_SWIGLU>(p, grid, smem, st);
-            case 2: return p.pro ? launch_t<F, 2, true, false, OUT_SWIGLU>(p, grid, smem, st) : launch_t<F, 2, false, false, OUT_SWIGLU>(p, grid, smem, st);
-            case 4: return p.pro ? launch_t<F, 4, true, false, OUT_SWIGLU>(p, grid, smem, st) : launch_t<F, 4, false, false, OUT_SWIGLU>(p, grid, smem, st);
+            case 1: return p.pro ? launch_t<F, 1, PRO_FUSED, false, OUT_SWIGLU>(p, grid, smem, st) : launch_t<F, 1, PRO_NONE, false, OUT_SWIGLU>(p, grid, smem, st);
+            case 2: return p.pro ? launch_t<F, 2, PRO_FUSED, false, OUT_SWIGLU>(p, grid, smem, st) : launch_t<F, 2, PRO_NONE, false, OUT_SWIGLU>(p, grid, smem, st);
+            case 4: return p.pro ? launch_t<F, 4, PRO_FUSED, false, OUT_SWIGLU>(p, grid, smem, st) : launch_t<F, 4, PRO_NONE, false, OUT_SWIGLU>(p, grid, smem, st);
             default: return cudaErrorInvalidValue;
         }
     }
     switch (mb) {
-        case 1: return p.pro ? launch_t<F, 1, true, false>(p, grid, smem, st) : launch_t<F, 1, false, false>(p, grid, smem, st);
-        case 2: return p.pro ? launch_t<F, 2, true, false>(p, grid, smem, st) : launch_t<F, 2, false, false>(p, grid, smem, st);
-        case 4: return p.pro ? launch_t<F, 4, true, false>(p, grid, smem, st) : launch_t<F, 4, false, false>(p, grid, smem, st);
+        case 1: return p.pro ? launch_t<F, 1, PRO_FUSED, false>(p, grid, smem, st) : launch_t<F, 1, PRO_NONE, false>(p, grid, smem, st);
+        case 2: return p.pro ? launch_t<F, 2, PRO_FUSED, false>(p, grid, smem, st) : launch_t<F, 2, PRO_NONE, false>(p, grid, smem, st);
+        case 4: return p.pro ? launch_t<F, 4, PRO_FUSED, false>(p, grid, smem, st) : launch_t<F, 4, PRO_NONE, false>(p, grid, smem, st);
         default: return cudaErrorInvalidValue;
     }
 }
