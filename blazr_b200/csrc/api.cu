@@ -547,8 +547,7 @@ int32_t b200q_matmul_path(const b200q_weight* w, int32_t path, const void* x, in
         size_t mv = align256(matvec_ws_bytes(w, M));
         size_t need = mv + align256(b200q_act_bytes(w->K, M));
         if (workspace_bytes < need) return fail(B200Q_ERR_WORKSPACE, "workspace too small: %zu < %zu", workspace_bytes, need);
-        MatvecPlan plan;
-        if (!w->pair && matvec_plan(w, M, &plan, 3) == cudaSuccess) {   // one launch: every CTA quantises what its own chunks need
+        if (matvec_quantises(w, M)) {   // one launch: every CTA quantises what its own chunks need
             FusedPrologue fp{3, nullptr, nullptr, nullptr, nullptr, 0.0f, nullptr, x, x_dtype, ldx};
             CUDA_TRY(launch_matvec(w, nullptr, M, y, y_dtype, ldy, (uint8_t*)workspace, st, &fp));
             return B200Q_OK;

@@ -5,6 +5,7 @@
 // next matvec consumes (so no separate quantise pass runs).  Every kernel is PDL-aware: it lets its
 // dependents launch immediately (the following matvec prefetches weights meanwhile) and waits for its own
 // producers before touching global memory.
+#include <atomic>
 #include <cooperative_groups.h>
 #include <cstdlib>
 
@@ -692,7 +693,13 @@ __global__ void embed_kernel(const __half* __restrict__ table, const int64_t* __
 
 int* decode_error_dev() {
     void* p = nullptr;
-    return cudaGetSymbolAddress(&p, g_decode_error) == cudaSuccess ? (int*)p : nullptr;
+    static std::atomic<int*> known[16];   // per device: asked for by every launch that can report a wait
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev < 16)
+        if (int* k = known[dev].load(std::memory_order_acquire)) return k;
+    if (cudaGetSymbolAddress(&p, g_decode_error) != cudaSuccess) return nullptr;
+    if (dev < 16) known[dev].store((int*)p, std::memory_order_release);
+    return (int*)p;
 }
 
 }  // namespace b200q

@@ -140,6 +140,10 @@ struct FmtQ4K {
     // matvec fast path: the byte offsets of (row r0 + 4 STEP, unit i) inside a chunk are lane constants, computed once per
     // thread and kept in registers; the hot loop only adds the stage base (same bytes / same arithmetic as load_unit<true, true>)
     static constexpr int NOFF = 5;
+    // planes of a chunk (bytes per row) and the plane of every offset: a slab of rows keeps the planes, shortened (matvec_slab.cuh)
+    static constexpr int NPLANES = 2;
+    __host__ __device__ static constexpr int plane_bytes(int pl, int) { return pl == 0 ? 128 : 16; }
+    __host__ __device__ static constexpr int plane_of(int q) { return q < 2 ? 0 : 1; }
     __device__ __forceinline__ static void unit_offsets(int r0, int i, FmtMeta, uint32_t (&o)[NOFF]) {
         o[0] = QS + r0 * 128 + 16 * swz8(r0, i);
         o[1] = QS + (r0 + 4) * 128 + 16 * swz8(r0 + 4, i);
@@ -235,6 +239,9 @@ struct FmtQ6K {
     }
 #ifndef B200Q_HOST_CHECK
     static constexpr int NOFF = 6;  // matvec fast path (see FmtQ4K)
+    static constexpr int NPLANES = 4;
+    __host__ __device__ static constexpr int plane_bytes(int pl, int) { return pl == 0 ? 128 : (pl == 1 ? 64 : (pl == 2 ? 16 : 2)); }
+    __host__ __device__ static constexpr int plane_of(int q) { return q < 2 ? 0 : (q < 4 ? 1 : q - 2); }
     __device__ __forceinline__ static void unit_offsets(int r0, int i, FmtMeta, uint32_t (&o)[NOFF]) {
         o[0] = QL + r0 * 128 + 16 * swz8(r0, i);
         o[1] = QL + (r0 + 4) * 128 + 16 * swz8(r0 + 4, i);
@@ -306,6 +313,9 @@ struct FmtQ8_0 {
     }
 #ifndef B200Q_HOST_CHECK
     static constexpr int NOFF = 5;  // matvec fast path (see FmtQ4K)
+    static constexpr int NPLANES = 2;
+    __host__ __device__ static constexpr int plane_bytes(int pl, int) { return pl == 0 ? 256 : 16; }
+    __host__ __device__ static constexpr int plane_of(int q) { return q < 4 ? 0 : 1; }
     __device__ __forceinline__ static void unit_offsets(int r0, int i, FmtMeta, uint32_t (&o)[NOFF]) {
         o[0] = QS + r0 * 256 + 16 * swz8(r0, 2 * i);
         o[1] = QS + (r0 + 4) * 256 + 16 * swz8(r0 + 4, 2 * i);
@@ -367,6 +377,9 @@ struct FmtG4 {
     }
 #ifndef B200Q_HOST_CHECK
     static constexpr int NOFF = 6;  // matvec fast path (see FmtQ4K)
+    static constexpr int NPLANES = 3;
+    __host__ __device__ static constexpr int plane_bytes(int pl, int gpc) { return pl == 0 ? 128 : (pl == 1 ? 2 * gpc : gpc); }
+    __host__ __device__ static constexpr int plane_of(int q) { return q >> 1; }
     __device__ __forceinline__ static void unit_offsets(int r0, int i, FmtMeta meta, uint32_t (&o)[NOFF]) {
         const int gq = (i * meta.gpc) >> 3;
         o[0] = QS + r0 * 128 + 16 * swz8(r0, i);

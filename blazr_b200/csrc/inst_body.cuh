@@ -2,13 +2,18 @@
 // B200Q_FMT / B200Q_FAM_ID / B200Q_HAS_GGML_REPACK defined), so formats compile as parallel translation units.
 #include "aux_impl.cuh"
 #include "gemm_impl.cuh"
-#include "matvec_impl.cuh"
+#include "matvec_slab.cuh"
 
 namespace b200q {
 
 template <>
 cudaError_t mv_launch<B200Q_FAM_ID>(const MatvecParams& p, int mb, int grid, int smem, cudaStream_t st) {
     return launch_f<B200Q_FMT>(p, mb, grid, smem, st);
+}
+template <>
+cudaError_t mv_slab_launch<B200Q_FAM_ID>(const MatvecParams& p, int mb, int grid, int smem, cudaStream_t st) {
+    if constexpr (FmtNoff<B200Q_FMT>::value > 0) return slab_launch_f<B200Q_FMT>(p, mb, grid, smem, st);
+    else return cudaErrorNotSupported;
 }
 template <>
 cudaError_t gemm_launch<B200Q_FAM_ID>(const GemmParams& p, int grid, int smem, cudaStream_t st) {

@@ -65,6 +65,7 @@ struct FusedPrologue {
     int64_t ldx = 0;
 };
 cudaError_t matvec_plan(const b200q_weight* w, int64_t M, MatvecPlan* plan, int pro = 0);
+bool matvec_quantises(const b200q_weight* w, int64_t M);   // launch_matvec takes FusedPrologue mode 3 (x itself) for M rows
 size_t matvec_ws_bytes(const b200q_weight* w, int64_t M);  // counters + partials (excludes the activation buffer)
 void set_matvec_trace(long long* dev_buf);
 cudaError_t launch_l2_prefetch(const b200q_weight* w, int64_t M, int64_t max_bytes, cudaStream_t st);

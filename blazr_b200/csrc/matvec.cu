@@ -47,6 +47,15 @@ static cudaError_t launch_family(int family, const MatvecParams& p, int mb, int 
         default: return cudaErrorInvalidValue;
     }
 }
+static cudaError_t slab_family(int family, const MatvecParams& p, int mb, int grid, int smem, cudaStream_t st) {
+    switch (family) {
+        case B200Q_FAM_Q4_K: return mv_slab_launch<B200Q_FAM_Q4_K>(p, mb, grid, smem, st);
+        case B200Q_FAM_Q6_K: return mv_slab_launch<B200Q_FAM_Q6_K>(p, mb, grid, smem, st);
+        case B200Q_FAM_Q8_0: return mv_slab_launch<B200Q_FAM_Q8_0>(p, mb, grid, smem, st);
+        case B200Q_FAM_G4: return mv_slab_launch<B200Q_FAM_G4>(p, mb, grid, smem, st);
+        default: return cudaErrorNotSupported;
+    }
+}
 static long long* g_trace = nullptr;
 static int g_trace_launch = 0;
 void set_matvec_trace(long long* p) { g_trace = p; g_trace_launch = 0; }
@@ -95,6 +104,38 @@ cudaError_t matvec_plan(const b200q_weight* w, int64_t M, MatvecPlan* plan, int 
     return cudaSuccess;
 }
 
+// Weights whose rows, dealt over the SMs, fit their shared memory whole (up to 28 MB): see matvec_slab.cuh
+struct SlabPlan {
+    int rows, slabs1, grid, xhat_bytes, smem_bytes;
+};
+static bool slab_plan(const b200q_weight* w, int64_t M, int pro, bool swiglu, SlabPlan* plan) {
+    const b200q_weight* w2 = dual_partner(w);
+    const int f = w->family;
+    if (f != B200Q_FAM_Q4_K && f != B200Q_FAM_Q6_K && f != B200Q_FAM_Q8_0 && f != B200Q_FAM_G4) return false;
+    if (M < 1 || M > 4 || pro == 2 || w->KC > 96 || (pro == 3 && (w2 || w->KC * M > MV_QUANT_RECORDS))) return false;
+    const int step = f == B200Q_FAM_G4 && w->gpc == 1 ? 16 : 8;   // a copy moves whole 16-byte pieces of every plane
+    int R = step;
+    auto slabs = [&](const b200q_weight* v) { return v ? (v->N + R - 1) / R : 0; };
+    while (R <= TILE_ROWS && slabs(w) + slabs(w2) > w->num_sms) R += step;
+    if (R > TILE_ROWS) return false;
+    if (swiglu) {   // whole tiles, as long as they cover the chip as well as smaller slabs do
+        if (w2 || w->T > w->num_sms || R < TILE_ROWS - 16) return false;
+        R = TILE_ROWS;
+    }
+    const int cb = (w2 && w2->chunk_bytes > w->chunk_bytes) ? w2->chunk_bytes : w->chunk_bytes;
+    const int64_t xhat = (w->KC * M * ACT_REC_BYTES + 127) & ~(int64_t)127, smem = 1024 + xhat + w->KC * R * (cb / TILE_ROWS) + ACT_REC_BYTES;
+    if (smem > 200 * 1024) return false;
+    plan->rows = R, plan->slabs1 = (int)slabs(w), plan->grid = (int)(slabs(w) + slabs(w2)), plan->xhat_bytes = (int)xhat, plan->smem_bytes = (int)smem;
+    if (plan->smem_bytes < 116 * 1024) plan->smem_bytes = 116 * 1024;   // > half an SM: see matvec_plan (4096 x 4096 Q4_K 5.7 us with what it needs, 4.6 so)
+    return true;
+}
+
+bool matvec_quantises(const b200q_weight* w, int64_t M) {
+    SlabPlan sp;
+    MatvecPlan mp;
+    return !w->pair && (slab_plan(w, M, 3, false, &sp) || matvec_plan(w, M, &mp, 3) == cudaSuccess);
+}
+
 size_t matvec_ws_bytes(const b200q_weight* w, int64_t M) {
     // counters (one per row tile, padded) + 2 partial slots per potential CTA
     size_t cnt = ((size_t)w->T * 4 + 255) & ~(size_t)255;
@@ -110,8 +151,11 @@ cudaError_t launch_matvec(const b200q_weight* w, const uint8_t* xq, int64_t M, v
     const b200q_weight* w2 = dual_partner(w);
     // a paired weight is launched together with its partner, by the plain / norm-prologue forms only; y holds N1 + N2 columns
     if (w2 && (ro || swiglu_xq_out || (fp && fp->mode != 1) || ldy < w->N + w2->N)) return cudaErrorInvalidValue;
-    cudaError_t e = matvec_plan(w, M, &plan, pro);
+    SlabPlan slab = {};
+    const bool whole = !ro && slab_plan(w, M, pro, swiglu_xq_out != nullptr, &slab);
+    cudaError_t e = whole ? cudaSuccess : matvec_plan(w, M, &plan, pro);
     if (e != cudaSuccess) return e;
+    if (whole) plan = MatvecPlan{}, plan.mb = M == 1 ? 1 : (M == 2 ? 2 : 4), plan.grid = slab.grid, plan.xhat_bytes = slab.xhat_bytes;
     MatvecParams p;
     p.w = w->data;
     p.xq = xq;
@@ -167,6 +211,14 @@ cudaError_t launch_matvec(const b200q_weight* w, const uint8_t* xq, int64_t M, v
     p.next_w = nullptr;
     p.next_C = p.next_KC = 0;
     p.next_chunk_bytes = p.next_G = p.next_pf = 0;
+    p.slab_rows = slab.rows;
+    p.slabs1 = slab.slabs1;
+    p.err = whole ? decode_error_dev() : nullptr;
+    if (whole) {
+        if (!w2) return slab_family(w->family, p, plan.mb, slab.grid, slab.smem_bytes, st);
+        if (w->family == B200Q_FAM_Q4_K && w2->family == B200Q_FAM_Q6_K) return mv_slab_launch_dual_q4k_q6k(p, plan.mb, slab.grid, slab.smem_bytes, st);
+        return cudaErrorInvalidValue;
+    }
     if (w->next && w->next->device == w->device && !pro) {
         // successor prefetch budget: what HBM can deliver during this launch's tail + the boundary (~6 us ~ 40 MB), well
         // inside the 126 MB L2.  B200Q_MV_NEXT_PF_MB overrides (0 disables).

@@ -66,6 +66,8 @@ struct MatvecParams {
     uint8_t* xq_out;
     int epi_F;      // rows of gate (= rows of up) = N / 2
     int epi_rows;   // record rows per k-chunk: M (plain) or n_slots (grouped)
+    int slab_rows, slabs1;   // matvec_slab.cuh: rows per CTA, CTAs of the first weight
+    int* err;                // device error word (b200q_decode_error)
     int plan32;     // (C + 1) * G < 2^32: the stream-K plan is computed with 32-bit divisions
     // dual-format launch (kernel template F2 != F; b200q_weight_set_pair): a second weight of another format whose output rows
     // directly follow the first one's (y2 = y + N1, N1 % 128 == 0) rides in the same stream-K grid -- tiles [0, T1) belong to w
@@ -85,6 +87,9 @@ struct MatvecParams {
 // per-format launcher, defined (explicitly specialised) in inst_<format>.cu so formats compile in parallel
 template <int FAMILY>
 cudaError_t mv_launch(const MatvecParams& p, int mb, int grid, int smem, cudaStream_t st);
+template <int FAMILY>
+cudaError_t mv_slab_launch(const MatvecParams& p, int mb, int grid, int smem, cudaStream_t st);   // cudaErrorNotSupported: a format without planes
+cudaError_t mv_slab_launch_dual_q4k_q6k(const MatvecParams& p, int mb, int grid, int smem, cudaStream_t st);
 // dual-format launcher (inst_q4k_q6k.cu): first weight Q4_K, second Q6_K
 cudaError_t mv_launch_dual_q4k_q6k(const MatvecParams& p, int mb, int grid, int smem, cudaStream_t st);
 

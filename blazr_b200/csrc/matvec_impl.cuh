@@ -282,6 +282,34 @@ __device__ __forceinline__ double i2d(int s) { return __hiloint2double(0x4330000
 __device__ __forceinline__ double i2d(int s) { return (double)s; }
 #endif
 
+// the terms of one unit (32 k of one row) for one activation row; b?: sums of the activations' halves
+template <class FF>
+__device__ __forceinline__ double unit_terms(const Unit& u, const uint4& xa, const uint4& xb, float dx, int bsA, int bsB, double a_) {
+    int sA = 0, sB = 0;
+    sA = __dp4a((int)u.v[0], (int)xa.x, sA); sA = __dp4a((int)u.v[1], (int)xa.y, sA);
+    sA = __dp4a((int)u.v[2], (int)xa.z, sA); sA = __dp4a((int)u.v[3], (int)xa.w, sA);
+    if constexpr (FF::NIB) {  // bytes hold 16 x q (unsigned): exact u8 x s8 dot, one arithmetic shift back
+        sB = dp4a_us(u.v[4], xb.x, sB); sB = dp4a_us(u.v[5], xb.y, sB);
+        sB = dp4a_us(u.v[6], xb.z, sB); sB = dp4a_us(u.v[7], xb.w, sB);
+        sB >>= 4;
+    } else {
+        sB = __dp4a((int)u.v[4], (int)xb.x, sB); sB = __dp4a((int)u.v[5], (int)xb.y, sB);
+        sB = __dp4a((int)u.v[6], (int)xb.z, sB); sB = __dp4a((int)u.v[7], (int)xb.w, sB);
+    }
+    sA -= u.off[0] * bsA;
+    sB -= u.off[1] * bsB;
+    if (FF::SUB == 32) {  // one scale per 32 weights
+        a_ = fma((double)__fmul_rn(u.a[0], dx), i2d(sA + sB), a_);
+        if (FF::HAS_MIN) a_ = fma(-(double)__fmul_rn(u.b[0], dx), i2d(bsA + bsB), a_);
+    } else {             // two 16-wide sub-blocks with their own scales
+        a_ = fma((double)__fmul_rn(u.a[0], dx), i2d(sA), a_);
+        if (FF::HAS_MIN) a_ = fma(-(double)__fmul_rn(u.b[0], dx), i2d(bsA), a_);
+        a_ = fma((double)__fmul_rn(u.a[1], dx), i2d(sB), a_);
+        if (FF::HAS_MIN) a_ = fma(-(double)__fmul_rn(u.b[1], dx), i2d(bsB), a_);
+    }
+    return a_;
+}
+
 // Per-CTA globaltimer trace and the "skip the math" debug flag cost 3-12 % in the consumer loop: they are
 // compiled in only with -DB200Q_MV_TRACE (make TRACE=1).
 #ifdef B200Q_MV_TRACE
@@ -333,15 +361,16 @@ enum { OUT_PLAIN = 0, OUT_REMOTE = 1 /* fused tensor-parallel exchange */, OUT_S
 // ---- OUT_SWIGLU: one finished 128-row tile (64 gate / 64 up rows interleaved, f32 in shared memory) -> 64 activations
 // silu(gate) * up -> two quantised 32-blocks of the next matvec's records.  Executed by the fix-up warp; arithmetic identical
 // to swiglu_quant_kernel (decode_ops.cu), so the records carry the same bits as the separate operator. ----
+__device__ __forceinline__ void swiglu_block_epilogue(const MatvecParams& p, const float* sy /*[TILE_ROWS]*/, int64_t tile_in_weight, int rec_row, int b, int lane) {
+    const int j = 32 * b + lane, w_ = j >> 2, g_ = j & 3;
+    const float gv = sy[8 * w_ + g_], uv = sy[8 * w_ + 4 + g_];
+    const float v = __fmul_rn(__fdiv_rn(gv, __fadd_rn(1.0f, det_expf(-gv))), uv);
+    const int64_t f = 64 * tile_in_weight + 32 * b;  // first ffn index of this block (F % 64 == 0: blocks are all-valid or absent)
+    if (f < p.epi_F) quant_block_to_record(v, p.xq_out + ((size_t)(f / CHUNK_K) * p.epi_rows + rec_row) * ACT_REC_BYTES, (int)((f % CHUNK_K) / 32), lane);
+}
 __device__ __forceinline__ void swiglu_tile_epilogue(const MatvecParams& p, const float* sy /*[TILE_ROWS]*/, int64_t tile_in_weight, int rec_row, int lane) {
 #pragma unroll
-    for (int b = 0; b < 2; b++) {
-        const int j = 32 * b + lane, w_ = j >> 2, g_ = j & 3;
-        const float gv = sy[8 * w_ + g_], uv = sy[8 * w_ + 4 + g_];
-        const float v = __fmul_rn(__fdiv_rn(gv, __fadd_rn(1.0f, det_expf(-gv))), uv);
-        const int64_t f = 64 * tile_in_weight + 32 * b;  // first ffn index of this block (F % 64 == 0: blocks are all-valid or absent)
-        if (f < p.epi_F) quant_block_to_record(v, p.xq_out + ((size_t)(f / CHUNK_K) * p.epi_rows + rec_row) * ACT_REC_BYTES, (int)((f % CHUNK_K) / 32), lane);
-    }
+    for (int b = 0; b < 2; b++) swiglu_block_epilogue(p, sy, tile_in_weight, rec_row, b, lane);
 }
 
 
@@ -743,32 +772,7 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_kernel(const MatvecParam
                     FF::template load_unit<true, FF::NIB>(wc, r, i, u, mt);
                 }
 #pragma unroll
-                for (int m = 0; m < MB; m++) {
-                    int sA = 0, sB = 0;
-                    sA = __dp4a((int)u.v[0], (int)xa[m].x, sA); sA = __dp4a((int)u.v[1], (int)xa[m].y, sA);
-                    sA = __dp4a((int)u.v[2], (int)xa[m].z, sA); sA = __dp4a((int)u.v[3], (int)xa[m].w, sA);
-                    if constexpr (FF::NIB) {  // bytes hold 16 x q (unsigned): exact u8 x s8 dot, one arithmetic shift back
-                        sB = dp4a_us(u.v[4], xb[m].x, sB); sB = dp4a_us(u.v[5], xb[m].y, sB);
-                        sB = dp4a_us(u.v[6], xb[m].z, sB); sB = dp4a_us(u.v[7], xb[m].w, sB);
-                        sB >>= 4;
-                    } else {
-                        sB = __dp4a((int)u.v[4], (int)xb[m].x, sB); sB = __dp4a((int)u.v[5], (int)xb[m].y, sB);
-                        sB = __dp4a((int)u.v[6], (int)xb[m].z, sB); sB = __dp4a((int)u.v[7], (int)xb[m].w, sB);
-                    }
-                    sA -= u.off[0] * bsA[m];
-                    sB -= u.off[1] * bsB[m];
-                    double a_ = acc[s4][m];
-                    if (FF::SUB == 32) {  // one scale per 32 weights
-                        a_ = fma((double)__fmul_rn(u.a[0], dx[m]), i2d(sA + sB), a_);
-                        if (FF::HAS_MIN) a_ = fma(-(double)__fmul_rn(u.b[0], dx[m]), i2d(bsA[m] + bsB[m]), a_);
-                    } else {             // two 16-wide sub-blocks with their own scales
-                        a_ = fma((double)__fmul_rn(u.a[0], dx[m]), i2d(sA), a_);
-                        if (FF::HAS_MIN) a_ = fma(-(double)__fmul_rn(u.b[0], dx[m]), i2d(bsA[m]), a_);
-                        a_ = fma((double)__fmul_rn(u.a[1], dx[m]), i2d(sB), a_);
-                        if (FF::HAS_MIN) a_ = fma(-(double)__fmul_rn(u.b[1], dx[m]), i2d(bsB[m]), a_);
-                    }
-                    acc[s4][m] = a_;
-                }
+                for (int m = 0; m < MB; m++) acc[s4][m] = unit_terms<FF>(u, xa[m], xb[m], dx[m], bsA[m], bsB[m], acc[s4][m]);
             }
         };
         if (!MV_DEBUG_SKIP(p) && !skip_chunk) {
