@@ -578,6 +578,28 @@ int32_t b200q_matmul(const b200q_weight* w, const void* x, int32_t x_dtype, int6
     return b200q_matmul_path(w, 0, x, x_dtype, M, ldx, y, y_dtype, ldy, workspace, workspace_bytes, stream);
 }
 
+size_t b200q_expand_bytes(const b200q_weight* w, int64_t M) { return w && M > 0 ? gemm_wide_panel_bytes(w, M) : 0; }
+int32_t b200q_gated_rows_ok(const b200q_weight* w, int64_t M) { return w && M > 0 && gemm_wide_gated_ok(w, M) ? 1 : 0; }
+int32_t b200q_expand(const b200q_weight* w, int64_t M, void* panel, int32_t beside, void* stream) {
+    if (!w || !panel || M <= 0 || ((uintptr_t)panel & 255) != 0) return fail(B200Q_ERR_INVALID_ARG, "expand: bad arguments");
+    if (!gemm_wide_panel_bytes(w, M)) return fail(B200Q_ERR_UNSUPPORTED, "expand: a step of %lld rows does not expand this weight", (long long)M);
+    CUDA_TRY(launch_expand(w, M, panel, beside != 0, (cudaStream_t)stream));
+    return B200Q_OK;
+}
+int32_t b200q_matmul_rows(const b200q_weight* w, const void* x16, int32_t x_ready, int64_t M, int64_t ldx, const void* panel, float* y, void* act16, int64_t ld, void* workspace,
+                          size_t workspace_bytes, void* stream) {
+    if (!w || !x16 || !workspace || M <= 0 || (!y) == (!act16)) return fail(B200Q_ERR_INVALID_ARG, "matmul_rows: bad arguments");
+    if (ldx < w->K || ld < (act16 ? w->N / 2 : w->N)) return fail(B200Q_ERR_INVALID_ARG, "matmul_rows: rows shorter than K / N");
+    if (((uintptr_t)workspace & 255) != 0 || ((uintptr_t)panel & 255) != 0) return fail(B200Q_ERR_WORKSPACE, "workspace and panel must be 256-byte aligned");
+    if (act16 && (!panel || !gemm_wide_gated_ok(w, M))) return fail(B200Q_ERR_UNSUPPORTED, "matmul_rows: gated rows need an expanded panel and whole products");
+    if (!panel) return b200q_matmul(w, x16, B200Q_F16, M, ldx, y, B200Q_F32, ld, workspace, workspace_bytes, stream);
+    const size_t wide = gemm_wide_ws_bytes(w, M);
+    if (wide == 0) return fail(B200Q_ERR_UNSUPPORTED, "matmul_rows: a step of %lld rows does not expand this weight", (long long)M);
+    if (workspace_bytes < wide) return fail(B200Q_ERR_WORKSPACE, "workspace too small: %zu < %zu", workspace_bytes, wide);
+    CUDA_TRY(launch_gemm_wide(w, x16, B200Q_F16, M, ldx, y, B200Q_F32, ld, (uint8_t*)workspace, (cudaStream_t)stream, panel, x_ready != 0, act16));
+    return B200Q_OK;
+}
+
 int32_t b200q_dequantize(const b200q_weight* w, void* out, int32_t dtype, void* stream) {
     if (!w || !out || dtype < 0 || dtype > 2) return fail(B200Q_ERR_INVALID_ARG, "bad dequantize arguments");
     CUDA_TRY(launch_dequantize(w, out, dtype, (cudaStream_t)stream));

@@ -691,6 +691,22 @@ __global__ void embed_kernel(const __half* __restrict__ table, const int64_t* __
     if (k < H) h[(size_t)m * H + k] = __half2float(table[(size_t)ids[m] * H + k]);
 }
 
+// the same, eight columns per thread (whole 16-byte pieces): 2048 rows of 2048 19.7 us, now 9.1
+__global__ void __launch_bounds__(256) embed8_kernel(const __half* __restrict__ table, const int64_t* __restrict__ ids, int H, float* __restrict__ h) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+    if (k >= H) return;
+    const uint4 u = *reinterpret_cast<const uint4*>(table + (size_t)ids[blockIdx.y] * H + k);
+    const uint32_t wd[4] = {u.x, u.y, u.z, u.w};
+    float4* o = reinterpret_cast<float4*>(h + (size_t)blockIdx.y * H + k);
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&wd[2 * j])), b = __half22float2(*reinterpret_cast<const __half2*>(&wd[2 * j + 1]));
+        o[j] = make_float4(a.x, a.y, b.x, b.y);
+    }
+}
+
 int* decode_error_dev() {
     void* p = nullptr;
     static std::atomic<int*> known[16];   // per device: asked for by every launch that can report a wait
@@ -946,6 +962,11 @@ int32_t b200q_moe_combine(const float* y, const float* gate_w, int64_t T, int64_
 
 int32_t b200q_embed(const void* table_f16, const int64_t* ids, int64_t H, int64_t M, float* h, void* stream) {
     if (!table_f16 || !ids || !h || H <= 0 || M <= 0) return B200Q_ERR_INVALID_ARG;
+    if (M > 1 && H % 8 == 0 && aligned16(table_f16) && aligned16(h)) {   // (one row: eight blocks of single columns start sooner)
+        const unsigned nt = H >= 2048 ? 256 : 128;
+        cudaError_t e8 = launch_pdl(embed8_kernel, dim3((unsigned)((H / 8 + nt - 1) / nt), (unsigned)M), dim3(nt), 0, (cudaStream_t)stream, (const __half*)table_f16, ids, (int)H, h);
+        return e8 == cudaSuccess ? B200Q_OK : B200Q_ERR_CUDA;
+    }
     cudaError_t e = launch_pdl(embed_kernel, dim3((unsigned)((H + 255) / 256), (unsigned)M), dim3(256), 0, (cudaStream_t)stream,
                                (const __half*)table_f16, ids, (int)H, h);
     return e == cudaSuccess ? B200Q_OK : B200Q_ERR_CUDA;

@@ -207,9 +207,9 @@ __global__ void __launch_bounds__(DQ16_THREADS) dequant_f16_kernel(const uint8_t
     pdl_wait();
 }
 template <int FAMILY>
-cudaError_t dequant_f16_launch(const b200q_weight* w, int tile0, int ntiles, __half* out, cudaStream_t st);
+cudaError_t dequant_f16_launch(const b200q_weight* w, int tile0, int ntiles, __half* out, bool beside, cudaStream_t st);   // beside: may start before the launch ahead ends
 template <class F>
-static cudaError_t launch_dequant_f16(const b200q_weight* w, int tile0, int ntiles, __half* out, cudaStream_t st) {
+static cudaError_t launch_dequant_f16(const b200q_weight* w, int tile0, int ntiles, __half* out, bool beside, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     const int64_t chunks = (int64_t)ntiles * w->KC, most = 2 * (int64_t)w->num_sms;   // two blocks are resident beside a GEMM CTA; more would queue behind blocks that wait
     cfg.gridDim = dim3((unsigned)(chunks < most ? chunks : most));
@@ -219,7 +219,7 @@ static cudaError_t launch_dequant_f16(const b200q_weight* w, int tile0, int ntil
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = beside ? 1 : 0;
     cudaError_t e = cudaLaunchKernelEx(&cfg, dequant_f16_kernel<F>, (const uint8_t*)w->data, w->KC, w->chunk_bytes, tile0, ntiles, out, w->K_pad, FmtMeta{w->gpc});
     count_launch();
     return e != cudaSuccess ? e : cudaGetLastError();

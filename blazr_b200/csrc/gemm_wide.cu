@@ -105,6 +105,31 @@ struct EpiOut {
     }
 };
 
+// act[m][f] = f16(silu(gate) * up) of an interleaved weight: rows 8 i + 0 .. 3 of a tile are gates, 8 i + 4 .. 7 their ups (b200q_gate_up_row), in lanes
+// four apart.  The gate's lane takes the first 16 tokens, the up's lane the others.  Same operations as swiglu_rows_kernel on the stored products, whose
+// 134 MB (2048 tokens, 2 x 8192) are neither written nor read again: product and activation 102 + 32 us, now 99.
+struct EpiGatedRows {
+    __half* act;
+    int64_t ld;
+    const float* bias;
+    int N, n0;
+    __device__ __forceinline__ void store(float (&v)[32], int n, int m, int m_end, int lane) const {
+        n += n0;
+        if (n >= N) return;      // (N % 128 == 0: the same for the whole warp)
+        const float b = bias ? bias[n] : 0.0f;
+        const bool up = (lane & 4) != 0;
+        const int m0 = m + (up ? 16 : 0);
+        __half* o = act + (int64_t)m0 * ld + (n >> 7) * 64 + ((n & 127) >> 3) * 4 + (n & 3);
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            const float lo = v[j] + b, hi = v[16 + j] + b, got = __shfl_xor_sync(0xffffffffu, up ? lo : hi, 4);
+            const float g = up ? got : lo, u = up ? hi : got;
+            const float a = __fmul_rn(__fdiv_rn(g, __fadd_rn(1.0f, det_expf(-g))), u);
+            if (m0 + j < m_end) o[(int64_t)j * ld] = __float2half_rn(fminf(fmaxf(a, -65504.0f), 65504.0f));
+        }
+    }
+};
+
 struct WidePlan {
     int bt;            // token rows per tile
     int per, panels;   // weight tiles of 256 rows per panel (the last one has the rest)
@@ -169,47 +194,70 @@ size_t gemm_wide_ws_bytes(const b200q_weight* w, int64_t M) {
     return wide_wins(w, M, p) ? p.bytes() : 0;
 }
 
-static cudaError_t dequant_f16_family(const b200q_weight* w, int tile0, int ntiles, __half* out, cudaStream_t st) {
+size_t gemm_wide_panel_bytes(const b200q_weight* w, int64_t M) { return gemm_wide_ws_bytes(w, M) ? wide_plan(w, M).buf_bytes : 0; }
+bool gemm_wide_gated_ok(const b200q_weight* w, int64_t M) { return w->N % TILE_ROWS == 0 && gemm_wide_ws_bytes(w, M) && wide_plan(w, M).parts == 1; }
+
+static cudaError_t dequant_f16_family(const b200q_weight* w, int tile0, int ntiles, __half* out, bool beside, cudaStream_t st) {
     switch (w->family) {
-        case B200Q_FAM_Q4_K: return dequant_f16_launch<B200Q_FAM_Q4_K>(w, tile0, ntiles, out, st);
-        case B200Q_FAM_Q6_K: return dequant_f16_launch<B200Q_FAM_Q6_K>(w, tile0, ntiles, out, st);
-        case B200Q_FAM_Q8_0: return dequant_f16_launch<B200Q_FAM_Q8_0>(w, tile0, ntiles, out, st);
-        case B200Q_FAM_Q5_K: return dequant_f16_launch<B200Q_FAM_Q5_K>(w, tile0, ntiles, out, st);
-        case B200Q_FAM_Q4_1: return dequant_f16_launch<B200Q_FAM_Q4_1>(w, tile0, ntiles, out, st);
-        case B200Q_FAM_Q5_1: return dequant_f16_launch<B200Q_FAM_Q5_1>(w, tile0, ntiles, out, st);
-        case B200Q_FAM_Q2_K: return dequant_f16_launch<B200Q_FAM_Q2_K>(w, tile0, ntiles, out, st);
-        case B200Q_FAM_Q3_K: return dequant_f16_launch<B200Q_FAM_Q3_K>(w, tile0, ntiles, out, st);
-        case B200Q_FAM_IQ4_XS: return dequant_f16_launch<B200Q_FAM_IQ4_XS>(w, tile0, ntiles, out, st);
-        case B200Q_FAM_TQ2_0: return dequant_f16_launch<B200Q_FAM_TQ2_0>(w, tile0, ntiles, out, st);
-        case B200Q_FAM_I8S: return dequant_f16_launch<B200Q_FAM_I8S>(w, tile0, ntiles, out, st);
-        case B200Q_FAM_G4: return dequant_f16_launch<B200Q_FAM_G4>(w, tile0, ntiles, out, st);
+        case B200Q_FAM_Q4_K: return dequant_f16_launch<B200Q_FAM_Q4_K>(w, tile0, ntiles, out, beside, st);
+        case B200Q_FAM_Q6_K: return dequant_f16_launch<B200Q_FAM_Q6_K>(w, tile0, ntiles, out, beside, st);
+        case B200Q_FAM_Q8_0: return dequant_f16_launch<B200Q_FAM_Q8_0>(w, tile0, ntiles, out, beside, st);
+        case B200Q_FAM_Q5_K: return dequant_f16_launch<B200Q_FAM_Q5_K>(w, tile0, ntiles, out, beside, st);
+        case B200Q_FAM_Q4_1: return dequant_f16_launch<B200Q_FAM_Q4_1>(w, tile0, ntiles, out, beside, st);
+        case B200Q_FAM_Q5_1: return dequant_f16_launch<B200Q_FAM_Q5_1>(w, tile0, ntiles, out, beside, st);
+        case B200Q_FAM_Q2_K: return dequant_f16_launch<B200Q_FAM_Q2_K>(w, tile0, ntiles, out, beside, st);
+        case B200Q_FAM_Q3_K: return dequant_f16_launch<B200Q_FAM_Q3_K>(w, tile0, ntiles, out, beside, st);
+        case B200Q_FAM_IQ4_XS: return dequant_f16_launch<B200Q_FAM_IQ4_XS>(w, tile0, ntiles, out, beside, st);
+        case B200Q_FAM_TQ2_0: return dequant_f16_launch<B200Q_FAM_TQ2_0>(w, tile0, ntiles, out, beside, st);
+        case B200Q_FAM_I8S: return dequant_f16_launch<B200Q_FAM_I8S>(w, tile0, ntiles, out, beside, st);
+        case B200Q_FAM_G4: return dequant_f16_launch<B200Q_FAM_G4>(w, tile0, ntiles, out, beside, st);
         default: return cudaErrorNotSupported;
     }
 }
 
-cudaError_t launch_gemm_wide(const b200q_weight* w, const void* x, int x_dtype, int64_t M, int64_t ldx, void* y, int y_dtype, int64_t ldy, uint8_t* ws, cudaStream_t st) {
+static int panel_tiles(const b200q_weight* w, const WidePlan& p, int nt0, int* nt) {   // weight tiles of 128 rows of the panel that starts at the pair nt0
+    const int left = (int)((w->T + 1) / 2) - nt0;
+    *nt = left < p.per ? left : p.per;
+    return (int)(w->T - 2 * nt0 < 2 * *nt ? w->T - 2 * nt0 : 2 * *nt);
+}
+
+cudaError_t launch_expand(const b200q_weight* w, int64_t M, void* panel, bool beside, cudaStream_t st) {
     const WidePlan p = wide_plan(w, M);
-    __half* xr = reinterpret_cast<__half*>(ws);
-    cudaError_t e = launch_stage_rows(x, x_dtype, M, w->K, ldx, w->perm, w->K_pad, xr, st);
+    int nt;
+    return dequant_f16_family(w, 0, panel_tiles(w, p, 0, &nt), reinterpret_cast<__half*>(panel), beside, st);
+}
+
+cudaError_t launch_gemm_wide(const b200q_weight* w, const void* x, int x_dtype, int64_t M, int64_t ldx, void* y, int y_dtype, int64_t ldy, uint8_t* ws, cudaStream_t st, const void* panel,
+                             bool x_ready, void* act) {
+    const WidePlan p = wide_plan(w, M);
+    // Rows that are read in place need the expansion to be there already: one launched here would start beside the operator that makes the rows, which may
+    // itself still wait for the product whose panel this one overwrites (staging waits for that operator first).
+    const bool direct = x_ready && panel && x_dtype == 1 && !w->perm && w->K == w->K_pad && ((uintptr_t)x & 15) == 0 && ldx % 8 == 0;
+    __half* staged = reinterpret_cast<__half*>(ws);
+    const __half* xr = direct ? reinterpret_cast<const __half*>(x) : staged;
+    const int64_t ldr = direct ? ldx : w->K_pad;
+    cudaError_t e = direct ? cudaSuccess : launch_stage_rows(x, x_dtype, M, w->K, ldx, w->perm, w->K_pad, staged, st);
     int nt0 = 0;
     for (int i = 0; i < p.panels && e == cudaSuccess; i++) {
-        const int left = (int)((w->T + 1) / 2) - nt0, nt = left < p.per ? left : p.per;
-        const int tile0 = 2 * nt0, ntiles = (int)(w->T - tile0 < 2 * nt ? w->T - tile0 : 2 * nt);
-        __half* buf = reinterpret_cast<__half*>(ws + p.x_bytes + (i & 1) * p.buf_bytes);
-        e = dequant_f16_family(w, tile0, ntiles, buf, st);
+        int nt;
+        const int ntiles = panel_tiles(w, p, nt0, &nt);
+        __half* made = reinterpret_cast<__half*>(ws + p.x_bytes + (i & 1) * p.buf_bytes);
+        const __half* buf = i == 0 && panel ? reinterpret_cast<const __half*>(panel) : made;
+        if (buf == made) e = dequant_f16_family(w, 2 * nt0, ntiles, made, true, st);
         if (e != cudaSuccess) break;
         tcpair::Args a{};
         a.M = (int)M, a.N = ntiles * TILE_ROWS, a.K = (int)w->K_pad, a.E = 1, a.bt = p.bt, a.err = decode_error_dev(), a.err_bit = B200Q_DECODE_ERR_GEMM_WAIT;
         a.parts = p.parts;
-        auto run = [&](const auto& epi) { return tcpair::launch(buf, a.N, w->K_pad, xr, w->K_pad, a, epi, st, true); };
+        auto run = [&](const auto& epi) { return tcpair::launch(buf, a.N, w->K_pad, xr, ldr, a, epi, st, true); };
         const int n0 = nt0 * 256;
         if (p.parts > 1) {
             float* part = reinterpret_cast<float*>(ws + p.x_bytes + p.buf_bytes);
-            e = tcpair::launch<true>(buf, a.N, w->K_pad, xr, w->K_pad, a, EpiOut<float>{part, w->N, nullptr, (int)w->N, 0}, st, true);
+            e = tcpair::launch<true>(buf, a.N, w->K_pad, xr, ldr, a, EpiOut<float>{part, w->N, nullptr, (int)w->N, 0}, st, true);
             count_launch();
             return e != cudaSuccess ? e : launch_splitk_reduce(part, p.parts, M, w, y, y_dtype, ldy, st);
         }
-        if (y_dtype == 0) e = run(EpiOut<float>{(float*)y, ldy, w->bias, (int)w->N, n0});
+        if (act) e = run(EpiGatedRows{(__half*)act, ldy, w->bias, (int)w->N, n0});
+        else if (y_dtype == 0) e = run(EpiOut<float>{(float*)y, ldy, w->bias, (int)w->N, n0});
         else if (y_dtype == 1) e = run(EpiOut<__half>{(__half*)y, ldy, w->bias, (int)w->N, n0});
         else e = run(EpiOut<__nv_bfloat16>{(__nv_bfloat16*)y, ldy, w->bias, (int)w->N, n0});
         count_launch();

@@ -20,8 +20,8 @@ cudaError_t gemm_launch<B200Q_FAM_ID>(const GemmParams& p, int grid, int smem, c
     return launch_gemm_t<B200Q_FMT>(p, grid, smem, st);
 }
 template <>
-cudaError_t dequant_f16_launch<B200Q_FAM_ID>(const b200q_weight* w, int tile0, int ntiles, __half* out, cudaStream_t st) {
-    return launch_dequant_f16<B200Q_FMT>(w, tile0, ntiles, out, st);
+cudaError_t dequant_f16_launch<B200Q_FAM_ID>(const b200q_weight* w, int tile0, int ntiles, __half* out, bool beside, cudaStream_t st) {
+    return launch_dequant_f16<B200Q_FMT>(w, tile0, ntiles, out, beside, st);
 }
 template <>
 cudaError_t dequant_launch<B200Q_FAM_ID>(const b200q_weight* w, void* out, int dtype, cudaStream_t st) {

@@ -87,7 +87,12 @@ int32_t set_error(int32_t code, const char* fmt, ...);  // api.cu: thread-local 
 // ---- gemm_wide.cu ----
 constexpr int64_t GEMM_WIDE_MIN_M = 512;   // ops.py: LARGE_STEP
 size_t gemm_wide_ws_bytes(const b200q_weight* w, int64_t M);   // 0: this M stays on the fused kernel
-cudaError_t launch_gemm_wide(const b200q_weight* w, const void* x, int x_dtype, int64_t M, int64_t ldx, void* y, int y_dtype, int64_t ldy, uint8_t* ws, cudaStream_t st);
+// panel: the first panel's expansion, made ahead (null: made here); x_ready: f16 rows without infinities, read in place; act: gated f16 rows instead of y
+cudaError_t launch_gemm_wide(const b200q_weight* w, const void* x, int x_dtype, int64_t M, int64_t ldx, void* y, int y_dtype, int64_t ldy, uint8_t* ws, cudaStream_t st,
+                             const void* panel = nullptr, bool x_ready = false, void* act = nullptr);
+size_t gemm_wide_panel_bytes(const b200q_weight* w, int64_t M);   // of the first panel; 0: this M stays on the fused kernel
+bool gemm_wide_gated_ok(const b200q_weight* w, int64_t M);
+cudaError_t launch_expand(const b200q_weight* w, int64_t M, void* panel, bool beside, cudaStream_t st);
 constexpr int B200Q_DECODE_ERR_GEMM_WAIT = 2;   // a bounded wait of the paired GEMM ran out: rows of its result are unwritten
 int* decode_error_dev();   // the device error word of b200q_decode_error (decode_ops.cu)
 

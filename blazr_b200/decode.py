@@ -738,14 +738,38 @@ class Decoder:
                      ws=torch.zeros(max(256, ws_bytes), dtype=torch.uint8, device=dev))
             b["xq1"] = torch.zeros(int(L.b200q_act_bytes(C.c_int64(H), C.c_int64(1))), dtype=torch.uint8, device=dev)
             b["h1"] = torch.empty((1, H), **f32)
+            # the expansions of a projection's weights are made one projection ahead, in turn in one of two buffers (they run beside the product before)
+            b["groups"] = [[(ln, (int(L.b200q_expand_bytes(ln.w.handle, C.c_int64(S))) + 255) & ~255 if rows is f16 else 0) for ln in lay[key]]
+                           for lay in self.layers for key in ("qkv", "o", "gu", "down")]
+            need = max((sum(n for _, n in g) for g in b["groups"]), default=0)
+            b["panels"] = [torch.empty(max(256, need), dtype=torch.uint8, device=dev) for _ in range(2)]
             b["logits1"] = torch.full((1, self.logits_local.shape[1]), float("-inf"), **f32)
             self._pf = b
         ids_d = torch.from_numpy(ids_h).to(dev)
         ops._check(L.b200q_embed(P(self.embed), P(ids_d), C.c_int64(H), C.c_int64(S), P(b["h"]), st))
         hin, hout = b["h"], b["h2"]
         delta = None
-        def gemm(lins, x, out):
-            for ln in lins:
+        def expand(i):
+            """expansion of projection group i, if there is one, right behind the product of group i - 1 and beside it where that has a panel of its own"""
+            if i < len(b["groups"]):
+                at, beside = b["panels"][i & 1].data_ptr(), i > 0 and b["groups"][i - 1][-1][1] > 0
+                for ln, n in b["groups"][i]:
+                    if n:
+                        ops._check(L.b200q_expand(ln.w.handle, C.c_int64(S), C.c_void_p(at), C.c_int32(1 if beside else 0), st))
+                    at += n
+
+        def gemm(i, x, out, ready=False, act=None):
+            """product of group i (its panels are there) and the expansion of the next one; ready: x was written by this library's operators"""
+            if rows is f16:
+                at = b["panels"][i & 1].data_ptr()
+                for ln, n in b["groups"][i]:
+                    to = act if act is not None else out
+                    ops._check(L.b200q_matmul_rows(ln.w.handle, P(x), C.c_int32(1 if ready else 0), C.c_int64(S), C.c_int64(x.stride(0)), C.c_void_p(at) if n else None,
+                                                   None if act is not None else C.c_void_p(out.data_ptr() + 4 * ln.col0), P(act) if act is not None else None,
+                                                   C.c_int64(to.stride(0)), P(b["ws"]), C.c_size_t(b["ws"].numel()), st))
+                    at += n
+                return expand(i + 1)
+            for ln, _ in b["groups"][i]:
                 ops._check(L.b200q_matmul(ln.w.handle, P(x), C.c_int32(ops._TORCH2DT[x.dtype]), C.c_int64(S), C.c_int64(x.stride(0)),
                                           C.c_void_p(out.data_ptr() + 4 * ln.col0), C.c_int32(ops.F32), C.c_int64(out.stride(0)), P(b["ws"]),
                                           C.c_size_t(b["ws"].numel()), st))
@@ -762,9 +786,11 @@ class Decoder:
                     b["xn"].copy_(x32.clamp_(-65504.0, 65504.0))
             hin, hout = hout, hin
 
-        for lay in self.layers:
+        normed = rows is f16 and H <= 8192      # the rows of b["xn"] come from add_rmsnorm_f16
+        expand(0)
+        for li, lay in enumerate(self.layers):
             norm(lay["attn_norm"])
-            gemm(lay["qkv"], b["xn"], b["qkv"])
+            gemm(4 * li, b["xn"], b["qkv"], normed)
             if self.paged:
                 ck, cv, table = lay["ck"], lay["cv"], self.block_table[seq]
             else:
@@ -774,18 +800,21 @@ class Decoder:
             o = Fnn.scaled_dot_product_attention(b["q16"].transpose(0, 1)[None], b["k16"].transpose(0, 1)[None], b["v16"].transpose(0, 1)[None], is_causal=True,
                                                  enable_gqa=(nh != nkv))
             attn = o[0].transpose(0, 1).reshape(S, self.qd)
-            gemm(lay["o"], attn, b["delta"])
+            gemm(4 * li + 1, attn, b["delta"])
             if self.world > 1:
                 torch.distributed.all_reduce(b["delta"], group=self.group)   # prefill-size message: NCCL over NVLink
             delta = b["delta"]
             norm(lay["mlp_norm"])
-            gemm(lay["gu"], b["xn"], b["gu"])
-            if rows is f16:
+            gated = rows is f16 and lay["swiglu_epi"] and len(lay["gu"]) == 1 and L.b200q_gated_rows_ok(lay["gu"][0].w.handle, C.c_int64(S))
+            gemm(4 * li + 2, b["xn"], b["gu"], normed, b["act"] if gated else None)
+            if gated:
+                pass                                     # the product's epilogue has written the activations
+            elif rows is f16:
                 ops._check(L.b200q_swiglu_f16(P(b["gu"]), C.c_int64(ff), C.c_int64(S), C.c_int32(1 if lay["swiglu_epi"] else 0), P(b["act"]), st))
             else:
                 sw = L.b200q_swiglu_f32_interleaved if lay["swiglu_epi"] else L.b200q_swiglu_f32
                 ops._check(sw(P(b["gu"]), C.c_int64(ff), C.c_int64(S), P(b["act"]), st))
-            gemm(lay["down"], b["act"], b["delta2"])
+            gemm(4 * li + 3, b["act"], b["delta2"], rows is f16)
             if self.world > 1:
                 torch.distributed.all_reduce(b["delta2"], group=self.group)
             delta = b["delta2"]

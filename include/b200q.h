@@ -298,6 +298,17 @@ int32_t b200q_swiglu_f32_interleaved(const float* gate_up, int64_t F, int64_t M,
  * All rows 16-byte aligned (B200Q_ERR_UNSUPPORTED otherwise). */
 int32_t b200q_add_rmsnorm_f16(const float* h_in, const float* delta, float* h_out, const float* w, float eps, int64_t H, int64_t M, void* x16, void* stream);
 int32_t b200q_swiglu_f16(const float* gate_up, int64_t F, int64_t M, int32_t interleaved, void* act16, void* stream);
+/* A prompt's products with the weight's expansion taken out of them, for callers that run several in a row: b200q_expand writes the f16 rows that a
+ * step of M rows reads first (b200q_expand_bytes of them; 0: this step does not expand, no call); beside: the launch before it in the stream is
+ * b200q_matmul_rows with another panel, and the two may run side by side (the panel of the product before that one may be overwritten: it has ended);
+ * otherwise the expansion starts when all before it has ended.  b200q_matmul_rows is b200q_matmul for f16 rows with the expansion in `panel` (or null).
+ * x_ready: the rows are finite, as the operators above write them, and are read where they lie.  act16 (with y null): w holds gate|up rows in the order of b200q_gate_up_row, act16[M][ld] = f16(silu(gate) * up) is written instead of the
+ * product (needs a panel and a step whose K is not cut: b200q_gated_rows_ok). */
+size_t b200q_expand_bytes(const b200q_weight* w, int64_t M);
+int32_t b200q_expand(const b200q_weight* w, int64_t M, void* panel, int32_t beside, void* stream);
+int32_t b200q_gated_rows_ok(const b200q_weight* w, int64_t M);
+int32_t b200q_matmul_rows(const b200q_weight* w, const void* x16, int32_t x_ready, int64_t M, int64_t ldx, const void* panel, float* y, void* act16, int64_t ld,
+                          void* workspace, size_t workspace_bytes, void* stream);
 int32_t b200q_rope_kv_prefill(const float* qkv, const float* rope_table, int32_t n_heads, int32_t n_kv_heads, int32_t head_dim, int64_t S, void* q16, void* k16,
                               void* v16, float* k_cache, float* v_cache, const int32_t* block_table, int32_t block_size, void* stream);
 /* RoPE (adjacent pairs; cos/sin from rope_table [max_ctx][hd/2][2] f32) on q and the new k, KV append at pos[m],

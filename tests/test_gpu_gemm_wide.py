@@ -153,3 +153,49 @@ def test_large_steps_leave_no_scratch_behind(client):
         client.quant_matmul(x[:M], w, out=y[:M])
     torch.cuda.synchronize()
     assert torch.cuda.memory_allocated() == held
+
+
+@pytest.mark.parametrize("fmt,N,K,M", [("Q4_K", 2048, 2048, 513), ("Q6_K", 512, 2048, 2048), ("Q6_K", 14336, 4096, 2048), ("Q8_0", 1000, 1024, 2048), ("AWQ", 6144, 4096, 1531)])
+def test_rows_with_the_expansion_made_ahead(client, fmt, N, K, M):
+    """b200q_expand + b200q_matmul_rows, rows staged or read in place (also with a longer stride), give the bits of b200q_matmul: whole weights, cut K, several panels."""
+    from blazr_b200 import ops
+    from blazr_b200 import synth
+    if fmt in synth.GGML:
+        w = client.weight_from_ggml(synth.GGML[fmt], synth.random_ggml(synth.GGML[fmt], N, K, seed=4), N, K)
+    else:
+        w = client.weight_from_decomposed(ops.DecomposedQuantTensor(*synth.random_awq(N, K, 128, seed=4), None, ops.DecomposedQuantMethod("awq", 128), (N, K)))
+    L, P = ops.lib(), lambda t: C.c_void_p(t.data_ptr())
+    n = int(L.b200q_expand_bytes(w.handle, C.c_int64(M)))
+    assert n > 0
+    x = torch.randn((M, K + 8), device="cuda", generator=torch.Generator(device="cuda").manual_seed(M)).half()
+    want = client.quant_matmul(x[:, :K].contiguous(), w, out_dtype=torch.float32)
+    panel, ws = torch.empty(n, dtype=torch.uint8, device="cuda"), torch.zeros(w.workspace_bytes(M), dtype=torch.uint8, device="cuda")
+    for rows in (x[:, :K].contiguous(), x[:, :K]):
+        for ready in (0, 1):
+            for beside in (0, 1):
+                panel.zero_()
+                got = torch.zeros((M, N), device="cuda")
+                ops._check(L.b200q_expand(w.handle, C.c_int64(M), P(panel), C.c_int32(beside), None))
+                ops._check(L.b200q_matmul_rows(w.handle, P(rows), C.c_int32(ready), C.c_int64(M), C.c_int64(rows.stride(0)), P(panel), P(got), None, C.c_int64(N), P(ws), C.c_size_t(ws.numel()), None))
+                assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.parametrize("F,K,M", [(8192, 2048, 1001), (5504, 2048, 777), (7168, 4096, 2047)])
+def test_gated_rows(client, F, K, M):
+    """The gated epilogue writes what the product and b200q_swiglu_f16 write, a step whose last tokens end inside a group of 16 included."""
+    from blazr_b200 import ops, synth
+    t, N = synth.GGML["Q4_K"], 2 * F
+    w = client.weight_from_ggml(t, synth.random_ggml(t, N, K, seed=F), N, K)
+    L, P = ops.lib(), lambda t_: C.c_void_p(t_.data_ptr())
+    while L.b200q_expand_bytes(w.handle, C.c_int64(M)) == 0:   # (from where on a step expands is a rule on measured times)
+        M += 256
+    n = int(L.b200q_expand_bytes(w.handle, C.c_int64(M)))
+    assert M < 8192 and L.b200q_gated_rows_ok(w.handle, C.c_int64(M)) == 1
+    x = (3.0 * torch.randn((M, K), device="cuda", generator=torch.Generator(device="cuda").manual_seed(F))).half()
+    gu = client.quant_matmul(x, w, out_dtype=torch.float32)
+    want, got = torch.zeros((M, F), dtype=torch.float16, device="cuda"), torch.zeros((M + 3, F), dtype=torch.float16, device="cuda")
+    ops._check(L.b200q_swiglu_f16(P(gu), C.c_int64(F), C.c_int64(M), C.c_int32(1), P(want), None))
+    panel, ws = torch.empty(n, dtype=torch.uint8, device="cuda"), torch.zeros(w.workspace_bytes(M), dtype=torch.uint8, device="cuda")
+    ops._check(L.b200q_expand(w.handle, C.c_int64(M), P(panel), C.c_int32(0), None))
+    ops._check(L.b200q_matmul_rows(w.handle, P(x), C.c_int32(1), C.c_int64(M), C.c_int64(K), P(panel), None, P(got), C.c_int64(F), P(ws), C.c_size_t(ws.numel()), None))
+    assert torch.equal(got[:M].view(torch.int16), want.view(torch.int16)) and not bool(got[M:].any())
