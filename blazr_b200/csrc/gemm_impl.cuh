@@ -124,6 +124,12 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t* r) {
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tc_ld8(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -143,12 +149,15 @@ __device__ __forceinline__ uint64_t make_b_desc(uint32_t saddr) {
 // exact __hsub2 and the scale/min applied with one __hfma2: a byte permutation, a subtraction and a multiply-add per pair of weights.
 // Pair order: word k yields (e0,e2) then (e1,e3) -- the activation staging kernel applies the same [0,2,1,3]
 // permutation inside every group of 4 k, so the contraction is unchanged.
-template <bool SIGNED>
+// RAWHI: the second half's bytes hold 16 x the integer (the matvec's loads); 1024 + 16 v is brought to v - off by one exact multiply-add.
+template <bool SIGNED, bool RAWHI = false>
 __device__ __forceinline__ void unit_to_f16(const Unit& u, uint32_t* out) {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-        const float offf = 1024.0f + (float)u.off[h] + (SIGNED ? 128.0f : 0.0f);
-        const __half2 off2 = __float2half2_rn(offf);         // integer <= 2047: exact in f16
+        const bool raw = RAWHI && h == 1;
+        const float offf = (raw ? 64.0f : 1024.0f) + (float)u.off[h] + (SIGNED ? 128.0f : 0.0f);
+        const __half2 off2 = __float2half2_rn(raw ? -offf : offf);         // integer <= 2047: exact in f16
+        const __half2 sixteenth = __float2half2_rn(0.0625f);
         const __half2 a2 = __float2half2_rn(u.a[h]);
         const __half2 nb2 = __float2half2_rn(-u.b[h]);
 #pragma unroll
@@ -156,8 +165,8 @@ __device__ __forceinline__ void unit_to_f16(const Unit& u, uint32_t* out) {
             const uint32_t wv = SIGNED ? (u.v[k] ^ 0x80808080u) : u.v[k];
             uint32_t p02 = __byte_perm(wv, 0x64646464u, 0x4240);      // bytes [e0, 0x64, e2, 0x64] = (1024 + e0, 1024 + e2): one PRMT
             uint32_t p13 = __byte_perm(wv, 0x64646464u, 0x4341);      // (1024 + e1, 1024 + e3)
-            __half2 x02 = __hsub2(*reinterpret_cast<__half2*>(&p02), off2);
-            __half2 x13 = __hsub2(*reinterpret_cast<__half2*>(&p13), off2);
+            __half2 x02 = raw ? __hfma2(*reinterpret_cast<__half2*>(&p02), sixteenth, off2) : __hsub2(*reinterpret_cast<__half2*>(&p02), off2);
+            __half2 x13 = raw ? __hfma2(*reinterpret_cast<__half2*>(&p13), sixteenth, off2) : __hsub2(*reinterpret_cast<__half2*>(&p13), off2);
             x02 = __hfma2(x02, a2, nb2);
             x13 = __hfma2(x13, a2, nb2);
             out[2 * k] = *reinterpret_cast<uint32_t*>(&x02);
@@ -207,7 +216,7 @@ __global__ void __launch_bounds__(DQ16_THREADS) dequant_f16_kernel(const uint8_t
     pdl_wait();
 }
 template <int FAMILY>
-cudaError_t dequant_f16_launch(const b200q_weight* w, int tile0, int ntiles, __half* out, bool beside, cudaStream_t st);   // beside: may start before the launch ahead ends
+cudaError_t dequant_f16_launch(const b200q_weight* w, int tile0, int ntiles, __half* out, bool beside, cudaStream_t st);   // beside: may start before the launch ahead ends   // beside: may start before the launch ahead ends
 template <class F>
 static cudaError_t launch_dequant_f16(const b200q_weight* w, int tile0, int ntiles, __half* out, bool beside, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
@@ -223,6 +232,34 @@ static cudaError_t launch_dequant_f16(const b200q_weight* w, int tile0, int ntil
     cudaError_t e = cudaLaunchKernelEx(&cfg, dequant_f16_kernel<F>, (const uint8_t*)w->data, w->KC, w->chunk_bytes, tile0, ntiles, out, w->K_pad, FmtMeta{w->gpc});
     count_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+// NC columns (token rows) of a work item's accumulator, from column cb on: lane = weight row n.  The type of y is asked for once per NC columns and the
+// rows are walked by pointer: with both asked and made for every element 32 columns took 2.4 us of a 17 us launch, 64 columns 4.6.
+template <int NC, typename T>
+__device__ __forceinline__ void store_cols(T* o, int64_t step, const uint32_t (&v)[NC], float bv, int nm) {
+#pragma unroll
+    for (int c = 0; c < NC; c++)
+        if (c < nm) {
+            const float f = __uint_as_float(v[c]) + bv;
+            if constexpr (sizeof(T) == 4) o[c * step] = f;
+            else if constexpr (std::is_same<T, __half>::value) o[c * step] = __float2half_rn(f);
+            else o[c * step] = __float2bfloat16_rn(f);
+        }
+}
+template <int NC>
+__device__ __forceinline__ void store_item(const GemmParams& p, const GemmItem& gi, uint32_t taddr, int r, float bv, int cb) {
+    uint32_t v[NC];
+    if constexpr (NC == 16) tc_ld16(taddr + cb, v);
+    else tc_ld8(taddr + cb, v);
+    tc_wait_ld();
+    const int64_t n = (int64_t)gi.t * TILE_ROWS + r, m = (int64_t)gi.mt * p.Mt + cb;
+    if (n >= p.N || m >= p.M) return;
+    const int nm = (int)(p.M - m < NC ? p.M - m : NC);
+    if (gi.nsp > 1) store_cols<NC>(gemm_partial_ptr(p, gi, r, n, m, cb), gi.tail >= 0 ? 1 : p.N, v, 0.0f, nm);
+    else if (p.y_dtype == 0) store_cols<NC>(reinterpret_cast<float*>(p.y) + m * p.ldy + n, p.ldy, v, bv, nm);
+    else if (p.y_dtype == 1) store_cols<NC>(reinterpret_cast<__half*>(p.y) + m * p.ldy + n, p.ldy, v, bv, nm);
+    else store_cols<NC>(reinterpret_cast<__nv_bfloat16*>(p.y) + m * p.ldy + n, p.ldy, v, bv, nm);
 }
 
 // EPI: four dedicated epilogue warps (one per TMEM lane quarter) and two accumulator buffers (Mt <= 128), so the
@@ -370,34 +407,17 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
         int acc = 0;
         uint32_t ph0 = 0, ph1 = 0;
         pdl_wait();  // y / partial may still be read by the preceding kernels
-        for (int tile = it0; tile < total_tiles; tile += its) {
+        for (int tile = it0; tile + its < total_tiles; tile += its) {   // (the last item: the dequant warps, which are done)
             const GemmItem gi = gemm_item(p, tile);
-            const int t = gi.t, mt = gi.mt;
             mbar_wait(&d_full[acc], acc ? ph1 : ph0);
             if (acc) ph1 ^= 1u; else ph0 ^= 1u;
             tc_fence_after();
-            const int64_t n = (int64_t)t * TILE_ROWS + r;
+            const int64_t n = (int64_t)gi.t * TILE_ROWS + r;
             const float bv = (p.bias && n < p.N) ? p.bias[n] : 0.0f;
-            for (int cb = 0; cb < p.Mt; cb += 16) {
-                uint32_t v[16];
-                tc_ld16(lane_base + GT_D_COL + acc * p.Mt + cb, v);
-                tc_wait_ld();
-                if (cb + 16 >= p.Mt) {  // last read of this buffer: hand it back to the MMA issuer before the stores
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&d_empty[acc]);
-                }
-                if (n < p.N) {
-#pragma unroll
-                    for (int c = 0; c < 16; c++) {
-                        const int64_t m = (int64_t)mt * p.Mt + cb + c;
-                        if (m < p.M) {
-                            if (gi.nsp > 1) *gemm_partial_ptr(p, gi, r, n, m, cb + c) = __uint_as_float(v[c]);
-                            else store_out(p.y, p.y_dtype, m * p.ldy + n, __uint_as_float(v[c]) + bv);
-                        }
-                    }
-                }
-            }
+            for (int cb = 0; cb < p.Mt; cb += 16) store_item<16>(p, gi, lane_base + GT_D_COL + acc * p.Mt, r, bv, cb);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&d_empty[acc]);   // the MMA issuer may have this buffer back
             acc ^= 1;
         }
     } else if (warp >= 4) {
@@ -408,23 +428,52 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
         const FmtMeta meta{p.gpc};
         int ws = 0, as = 0;
         uint32_t wph = 0, aph = 1, dph = 0;
+        // Formats with lane constants for their offsets (formats.cuh: unit_offsets) have them for all units of the thread in registers, and a chunk's units
+        // are all requested before the first is expanded: with the addresses made again for every unit and one unit after another the skinny
+        // launches (Q6_K, 32 rows) issued in 56 % of the cycles, waiting for shared memory and for their own arithmetic.
+        constexpr int NU = 8 / KG, NOFF = FmtNoff<F>::value;
+        uint32_t uo[NU][NOFF > 0 ? NOFF : 1];
+        if constexpr (NOFF > 0) {
+#pragma unroll
+            for (int j = 0; j < NU; j++) {
+                F::unit_offsets(r, KG * j + h, meta, uo[j]);
+#pragma unroll
+                for (int q = 0; q < NOFF; q++) uo[j][q] += smem_u32(wst);
+            }
+        }
         if (!EPI) pdl_wait();  // these warps also run the epilogue (stores to y / partial)
         for (int tile = it0; tile < total_tiles; tile += its) {
             const GemmItem gi = gemm_item(p, tile);
-            const int t = gi.t, mt = gi.mt;
+            const int t = gi.t;
             const int kc0 = gi.kc0, kc1 = gi.kc1;
             for (int kc = kc0; kc < kc1; kc++) {
                 mbar_wait(&full_w[ws], wph);
                 const uint8_t* wc = wst + (size_t)ws * p.w_stage_bytes;
                 mbar_wait(&a_empty[as], aph);  // the MMAs that read this TMEM slot two/three chunks ago are done
                 tc_fence_after();
+                if constexpr (NOFF > 0) {
+                    constexpr int AHEAD = NU < 2 ? NU : 2;
+                    Unit u[AHEAD];
+#pragma unroll
+                    for (int j0 = 0; j0 < NU; j0 += AHEAD) {
+#pragma unroll
+                        for (int j = 0; j < AHEAD; j++) F::template load_unit_at<0>((uint32_t)(ws * p.w_stage_bytes), uo[j0 + j], KG * (j0 + j) + h, u[j], meta);
+#pragma unroll
+                        for (int j = 0; j < AHEAD; j++) {
+                            uint32_t pk[16];
+                            unit_to_f16<F::SIGNED, F::NIB>(u[j], pk);
+                            tc_st16(lane_base + p.a_col + as * 128 + (KG * (j0 + j) + h) * 16, pk);
+                        }
+                    }
+                } else {
 #pragma unroll 1
-                for (int j = 0; j < 8 / KG; j++) {
-                    Unit u;
-                    F::template load_unit<true>(wc, r, KG * j + h, u, meta);
-                    uint32_t pk[16];
-                    unit_to_f16<F::SIGNED>(u, pk);
-                    tc_st16(lane_base + p.a_col + as * 128 + (KG * j + h) * 16, pk);
+                    for (int j = 0; j < NU; j++) {
+                        Unit u;
+                        F::template load_unit<true>(wc, r, KG * j + h, u, meta);
+                        uint32_t pk[16];
+                        unit_to_f16<F::SIGNED>(u, pk);
+                        tc_st16(lane_base + p.a_col + as * 128 + (KG * j + h) * 16, pk);
+                    }
                 }
                 tc_wait_st();
                 tc_fence_before();
@@ -435,7 +484,19 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
                 if (lane == 0) mbar_arrive(&empty_w[ws]);
                 if (++ws == p.nw) { ws = 0; wph ^= 1u; }
             }
-            if (EPI) continue;  // the dedicated epilogue warps drain the accumulator
+            if (EPI) {
+                if (tile + its < total_tiles) continue;  // the dedicated epilogue warps drain the accumulator
+                // the CTA's last item: these warps have nothing left to expand and share its columns, eight at a time
+                const int k = (tile - it0) / its, buf = k & 1;
+                pdl_wait();     // y / partial may still be read by the preceding kernels
+                mbar_wait(&d_full[buf], (k >> 1) & 1);
+                tc_fence_after();
+                const int64_t n = (int64_t)t * TILE_ROWS + r;
+                const float bv = (p.bias && n < p.N) ? p.bias[n] : 0.0f;
+                for (int cb = 8 * h; cb < p.Mt; cb += 8 * KG) store_item<8>(p, gi, lane_base + GT_D_COL + buf * p.Mt, r, bv, cb);
+                tc_fence_before();
+                continue;
+            }
             // ---- epilogue: accumulator rows = n, columns = m ----
             mbar_wait(&d_full[0], dph);
             dph ^= 1u;
@@ -443,21 +504,7 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
             const int64_t n = (int64_t)t * TILE_ROWS + r;
             const float bv = (p.bias && n < p.N) ? p.bias[n] : 0.0f;
             const int half_cols = p.Mt >> 1;
-            for (int cb = 0; cb < (h < 2 ? half_cols : 0); cb += 16) {
-                uint32_t v[16];
-                tc_ld16(lane_base + GT_D_COL + h * half_cols + cb, v);
-                tc_wait_ld();
-                if (n < p.N) {
-#pragma unroll
-                    for (int c = 0; c < 16; c++) {
-                        const int64_t m = (int64_t)mt * p.Mt + h * half_cols + cb + c;
-                        if (m < p.M) {
-                            if (gi.nsp > 1) *gemm_partial_ptr(p, gi, r, n, m, h * half_cols + cb + c) = __uint_as_float(v[c]);
-                            else store_out(p.y, p.y_dtype, m * p.ldy + n, __uint_as_float(v[c]) + bv);
-                        }
-                    }
-                }
-            }
+            for (int cb = 0; cb < (h < 2 ? half_cols : 0); cb += 16) store_item<16>(p, gi, lane_base + GT_D_COL, r, bv, h * half_cols + cb);
             tc_fence_before();
         }
     }

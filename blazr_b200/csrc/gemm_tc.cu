@@ -9,22 +9,48 @@ namespace b200q {
 // ------------------------------------------------------------------------------------------------
 // activation staging: x[M,K] (f32/f16/bf16) -> f16 UMMA tiles  xs[mt][ks][Mt rows x 128 B, SW128]
 // ------------------------------------------------------------------------------------------------
-__global__ void stage_x_kernel(const void* __restrict__ x, int x_dtype, int64_t M, int64_t K, int64_t ldx, const int32_t* __restrict__ perm,
-                               int Mt, int KS, uint8_t* __restrict__ xs) {
+// A thread makes one 16-byte piece of a tile row: eight columns, in the order 0 2 1 3 of every four (see unit_to_f16); eight threads a row's 64 columns.
+// vec: 16-byte loads (rows and row stride aligned, no gather).  One column per thread (2-byte stores) took 13 us more for 400 x 8192.
+__global__ void __launch_bounds__(256) stage_x_kernel(const void* __restrict__ x, int x_dtype, int64_t M, int64_t K, int64_t ldx, const int32_t* __restrict__ perm, int Mt, int KS,
+                                                      int64_t pieces, int vec, uint8_t* __restrict__ xs) {
     pdl_launch_dependents();
+    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= pieces) return;
+    const int64_t row = idx / (8 * KS), mt = row / Mt;      // row in padded space
+    const int piece = (int)(idx - row * (8 * KS)), ks = piece >> 3, c8 = piece & 7, mr = (int)(row - mt * Mt);
+    const int64_t k = (int64_t)piece * 8;
     pdl_wait();  // x is written by the operator just ahead in the stream
-    const int ks = blockIdx.x;
-    const int64_t m = (int64_t)blockIdx.y * blockDim.y + threadIdx.y;  // row in padded space
-    const int kk = threadIdx.x;                                          // 0..63
-    const int64_t mt = m / Mt;
-    const int mr = (int)(m % Mt);
-    // position kk of the sub-stage holds source element (kk & ~3) | {0,2,1,3}[kk & 3]  (see unit_to_f16)
-    const int64_t k = (int64_t)ks * 64 + ((kk & ~3) | (((kk & 1) << 1) | ((kk >> 1) & 1)));
-    float v = 0.0f;
-    if (m < M && k < K) v = load_in(x, x_dtype, m * ldx + (perm ? perm[k] : k));
-    v = fminf(fmaxf(v, -65504.0f), 65504.0f);
-    uint8_t* dst = xs + ((size_t)(mt * KS + ks) * Mt) * 128 + (size_t)mr * 128 + ((((kk >> 3) ^ (mr & 7)) << 4) + ((kk & 7) << 1));
-    *reinterpret_cast<__half*>(dst) = __float2half_rn(v);
+    float v[8];
+    if (row < M && vec && k + 8 <= K) {
+        if (x_dtype == 0) {
+            const float4* p = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + row * ldx + k);
+            const float4 a = p[0], b = p[1];
+            v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+        } else {
+            const uint4 u = *reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(x) + row * ldx + k);
+            const uint32_t wd[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (x_dtype == 1) {
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&wd[j]));
+                    v[2 * j] = f.x, v[2 * j + 1] = f.y;
+                } else {
+                    v[2 * j] = __uint_as_float(wd[j] << 16), v[2 * j + 1] = __uint_as_float(wd[j] & 0xFFFF0000u);
+                }
+            }
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = row < M && k + j < K ? load_in(x, x_dtype, row * ldx + (perm ? perm[k + j] : k + j)) : 0.0f;
+    }
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const int e = 4 * (j >> 1) + (j & 1);      // columns e, e + 2
+        const __half2 hh = __floats2half2_rn(fminf(fmaxf(v[e], -65504.0f), 65504.0f), fminf(fmaxf(v[e + 2], -65504.0f), 65504.0f));
+        o[j] = *reinterpret_cast<const uint32_t*>(&hh);
+    }
+    *reinterpret_cast<uint4*>(xs + ((size_t)(mt * KS + ks) * Mt + mr) * 128 + ((c8 ^ (mr & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 // split-K reduction: y[m,n] = sum_s partial[s][m][n] (+ bias), summed in split order (deterministic)
@@ -133,6 +159,7 @@ static int pick_splits(const b200q_weight* w, int MT, int64_t M) {
     }
     int best = 1;
     double best_eff = 0.0;
+    if (tiles * smax > sms) smax = (int)(sms / tiles) > 1 ? (int)(sms / tiles) : 1;   // in one wave: a second wave and the pass over the parts cost more than idle SMs (112 tiles, 5 rows: cut in five 18.2 us, whole 15.9)
     for (int s = 1; s <= smax; s++) {
         const int64_t items = tiles * s;
         const int64_t waves = (items + sms - 1) / sms;
@@ -197,9 +224,9 @@ cudaError_t launch_gemm_tc(const b200q_weight* w, const void* x, int x_dtype, in
     const int KS = (int)w->KC * 4;
     // 1. stage activations as f16 UMMA tiles
     {
-        dim3 block(64, 4);
-        dim3 grid((unsigned)KS, (unsigned)((int64_t)MT * Mt / 4));
-        cudaError_t e = launch_pdl_g(stage_x_kernel, grid, block, 0, st, x, x_dtype, M, w->K, ldx, w->perm, Mt, KS, ws);
+        const int64_t pieces = (int64_t)MT * Mt * KS * 8;
+        const int vec = !w->perm && ((uintptr_t)x & 15) == 0 && (ldx * (x_dtype == 0 ? 4 : 2)) % 16 == 0;
+        cudaError_t e = launch_pdl_g(stage_x_kernel, dim3((unsigned)((pieces + 255) / 256)), dim3(256), 0, st, x, x_dtype, M, w->K, ldx, w->perm, Mt, KS, pieces, vec, ws);
         if (e != cudaSuccess) return e;
     }
     // 2. GEMM
