@@ -59,6 +59,28 @@ def test_grouped_matvec_skips_negative_slots(client):
             assert_bit_exact(y[s:s + 1], oracle.matmul_q8(qi, a, b, sub, x), f"slot {s}")
 
 
+@pytest.mark.parametrize("fmt,N,K,n_slots,div", [("Q4_K", 200, 768, 300, 3), ("Q8_0", 128, 96, 741, 1), ("Q6_K", 384, 512, 97, 97), ("Q4_K", 128, 256, 148, 2)])
+def test_grouped_matvec_of_many_slots_a_block(client, fmt, N, K, n_slots, div):
+    """ranges that begin in one slot, end in another and hold whole slots between them, taken in another order than they lie in; slots skipped among them"""
+    E = 5
+    _, ws, _ = _bank(client, fmt, E, N, K, 250)
+    bank = ops.ExpertBank(ws)
+    rows = -(-n_slots // div)
+    rng = np.random.default_rng(n_slots)
+    sel_h = rng.integers(-1, E + 1, n_slots).astype(np.int32)             # -1 and E: not in the bank
+    x = synth.random_act(rows, K, seed=9)
+    y = bank.matmul_q8(torch.from_numpy(sel_h).cuda(), client.quantize_act(torch.from_numpy(x).cuda()), rows, div).cpu().numpy()
+    single = np.zeros((E, rows, N), dtype=np.float32)
+    for r in range(0, rows, 4):
+        xr = torch.from_numpy(x[r:r + 4]).cuda()
+        q = client.quantize_act(xr)
+        for e in range(E):
+            single[e, r:r + 4] = client.matmul_q8(q, xr.shape[0], ws[e]).cpu().numpy()
+    for s in range(n_slots):
+        want = single[sel_h[s], s // div] if 0 <= sel_h[s] < E else np.zeros(N, dtype=np.float32)
+        assert np.array_equal(want.view(np.uint32), y[s].view(np.uint32)), s
+
+
 def test_bank_set_swaps_an_expert(client):
     """set_expert_weights analogue (reference executor_cache.rs:283): the pointer table entry changes, nothing else"""
     E, N, K = 3, 256, 256
