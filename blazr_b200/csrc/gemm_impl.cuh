@@ -278,16 +278,18 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
     uint64_t* a_empty = a_full + GT_ASLOTS;
     uint64_t* d_full = a_empty + GT_ASLOTS;   // [2]
     uint64_t* d_empty = d_full + 2;           // [2]
-    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(d_empty + 2);
+    uint64_t* d_last = d_empty + 2;           // EPI: the last item's products, used once
+    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(d_last + 1);
     uint8_t* xst = smem + GT_HDR;
     uint8_t* wst = xst + (size_t)p.nx * p.x_stage_bytes;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0) {
-        for (int s = 0; s < p.nw; s++) { mbar_init(&full_w[s], 1); mbar_init(&empty_w[s], GT_DQ_WARPS); }
-        for (int s = 0; s < p.nx; s++) { mbar_init(&full_x[s], 1); mbar_init(&empty_x[s], 1); }
-        for (int s = 0; s < p.nslots; s++) { mbar_init(&a_full[s], GT_DQ_WARPS); mbar_init(&a_empty[s], 1); }
-        for (int s = 0; s < 2; s++) { mbar_init(&d_full[s], 1); mbar_init(&d_empty[s], 4); }
+    if (warp == 0) {   // (a lane each: one after another they held the first requests back)
+        if (lane < p.nw) mbar_init(&full_w[lane], 1), mbar_init(&empty_w[lane], GT_DQ_WARPS);
+        if (lane < p.nx) mbar_init(&full_x[lane], 1), mbar_init(&empty_x[lane], 1);
+        if (lane < p.nslots) mbar_init(&a_full[lane], GT_DQ_WARPS), mbar_init(&a_empty[lane], 1);
+        if (lane < 2) mbar_init(&d_full[lane], 1), mbar_init(&d_empty[lane], 4);
+        if (lane == 0) mbar_init(d_last, 1);
         fence_mbar_init();
         fence_proxy_async();
     }
@@ -395,7 +397,7 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
                     tc_commit(&a_empty[as]);
                     if (++as == p.nslots) { as = 0; aph ^= 1u; }
                 }
-                tc_commit(&d_full[acc]);
+                tc_commit(EPI && tile + its >= total_tiles ? d_last : &d_full[acc]);   // (nobody waits for the last phase of d_full)
                 if (EPI) acc ^= 1;
             }
         }
@@ -486,10 +488,12 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
             }
             if (EPI) {
                 if (tile + its < total_tiles) continue;  // the dedicated epilogue warps drain the accumulator
-                // the CTA's last item: these warps have nothing left to expand and share its columns, eight at a time
-                const int k = (tile - it0) / its, buf = k & 1;
+                // The CTA's last item: these warps have nothing left to expand and share its columns, eight at a time.  It has a barrier of its own: they
+                // follow no phase of d_full, and run up to three items ahead of the products where an item is one chunk, so that a parity of d_full
+                // could be that of an item two phases back.
+                const int buf = ((tile - it0) / its) & 1;
                 pdl_wait();     // y / partial may still be read by the preceding kernels
-                mbar_wait(&d_full[buf], (k >> 1) & 1);
+                mbar_wait(d_last, 0);
                 tc_fence_after();
                 const int64_t n = (int64_t)t * TILE_ROWS + r;
                 const float bv = (p.bias && n < p.N) ? p.bias[n] : 0.0f;

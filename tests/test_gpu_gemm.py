@@ -105,3 +105,26 @@ def test_gemm_tail_split_k_wave_quantisation(client, fmt, bias, monkeypatch):
     x = synth.random_act(M, K, seed=5)
     y = client.quant_matmul(torch.from_numpy(x).cuda(), c.w).cpu().numpy()
     assert rel_err(y, c.oracle_a(x)) < TOL
+
+
+# One chunk of K per item and three or more items per CTA (148 SMs: more than 37 888 rows): the warps that expand the weight, which also store the CTA's last
+# item, reach it up to three items ahead of the products.  A row's result does not depend on the rows beside it, so it is that of the same row in a
+# weight whose CTAs have one item each, bit for bit.
+@pytest.mark.parametrize("fmt,K", [("Q4_K", 256), ("Q6_K", 256), ("Q8_0", 96), ("Q8_0", 256), ("AWQ", 256), ("Q5_K", 256), ("Q4_1", 96), ("Q3_K", 256), ("IQ4_XS", 256), ("TQ2_0", 256)])
+@pytest.mark.parametrize("N", [37904, 57000, 130000])
+def test_gemm_many_items_of_one_chunk(client, fmt, K, N):
+    if fmt == "AWQ":
+        qw, sc, zr = synth.random_awq(N, K, 128, seed=N)
+        dq = ops.DecomposedQuantTensor(qw, sc, zr, None, ops.DecomposedQuantMethod("awq", 128), (N, K))
+        part = lambda a, b: client.weight_from_decomposed(dq, rows=(a, b))
+    else:
+        blk = synth.random_ggml(synth.GGML[fmt], N, K, seed=N)
+        part = lambda a, b: client.weight_from_ggml(synth.GGML[fmt], np.ascontiguousarray(blk[a:b]), b - a, K)
+    w, cuts = part(0, N), list(range(0, N, 18432)) + [N]                 # 144 tiles of 128 rows
+    small = [part(a, b) for a, b in zip(cuts, cuts[1:])]
+    for M in (5, 32, 64, 128):
+        xs = [torch.randn((M, K), device="cuda", generator=torch.Generator(device="cuda").manual_seed(i)) for i in range(4)]
+        ys = [client.quant_matmul(x, w) for x in xs]                       # back to back: each is launched beside the end of the one before
+        for x, y in zip(xs, ys):
+            want = torch.cat([client.quant_matmul(x, s) for s in small], 1)
+            assert torch.equal(y.view(torch.int32), want.view(torch.int32)), (fmt, N, M)
