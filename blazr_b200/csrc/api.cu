@@ -533,6 +533,17 @@ int32_t b200q_moe_matmul_q8_swiglu(const b200q_bank* b, const int32_t* sel_dev, 
     return B200Q_OK;
 }
 
+// M rows of x and of y share bytes (rows of one pitch that lie beside each other in it do not)
+static bool rows_overlap(const void* x, int x_dtype, int64_t ldx, int64_t K, const void* y, int y_dtype, int64_t ldy, int64_t N, int64_t M) {
+    const int64_t ex = x_dtype == B200Q_F32 ? 4 : 2, ey = y_dtype == B200Q_F32 ? 4 : 2;
+    const uintptr_t x0 = (uintptr_t)x, y0 = (uintptr_t)y, x1 = x0 + (size_t)((M - 1) * ldx + K) * ex, y1 = y0 + (size_t)((M - 1) * ldy + N) * ey;
+    if (x0 >= y1 || y0 >= x1) return false;
+    const int64_t pitch = ldx * ex;
+    if (ldy * ey != pitch) return true;
+    const int64_t d = (((int64_t)(y0 - x0)) % pitch + pitch) % pitch;      // where a row of y begins, from the beginning of a row of x
+    return d < K * ex || d + N * ey > pitch;
+}
+
 int32_t b200q_matmul_path(const b200q_weight* w, int32_t path, const void* x, int32_t x_dtype, int64_t M, int64_t ldx, void* y,
                           int32_t y_dtype, int64_t ldy, void* workspace, size_t workspace_bytes, void* stream) {
     if (!w || !x || !y || !workspace) return fail(B200Q_ERR_INVALID_ARG, "null argument");
@@ -547,7 +558,8 @@ int32_t b200q_matmul_path(const b200q_weight* w, int32_t path, const void* x, in
         size_t mv = align256(matvec_ws_bytes(w, M));
         size_t need = mv + align256(b200q_act_bytes(w->K, M));
         if (workspace_bytes < need) return fail(B200Q_ERR_WORKSPACE, "workspace too small: %zu < %zu", workspace_bytes, need);
-        if (matvec_quantises(w, M)) {   // one launch: every CTA quantises what its own chunks need
+        // one launch: every CTA quantises what its own chunks need -- of rows that no other CTA writes meanwhile
+        if (matvec_quantises(w, M) && !rows_overlap(x, x_dtype, ldx, w->K, y, y_dtype, ldy, w->N, M)) {
             FusedPrologue fp{3, nullptr, nullptr, nullptr, nullptr, 0.0f, nullptr, x, x_dtype, ldx};
             CUDA_TRY(launch_matvec(w, nullptr, M, y, y_dtype, ldy, (uint8_t*)workspace, st, &fp));
             return B200Q_OK;

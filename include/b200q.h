@@ -147,7 +147,7 @@ int32_t b200q_shard_range_blocks(int64_t total, int64_t granule, int64_t rank, i
 /* M >= 512: may include the expanded weight (2 bytes per element, up to 2 x 64 MB); the scratch of such a call holds nothing afterwards and need not be
  * zero-filled, and b200q_matmul also accepts that of the GEMM that expands its weight tile by tile */
 size_t b200q_workspace_bytes(const b200q_weight* w, int64_t M);
-/* Y[M,N] (ldy elements between rows) = X[M,K] (ldx) . dequant(W)^T (+bias).  x,y,workspace: device memory.
+/* Y[M,N] (ldy elements between rows) = X[M,K] (ldx) . dequant(W)^T (+bias).  x,y,workspace: device memory; y may lie over x.
  * M == 1..4 : dp4a stream-K matvec on int8-quantised activations (decode);
  * M >= 5    : tcgen05/TMEM dequant-GEMM on bf16 activations (batched decode and prefill). */
 int32_t b200q_matmul(const b200q_weight* w, const void* x, int32_t x_dtype, int64_t M, int64_t ldx, void* y, int32_t y_dtype,
@@ -302,7 +302,8 @@ int32_t b200q_swiglu_f16(const float* gate_up, int64_t F, int64_t M, int32_t int
  * step of M rows reads first (b200q_expand_bytes of them; 0: this step does not expand, no call); beside: the launch before it in the stream is
  * b200q_matmul_rows with another panel, and the two may run side by side (the panel of the product before that one may be overwritten: it has ended);
  * otherwise the expansion starts when all before it has ended.  b200q_matmul_rows is b200q_matmul for f16 rows with the expansion in `panel` (or null).
- * x_ready: the rows are finite, as the operators above write them, and are read where they lie.  act16 (with y null): w holds gate|up rows in the order of b200q_gate_up_row, act16[M][ld] = f16(silu(gate) * up) is written instead of the
+ * x_ready: the rows are finite, as the operators above write them, and are read where they lie (what is written must not overlap them).
+ * act16 (with y null): w holds gate|up rows in the order of b200q_gate_up_row, act16[M][ld] = f16(silu(gate) * up) is written instead of the
  * product (needs a panel and a step whose K is not cut: b200q_gated_rows_ok). */
 size_t b200q_expand_bytes(const b200q_weight* w, int64_t M);
 int32_t b200q_expand(const b200q_weight* w, int64_t M, void* panel, int32_t beside, void* stream);

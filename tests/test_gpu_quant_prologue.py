@@ -54,3 +54,41 @@ def test_act_order_and_bias(client, fmt):
     perm = None if c.perm is None else torch.from_numpy(np.ascontiguousarray(c.perm, dtype=np.int32)).cuda()
     for M in (1, 4):
         same(client, c.w, torch.randn((M, 1024), device="cuda"), M, 1024, perm)
+
+
+@pytest.mark.parametrize("N", [2048, 4096, 20480])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_results_over_the_rows_they_come_from(client, N, dtype):
+    """y on x itself, y a row further on in x's buffer, y of a wider type that begins inside x: what the call gives with an output of its own"""
+    from blazr_b200 import synth
+    K = min(N, 4096)
+    t = synth.GGML["Q4_K"]
+    w = client.weight_from_ggml(t, synth.random_ggml(t, N, K, seed=6), N, K)
+    g = torch.Generator(device="cuda").manual_seed(N)
+    for M in (1, 2, 3, 4):
+        for rep in range(20):
+            buf = torch.randn((M + 2, N), device="cuda", generator=g).to(dtype)
+            x = buf[:M, :K]
+            want = client.quant_matmul(x.clone(), w, out_dtype=dtype)
+            for row in (0, 1):
+                b = buf.clone()
+                got = client.quant_matmul(b[:M, :K], w, out=b[row:row + M])
+                assert torch.equal(got, want), (M, rep, row)
+            flat = torch.zeros(2 * M * N + 64, device="cuda")            # f32
+            src = flat.view(dtype)[:M * K].view(M, K)
+            src.copy_(x)
+            wide = client.quant_matmul(x.clone(), w, out_dtype=torch.float32)
+            assert torch.equal(client.quant_matmul(src, w, out=flat[32:32 + M * N].view(M, N)), wide)
+
+
+def test_rows_side_by_side_in_one_buffer(client):
+    """x and y as columns of one buffer share no bytes: one launch, as ever, and the same bits"""
+    from blazr_b200 import ops, synth
+    t = synth.GGML["Q6_K"]
+    w = client.weight_from_ggml(t, synth.random_ggml(t, 1024, 2048, seed=7), 1024, 2048)
+    for first in (0, 1024):
+        buf = torch.randn((4, 3072), device="cuda")
+        x, y = buf[:, first:first + 2048], buf[:, 2048 if first == 0 else 0:][:, :1024]
+        want = client.quant_matmul(x.clone(), w)
+        n0 = ops.launch_count()
+        assert torch.equal(client.quant_matmul(x, w, out=y), want) and ops.launch_count() - n0 == 1
