@@ -142,7 +142,9 @@ static void tail_plan(const b200q_weight* w, int MT, int64_t M, int grid, int* f
 
 // split-K factor: the work items (tiles x splits) should fill whole waves of the SMs.  Wide-M launches only split
 // when there are fewer tiles than SMs; skinny launches (one M tile, HBM-bound) pick the split with the least wave
-// quantisation loss, since a 112-tile weight on 148 SMs otherwise idles a quarter of the machine.
+// quantisation loss, since a 112-tile weight on 148 SMs otherwise idles a quarter of the machine.  Cutting only where one wave covers the parts
+// would be faster for 14336 x 4096 (Q8_0, 5 rows: cut in five 17.2 us, whole 13.9) and slower for 10240 x 8192 (cut in seven 21.6, whole 22.1; Q4_K 19.9 and
+// 23.2), but it leaves one accumulator, which truncates, with all of K: error against 64 bits 1.0e-6 and 1.4e-6 cut, 4.9e-6 and 9.6e-6 whole.
 static int pick_splits(const b200q_weight* w, int MT, int64_t M) {
     const int64_t tiles = w->T * MT;
     const int sms = w->num_sms;
@@ -159,7 +161,6 @@ static int pick_splits(const b200q_weight* w, int MT, int64_t M) {
     }
     int best = 1;
     double best_eff = 0.0;
-    if (tiles * smax > sms) smax = (int)(sms / tiles) > 1 ? (int)(sms / tiles) : 1;   // in one wave: a second wave and the pass over the parts cost more than idle SMs (112 tiles, 5 rows: cut in five 18.2 us, whole 15.9)
     for (int s = 1; s <= smax; s++) {
         const int64_t items = tiles * s;
         const int64_t waves = (items + sms - 1) / sms;

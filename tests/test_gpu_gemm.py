@@ -128,3 +128,18 @@ def test_gemm_many_items_of_one_chunk(client, fmt, K, N):
         for x, y in zip(xs, ys):
             want = torch.cat([client.quant_matmul(x, s) for s in small], 1)
             assert torch.equal(y.view(torch.int32), want.view(torch.int32)), (fmt, N, M)
+
+
+@pytest.mark.parametrize("N,K,M,parts", [(14336, 4096, 5, 5), (14336, 4096, 16, 5), (28672, 4096, 16, 3), (10240, 8192, 5, 7), (10240, 8192, 16, 5), (10240, 8192, 128, 3), (4096, 4096, 32, 4)])
+def test_skinny_products_are_cut_along_k(client, N, K, M, parts):
+    """Weights of one, 65504 in the first chunk of K and 1 / 64 in the others.  Beside the large sum (2^24: its unit is 1) the 16 products that a tensor-core
+    step adds (1 / 4) are lost; the parts of K that do not hold the first chunk arrive whole, 4 for each of their chunks."""
+    blk = np.zeros((N, K // 32, 34), np.uint8)
+    blk[:, :, :2] = np.frombuffer(np.float16(1.0).tobytes(), np.uint8)
+    blk[:, :, 2:] = 1
+    w = client.weight_from_ggml(8, blk.reshape(N, -1), N, K)
+    x = torch.full((M, K), 2.0 ** -6, device="cuda")
+    x[:, :256] = 65504.0
+    more = client.quant_matmul(x, w).double() - 256 * 65504.0
+    chunks = K // 256
+    assert more.min().item() >= 4 * (chunks - -(-chunks // parts)) and more.max().item() <= 4 * (chunks - 1)
