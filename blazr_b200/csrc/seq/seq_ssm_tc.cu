@@ -400,16 +400,6 @@ __device__ __noinline__ void recur_head(const SsmArgs& a, int row0, int len, int
     }
 }
 
-// x / (1 + exp(-x)) by a reciprocal and two corrections; below -85 the result is x 1e-37 instead of something smaller
-__device__ __forceinline__ float silu_near(float x) {
-    const float d = fminf(1.f + expf(-x), 1e37f);
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    r = fmaf(fmaf(-d, r, 1.f), r, r);
-    const float y = x * r;
-    return fabsf(x) < 1e30f ? fmaf(fmaf(-d, y, x), r, y) : y;   // (no residue of an infinity)
-}
-
 // 2^a and 2^b for arguments up to 0 (what lies above is not used): to the nearest whole number by the addition of 1.5 2^23, then 1 + f q(f) with a
 // polynomial of degree 5 (fitted by iterated weighted least squares on |f| <= 1/2: 2e-9 of the result), at half the instructions of two expf calls and
 // closer to 64 bits than ex2.approx, whose errors alone made the outputs' 1.2e-7 to 1.4e-7
@@ -573,8 +563,8 @@ __global__ void __launch_bounds__(THREADS_SSM, 1) ssm_tc_out_kernel(const __grid
                     const int r = r0 + 32 * i;
                     if (r < len) {
                         const float4 o = *reinterpret_cast<const float4*>(&Y[r * YLD + c]);
-                        *reinterpret_cast<float4*>(ob + (int64_t)r * inner) = make_float4(fmaf(Dh, x[i].x, o.x) * silu_near(z[i].x), fmaf(Dh, x[i].y, o.y) * silu_near(z[i].y),
-                                                                                          fmaf(Dh, x[i].z, o.z) * silu_near(z[i].z), fmaf(Dh, x[i].w, o.w) * silu_near(z[i].w));
+                        *reinterpret_cast<float4*>(ob + (int64_t)r * inner) = make_float4(fmaf(Dh, x[i].x, o.x) * siluf_acc(z[i].x), fmaf(Dh, x[i].y, o.y) * siluf_acc(z[i].y),
+                                                                                          fmaf(Dh, x[i].z, o.z) * siluf_acc(z[i].z), fmaf(Dh, x[i].w, o.w) * siluf_acc(z[i].w));
                     }
                 }
             }

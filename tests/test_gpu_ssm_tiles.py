@@ -18,8 +18,8 @@ def ops():
     return seqops
 
 
-def scan(ops, lens, H, V, N, G, speed, plant=None):
-    """(outputs, states) of the kernel and of the recurrence in float64; plant(xbc, A_log, Dp) changes the inputs first"""
+def scan(ops, lens, H, V, N, G, speed, plant=None, gates=None):
+    """(outputs, states) of the kernel and of the recurrence in float64; plant(xbc, A_log, Dp) and gates(proj) change the inputs first"""
     from blazr_b200.batch import StepEntry, build_step
     g = torch.Generator(device=DEV)
     g.manual_seed(H * V + N)
@@ -34,6 +34,8 @@ def scan(ops, lens, H, V, N, G, speed, plant=None):
     dt0 = 2 * inner + 2 * G * N
     if plant is not None:
         plant(xbc, A_log, Dp)
+    if gates is not None:
+        gates(proj)
     state = rnd(B, H, N, V)
     ref_state, ref = state.double().clone(), torch.empty(T, inner, dtype=torch.float64, device=DEV)
     x = xbc[:, :inner].double().reshape(T, H, V)
@@ -100,3 +102,33 @@ def test_decays_that_forget_at_once(ops):
     for got, want in scan(ops, [300, 40], 4, 64, 64, 2, 0.0, plant):
         assert bool(torch.isfinite(got).all())
         assert (got.double() - want).abs().max().item() / want.abs().max().item() < 3e-6
+
+
+@pytest.mark.parametrize("lens", [[31], [32], [128], [300]])
+def test_gates_of_every_size(ops, lens):
+    """Outputs that are x silu(z) alone (no states, D 1, x 1), z over all of f32: the recurrence (31 tokens) and the tiles give the same value for the same gate.
+    Bound: z / (1 + exp(-z)) with an exponential, a sum and a quotient in f32, 2 + 1/2 + 1/2 units of 2^-23; what lies below f32's normal numbers may be 0."""
+    H, V = 4, 64
+    z = torch.cat([torch.linspace(-104, 104, 4001), torch.tensor([0.0, -0.0, 1e-30, -1e-30, 1e30, -1e30, 3e38, -3e38, float("inf"), -float("inf"), float("nan")]), -torch.logspace(0, 38.4, 900),
+                   torch.logspace(-38, 38, 900)]).to(DEV)
+    seen = torch.empty_like(z)
+    per = sum(lens) * H * V
+    for at in range(0, z.numel(), per):
+        part = torch.zeros(per, device=DEV)
+        n = min(per, z.numel() - at)
+        part[:n] = z[at:at + n]
+
+        def plant(xbc, A_log, Dp):
+            xbc[:, :H * V], xbc[:, H * V:] = 1.0, 0.0
+            Dp.fill_(1.0)
+
+        def gates(proj):
+            proj[:, :H * V] = part.view(sum(lens), H * V)
+        (out, _), _ = scan(ops, lens, H, V, 64, 2, 0.0, plant, gates)
+        seen[at:at + n] = out.reshape(-1)[:n]
+    want = z.double() / (1 + torch.exp(-z.double()))
+    wild = z.isnan() | (z == -float("inf"))                       # -inf / inf, as the quotient has it
+    assert torch.equal(seen.isnan(), wild)
+    tame = ~wild & want.isfinite()
+    assert torch.equal(seen[~wild & ~tame], want[~wild & ~tame].float())
+    assert ((seen.double() - want).abs()[tame] <= 3.0 * 2.0 ** -23 * want.abs()[tame] + 2.0 ** -126 * 128).all()
