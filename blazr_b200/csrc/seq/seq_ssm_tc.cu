@@ -400,13 +400,18 @@ __device__ __noinline__ void recur_head(const SsmArgs& a, int row0, int len, int
     }
 }
 
-// 2^a and 2^b for arguments up to 0 (what lies above is not used): to the nearest whole number by the addition of 1.5 2^23, then 1 + f q(f) with a
+__device__ __forceinline__ float max_nan(float a, float b) {   // NaN if either is
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+// 2^a and 2^b for arguments up to 0, NaN for NaN (what lies above is not used): to the nearest whole number by the addition of 1.5 2^23, then 1 + f q(f) with a
 // polynomial of degree 5 (fitted by iterated weighted least squares on |f| <= 1/2: 2e-9 of the result), at half the instructions of two expf calls and
 // closer to 64 bits than ex2.approx, whose errors alone made the outputs' 1.2e-7 to 1.4e-7
 __device__ __forceinline__ uint64_t exp2_pair(uint64_t u) {
     float a, b;
     upk(u, a, b);
-    u = pk(fmaxf(a, -127.f), fmaxf(b, -127.f));
+    u = pk(max_nan(a, -127.f), max_nan(b, -127.f));
     constexpr float MAGIC = 12582912.f;
     const uint64_t j = add2(u, pk(MAGIC, MAGIC)), f = fma2(add2(j, pk(-MAGIC, -MAGIC)), pk(-1.f, -1.f), u);
     uint64_t q = pk(0x1.41fbbcp-13f, 0x1.41fbbcp-13f);

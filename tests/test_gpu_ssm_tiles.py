@@ -132,3 +132,14 @@ def test_gates_of_every_size(ops, lens):
     tame = ~wild & want.isfinite()
     assert torch.equal(seen[~wild & ~tame], want[~wild & ~tame].float())
     assert ((seen.double() - want).abs()[tame] <= 3.0 * 2.0 ** -23 * want.abs()[tame] + 2.0 ** -126 * 128).all()
+
+
+@pytest.mark.parametrize("lens", [[20], [20, 44], [32], [40], [129]])
+def test_a_rate_that_is_not_a_number(ops, lens):
+    """A head whose rate is NaN has NaN outputs and states from its first token on, as the recurrence has it; the other heads are what they are."""
+    def plant(xbc, A_log, Dp):
+        A_log[1] = float("nan")
+    for got, want in scan(ops, lens, 4, 64, 64, 2, 0.0, plant):
+        fine = want.isfinite()
+        assert torch.equal(got.isfinite(), fine) and bool((~fine).any())
+        assert (got.double() - want).abs()[fine].max().item() / want[fine].abs().max().item() < 3e-6
