@@ -214,12 +214,7 @@ cudaError_t launch_matvec(const b200q_weight* w, const uint8_t* xq, int64_t M, v
     p.slab_rows = slab.rows;
     p.slabs1 = slab.slabs1;
     p.err = whole ? decode_error_dev() : nullptr;
-    if (whole) {
-        if (!w2) return slab_family(w->family, p, plan.mb, slab.grid, slab.smem_bytes, st);
-        if (w->family == B200Q_FAM_Q4_K && w2->family == B200Q_FAM_Q6_K) return mv_slab_launch_dual_q4k_q6k(p, plan.mb, slab.grid, slab.smem_bytes, st);
-        return cudaErrorInvalidValue;
-    }
-    if (w->next && w->next->device == w->device && !pro) {
+    if (w->next && !w2 && w->next->device == w->device && (pro == 0 || pro == 3)) {
         // successor prefetch budget: what HBM can deliver during this launch's tail + the boundary (~6 us ~ 40 MB), well
         // inside the 126 MB L2.  B200Q_MV_NEXT_PF_MB overrides (0 disables).
         static const double pf_mb = [] { const char* e = getenv("B200Q_MV_NEXT_PF_MB"); return e ? atof(e) : 32.0; }();
@@ -236,6 +231,11 @@ cudaError_t launch_matvec(const b200q_weight* w, const uint8_t* xq, int64_t M, v
             }
         }
     }
+    if (whole) {
+        if (!w2) return slab_family(w->family, p, plan.mb, slab.grid, slab.smem_bytes, st);
+        if (w->family == B200Q_FAM_Q4_K && w2->family == B200Q_FAM_Q6_K) return mv_slab_launch_dual_q4k_q6k(p, plan.mb, slab.grid, slab.smem_bytes, st);
+        return cudaErrorInvalidValue;
+    }
     {
         // L2 prefetch budget: at most ~64 MB per launch so a huge weight (lm_head) cannot thrash the 126 MB L2
         int64_t per_cta = (64ll << 20) / ((int64_t)plan.grid * p.chunk_bytes);
@@ -245,7 +245,6 @@ cudaError_t launch_matvec(const b200q_weight* w, const uint8_t* xq, int64_t M, v
     }
     if (const char* e = getenv("B200Q_MV_DEBUG")) p.debug_flags = atoi(e);
     if (w2) {
-        p.next_w = nullptr; p.next_pf = 0;
         if (w->family == B200Q_FAM_Q4_K && w2->family == B200Q_FAM_Q6_K) return mv_launch_dual_q4k_q6k(p, plan.mb, plan.grid, plan.smem_bytes, st);
         return cudaErrorInvalidValue;
     }

@@ -103,8 +103,9 @@ __device__ __forceinline__ void slab_math(uint32_t w_sa, int stride, int R, int 
     }
 }
 
-// OUT_SWIGLU: gate|up rows interleaved per tile, a CTA has a whole tile (R = 128) and quantises its 64 activations
-template <class F, int MB, int PRO, int OUT, class F2 = F>
+// OUT_SWIGLU: gate|up rows interleaved per tile, a CTA has a whole tile (R = 128) and quantises its 64 activations.
+// NEXT: the launch has a successor hint (a form of its own: as a branch it cost every launch 0.05 us)
+template <class F, int MB, int PRO, int OUT, class F2 = F, bool NEXT = false>
 __global__ void __launch_bounds__(SLAB_THREADS, 1) matvec_slab_kernel(const MatvecParams p) {
     constexpr bool DUAL = !std::is_same<F, F2>::value;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -125,6 +126,8 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) matvec_slab_kernel(const Matv
     // the weights are static: requested before anything is waited for
     if (second) slab_request<F2>(p.w2, KC, cb, row0, rows, R, gpc, slab, stride, wbar, warp, lane);
     else slab_request<F>(p.w, KC, cb, row0, rows, R, gpc, slab, stride, wbar, warp, lane);
+    if constexpr (NEXT)
+        if (tid == SLAB_THREADS - 1) prefetch_next(p, g, gridDim.x);
     if (PRO == PRO_NONE && tid == 0) {
         mbar_init(xbar, 1);
         fence_mbar_init();
@@ -195,13 +198,15 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) matvec_slab_kernel(const Matv
     }
 }
 
-template <class F, int MB, int PRO, int OUT = OUT_PLAIN, class F2 = F>
+template <class F, int MB, int PRO, int OUT = OUT_PLAIN, class F2 = F, bool NEXT = false>
 static cudaError_t slab_launch_t(const MatvecParams& p, int grid, int smem, cudaStream_t st) {
+    if constexpr (!NEXT && PRO != PRO_FUSED && std::is_same<F, F2>::value)
+        if (p.next_pf > 0) return slab_launch_t<F, MB, PRO, OUT, F2, true>(p, grid, smem, st);
     static std::atomic<bool> configured[16];   // per device; racing first calls both set the attribute (idempotent): re-entrant
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 16 || !configured[dev].load(std::memory_order_acquire)) {
-        cudaError_t e = cudaFuncSetAttribute(matvec_slab_kernel<F, MB, PRO, OUT, F2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
+        cudaError_t e = cudaFuncSetAttribute(matvec_slab_kernel<F, MB, PRO, OUT, F2, NEXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
         if (e != cudaSuccess) return e;
         if (dev < 16) configured[dev].store(true, std::memory_order_release);
     }
@@ -215,7 +220,7 @@ static cudaError_t slab_launch_t(const MatvecParams& p, int grid, int smem, cuda
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaError_t le = cudaLaunchKernelEx(&cfg, matvec_slab_kernel<F, MB, PRO, OUT, F2>, p);
+    cudaError_t le = cudaLaunchKernelEx(&cfg, matvec_slab_kernel<F, MB, PRO, OUT, F2, NEXT>, p);
     if (le != cudaSuccess) return le;
     count_launch();
     return cudaGetLastError();

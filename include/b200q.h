@@ -125,7 +125,8 @@ int32_t b200q_weight_info(const b200q_weight* w, b200q_weight_info_t* info);
 int32_t b200q_weight_set_bias(b200q_weight* w, const float* bias, int32_t src_on_device, void* stream);
 /* Streaming-order hint (performance only; results never depend on it): `next` is the weight the caller will run through
  * b200q_matmul_q8 right after `w` (the model's projection order: qkv -> o -> gate|up -> down -> next layer's qkv ...).
- * A decode matvec on `w` then prefetches the first chunks of `next` into L2 once its own weight stream is fully requested,
+ * A decode matvec on `w` (b200q_matmul_q8, b200q_matmul_q8_swiglu, b200q_matmul of up to four rows; not the norm-prologue, paired and grouped forms)
+ * then prefetches the first chunks of `next` into L2 once its own weight stream is fully requested,
  * so HBM keeps streaming across the kernel boundary and the glue operators in between.  `next` is not owned: clear the
  * hint (next = NULL) before freeing it.  The one mutable field of a handle; set it before the handle is shared. */
 int32_t b200q_weight_set_next(b200q_weight* w, const b200q_weight* next);

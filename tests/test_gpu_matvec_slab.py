@@ -74,3 +74,20 @@ def test_gated_tiles(client, fmt, F, M):
     ws = mixed.workspace(M)
     ops._check(L.b200q_matmul_q8_swiglu(mixed.handle, P(xq), C.c_int64(M), P(got), P(ws), C.c_size_t(ws.numel()), None))
     assert torch.equal(got, want)
+
+
+def test_the_next_weights_hint_changes_no_result(client):
+    """b200q_weight_set_next on a weight of this kernel, on a larger one, on the quantising forms and on a chain that ends where it began"""
+    from blazr_b200 import synth
+    t, K = synth.GGML["Q4_K"], 2048
+    ws = [client.weight_from_ggml(t, synth.random_ggml(t, N, K, seed=N), N, K) for N in (2048, 20480, 1000, 8192)]
+    x = torch.randn((2, K), device="cuda")
+    xq = client.quantize_act(x)
+    want = [(client.matmul_q8(xq, 2, w), client.quant_matmul(x, w)) for w in ws]
+    for a, b in zip(ws, ws[1:] + ws[:1]):
+        a.set_next(b)
+    for _ in range(3):
+        got = [(client.matmul_q8(xq, 2, w), client.quant_matmul(x, w)) for w in ws]
+        assert all(torch.equal(g, v) for gs, vs in zip(got, want) for g, v in zip(gs, vs))
+    for w in ws:
+        w.set_next(None)
