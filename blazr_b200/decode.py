@@ -730,10 +730,12 @@ class Decoder:
         rows = f32 if S <= 4 else f16    # what the products read: the GEMM rounds its activations to f16 anyway, the matvec quantises f32 rows
         b = getattr(self, "_pf", None)
         if b is None or b["S"] != S:
+            # gate|up products that leave as activations (the GEMM's epilogue) need no rows of their own
+            gated = [rows is f16 and lay["swiglu_epi"] and len(lay["gu"]) == 1 and bool(L.b200q_gated_rows_ok(lay["gu"][0].w.handle, C.c_int64(S))) for lay in self.layers]
             ws_bytes = max(ln.w.workspace_bytes(S) for lay in self.layers for key in ("qkv", "o", "gu", "down") for ln in lay[key])
             b = dict(S=S, h=torch.empty((S, H), **f32), h2=torch.empty((S, H), **f32), xn=torch.empty((S, H), **rows),
                      qkv=torch.empty((S, self.qd + 2 * self.kvd), **f32), delta=torch.empty((S, H), **f32),
-                     delta2=torch.empty((S, H), **f32), gu=torch.empty((S, 2 * ff), **f32), act=torch.empty((S, ff), **rows),
+                     delta2=torch.empty((S, H), **f32), gated=gated, gu=None if all(gated) else torch.empty((S, 2 * ff), **f32), act=torch.empty((S, ff), **rows),
                      q16=torch.empty((S, nh, hd), **f16), k16=torch.empty((S, nkv, hd), **f16), v16=torch.empty((S, nkv, hd), **f16),
                      ws=torch.zeros(max(256, ws_bytes), dtype=torch.uint8, device=dev))
             b["xq1"] = torch.zeros(int(L.b200q_act_bytes(C.c_int64(H), C.c_int64(1))), dtype=torch.uint8, device=dev)
@@ -741,8 +743,7 @@ class Decoder:
             # the expansions of a projection's weights are made one projection ahead, in turn in one of two buffers (they run beside the product before)
             b["groups"] = [[(ln, (int(L.b200q_expand_bytes(ln.w.handle, C.c_int64(S))) + 255) & ~255 if rows is f16 else 0) for ln in lay[key]]
                            for lay in self.layers for key in ("qkv", "o", "gu", "down")]
-            need = max((sum(n for _, n in g) for g in b["groups"]), default=0)
-            b["panels"] = [torch.empty(max(256, need), dtype=torch.uint8, device=dev) for _ in range(2)]
+            b["panels"] = [torch.empty(max([256] + [sum(n for _, n in g) for g in b["groups"][p::2]]), dtype=torch.uint8, device=dev) for p in range(2)]
             b["logits1"] = torch.full((1, self.logits_local.shape[1]), float("-inf"), **f32)
             self._pf = b
         ids_d = torch.from_numpy(ids_h).to(dev)
@@ -805,9 +806,8 @@ class Decoder:
                 torch.distributed.all_reduce(b["delta"], group=self.group)   # prefill-size message: NCCL over NVLink
             delta = b["delta"]
             norm(lay["mlp_norm"])
-            gated = rows is f16 and lay["swiglu_epi"] and len(lay["gu"]) == 1 and L.b200q_gated_rows_ok(lay["gu"][0].w.handle, C.c_int64(S))
-            gemm(4 * li + 2, b["xn"], b["gu"], normed, b["act"] if gated else None)
-            if gated:
+            gemm(4 * li + 2, b["xn"], b["gu"], normed, b["act"] if b["gated"][li] else None)
+            if b["gated"][li]:
                 pass                                     # the product's epilogue has written the activations
             elif rows is f16:
                 ops._check(L.b200q_swiglu_f16(P(b["gu"]), C.c_int64(ff), C.c_int64(S), C.c_int32(1 if lay["swiglu_epi"] else 0), P(b["act"]), st))

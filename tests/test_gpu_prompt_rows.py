@@ -134,3 +134,25 @@ def test_prompts_of_heads_that_are_not_a_multiple_of_four():
         want = oracle.step(int(t))
     want = torch.as_tensor(want).double().reshape(-1)
     assert ((got - want).norm() / want.norm()).item() < 1e-2
+
+
+def test_prompt_buffers_are_those_that_the_pass_uses(monkeypatch):
+    """Gate|up products that leave as activations keep no rows of their own, and each of the two expansion buffers has the size of the projections that use
+    it; without that epilogue the rows are there, and the logits are the same, bit for bit."""
+    import dataclasses
+    from blazr_b200 import decode, ops
+    cfg = dataclasses.replace(decode.PRESETS["small-1b"], n_layers=2)
+    hm = decode.build_host_model(cfg, "Q4_K", seed=9)
+    client = ops.B200Client(0)
+    prompt = (torch.arange(2048) * 37 % cfg.vocab).numpy()
+    got = []
+    for epi in ("1", "0"):
+        monkeypatch.setenv("B200Q_SWIGLU_EPI", epi)
+        dec = decode.Decoder(client, cfg, "Q4_K", batch=1, max_ctx=2048, host=hm)
+        got.append(dec.prefill(prompt).clone())
+        b = dec._pf
+        assert (b["gu"] is None) == (epi == "1") == all(b["gated"])
+        for p in range(2):
+            assert b["panels"][p].numel() == max([256] + [sum(n for _, n in g) for g in b["groups"][p::2]])
+        assert b["panels"][0].numel() > 256
+    assert torch.equal(got[0], got[1])
