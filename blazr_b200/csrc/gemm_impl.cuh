@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(DQ16_THREADS) dequant_f16_kernel(const uint8_t
     pdl_wait();
 }
 template <int FAMILY>
-cudaError_t dequant_f16_launch(const b200q_weight* w, int tile0, int ntiles, __half* out, bool beside, cudaStream_t st);   // beside: may start before the launch ahead ends   // beside: may start before the launch ahead ends
+cudaError_t dequant_f16_launch(const b200q_weight* w, int tile0, int ntiles, __half* out, bool beside, cudaStream_t st);   // beside: may start before the launch ahead ends
 template <class F>
 static cudaError_t launch_dequant_f16(const b200q_weight* w, int tile0, int ntiles, __half* out, bool beside, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
@@ -430,8 +430,8 @@ __global__ void __launch_bounds__((4 + DQW + (EPI ? 4 : 0)) * 32, 1) gemm_tc_ker
         const FmtMeta meta{p.gpc};
         int ws = 0, as = 0;
         uint32_t wph = 0, aph = 1, dph = 0;
-        // Formats with lane constants for their offsets (formats.cuh: unit_offsets) have them for all units of the thread in registers, and a chunk's units
-        // are all requested before the first is expanded: with the addresses made again for every unit and one unit after another the skinny
+        // Formats with lane constants for their offsets (formats.cuh: unit_offsets) have them for all units of the thread in registers, and two
+        // units are requested before the first of them is expanded: with the addresses made again for every unit and one unit after another the skinny
         // launches (Q6_K, 32 rows) issued in 56 % of the cycles, waiting for shared memory and for their own arithmetic.
         constexpr int NU = 8 / KG, NOFF = FmtNoff<F>::value;
         uint32_t uo[NU][NOFF > 0 ? NOFF : 1];

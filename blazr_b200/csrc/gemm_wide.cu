@@ -179,8 +179,8 @@ static WidePlan wide_plan(const b200q_weight* w, int64_t M) {
 // 120 / 67; 4096 x 4096, 512 rows 49.0 / 47.0.
 // The fused kernel's times are those from before all its warps stored results and its staging moved 16-byte pieces.  Now it would be the better one well
 // above these lines (fused / expanded in a loop of seconds, us: AWQ 6144 x 4096, 1531 rows 73 / 86; Q6_K 14336 x 4096, 1000 rows 130 / 151; 28672 x 4096, 1280
-// rows 287 / 320; 8192 x 8192, 1536 rows 195 / 230; 2048 x 8192, 2048 rows 76 / 84).  The lines are where they were: which sizes take the expanded path, and
-// with it the workspace that callers are told to bring, is fixed by tests of that path at such sizes.  Both kernels give the same bits.
+// rows 287 / 320; 8192 x 8192, 1536 rows 195 / 230; 2048 x 8192, 2048 rows 76 / 84).  The lines are still those of the older
+// times, and stand to be drawn again.  A caller who brings the smaller workspace has the fused kernel; both give the same bits.
 static bool wide_wins(const b200q_weight* w, int64_t M, const WidePlan& p) {
     const int64_t mt = (M + 255) / 256, rows = ((M + mt - 1) / mt + 31) / 32 * 32, items = w->T * mt;
     const double wave = (12.0 + 0.1 * (double)rows) * (double)w->K_pad / 4096.0;

@@ -52,6 +52,8 @@ cudaError_t launch_to_bf16(const void* x, int x_dtype, int64_t M, int64_t K, int
 struct MatvecPlan {
     int grid, nstages, stage_bytes, smem_bytes, mb, xhat_bytes;
 };
+// matvec_slab.cuh: most k-chunks of a weight, bytes ahead of the records
+constexpr int SLAB_MAX_KC = 96, SLAB_HDR = 1024;
 struct FusedPrologue {
     int mode;  // 1 = add + rmsnorm + quant, 2 = swiglu + quant, 3 = quant of x
     const float* h_in;

@@ -104,7 +104,8 @@ cudaError_t matvec_plan(const b200q_weight* w, int64_t M, MatvecPlan* plan, int 
     return cudaSuccess;
 }
 
-// Weights whose rows, dealt over the SMs, fit their shared memory whole (up to 28 MB): see matvec_slab.cuh
+// Weights whose rows, dealt over the SMs, fit their shared memory whole (up to 28 MB): see matvec_slab.cuh (B200Q_MV_GRID, _SMEM_KB and _STAGES shape the
+// stream-K launch of the others)
 struct SlabPlan {
     int rows, slabs1, grid, xhat_bytes, smem_bytes;
 };
@@ -112,7 +113,7 @@ static bool slab_plan(const b200q_weight* w, int64_t M, int pro, bool swiglu, Sl
     const b200q_weight* w2 = dual_partner(w);
     const int f = w->family;
     if (f != B200Q_FAM_Q4_K && f != B200Q_FAM_Q6_K && f != B200Q_FAM_Q8_0 && f != B200Q_FAM_G4) return false;
-    if (M < 1 || M > 4 || pro == 2 || w->KC > 96 || (pro == 3 && (w2 || w->KC * M > MV_QUANT_RECORDS))) return false;
+    if (M < 1 || M > 4 || pro == 2 || w->KC > SLAB_MAX_KC || (pro == 3 && (w2 || w->KC * M > MV_QUANT_RECORDS))) return false;
     const int step = f == B200Q_FAM_G4 && w->gpc == 1 ? 16 : 8;   // a copy moves whole 16-byte pieces of every plane
     int R = step;
     auto slabs = [&](const b200q_weight* v) { return v ? (v->N + R - 1) / R : 0; };
@@ -123,7 +124,7 @@ static bool slab_plan(const b200q_weight* w, int64_t M, int pro, bool swiglu, Sl
         R = TILE_ROWS;
     }
     const int cb = (w2 && w2->chunk_bytes > w->chunk_bytes) ? w2->chunk_bytes : w->chunk_bytes;
-    const int64_t xhat = (w->KC * M * ACT_REC_BYTES + 127) & ~(int64_t)127, smem = 1024 + xhat + w->KC * R * (cb / TILE_ROWS) + ACT_REC_BYTES;
+    const int64_t xhat = (w->KC * M * ACT_REC_BYTES + 127) & ~(int64_t)127, smem = SLAB_HDR + xhat + w->KC * R * (cb / TILE_ROWS) + ACT_REC_BYTES;
     if (smem > 200 * 1024) return false;
     plan->rows = R, plan->slabs1 = (int)slabs(w), plan->grid = (int)(slabs(w) + slabs(w2)), plan->xhat_bytes = (int)xhat, plan->smem_bytes = (int)smem;
     if (plan->smem_bytes < 116 * 1024) plan->smem_bytes = 116 * 1024;   // > half an SM: see matvec_plan (4096 x 4096 Q4_K 5.7 us with what it needs, 4.6 so)

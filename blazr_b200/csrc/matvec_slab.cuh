@@ -12,8 +12,7 @@
 
 namespace b200q {
 
-constexpr int SLAB_MAX_KC = 96;
-constexpr int SLAB_HDR = 1024;      // barriers: records, then one per k-chunk
+static_assert((1 + SLAB_MAX_KC) * 8 <= SLAB_HDR, "barriers: records, then one per k-chunk");
 constexpr int SLAB_THREADS = MV_CONSUMER_WARPS * 32;
 
 // bounded: copies that never arrive are reported, not waited for

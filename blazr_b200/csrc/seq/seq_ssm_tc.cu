@@ -7,7 +7,7 @@
 // product runs as six (tc_split.cuh).  The leading one (x1 y1) has accumulators of its own and the five small ones share another; they are added in
 // registers.  Products of 8-bit parts leave room in 24 bits, so a short leading sum loses little to the tensor core's truncation, and what the small
 // ones lose is 2^-8 of that.  Sums of values that have one sign more often than not grow with every step and drop bits of what they add: those of C . B
-// are cut into steps of 32, those of C S into 64.  Error against 64 bits, 4096 tokens of 64 heads:
+// are cut into steps of 16, the others into 32.  Error against 64 bits, 4096 tokens of 64 heads:
 // outputs 1.14e-7, states 9.3e-8 (f32 multiply-add tiles: 1.14e-7, 8.8e-8; with one accumulator for each of the leading and the small products 1.6e-7).
 // Decays are exponentials of differences of the sums (never above 1), the sums kept as a float pair of the f64 running sum, so that a difference late in
 // the segment is as exact as an early one.

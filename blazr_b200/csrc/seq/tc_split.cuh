@@ -79,7 +79,7 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& p1, uint32_t&
     upk(fma2(pk(__uint_as_float(p2 << 16), __uint_as_float(p2 & 0xFFFF0000u)), minus1, pk(ra, rb)), sa_, sb_);
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p3) : "f"(sb_), "f"(sa_));
 }
-// a pair of weights (>= 0) -> three packed bf16 pairs by truncation: 8 + 8 + 8 significant bits, no conversion instruction
+// a pair of values -> three packed bf16 pairs by truncation (toward zero, either sign): 8 + 8 + 8 significant bits, no conversion instruction
 __device__ __forceinline__ void cut2(float x, float y, uint64_t minus1, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
     const float x1 = __uint_as_float(__float_as_uint(x) & 0xFFFF0000u), y1 = __uint_as_float(__float_as_uint(y) & 0xFFFF0000u);
     float rx, ry, sx, sy;
