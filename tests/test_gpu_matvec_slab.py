@@ -59,13 +59,21 @@ def test_norm_prologue(client, fmt, K):
         assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1].view(torch.int32), res[1][1].view(torch.int32))
 
 
-@pytest.mark.parametrize("fmt,F,M", [("Q4_K", 8192, 1), ("Q6_K", 7232, 2), ("Q8_0", 9472, 4)])
-def test_gated_tiles(client, fmt, F, M):
+def gated_pair(client, fmt, F, K):
+    """a gate|up weight with its rows as they lie in a file, and the same in the order of whole tiles; the sizes at which a CTA takes a whole tile"""
     from blazr_b200 import ops, synth
-    t, K = synth.GGML[fmt], 512
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert 104 * sms < 2 * F <= 128 * sms
+    t = synth.GGML[fmt]
     blk = synth.random_ggml(t, 2 * F, K, seed=F)
-    plain = client.weight_from_ggml(t, blk, 2 * F, K)
-    mixed = client.weight_from_ggml(t, np.ascontiguousarray(blk[ops.gate_up_row_order(F)]), 2 * F, K)
+    return client.weight_from_ggml(t, blk, 2 * F, K), client.weight_from_ggml(t, np.ascontiguousarray(blk[ops.gate_up_row_order(F)]), 2 * F, K)
+
+
+@pytest.mark.parametrize("fmt,F,M", [("Q4_K", 8192, 1), ("Q6_K", 7744, 2), ("Q6_K", 9472, 3), ("Q8_0", 9472, 4)])
+def test_gated_tiles(client, fmt, F, M):
+    from blazr_b200 import ops
+    K = 512
+    plain, mixed = gated_pair(client, fmt, F, K)
     L, P = ops.lib(), lambda t_: C.c_void_p(t_.data_ptr())
     xq = client.quantize_act(torch.randn((M, K), device="cuda"))
     gu = client.matmul_q8(xq, M, plain)
@@ -74,6 +82,23 @@ def test_gated_tiles(client, fmt, F, M):
     ws = mixed.workspace(M)
     ops._check(L.b200q_matmul_q8_swiglu(mixed.handle, P(xq), C.c_int64(M), P(got), P(ws), C.c_size_t(ws.numel()), None))
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("fmt,F,K,M", [("Q4_K", 8192, 2048, 1), ("Q6_K", 7744, 1024, 2), ("Q8_0", 9472, 512, 3), ("Q4_K", 9472, 512, 4)])
+def test_norm_and_gated_tiles(client, fmt, F, K, M):
+    from blazr_b200 import ops
+    plain, mixed = gated_pair(client, fmt, F, K)
+    L, P = ops.lib(), lambda t_: C.c_void_p(t_.data_ptr())
+    h, d, nw = torch.randn((M, K), device="cuda"), torch.randn((M, K), device="cuda"), torch.randn(K, device="cuda")
+    gu, xq = torch.zeros((M, 2 * F), device="cuda"), torch.zeros(int(L.b200q_act_bytes(C.c_int64(K), C.c_int64(M))), dtype=torch.uint8, device="cuda")
+    h1, h2 = torch.zeros_like(h), torch.zeros_like(h)
+    want, got = (torch.zeros(int(L.b200q_act_bytes(C.c_int64(F), C.c_int64(M))), dtype=torch.uint8, device="cuda") for _ in range(2))
+    ops._check(L.b200q_add_rmsnorm_quant(P(h), P(d), P(h1), P(nw), C.c_float(1e-5), C.c_int64(K), C.c_int64(M), P(xq), None, None))
+    client.matmul_q8(xq, M, plain, out=gu)
+    ops._check(L.b200q_swiglu_quant(P(gu), C.c_int64(F), C.c_int64(M), P(want), None))
+    ws = mixed.workspace(M)
+    ops._check(L.b200q_matmul_norm_swiglu(mixed.handle, P(h), P(d), P(h2), P(nw), C.c_float(1e-5), C.c_int64(M), P(got), P(ws), C.c_size_t(ws.numel()), None))
+    assert torch.equal(got, want) and torch.equal(h1, h2)
 
 
 def test_the_next_weights_hint_changes_no_result(client):
