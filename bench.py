@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""bench.py -- decode tokens/s of the quantized linear-layer hot path on B200 (BASELINE.json metric).
+"""bench.py -- decode tokens/s of the quantized linear-layer hot path on B200.
 
 A *step* is one decode token of the named random-init model: every quantized projection of the model
 (4 fused matvec launches per layer + lm_head; 7L+1 projections) plus the glue operators, replayed from one
@@ -36,8 +36,8 @@ def parse_args():
     ap.add_argument("--steps", type=int, default=128)
     ap.add_argument("--warmup", type=int, default=16)
     ap.add_argument("--impl", default="b200", choices=["b200", "reference"])
-    ap.add_argument("--workload", default="llama-3-70b:Q4_K_M", help="<model preset>:<scheme>  e.g. mistral-7b:Q6_K, llama-3-8b:AWQ (default: the config "
-                    "BASELINE.json's target sentence names; it fits one B200 at 42 GB and runs tensor-parallel at --gpus N)")
+    ap.add_argument("--workload", default="llama-3-70b:Q4_K_M", help="<model preset>:<scheme>  e.g. mistral-7b:Q6_K, llama-3-8b:AWQ (default: the largest "
+                    "model; it fits one B200 at 42 GB and runs tensor-parallel at --gpus N)")
     ap.add_argument("--batch", type=int, default=1)
     ap.add_argument("--prompt", type=int, default=32, help="prompt tokens fed before the timed region (reference bench.rs:24)")
     ap.add_argument("--no-extra", action="store_true", help="skip the secondary measurements (prefill GEMM, batch-32)")
@@ -383,7 +383,7 @@ def time_decode(dec, steps: int, warmup: int = 6, prompt: int = 16):
 
 
 def matvec_shape_table(client, pk):
-    """kernel GB/s of the decode matvec for every projection shape of the 7B/8B configs x the north_star's lead formats:
+    """kernel GB/s of the decode matvec for every projection shape of the 7B/8B configs x the lead formats:
     one launch per rotating weight copy (copies > 2x L2), graph replay, CUDA events (tools/kbench.py method)."""
     import torch
 
@@ -439,7 +439,7 @@ def matvec_shape_table(client, pk):
 
 
 def extras(client, cfg, scheme, pk, args):
-    """secondary numbers of the north_star, all driver-run with the default command: (1) batch-1 decode tok/s of the other named
+    """secondary numbers, all run with the default command: (1) batch-1 decode tok/s of the other named
     configs, (2) the per-shape matvec table, (3) prefill dequant-GEMM TFLOP/s + prefill pass tokens/s, (4) batch-32 decode,
     (5) a DeepSeek-V2-Lite-shaped MoE layer."""
     import time
@@ -451,7 +451,7 @@ def extras(client, cfg, scheme, pk, args):
     out = {}
     t_start = time.perf_counter()
     budget_s = float(os.environ.get("B200Q_BENCH_EXTRA_S", "170"))   # the default run must end within minutes
-    # (1) the other BASELINE configs, batch-1 greedy decode, whole step from one CUDA graph
+    # (1) the other configurations, batch-1 greedy decode, whole step from one CUDA graph
     cfgs = []
     for wl in ("llama-3.2-1b:Q4_K_M", "mistral-7b:Q6_K", "mistral-7b:Q8_0", "mistral-7b:Q4_K", "llama-3-8b:AWQ", "llama-3-8b:GPTQ", "llama-3-70b:Q4_K_M"):
         if wl == args.workload or time.perf_counter() - t_start > budget_s:
@@ -501,7 +501,7 @@ def extras(client, cfg, scheme, pk, args):
             out["matvec_shapes"] = matvec_shape_table(client, pk)
         except Exception as ex:
             out["matvec_shapes"] = {"error": repr(ex)[:200]}
-    # (3)-(5) on the Mistral-7B shapes (BASELINE config 2) whatever the headline workload is
+    # (3)-(5) on the Mistral-7B shapes whatever the headline workload is
     cfg = decode.PRESETS["mistral-7b"]
     scheme = "Q6_K"
     # prefill dequant-GEMM (tcgen05/TMEM) on the gate projection shape: Mistral-7B Q6_K / Q8_0 at S = 2048 (config 2),
@@ -546,7 +546,7 @@ def extras(client, cfg, scheme, pk, args):
                 w.free()
         except Exception as ex:
             out[name] = {"error": repr(ex)[:200]}
-    # whole-step batched decode (BASELINE metric: "decode tok/s at batch 1 and batch 32"): 32 sequences, every
+    # whole-step batched decode (decode tokens/s at batch 1 and batch 32): 32 sequences, every
     # projection on the tcgen05 path, replayed from one CUDA graph
     try:
         B = 32
@@ -570,7 +570,7 @@ def extras(client, cfg, scheme, pk, args):
         del decb
     except Exception as ex:  # secondary number: never take the headline down with it
         out["decode_batch32_step"] = {"error": repr(ex)[:200]}
-    # MoE decode (BASELINE config 5 shapes: DeepSeek-V2-Lite, 64 routed experts + 2 shared halves, top-6; gate|up Q4_K
+    # MoE decode (shapes of DeepSeek-V2-Lite, 64 routed experts + 2 shared halves, top-6; gate|up Q4_K
     # [2816 x 2048] in the SwiGLU-epilogue row order, down Q8_0 [2048 x 1408] because K = 1408 is not a multiple of 256): one token
     # through the expert MLP = quantise, grouped gate|up + SwiGLU epilogue, grouped down, combine -- 4 PDL-chained launches,
     # 16 different routings captured in ONE CUDA graph (every expert weight is touched, > L2)

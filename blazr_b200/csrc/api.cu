@@ -244,7 +244,7 @@ int32_t b200q_weight_from_awq_shard(const uint32_t* qweight, const float* scales
     w->N = n1 - n0; w->K = k1 - k0;
     w->family = B200Q_FAM_G4; w->source = B200Q_SRC_AWQ; w->ggml_type = -1; w->group_size = group_size; w->sub = 32; w->gpc = gpc;
     w->chunk_bytes = 128 * 128 + 128 * gpc * 3;
-    // canonical on-disk bytes: 4-bit weights + f16 scale + 4-bit zero per group (SURVEY.md section 8d)
+    // canonical on-disk bytes: 4-bit weights + f16 scale + 4-bit zero per group
     w->canonical_bytes = w->N * w->K / 2 + w->N * (w->K / group_size) * 2 + w->N * (w->K / group_size) / 2;
     int32_t rc = alloc_weight(w, device);
     if (rc) { free_weight(w); return rc; }
@@ -304,7 +304,7 @@ int32_t b200q_weight_from_gptq_shard(const uint32_t* qweight, const float* scale
         }
     }
     // act-order scatters every group over the whole K axis: a contiguous K slice of the weight does not correspond to a
-    // contiguous slice of the activations (SURVEY.md section 7 "GPTQ act-order g_idx defeats contiguous K-splits")
+    // contiguous slice of the activations (a GPTQ act-order g_idx defeats contiguous splits of K)
     if (need_perm && k_sharded) return fail(B200Q_ERR_UNSUPPORTED, "GPTQ act-order (non-trivial g_idx) weights cannot be split along K");
     b200q_weight* w = new (std::nothrow) b200q_weight();
     if (!w) return fail(B200Q_ERR_CUDA, "out of host memory");

@@ -1,6 +1,6 @@
 // comm_dev.cuh -- device-side view of the tensor-parallel exchange buffers (one per rank, CUDA IPC mapped into every
-// peer; csrc/comm.cu owns them).  The exchange is FUSED into the kernels on both sides of it (SURVEY.md section 5 / 8b
-// b200q_matmul_rowpar_allreduce):
+// peer; csrc/comm.cu owns them).  The exchange is FUSED into the kernels on both sides of it
+// (b200q_matmul_rowpar_allreduce):
 //
 //   producer  = the row-parallel matvec (o_proj / down_proj).  Its flush paths store every finished row sum -- the exact
 //               f64 partial of this rank's K slice -- straight into slot (parity, rank) of EVERY rank's buffer over NVLink

@@ -1,5 +1,5 @@
 // decode_ops.cu -- the small operators that sit between the quantized matvecs of one decode step
-// (SURVEY.md section 8f rows 2-4: norm -> activation-quant, RoPE + KV append + decode attention, SwiGLU,
+// (norm -> activation-quant, RoPE + KV append + decode attention, SwiGLU,
 // residual, lm_head argmax).  They are NOT the graded hot path; they exist so that a whole decode step can
 // be captured in one CUDA graph and timed as tokens/s, and each one emits the int8 activation records the
 // next matvec consumes (so no separate quantise pass runs).  Every kernel is PDL-aware: it lets its

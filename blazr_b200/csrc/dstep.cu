@@ -1,5 +1,5 @@
 // dstep.cu -- host side of the EXPERIMENTAL persistent op-list kernel (dstep_impl.cuh): program builder + launcher.
-// Opt-in (blazr_b200/decode.py: B200Q_DSTEP=1); not yet run on hardware -- see DESIGN.md section 8 item 1.
+// Opt-in (blazr_b200/decode.py: B200Q_DSTEP=1); slower than the launches it replaces.
 #include <cstring>
 #include <new>
 #include <vector>

@@ -2,7 +2,7 @@
 // the decode step.  One CTA per SM walks a program of ops -- add+RMSNorm+quantise, quantised matvec, SwiGLU+quantise --
 // separated by grid barriers, while ONE producer thread per CTA keeps the TMA weight stream running across the
 // barriers (weights depend on nothing), so the 3-5 us of fixed cost that every separate launch / kernel boundary
-// pays today (DESIGN.md section 8 item 1) is replaced by a ~1 us barrier hidden behind a full shared-memory ring.
+// pays today is replaced by a ~1 us barrier hidden behind a full shared-memory ring.
 //
 // The arithmetic is copied from the verified kernels (matvec_impl.cuh consumer loop + fix-up, decode_ops.cu norm /
 // SwiGLU / quantiser): same operation order => same bits.  Differences: activation records of a matvec are pulled from

@@ -1,6 +1,6 @@
 // formats.cuh -- kernel-native tile layouts of the quantized weight formats.
 //
-// Device layout (DESIGN.md "Data layout in HBM"): a logical [N,K] weight is cut into tiles of
+// Device layout: a logical [N,K] weight is cut into tiles of
 // TILE_ROWS=128 rows x CHUNK_K=256 k ("chunks"), stored tile-row-major then k-chunk-major, each chunk one
 // contiguous, 16-byte aligned byte string that a single cp.async.bulk (TMA) copy brings into shared memory.
 // Inside a chunk the canonical ggml block is split into SoA planes over the 128 rows (so 210-byte Q6_K and
@@ -61,7 +61,7 @@ __device__ __forceinline__ uint16_t ld2(const uint8_t* p) { return *reinterpret_
 __device__ __forceinline__ int swz8(int r, int u) { return u ^ (r & 7); }          // planes with >= 128 B per row
 __device__ __forceinline__ int swz4(int r, int u) { return u ^ ((r >> 1) & 3); }   // planes with 64 B per row
 
-// Q4_K / Q5_K 6-bit scale+min unpack from the canonical 12 bytes (SURVEY.md Appendix A)
+// Q4_K / Q5_K 6-bit scale+min unpack from the canonical 12 bytes
 __device__ __forceinline__ void k4_scale_min(int j, const uint8_t* s, int& sc, int& m) {
     if (j < 4) {
         sc = s[j] & 63;
@@ -405,7 +405,7 @@ struct FmtG4 {
 };
 
 // ------------------------------------------------------------------------------------------------
-// Formats added after the headline three ("the remaining K formats").  Same micro-interface, so
+// Formats added after the headline three (the remaining K formats).  Same micro-interface, so
 // every kernel (dequantize, integer partials, matvec, grouped matvec, tcgen05 GEMM) is instantiated unchanged.  Their
 // repack_row / load_unit are verified on the CPU against the oracle (hostcheck/, tests/test_host_formats.py).
 // High-bit planes are re-encoded so that word K of a unit gets its 4 bits with one shift + mask:

@@ -1,7 +1,7 @@
 // gemm_tc.cu -- dequant-GEMM on the 5th-generation tensor cores (tcgen05 + TMEM) for M >= 5:
 // batched decode (HBM-bound) and prefill (tensor-bound) through one kernel.
 //
-// Design (DESIGN.md "Kernel 2"): Y^T tile = W_tile[128 n x K] . X_tile[Mt m x K]^T
+// Design: Y^T tile = W_tile[128 n x K] . X_tile[Mt m x K]^T
 //   * UMMA M = 128 weight rows, UMMA N = Mt <= 256 activation rows, K = 16 per instruction, f16 x f16 -> f32;
 //   * the weight operand never touches shared memory as f16: packed chunks arrive by cp.async.bulk (TMA
 //     engine), 8 dequant warps (thread == weight row, bank-conflict-free thanks to the upload swizzle) expand

@@ -20,7 +20,7 @@ struct b200q_weight {
     const b200q_weight* pair;  // dual-format partner (b200q_weight_set_pair), not owned: its rows follow this weight's in y; null = none
 };
 
-// Expert bank (SURVEY 8a row a9: boostr::ExpertWeights stacked [num_experts, ...]): E weights of one format and shape
+// Expert bank (boostr::ExpertWeights stacked [num_experts, ...]): E weights of one format and shape
 // addressed through a device-resident pointer table, so one grouped launch streams the selected experts.
 struct b200q_bank {
     int E;

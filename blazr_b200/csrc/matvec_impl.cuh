@@ -1,6 +1,6 @@
 // matvec.cu -- decode-time dequant-matvec (M = 1..4): the HBM-bound hot kernel.
 //
-// Design (DESIGN.md "Kernel 1"):
+// Design:
 //   * stream-K over the tile-major chunk array: CTA g owns the contiguous chunk range
 //     [g*C/G, (g+1)*C/G)  -> every SM streams one contiguous region of HBM, perfect balance for any N,K;
 //   * one producer thread feeds a ring of shared-memory stages with cp.async.bulk (TMA engine, 1-D,

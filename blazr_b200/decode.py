@@ -8,7 +8,7 @@ Per layer (batch-1..4 decode, everything enqueued on one stream, PDL-chained, gr
 then add+rmsnorm+quant -> lm_head matvec -> argmax (greedy, the configs' sampling mode).
 
 Projections of equal format are fused at upload (q,k,v / gate,up share one weight handle, i.e. one launch);
-the GGUF "Q4_K_M" mix keeps attn_v / ffn_down of the "more bits" layers in Q6_K (SURVEY.md Appendix B).
+the GGUF "Q4_K_M" mix keeps attn_v / ffn_down of the "more bits" layers in Q6_K.
 Tensor parallel (reference src/engine/tensor_parallel.rs, Megatron split): column-split q/k/v/gate/up by
 heads / rows, row-split o/down along K at block granularity, all-reduce after o and down, vocab-split
 lm_head + all-gather.
@@ -62,7 +62,7 @@ def rope_table(max_ctx: int, head_dim: int, theta: float) -> np.ndarray:
 
 
 def use_more_bits(i: int, n: int) -> bool:
-    """llama.cpp's layer rule for the *_M mixes (public convention, SURVEY.md Appendix B)"""
+    """llama.cpp's layer rule for the *_M mixes (public convention)"""
     return i < n // 8 or i >= 7 * n // 8 or (i - n // 8) % 3 == 2
 
 

@@ -1,4 +1,4 @@
-"""GGUF file parsing + direct upload of the raw quantized blocks (SURVEY.md section 8f rank 1).
+"""GGUF file parsing + direct upload of the raw quantized blocks.
 
 Mirrors the reference loader surface (src/loader/gguf.rs):
     Gguf.open(path)                       boostr::format::Gguf::open            (gguf.rs:29)
@@ -23,7 +23,7 @@ from typing import Dict, List, Optional, Tuple
 import numpy as np
 
 GGUF_MAGIC = 0x46554747
-# ggml type id -> (name, block elems, block bytes)   (public ggml spec; SURVEY.md Appendix A)
+# ggml type id -> (name, block elems, block bytes)   (public ggml spec)
 GGML_TYPE_INFO = {
     0: ("F32", 1, 4), 1: ("F16", 1, 2), 2: ("Q4_0", 32, 18), 3: ("Q4_1", 32, 20), 6: ("Q5_0", 32, 22), 7: ("Q5_1", 32, 24),
     8: ("Q8_0", 32, 34), 9: ("Q8_1", 32, 36), 10: ("Q2_K", 256, 84), 11: ("Q3_K", 256, 110), 12: ("Q4_K", 256, 144),

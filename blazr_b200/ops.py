@@ -1,8 +1,7 @@
 """Python harness over the C ABI of libb200q.so (include/b200q.h).
 
 PyTorch is used only for device memory, streams and torch.distributed; every compute call goes through
-ctypes into the shared library -- the same entry points a Rust host would bind over FFI
-(INTEGRATION.md).  The interface mirrors the reference operator boundary
+ctypes into the shared library -- the same entry points a Rust host would bind over FFI.  The interface mirrors the reference operator boundary
 (``boostr::quant::QuantMatmulOps`` / ``DequantOps`` bounds at reference src/loader/api.rs:25 and
 ``DecomposedQuantTensor::new`` at src/loader/safetensors/awq.rs:218, gptq.rs:252):
 
@@ -406,7 +405,7 @@ class ExpertWeights:
 class MoeMlp:
     """Decode-time mixture-of-experts MLP over two expert banks (gate|up fused, down), the operator behind
     get_expert_weights / set_expert_weights (reference executor_cache.rs:260,283).  `local` lists the expert ids this
-    rank hosts (expert parallelism, SURVEY 8e: each rank runs its local selected experts on the replicated hidden state;
+    rank hosts (expert parallelism: each rank runs its local selected experts on the replicated hidden state;
     blazr_b200/tp.py:ep_local_slots masks the non-local slots and the caller all-reduces the partial outputs)."""
 
     def __init__(self, client: "B200Client", experts, ffn: int, hidden: int, local=None):

@@ -1,4 +1,4 @@
-"""Synthetic packed weights / activations (SURVEY.md section 8d).
+"""Synthetic packed weights / activations.
 
 There are no checkpoints in this environment, so every test and bench builds *packed bytes directly*:
 quant payload bytes are uniform u8 (every bit pattern is a valid block), and the f16 super-block

@@ -62,7 +62,7 @@ def plan(hidden: int, n_heads: int, n_kv_heads: int, head_dim: int, ffn: int, vo
 
 
 # ------------------------------------------------------------------------------------------------
-# expert parallelism (SURVEY.md section 8e): experts are partitioned num_experts / world per rank with the same
+# expert parallelism: experts are partitioned num_experts / world per rank with the same
 # shard_range rule; for decode every rank runs its local selected experts on the replicated hidden state and the
 # partial outputs are all-reduced (single exchange).
 # ------------------------------------------------------------------------------------------------

@@ -2,7 +2,7 @@
  * b200q.h -- C ABI of libb200q.so: the B200 (sm_100a) replacement for blazr's quantized linear-layer
  * operator.  Plain pointers and sizes only; no torch / C++ types cross this boundary.
  *
- * What each entry point replaces in the reference (ml-rust/blazr, paths relative to /root/reference):
+ * What each entry point replaces in the reference (ml-rust/blazr, paths within its project):
  *
  *   blazr reaches the operator only through trait bounds on the backend client
  *   (`boostr::quant::QuantMatmulOps<R>` / `boostr::quant::DequantOps<R>`: src/loader/api.rs:25,45,67,90;
@@ -150,7 +150,7 @@ int32_t b200q_shard_range_blocks(int64_t total, int64_t granule, int64_t rank, i
 size_t b200q_workspace_bytes(const b200q_weight* w, int64_t M);
 /* Y[M,N] (ldy elements between rows) = X[M,K] (ldx) . dequant(W)^T (+bias).  x,y,workspace: device memory; y may lie over x.
  * M == 1..4 : dp4a stream-K matvec on int8-quantised activations (decode);
- * M >= 5    : tcgen05/TMEM dequant-GEMM on bf16 activations (batched decode and prefill). */
+ * M >= 5    : tcgen05/TMEM dequant-GEMM on f16 activations (batched decode and prefill). */
 int32_t b200q_matmul(const b200q_weight* w, const void* x, int32_t x_dtype, int64_t M, int64_t ldx, void* y, int32_t y_dtype,
                      int64_t ldy, void* workspace, size_t workspace_bytes, void* stream);
 /* Split form for callers that share one quantised activation among several weights (q,k,v / gate,up):
@@ -204,8 +204,8 @@ int32_t b200q_moe_matmul_q8(const b200q_bank* b, const int32_t* sel_dev, int64_t
 int32_t b200q_moe_combine(const float* y, const float* gate_w, int64_t T, int64_t top_k, int64_t H, float* out, void* stream);
 
 /* ---- tensor-parallel exchange over NVLink peer memory, FUSED into the kernels on both sides of it (replaces the NCCL
- * all-reduce blazr's TP issues after the row-parallel o_proj / down_proj, reference src/engine/tensor_parallel.rs:125-163;
- * SURVEY.md sections 5 and 8b/8e).  One process per GPU: create on every rank, all-gather the 64-byte IPC handles, connect.
+ * all-reduce blazr's TP issues after the row-parallel o_proj / down_proj, reference src/engine/tensor_parallel.rs:125-163).
+ * One process per GPU: create on every rank, all-gather the 64-byte IPC handles, connect.
  *   producer  b200q_matmul_q8_rowpar : the row-parallel matvec stores its exact f64 row sums [M, ld] straight into a slot of
  *             every rank's buffer (8-byte peer stores from the kernel's flush paths) and nothing else: the slot elements are
  *             their own ready flags (empty = +0.0 bits; an exact zero travels as -0.0), no fence, no flag, no extra launch.
@@ -275,7 +275,7 @@ int32_t b200q_act_unpack(const void* xq, int64_t M, int64_t K, int8_t* q, float*
 int32_t b200q_int_partials(const b200q_weight* w, const void* xq, int64_t M, int32_t* partials, void* stream);
 
 
-/* ---- decode-step glue operators (outside the quantized-matmul path; SURVEY.md section 8f "next") ----
+/* ---- decode-step glue operators (outside the quantized-matmul path) ----
  * They let one whole decode step be captured in a CUDA graph: each emits the int8 activation records
  * (b200q_act_bytes layout) that the following b200q_matmul_q8 consumes, so no separate quantise pass runs.
  * Reference call sites: src/engine/cuda_graphs.rs:101-130 (captured forward + argmax_to_buf). */

@@ -2,10 +2,10 @@
  * cpu_fast.c -- the TIMED CPU baseline (bench.py cpu_baseline / --impl reference): AVX2 + OpenMP kernels for the three
  * headline formats, written the way a tuned CPU inference path (ggml-style) computes a quantized matvec: weights stay
  * packed, activations are int8 with one f32 scale per 32 (orc_quantize_act), integer dot products per sub-block with
- * maddubs/madd, f32 accumulation.  TEST INFRASTRUCTURE / BASELINE ONLY -- the product never links this.
+ * maddubs/madd, f32 accumulation.  TEST INFRASTRUCTURE / CPU BASELINE ONLY -- the product never links this.
  * PARITY UNPINNED like the rest of the oracle (the reference's CPU kernels live in the un-vendored boostr/numr crates);
  * tests/test_oracle_golden.py holds it to the exact-accumulation oracle (orc_matmul_q8) within 1e-5.
- * Block layouts: public ggml spec (SURVEY.md Appendix A).
+ * Block layouts: public ggml spec.
  */
 #include <immintrin.h>
 #include <stdint.h>

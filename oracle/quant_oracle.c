@@ -7,7 +7,7 @@
  *
  * PARITY UNPINNED: the arithmetic of this path lives in the third-party crates boostr 0.1.0 /
  * numr 0.5.0 (Cargo.lock:352-353, 1940-1941 of the reference), whose sources are absent from
- * /root/reference, and the reference holds no numeric test or golden vector for it.  This file
+ * its tree, and the reference holds no numeric test or golden vector for it.  This file
  * therefore restates
  *   (1) the public ggml block formats that blazr uploads as raw bytes
  *       (reference src/loader/gguf.rs:29-43: VarMap::from_gguf keeps ggml blocks, f32 activations
@@ -95,7 +95,7 @@ int orc_type_sub(int t) {
     }
 }
 
-/* Q4_K / Q5_K 6-bit scale+min unpack (SURVEY Appendix A) */
+/* Q4_K / Q5_K 6-bit scale+min unpack */
 static void k4_scale_min(int j, const uint8_t* s, int* sc, int* m) {
     if (j < 4) {
         *sc = s[j] & 63;

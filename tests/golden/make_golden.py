@@ -1,7 +1,7 @@
 """Generates tests/golden/ggml_dequant.npz -- the fixture that pins the CPU oracle.
 
 The reference (blazr) holds no numeric golden vector for the quantized-matmul path and its arithmetic
-lives in un-vendored crates (SURVEY.md section 8c), so the oracle is pinned against the independent numpy
+lives in un-vendored crates, so the oracle is pinned against the independent numpy
 implementation of the public ggml formats that ships in this image: gguf 0.19.0 ``gguf.quants``.
 For every format: 64 random packed blocks (payload bytes uniform, f16 scales finite) and the f32
 values ``gguf.quants.dequantize`` returns for them.  AWQ nibble-order golden: AutoAWQ's documented

@@ -1,6 +1,6 @@
 """GPU: a whole decode step (quantized matvecs + the glue operators) against the CPU oracle model:
 logits within tolerance at every step, and greedy token streams identical over 128 tokens on a seed whose
-top-2 logit gaps are well above the arithmetic noise (SURVEY.md section 8c contract 4)."""
+top-2 logit gaps are well above the arithmetic noise."""
 import os
 
 import numpy as np
@@ -89,7 +89,7 @@ def test_batch_of_sequences(client):
 
 
 def test_greedy_stream_llama32_1b_shape_q4km(client):
-    """BASELINE config 1 structure (Llama-3.2-1B Q4_K_M mix: Q4_K + Q6_K for attn_v / ffn_down / output, 32 heads
+    """The structure of Llama-3.2-1B (Q4_K_M mix: Q4_K + Q6_K for attn_v / ffn_down / output, 32 heads
     x 64, GQA 4, ffn 8192) at a reduced depth/vocab the CPU oracle finishes in seconds: 32-token prompt
     (reference src/cli/bench.rs:24) then 128 greedy tokens."""
     cfg = decode.PRESETS["small-1b"]
@@ -122,7 +122,7 @@ def test_peer_allreduce_world1_and_f64_partials(client):
 @pytest.mark.parametrize("scheme", ["Q6_K", "Q4_K_M", "AWQ"])
 def test_batched_decode_gemm_path_matches_oracle_logits(client, scheme):
     """M = 8 decode (batch_decode.rs:115-147): every projection runs on the tcgen05 dequant-GEMM with f32 activations.
-    Tolerance contract (north_star): logits within 1e-2 relative of the CPU path, here after several dependent steps."""
+    Tolerance contract: logits within 1e-2 relative of the CPU path, here after several dependent steps."""
     cfg = decode.PRESETS["tiny"]
     hm = decode.build_host_model(cfg, scheme, seed=13)
     rng = np.random.Generator(np.random.PCG64(5))
@@ -148,7 +148,7 @@ def test_batched_decode_gemm_path_matches_oracle_logits(client, scheme):
 
 
 def test_load_gguf_file_and_decode(client, tmp_path):
-    """a GGUF file (written by the independent gguf package) -> parse -> upload raw blocks ->
+    """A GGUF file (written by the independent gguf package) -> parse -> upload raw blocks ->
     decode; the greedy stream equals the oracle's on the same weights (tied-embedding variant included: lm_head =
     token_embd stored as Q6_K and expanded through DequantOps for the embedding lookup)."""
     from blazr_b200 import gguf_loader

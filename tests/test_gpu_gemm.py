@@ -1,7 +1,7 @@
 """GPU parity tests for the tcgen05/TMEM dequant-GEMM path (M >= 5: batched decode and prefill) against
 the CPU oracle's f32 flavour A (dequantized weights x f32 activations, double accumulation).
 
-Tolerance (north_star): max-abs error / max-abs reference <= 1e-2.  The kernel rounds weights and
+Tolerance: max-abs error / max-abs reference <= 1e-2.  The kernel rounds weights and
 activations to f16 (2^-11 relative each) and accumulates in f32, so the observed error is ~1e-3.
 """
 import numpy as np
@@ -80,7 +80,7 @@ def test_gemm_act_order_permutation(client):
 
 
 def test_gemm_prefill_shape_property(client):
-    """BASELINE config shape (Mistral-7B q_proj, S = 2048): check sampled rows against the oracle and
+    """A projection's shape (Mistral-7B q_proj, S = 2048): check sampled rows against the oracle and
     linearity in the activations (scaling x by 2 is exact in f16/f32)"""
     N, K, M = 4096, 4096, 2048
     c = Case(client, "Q6_K", N, K, seed=42)

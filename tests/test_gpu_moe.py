@@ -1,6 +1,6 @@
 """GPU parity of the grouped expert-bank matvec (b200q_moe_matmul_q8) and the decode MoE MLP against the CPU
 oracle, on DeepSeek-V2-Lite-shaped experts (gate/up 1408 x 2048, down 2048 x 1408: K is not a multiple of
-256, so down is a 32-block format -- SURVEY.md section 7 "format corner cases").  Every slot must equal the
+256, so down is a 32-block format).  Every slot must equal the
 plain per-weight matvec bit for bit (same kernel arithmetic) and the oracle's int8 flavour."""
 import numpy as np
 import pytest

@@ -1,7 +1,7 @@
 """GPU parity tests (call through the C ABI): repack + dequantize, activation quantiser, integer partials
 and the dp4a stream-K matvec against the CPU oracle on identical synthetic packed weights.
 
-Contracts (BASELINE.json north_star / SURVEY.md section 8c):
+Contracts:
   #1 dequantized weights bit-exact          #2 integer dot partials bit-exact
   #3 Y within 1e-2 relative (max-abs / max-abs) of the f32 flavour A; we additionally hold the device
      result within 2e-4 of the oracle's int8-activation flavour B (same arithmetic, different f32 order).
@@ -19,7 +19,7 @@ from qcases import ALL, GGML_GPU, Case
 pytestmark = pytest.mark.gpu
 
 GOLD = np.load(os.path.join(os.path.dirname(__file__), "golden", "ggml_dequant.npz"))
-TOL_A = 1e-2   # north_star: 1e-2 relative on outputs vs the reference CPU (f32) path
+TOL_A = 1e-2   # 1e-2 relative on outputs vs the reference CPU (f32) path
 TOL_B = 1e-6   # same int8 arithmetic with exact f64 accumulation on both sides: bit-identical up to rare 1-ulp cases
 
 
@@ -207,7 +207,7 @@ def test_matvec_is_deterministic_and_workspace_self_cleaning(client):
 
 
 def test_matvec_linearity_at_full_size(client):
-    """size-independent property at a BASELINE config shape (Mistral-7B gate_proj, Q6_K): the int8
+    """size-independent property at a projection's shape (Mistral-7B gate_proj, Q6_K): the int8
     quantiser is scale-equivariant for powers of two, so W(2x) == 2 W(x) exactly."""
     N, K = 14336, 4096
     c = Case(client, "Q6_K", N, K, seed=77)

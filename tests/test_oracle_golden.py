@@ -94,7 +94,7 @@ def test_gptq_perm_rejects_ragged_groups():
 
 @pytest.mark.parametrize("name", ["Q8_0", "Q4_K", "Q6_K", "Q5_K", "Q2_K", "Q3_K", "Q4_0", "IQ4_XS"])
 def test_flavours_agree(name):
-    """int8-activation flavour B stays within the north_star tolerance (1e-2 rel) of the f32 flavour A"""
+    """int8-activation flavour B stays within the tolerance (1e-2 rel) of the f32 flavour A"""
     t = synth.GGML[name]
     N, K, M = 64, 1024, 3
     blk = synth.random_ggml(t, N, K, seed=11)

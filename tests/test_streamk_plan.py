@@ -1,5 +1,5 @@
 """CPU check of the matvec kernel's stream-K plan (blazr_b200/csrc/streamk_plan.cuh, compiled for the host): for every
-grid size and (tiles, k-chunks) combination -- including every projection shape of the BASELINE configs at TP 1/2/4/8 and
+grid size and (tiles, k-chunks) combination -- including every projection shape of the benchmarked models at TP 1/2/4/8 and
 the grouped MoE launches -- each chunk is streamed exactly once, the consumer walk flushes the tile it accumulated, and
 the fix-up's contributor range / count / partial-slot bookkeeping matches the CTAs that really contribute, and the wide
 reducer's premise holds (contributor gf + 1 of a tile split three or more ways owns chunks of that tile only)."""
@@ -36,7 +36,7 @@ def test_exhaustive_small(sk):
 
 
 def test_model_shapes_at_every_tp_degree(sk):
-    """(N, K) of q|k|v, o, gate|up, down, lm_head of the BASELINE models, sharded as blazr_b200/tp.py does"""
+    """(N, K) of q|k|v, o, gate|up, down, lm_head of the benchmarked models, sharded as blazr_b200/tp.py does"""
     models = [(2048, 32, 8, 64, 8192, 128256), (4096, 32, 8, 128, 14336, 32000), (4096, 32, 8, 128, 14336, 128256),
               (8192, 64, 8, 128, 28672, 128256)]
     for hidden, nh, nkv, hd, ffn, vocab in models:

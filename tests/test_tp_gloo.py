@@ -80,7 +80,7 @@ def test_tp_validation_matches_reference_rule():
     with pytest.raises(ValueError):
         tp.validate_tp_config(4, 32, 6)
     tp.validate_tp_config(1, 7, 3)
-    pl = tp.plan(8192, 64, 8, 128, 28672, 128256, 3, 8)  # Llama-3-70B at TP8 (SURVEY.md section 8 a8)
+    pl = tp.plan(8192, 64, 8, 128, 28672, 128256, 3, 8)  # Llama-3-70B at TP8
     assert pl.n_heads == 8 and pl.n_kv_heads == 1
     assert pl.q_rows == (3072, 4096) and pl.kv_rows == (384, 512)
     assert pl.down_cols == (10752, 14336) and (pl.down_cols[1] - pl.down_cols[0]) // 256 == 14
@@ -92,7 +92,7 @@ def _ep_worker(rank, world, port, ret):
     os.environ["MASTER_PORT"] = str(port)
     dist.init_process_group("gloo", rank=rank, world_size=world)
     try:
-        # expert parallelism (SURVEY.md section 8e): 8 experts over 2 ranks, top-3 routing of 2 tokens; every rank
+        # expert parallelism: 8 experts over 2 ranks, top-3 routing of 2 tokens; every rank
         # evaluates its local selected experts with the oracle on the replicated hidden state, all-reduce combines
         E, top_k, hidden, ffn = 8, 3, 256, 128
         t = synth.GGML["Q8_0"]

@@ -1,6 +1,6 @@
 """torchrun script: expert-parallel MoE decode over N GPUs (DeepSeek-V2-Lite expert shapes) == the 1-GPU layer.
 
-Placement (reference north_star: per-GPU expert placement; src/engine/executor_cache.rs:218-228 for the stacked layout):
+Placement (per-GPU expert placement; src/engine/executor_cache.rs:218-228 for the stacked layout):
 the 64 routed experts + 2 shared halves are partitioned with shard_range, every rank builds ONLY its experts, runs its
 local selected experts on the replicated hidden state (non-local slots masked to -1: the grouped kernel skips their weight
 stream) and the partial outputs are summed by the one-shot NVLink all-reduce (b200q_allreduce: push to every peer, flags,

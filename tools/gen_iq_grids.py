@@ -1,5 +1,5 @@
 """Generates the public ggml IQ codebook tables (iq2xxs / iq2xs / iq3xxs / iq2s / iq3s / iq1s grids, ksigns) as C headers from the
-`gguf` python package installed in this image (gguf 0.19.0, gguf/quants.py -- NOT from /root/reference):
+`gguf` python package installed in this image (gguf 0.19.0, gguf/quants.py; the reference has none of its own):
 
     python tools/gen_iq_grids.py      -> blazr_b200/csrc/iq_grids.h  (device + host-check builds)
                                          (oracle/quant_oracle.c includes the same file: oracle/Makefile -I../blazr_b200/csrc)

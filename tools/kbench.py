@@ -1,6 +1,6 @@
 """Kernel micro-benchmark: quant matvec GB/s per (format, shape, M) with CUDA-graph replay and L2 defeat.
 
-Timing method (SURVEY.md section 8d): a CUDA graph holding one launch per rotating weight copy (copies
+Timing method: a CUDA graph holding one launch per rotating weight copy (copies
 total > 2x L2 so every launch streams its weights from HBM), >= 20 warm-up replays, CUDA events on the
 launching stream around R replays.  Algorithmic bytes = canonical packed weight bytes + x + y.
 
