@@ -391,17 +391,6 @@ __device__ __forceinline__ void sk_tile_span(const MatvecParams& p, int64_t tq, 
 // for up to 16 contributors instead of one per 4 in the single fix-up warp (measured 4.6 us of tail on 17-way split tiles)
 constexpr int MV_WIDE_MIN = 3;
 
-// successor hint: this CTA's share (g of G) of the chunks that the next weight's CTAs take first, into L2 (one thread)
-__device__ __forceinline__ void prefetch_next(const MatvecParams& p, int64_t g, int64_t G) {
-    for (int64_t ng = g; ng < p.next_G; ng += G) {
-        const int64_t a0 = sk_begin(ng, p.next_C, p.next_G), a1 = sk_begin(ng + 1, p.next_C, p.next_G);
-        const SkPlan np_ = sk_plan(a0, a1, p.next_KC);
-        const int n = (int)(a1 - a0) < p.next_pf ? (int)(a1 - a0) : p.next_pf;
-        for (int j = 0; j < n; j++)
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.next_w + sk_chunk_at(np_, a0, j) * (int64_t)p.next_chunk_bytes), "r"(p.next_chunk_bytes) : "memory");
-    }
-}
-
 // PRO: PRO_FUSED = norm / SwiGLU prologue (p.pro 1, 2), PRO_QUANT = quantising prologue (p.pro 3)
 template <class F, int MB, int PRO, bool GRP, int OUT, class F2 = F>
 __global__ void __launch_bounds__(MV_THREADS, 1) matvec_kernel(const MatvecParams p) {
@@ -555,7 +544,17 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_kernel(const MatvecParam
                 if (++s == nst) { s = 0; ph ^= 1u; }
             }
             // every chunk of this launch is requested: keep HBM busy with the successor's first chunks (L2 prefetch)
-            if (!GRP && p.next_pf > 0) prefetch_next(p, g, G);
+            if (!GRP && p.next_pf > 0) {
+                for (int64_t ng = g; ng < p.next_G; ng += G) {
+                    const int64_t a0 = sk_begin(ng, p.next_C, p.next_G), a1 = sk_begin(ng + 1, p.next_C, p.next_G);
+                    const SkPlan np_ = sk_plan(a0, a1, p.next_KC);
+                    const int n = (int)(a1 - a0) < p.next_pf ? (int)(a1 - a0) : p.next_pf;
+                    for (int j = 0; j < n; j++)
+                        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.next_w + sk_chunk_at(np_, a0, j) * (int64_t)p.next_chunk_bytes),
+                                     "r"(p.next_chunk_bytes)
+                                     : "memory");
+                }
+            }
         }
         return;
     }
