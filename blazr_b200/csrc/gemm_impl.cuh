@@ -149,8 +149,9 @@ __device__ __forceinline__ uint64_t make_b_desc(uint32_t saddr) {
 // exact __hsub2 and the scale/min applied with one __hfma2: a byte permutation, a subtraction and a multiply-add per pair of weights.
 // Pair order: word k yields (e0,e2) then (e1,e3) -- the activation staging kernel applies the same [0,2,1,3]
 // permutation inside every group of 4 k, so the contraction is unchanged.
+// NAT: pairs (e0,e1) then (e2,e3) instead, for operands whose activations lie in k order.
 // RAWHI: the second half's bytes hold 16 x the integer (the matvec's loads); 1024 + 16 v is brought to v - off by one exact multiply-add.
-template <bool SIGNED, bool RAWHI = false>
+template <bool SIGNED, bool RAWHI = false, bool NAT = false>
 __device__ __forceinline__ void unit_to_f16(const Unit& u, uint32_t* out) {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -163,8 +164,8 @@ __device__ __forceinline__ void unit_to_f16(const Unit& u, uint32_t* out) {
 #pragma unroll
         for (int k = 4 * h; k < 4 * h + 4; k++) {
             const uint32_t wv = SIGNED ? (u.v[k] ^ 0x80808080u) : u.v[k];
-            uint32_t p02 = __byte_perm(wv, 0x64646464u, 0x4240);      // bytes [e0, 0x64, e2, 0x64] = (1024 + e0, 1024 + e2): one PRMT
-            uint32_t p13 = __byte_perm(wv, 0x64646464u, 0x4341);      // (1024 + e1, 1024 + e3)
+            uint32_t p02 = __byte_perm(wv, 0x64646464u, NAT ? 0x4140 : 0x4240);      // bytes [e0, 0x64, e2, 0x64] = (1024 + e0, 1024 + e2): one PRMT
+            uint32_t p13 = __byte_perm(wv, 0x64646464u, NAT ? 0x4342 : 0x4341);      // (1024 + e1, 1024 + e3)
             __half2 x02 = raw ? __hfma2(*reinterpret_cast<__half2*>(&p02), sixteenth, off2) : __hsub2(*reinterpret_cast<__half2*>(&p02), off2);
             __half2 x13 = raw ? __hfma2(*reinterpret_cast<__half2*>(&p13), sixteenth, off2) : __hsub2(*reinterpret_cast<__half2*>(&p13), off2);
             x02 = __hfma2(x02, a2, nb2);
@@ -201,13 +202,8 @@ __global__ void __launch_bounds__(DQ16_THREADS) dequant_f16_kernel(const uint8_t
             const int r = r0 + j * (DQ16_THREADS / 8);
             Unit u;
             F::template load_unit<false>(chunk, r, i, u, meta);
-            uint32_t pk[16], nat[16];
-            unit_to_f16<F::SIGNED>(u, pk);
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                nat[2 * k] = __byte_perm(pk[2 * k], pk[2 * k + 1], 0x5410);
-                nat[2 * k + 1] = __byte_perm(pk[2 * k], pk[2 * k + 1], 0x7632);
-            }
+            uint32_t nat[16];
+            unit_to_f16<F::SIGNED, false, true>(u, nat);
             __half* dst = o + (int64_t)r * K_pad;
             st_global_32b(dst, nat);
             st_global_32b(dst + 16, nat + 8);

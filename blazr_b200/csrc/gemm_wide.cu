@@ -71,7 +71,8 @@ static cudaError_t launch_pdl_w(void (*kern)(KArgs...), int64_t blocks, int thre
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-static cudaError_t launch_stage_rows(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, const int32_t* perm, int64_t K_pad, __half* out, cudaStream_t st) {
+cudaError_t launch_stage_rows(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, const int32_t* perm, int64_t K_pad, void* rows, cudaStream_t st) {
+    __half* out = reinterpret_cast<__half*>(rows);
     const int64_t es = x_dtype == 0 ? 4 : 2;
     const bool vec = !perm && ((uintptr_t)x & 15) == 0 && (ldx * es) % 16 == 0;
     const int64_t blocks = (M * (K_pad / 8) + 255) / 256;

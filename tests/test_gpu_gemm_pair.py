@@ -1,0 +1,58 @@
+"""The dequant-GEMM on pairs of SMs (csrc/gemm_pair.cuh) where it can go wrong: every format, one chunk of K and several, one tile and several to a pair of
+CTAs, token tiles that end inside 16, 32 and 64 columns, f32 / f16 / bf16 rows with any start and stride, results in every type.  It expands weights to the
+operands of the other two kernels and sums in their order of k, so its results are theirs, bit for bit (rows of 160 take the fused kernel; 80 and more
+weight tiles are not cut along K there).  Bound against 64 bits: weights and activations are rounded to f16 (2^-11 each), see test_gpu_gemm_wide.py."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+FORMATS = ["Q4_K", "Q6_K", "Q8_0", "Q5_K", "Q4_1", "Q5_1", "Q2_K", "Q3_K", "IQ4_XS", "TQ2_0", "IQ2_S", "AWQ", "GPTQ"]
+
+
+@pytest.fixture(scope="module")
+def client():
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    from blazr_b200 import ops
+    return ops.B200Client(0)
+
+
+def weight(client, fmt, N, K):
+    from blazr_b200 import ops, synth
+    if fmt in synth.GGML:
+        t = synth.GGML[fmt]
+        return client.weight_from_ggml(t, synth.random_ggml(t, N, K, seed=N + K), N, K), None
+    if fmt == "AWQ":
+        return client.weight_from_decomposed(ops.DecomposedQuantTensor(*synth.random_awq(N, K, 128, seed=5), None, ops.DecomposedQuantMethod("awq", 128), (N, K))), None
+    qw, sc, qz, gi, b = synth.random_gptq(N, K, 128, seed=6, act_order=True, bias=True)
+    return client.weight_from_decomposed(ops.DecomposedQuantTensor(qw, sc, qz, gi, ops.DecomposedQuantMethod("gptq", 128), (N, K), bias=b)), torch.from_numpy(np.asarray(b)).cuda()
+
+
+@pytest.mark.parametrize("fmt", FORMATS)
+@pytest.mark.parametrize("N,K,M", [(10240, 256, 513), (10240, 1024, 785)])
+def test_the_bits_of_the_fused_kernel(client, fmt, N, K, M):
+    from blazr_b200 import ops
+    w, _ = weight(client, fmt, N, K)
+    x = torch.randn((M, K + 3), device="cuda:0", generator=torch.Generator(device="cuda:0").manual_seed(1)).half()[:, 1:K + 1]
+    y = torch.full((M + 1, N + 8), 7.0, dtype=torch.float16, device="cuda:0")
+    n0 = ops.launch_count()
+    client.quant_matmul(x, w, out=y[:M, :N])
+    assert ops.launch_count() - n0 == 2                                   # rows staged, one GEMM
+    for a in range(0, M, 160):
+        assert torch.equal(y[a:min(a + 160, M), :N], client.quant_matmul(x[a:a + 160].contiguous(), w))
+    assert bool((y[M] == 7).all()) and bool((y[:, N:] == 7).all())
+
+
+@pytest.mark.parametrize("fmt,N,K,M", [("Q4_K", 256, 512, 512), ("Q6_K", 512, 256, 4099), ("Q8_0", 2560, 1056, 1537), ("GPTQ", 20480, 512, 1300), ("AWQ", 28672, 640, 260), ("Q6_K", 28672, 768, 250)])
+@pytest.mark.parametrize("dt", [torch.float32, torch.float16, torch.bfloat16])
+def test_against_the_dequantized_weight(client, fmt, N, K, M, dt):
+    w, b = weight(client, fmt, N, K)
+    x = torch.randn((M, K), device="cuda:0", generator=torch.Generator(device="cuda:0").manual_seed(2)).to(dt)
+    ref = x.double() @ client.dequantize(w).double().T + (b.double() if b is not None else 0.0)
+    ws = torch.zeros(w.workspace_bytes(M), dtype=torch.uint8, device="cuda:0")
+    for out in (torch.float32, torch.float16, torch.bfloat16):
+        y = client.quant_matmul(x, w, out_dtype=out, workspace=ws)
+        assert ((y.double() - ref).norm() / ref.norm()).item() < 8.3e-4 + {torch.float32: 0.0, torch.float16: 2 ** -11, torch.bfloat16: 2 ** -9}[out]
+    from blazr_b200 import ops
+    ops.check_device_errors()
