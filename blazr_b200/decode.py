@@ -725,29 +725,29 @@ class Decoder:
         H, hd, nh, nkv, ff = cfg.hidden, cfg.head_dim, self.nh, self.nkv, self.ff
         dev = self.dev
         st = ops._stream_ptr(dev)
-        P = lambda t: C.c_void_p(t.data_ptr())
+        P = lambda t: t.data_ptr()      # (every call below has declared argument types: ops.SIGNATURES)
         f32, f16 = dict(dtype=torch.float32, device=dev), dict(dtype=torch.float16, device=dev)
         rows = f32 if S <= 4 else f16    # what the products read: the GEMM rounds its activations to f16 anyway, the matvec quantises f32 rows
         b = getattr(self, "_pf", None)
         if b is None or b["S"] != S:
             # gate|up products that leave as activations (the GEMM's epilogue) need no rows of their own
-            gated = [rows is f16 and lay["swiglu_epi"] and len(lay["gu"]) == 1 and bool(L.b200q_gated_rows_ok(lay["gu"][0].w.handle, C.c_int64(S))) for lay in self.layers]
+            gated = [rows is f16 and lay["swiglu_epi"] and len(lay["gu"]) == 1 and bool(L.b200q_gated_rows_ok(lay["gu"][0].w.handle, S)) for lay in self.layers]
             ws_bytes = max(ln.w.workspace_bytes(S) for lay in self.layers for key in ("qkv", "o", "gu", "down") for ln in lay[key])
             b = dict(S=S, h=torch.empty((S, H), **f32), h2=torch.empty((S, H), **f32), xn=torch.empty((S, H), **rows),
                      qkv=torch.empty((S, self.qd + 2 * self.kvd), **f32), delta=torch.empty((S, H), **f32),
                      delta2=torch.empty((S, H), **f32), gated=gated, gu=None if all(gated) else torch.empty((S, 2 * ff), **f32), act=torch.empty((S, ff), **rows),
                      q16=torch.empty((S, nh, hd), **f16), k16=torch.empty((S, nkv, hd), **f16), v16=torch.empty((S, nkv, hd), **f16),
                      ws=torch.zeros(max(256, ws_bytes), dtype=torch.uint8, device=dev))
-            b["xq1"] = torch.zeros(int(L.b200q_act_bytes(C.c_int64(H), C.c_int64(1))), dtype=torch.uint8, device=dev)
+            b["xq1"] = torch.zeros(int(L.b200q_act_bytes(H, 1)), dtype=torch.uint8, device=dev)
             b["h1"] = torch.empty((1, H), **f32)
             # the expansions of a projection's weights are made one projection ahead, in turn in one of two buffers (they run beside the product before)
-            b["groups"] = [[(ln, (int(L.b200q_expand_bytes(ln.w.handle, C.c_int64(S))) + 255) & ~255 if rows is f16 else 0) for ln in lay[key]]
+            b["groups"] = [[(ln, (int(L.b200q_expand_bytes(ln.w.handle, S)) + 255) & ~255 if rows is f16 else 0) for ln in lay[key]]
                            for lay in self.layers for key in ("qkv", "o", "gu", "down")]
             b["panels"] = [torch.empty(max([256] + [sum(n for _, n in g) for g in b["groups"][p::2]]), dtype=torch.uint8, device=dev) for p in range(2)]
             b["logits1"] = torch.full((1, self.logits_local.shape[1]), float("-inf"), **f32)
             self._pf = b
         ids_d = torch.from_numpy(ids_h).to(dev)
-        ops._check(L.b200q_embed(P(self.embed), P(ids_d), C.c_int64(H), C.c_int64(S), P(b["h"]), st))
+        ops._check(L.b200q_embed(P(self.embed), P(ids_d), H, S, P(b["h"]), st))
         hin, hout = b["h"], b["h2"]
         delta = None
         def expand(i):
@@ -756,7 +756,7 @@ class Decoder:
                 at, beside = b["panels"][i & 1].data_ptr(), i > 0 and b["groups"][i - 1][-1][1] > 0
                 for ln, n in b["groups"][i]:
                     if n:
-                        ops._check(L.b200q_expand(ln.w.handle, C.c_int64(S), C.c_void_p(at), C.c_int32(1 if beside else 0), st))
+                        ops._check(L.b200q_expand(ln.w.handle, S, at, 1 if beside else 0, st))
                     at += n
 
         def gemm(i, x, out, ready=False, act=None):
@@ -765,24 +765,24 @@ class Decoder:
                 at = b["panels"][i & 1].data_ptr()
                 for ln, n in b["groups"][i]:
                     to = act if act is not None else out
-                    ops._check(L.b200q_matmul_rows(ln.w.handle, P(x), C.c_int32(1 if ready else 0), C.c_int64(S), C.c_int64(x.stride(0)), C.c_void_p(at) if n else None,
-                                                   None if act is not None else C.c_void_p(out.data_ptr() + 4 * ln.col0), P(act) if act is not None else None,
-                                                   C.c_int64(to.stride(0)), P(b["ws"]), C.c_size_t(b["ws"].numel()), st))
+                    ops._check(L.b200q_matmul_rows(ln.w.handle, P(x), 1 if ready else 0, S, x.stride(0), at if n else None,
+                                                   None if act is not None else out.data_ptr() + 4 * ln.col0, P(act) if act is not None else None,
+                                                   to.stride(0), P(b["ws"]), b["ws"].numel(), st))
                     at += n
                 return expand(i + 1)
             for ln, _ in b["groups"][i]:
-                ops._check(L.b200q_matmul(ln.w.handle, P(x), C.c_int32(ops._TORCH2DT[x.dtype]), C.c_int64(S), C.c_int64(x.stride(0)),
-                                          C.c_void_p(out.data_ptr() + 4 * ln.col0), C.c_int32(ops.F32), C.c_int64(out.stride(0)), P(b["ws"]),
-                                          C.c_size_t(b["ws"].numel()), st))
+                ops._check(L.b200q_matmul(ln.w.handle, P(x), ops._TORCH2DT[x.dtype], S, x.stride(0),
+                                          out.data_ptr() + 4 * ln.col0, ops.F32, out.stride(0), P(b["ws"]),
+                                          b["ws"].numel(), st))
 
         def norm(w):
             nonlocal hin, hout
             if rows is f16 and H <= 8192:
-                ops._check(L.b200q_add_rmsnorm_f16(P(hin), P(delta) if delta is not None else None, P(hout), P(w), C.c_float(cfg.eps), C.c_int64(H), C.c_int64(S), P(b["xn"]), st))
+                ops._check(L.b200q_add_rmsnorm_f16(P(hin), P(delta) if delta is not None else None, P(hout), P(w), cfg.eps, H, S, P(b["xn"]), st))
             else:
                 x32 = b["xn"] if rows is f32 else torch.empty((S, H), **f32)
-                ops._check(L.b200q_add_rmsnorm_quant(P(hin), P(delta) if delta is not None else None, P(hout), P(w), C.c_float(cfg.eps), C.c_int64(H),
-                                                     C.c_int64(S), None, P(x32), st))
+                ops._check(L.b200q_add_rmsnorm_quant(P(hin), P(delta) if delta is not None else None, P(hout), P(w), cfg.eps, H,
+                                                     S, None, P(x32), st))
                 if rows is f16:
                     b["xn"].copy_(x32.clamp_(-65504.0, 65504.0))
             hin, hout = hout, hin
@@ -796,8 +796,8 @@ class Decoder:
                 ck, cv, table = lay["ck"], lay["cv"], self.block_table[seq]
             else:
                 ck, cv, table = lay["ck"][seq], lay["cv"][seq], None
-            ops._check(L.b200q_rope_kv_prefill(P(b["qkv"]), P(self.rope), C.c_int32(nh), C.c_int32(nkv), C.c_int32(hd), C.c_int64(S), P(b["q16"]), P(b["k16"]), P(b["v16"]),
-                                               P(ck), P(cv), P(table) if table is not None else None, C.c_int32(self.block_size), st))
+            ops._check(L.b200q_rope_kv_prefill(P(b["qkv"]), P(self.rope), nh, nkv, hd, S, P(b["q16"]), P(b["k16"]), P(b["v16"]),
+                                               P(ck), P(cv), P(table) if table is not None else None, self.block_size, st))
             o = Fnn.scaled_dot_product_attention(b["q16"].transpose(0, 1)[None], b["k16"].transpose(0, 1)[None], b["v16"].transpose(0, 1)[None], is_causal=True,
                                                  enable_gqa=(nh != nkv))
             attn = o[0].transpose(0, 1).reshape(S, self.qd)
@@ -810,21 +810,21 @@ class Decoder:
             if b["gated"][li]:
                 pass                                     # the product's epilogue has written the activations
             elif rows is f16:
-                ops._check(L.b200q_swiglu_f16(P(b["gu"]), C.c_int64(ff), C.c_int64(S), C.c_int32(1 if lay["swiglu_epi"] else 0), P(b["act"]), st))
+                ops._check(L.b200q_swiglu_f16(P(b["gu"]), ff, S, 1 if lay["swiglu_epi"] else 0, P(b["act"]), st))
             else:
                 sw = L.b200q_swiglu_f32_interleaved if lay["swiglu_epi"] else L.b200q_swiglu_f32
-                ops._check(sw(P(b["gu"]), C.c_int64(ff), C.c_int64(S), P(b["act"]), st))
+                ops._check(sw(P(b["gu"]), ff, S, P(b["act"]), st))
             gemm(4 * li + 3, b["act"], b["delta2"], rows is f16)
             if self.world > 1:
                 torch.distributed.all_reduce(b["delta2"], group=self.group)
             delta = b["delta2"]
         # last position only: final norm + quantise -> lm_head on the decode matvec (M = 1) -> greedy token
         last_h, last_d = hin[S - 1:S], delta[S - 1:S]
-        ops._check(L.b200q_add_rmsnorm_quant(P(last_h), P(last_d), P(b["h1"]), P(self.final_norm), C.c_float(cfg.eps), C.c_int64(H), C.c_int64(1),
+        ops._check(L.b200q_add_rmsnorm_quant(P(last_h), P(last_d), P(b["h1"]), P(self.final_norm), cfg.eps, H, 1,
                                              P(b["xq1"]), None, st))
         for ln in self.head:
-            ops._check(L.b200q_matmul_q8(ln.w.handle, P(b["xq1"]), C.c_int64(1), C.c_void_p(b["logits1"].data_ptr() + 4 * ln.col0), C.c_int32(ops.F32),
-                                         C.c_int64(b["logits1"].stride(0)), P(ln.ws), C.c_size_t(ln.ws.numel()), st))
+            ops._check(L.b200q_matmul_q8(ln.w.handle, P(b["xq1"]), 1, b["logits1"].data_ptr() + 4 * ln.col0, ops.F32,
+                                         b["logits1"].stride(0), P(ln.ws), ln.ws.numel(), st))
         logits = b["logits1"][0]
         if self.world > 1:
             parts = [torch.empty_like(b["logits1"]) for _ in range(self.world)]

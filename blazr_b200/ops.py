@@ -60,6 +60,15 @@ EXPORTS = [
     "b200q_bank_create", "b200q_bank_free", "b200q_bank_set", "b200q_bank_get", "b200q_bank_workspace_bytes", "b200q_moe_matmul_q8", "b200q_moe_combine",
 ]
 
+# argument types of the calls that a projection, a prompt and an expert step are made of (p pointer, i int32, l int64, z size_t, f float): plain numbers, converted
+# once by ctypes
+_ARG = dict(p=C.c_void_p, i=C.c_int32, l=C.c_int64, z=C.c_size_t, f=C.c_float)
+SIGNATURES = {
+    "matmul": "ppillpilpzp", "matmul_q8": "pplpilpzp", "matmul_rows": "ppillppplpzp", "expand": "plpip", "expand_bytes": "pl", "gated_rows_ok": "pl",
+    "embed": "ppllpp", "add_rmsnorm_f16": "ppppfllpp", "add_rmsnorm_quant": "ppppfllppp", "rope_kv_prefill": "ppiiilppppppip", "swiglu_f16": "pllipp",
+    "swiglu_f32": "pllpp", "swiglu_f32_interleaved": "pllpp", "quantize_act": "pilllppp", "moe_matmul_q8": "pplpllpilpzp", "moe_matmul_q8_swiglu": "pplpllppzp",
+    "moe_combine": "pplllpp", "matmul_path": "pipillpilpzp"
+}
 _lib = None
 
 
@@ -83,8 +92,8 @@ def lib() -> C.CDLL:
         L.b200q_weight_set_next.argtypes = [C.c_void_p, C.c_void_p]
         L.b200q_gate_up_row.restype = C.c_int64
         L.b200q_gate_up_row.argtypes = [C.c_int64, C.c_int64]
-        p, i32, i64, sz = C.c_void_p, C.c_int32, C.c_int64, C.c_size_t      # the call of every projection: plain numbers, converted once by ctypes
-        L.b200q_matmul_path.argtypes = [p, i32, p, i32, i64, i64, p, i32, i64, p, sz, p]
+        for name, args in SIGNATURES.items():
+            getattr(L, "b200q_" + name).argtypes = [_ARG[a] for a in args]
         _lib = L
     return _lib
 
@@ -450,22 +459,22 @@ class MoeMlp:
         T, top_k = sel.shape
         n = T * top_k
         L = lib()
-        P = lambda t_: C.c_void_p(t_.data_ptr())
+        P = lambda t_: t_.data_ptr()
         st = _stream_ptr(x.device)
         b = self._buffers(T, top_k, x.device)
         x = x.contiguous()
         sel_flat, gw = sel.reshape(-1), gate_w.contiguous()
-        _check(L.b200q_quantize_act(P(x), C.c_int32(F32), C.c_int64(T), C.c_int64(self.hidden), C.c_int64(self.hidden), None, P(b["xq"]), st))
+        _check(L.b200q_quantize_act(P(x), F32, T, self.hidden, self.hidden, None, P(b["xq"]), st))
         if self.interleaved:
-            _check(L.b200q_moe_matmul_q8_swiglu(self.gu.handle, P(sel_flat), C.c_int64(n), P(b["xq"]), C.c_int64(T), C.c_int64(top_k), P(b["aq"]),
-                                                P(b["ws_gu"]), C.c_size_t(b["ws_gu"].numel()), st))
+            _check(L.b200q_moe_matmul_q8_swiglu(self.gu.handle, P(sel_flat), n, P(b["xq"]), T, top_k, P(b["aq"]),
+                                                P(b["ws_gu"]), b["ws_gu"].numel(), st))
         else:
-            _check(L.b200q_moe_matmul_q8(self.gu.handle, P(sel_flat), C.c_int64(n), P(b["xq"]), C.c_int64(T), C.c_int64(top_k), P(b["gu"]), C.c_int32(F32),
-                                         C.c_int64(2 * self.ffn), P(b["ws_gu"]), C.c_size_t(b["ws_gu"].numel()), st))
-            _check(L.b200q_swiglu_quant(P(b["gu"]), C.c_int64(self.ffn), C.c_int64(n), P(b["aq"]), st))
-        _check(L.b200q_moe_matmul_q8(self.down.handle, P(sel_flat), C.c_int64(n), P(b["aq"]), C.c_int64(n), C.c_int64(1), P(b["y"]), C.c_int32(F32),
-                                     C.c_int64(self.hidden), P(b["ws_dn"]), C.c_size_t(b["ws_dn"].numel()), st))
-        _check(L.b200q_moe_combine(P(b["y"]), P(gw), C.c_int64(T), C.c_int64(top_k), C.c_int64(self.hidden), P(b["out"]), st))
+            _check(L.b200q_moe_matmul_q8(self.gu.handle, P(sel_flat), n, P(b["xq"]), T, top_k, P(b["gu"]), F32,
+                                         2 * self.ffn, P(b["ws_gu"]), b["ws_gu"].numel(), st))
+            _check(L.b200q_swiglu_quant(C.c_void_p(P(b["gu"])), C.c_int64(self.ffn), C.c_int64(n), C.c_void_p(P(b["aq"])), st))
+        _check(L.b200q_moe_matmul_q8(self.down.handle, P(sel_flat), n, P(b["aq"]), n, 1, P(b["y"]), F32,
+                                     self.hidden, P(b["ws_dn"]), b["ws_dn"].numel(), st))
+        _check(L.b200q_moe_combine(P(b["y"]), P(gw), T, top_k, self.hidden, P(b["out"]), st))
         return b["out"]
 
 

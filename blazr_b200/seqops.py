@@ -46,6 +46,24 @@ EXPORTS = ["b200seq_last_error", "b200seq_version", "b200seq_launch_count", "b20
            "b200seq_token_gate", "b200seq_side_close", "b200seq_linear_silu", "b200seq_moe_route_rule", "b200seq_moe_router_rule", "b200seq_retention_partials",
            "b200seq_selective_scan", "b200seq_scan_scratch_floats", "b200seq_parallel_close"]
 
+# argument types of the operators' C entries (include/b200seq.h): p pointer, i int, l int64, z size_t, f float.  Declared, plain numbers are converted by ctypes
+# as they are passed; an object made for each of them and a stream object looked up for each call took half of a call's 4 - 8 us.
+_ARG = dict(p=C.c_void_p, i=C.c_int, l=C.c_int64, z=C.c_size_t, f=C.c_float)
+SIGNATURES = {
+    "error_flags": "p", "embed_streams": "ppfiiipp", "hc_norm": "pppppiiifpipip", "hc_norm_conv": "pppppiiifpppipip", "causal_conv": "plppppiiipilp",
+    "group_rmsnorm": "plpiiifpip", "gated_act": "pliifffipip", "linear": "pilpiiiplip", "linear_silu": "pilpiiipliiip", "linear_gated": "pilpiiifffpilp",
+    "attn_prep": "plpppiiiifp", "attn": "plpppiiiifiiipipzp", "ssm_scan": "pliiplpppppiiiippzp", "linear_act": "pilpiiiifffpilp", "act": "pliiifffpilp",
+    "depth_norm": "plippppppifpppippip", "attn_prep_ex": "plppppppp", "attn_ex": "plpppppppipzp", "latent_prep": "pliiplpiiiipfpfpplpip",
+    "latent_gather": "plpiipip", "head_linear": "pilpiiiiipillp", "rotary": "pliiipiipffp", "retention_partials": "iiii", "retention": "plppppipzp",
+    "token_shift": "pipppppip", "post_norm": "ppplpfppfipippipppppp", "moe_route": "pliiiiipppp", "moe_router": "pilpiiiiiiiplppp", "moe_table_route": "ppiiipppp",
+    "moe_sort": "piippppp", "moe_linear": "pilippppiiiiipilp", "moe_linear_act": "pilippppiiiiifffpilp", "moe_gather": "plpiiiplp", "moe_combine": "pppiiipplpp",
+    "moe_route_ex": "pliiiiiippppp", "moe_router_ex": "pilpiiiiiiiipplppp", "moe_route_rule": "plippppp", "moe_router_rule": "pilpiiipplppp",
+    "moe_combine_ex": "ppppipiiipplpp", "causal_conv_ex": "plpppppiiipilpilp", "embed_bigram": "pppppfiiiippip", "branch_norm": "ppppfppfpfipippipp",
+    "polynorm": "pliipfpilp", "softcap": "plfp", "diff_combine": "piiiifffpip", "min_gru": "pliiipppipip", "rg_lru": "plplppfplipppiipip", "delta": "plppplppipzp",
+    "embed_pos": "pppfpippppfpip", "sandwich_norm": "pppfppipippipp", "token_gate": "pliiplippip", "side_close": "pppfpppliippppipippipp",
+    "selective_scan": "piplpplppppipzp", "parallel_close": "pp", "argmax": "piipp"
+}
+
 
 class SeqError(RuntimeError):
     def __init__(self, code: int, msg: str):
@@ -184,6 +202,8 @@ def lib() -> C.CDLL:
         L = C.CDLL(LIB_PATH)
         L.b200seq_last_error.restype = C.c_char_p
         L.b200seq_launch_count.restype = C.c_int64
+        for name, args in SIGNATURES.items():
+            getattr(L, "b200seq_" + name).argtypes = [_ARG[a] for a in args]
         _lib = L
     return _lib
 
@@ -193,12 +213,15 @@ def _check(rc: int):
         raise SeqError(rc, lib().b200seq_last_error().decode())
 
 
-def _st(t: torch.Tensor) -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+def _st(t: torch.Tensor) -> int:
+    dev = t.device
+    if dev.type != "cuda":
+        raise ValueError(f"Expected a cuda device, but got: {dev}")
+    return torch._C._cuda_getCurrentRawStream(dev.index)
 
 
 def _p(t: Optional[torch.Tensor]):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def launch_count() -> int:
@@ -212,8 +235,9 @@ def error_flags() -> int:
 
 
 def _rows2d(t: torch.Tensor):
-    assert t.dim() == 2 and t.stride(1) == 1, "row-major 2-D view expected"
-    return t.shape[0], t.shape[1], t.stride(0)
+    shape, strides = t.shape, t.stride()
+    assert len(shape) == 2 and strides[1] == 1, "row-major 2-D view expected"
+    return shape[0], shape[1], strides[0]
 
 
 # ---- per-operator timeline (bench / profiling aid): set `timeline = []` and every operator call appends
@@ -247,7 +271,7 @@ def _timed(fn):
 @_timed
 def embed_streams(table: torch.Tensor, ids: torch.Tensor, scale: float, X: torch.Tensor):
     T, S, W = X.shape
-    _check(lib().b200seq_embed_streams(_p(table), _p(ids), C.c_float(scale), T, S, W, _p(X), _st(X)))
+    _check(lib().b200seq_embed_streams(_p(table), _p(ids), scale, T, S, W, _p(X), _st(X)))
 
 
 @_timed
@@ -255,7 +279,7 @@ def hc_norm(X: torch.Tensor, y: Optional[torch.Tensor], post: Optional[torch.Ten
             groups: int, eps: float, out: Optional[torch.Tensor], rows: Optional[torch.Tensor] = None):
     T, S, W = X.shape
     R = T if rows is None else rows.numel()
-    _check(lib().b200seq_hc_norm(_p(X), _p(y), _p(post), _p(in_w), _p(norm_w), S, W, groups, C.c_float(eps), _p(rows), R, _p(out), _DT[out.dtype] if out is not None else F32, _st(X)))
+    _check(lib().b200seq_hc_norm(_p(X), _p(y), _p(post), _p(in_w), _p(norm_w), S, W, groups, eps, _p(rows), R, _p(out), _DT[out.dtype] if out is not None else F32, _st(X)))
 
 
 @_timed
@@ -263,7 +287,7 @@ def hc_norm_conv(X: torch.Tensor, y: Optional[torch.Tensor], post: Optional[torc
                  conv_w: torch.Tensor, conv_state: torch.Tensor, step: "StepDesc", out: torch.Tensor):
     """hc_norm followed by the residual carried convolution in one kernel; only for steps in which every entry brings one token"""
     T, S, W = X.shape
-    _check(lib().b200seq_hc_norm_conv(_p(X), _p(y), _p(post), _p(in_w), _p(norm_w), S, W, groups, C.c_float(eps), _p(conv_w), _p(conv_state), C.byref(step),
+    _check(lib().b200seq_hc_norm_conv(_p(X), _p(y), _p(post), _p(in_w), _p(norm_w), S, W, groups, eps, _p(conv_w), _p(conv_state), C.byref(step),
                                       conv_w.shape[1], _p(out), _DT[out.dtype], _st(X)))
 
 
@@ -271,22 +295,22 @@ def hc_norm_conv(X: torch.Tensor, y: Optional[torch.Tensor], post: Optional[torc
 def causal_conv(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], state: Optional[torch.Tensor], step: "StepDesc", mode: int, out: torch.Tensor):
     T, Cn, ldx = _rows2d(x)
     _, _, ldo = _rows2d(out)
-    _check(lib().b200seq_causal_conv(_p(x), C.c_int64(ldx), _p(w), _p(bias), _p(state), C.byref(step), Cn, w.shape[1], mode, _p(out), _DT[out.dtype],
-                                     C.c_int64(ldo), _st(x)))
+    _check(lib().b200seq_causal_conv(_p(x), ldx, _p(w), _p(bias), _p(state), C.byref(step), Cn, w.shape[1], mode, _p(out), _DT[out.dtype],
+                                     ldo, _st(x)))
 
 
 @_timed
 def group_rmsnorm(x: torch.Tensor, w: Optional[torch.Tensor], groups: int, eps: float, out: torch.Tensor):
     T, D, ldx = _rows2d(x)
     assert out.is_contiguous()
-    _check(lib().b200seq_group_rmsnorm(_p(x), C.c_int64(ldx), _p(w), T, D, groups, C.c_float(eps), _p(out), _DT[out.dtype], _st(x)))
+    _check(lib().b200seq_group_rmsnorm(_p(x), ldx, _p(w), T, D, groups, eps, _p(out), _DT[out.dtype], _st(x)))
 
 
 @_timed
 def gated_act(gu: torch.Tensor, limit: float, alpha: float, up_shift: float, out: torch.Tensor, interleaved: bool = False):
     T, F2, ldg = _rows2d(gu)
     assert out.is_contiguous() and out.shape[1] * 2 == F2
-    _check(lib().b200seq_gated_act(_p(gu), C.c_int64(ldg), T, F2 // 2, C.c_float(limit), C.c_float(alpha), C.c_float(up_shift), int(interleaved), _p(out), _DT[out.dtype], _st(gu)))
+    _check(lib().b200seq_gated_act(_p(gu), ldg, T, F2 // 2, limit, alpha, up_shift, int(interleaved), _p(out), _DT[out.dtype], _st(gu)))
 
 
 @_timed
@@ -295,7 +319,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor, path: int = PATH_A
     M, K, ldx = _rows2d(x)
     _, N, ldy = _rows2d(y)
     assert w.dtype == torch.bfloat16 and w.is_contiguous() and tuple(w.shape) == (N, K) and y.dtype == torch.float32 and y.shape[0] == M
-    _check(lib().b200seq_linear_silu(_p(x), _DT[x.dtype], C.c_int64(ldx), _p(w), M, N, K, _p(y), C.c_int64(ldy), silu[0], silu[1], path, _st(x)))
+    _check(lib().b200seq_linear_silu(_p(x), _DT[x.dtype], ldx, _p(w), M, N, K, _p(y), ldy, silu[0], silu[1], path, _st(x)))
 
 
 @_timed
@@ -305,8 +329,8 @@ def linear_gated(x: torch.Tensor, w_il: torch.Tensor, limit: float, alpha: float
     M, K, ldx = _rows2d(x)
     _, F, ldo = _rows2d(out)
     assert w_il.dtype == torch.bfloat16 and w_il.is_contiguous() and tuple(w_il.shape) == (2 * F, K) and out.shape[0] == M
-    _check(lib().b200seq_linear_gated(_p(x), _DT[x.dtype], C.c_int64(ldx), _p(w_il), M, F, K, C.c_float(limit), C.c_float(alpha), C.c_float(up_shift), _p(out),
-                                      _DT[out.dtype], C.c_int64(ldo), _st(x)))
+    _check(lib().b200seq_linear_gated(_p(x), _DT[x.dtype], ldx, _p(w_il), M, F, K, limit, alpha, up_shift, _p(out),
+                                      _DT[out.dtype], ldo, _st(x)))
 
 
 @_timed
@@ -317,8 +341,8 @@ def linear_act(x: torch.Tensor, w: torch.Tensor, act: int, out: torch.Tensor, li
     _, F, ldo = _rows2d(out)
     N = w.shape[0]
     assert w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] == K and out.shape[0] == M and F == (N // 2 if act in ACT_GATED else N)
-    _check(lib().b200seq_linear_act(_p(x), _DT[x.dtype], C.c_int64(ldx), _p(w), M, N, K, act, C.c_float(limit), C.c_float(alpha), C.c_float(shift), _p(out),
-                                    _DT[out.dtype], C.c_int64(ldo), _st(x)))
+    _check(lib().b200seq_linear_act(_p(x), _DT[x.dtype], ldx, _p(w), M, N, K, act, limit, alpha, shift, _p(out),
+                                    _DT[out.dtype], ldo, _st(x)))
 
 
 @_timed
@@ -326,7 +350,7 @@ def act(z: torch.Tensor, kind: int, out: torch.Tensor, limit: float = 0.0, alpha
     """the same activation on a product that is in memory (z f32 [T, N]; gated kinds read interleaved pairs)"""
     T, N, ldz = _rows2d(z)
     _, _, ldo = _rows2d(out)
-    _check(lib().b200seq_act(_p(z), C.c_int64(ldz), T, N, kind, C.c_float(limit), C.c_float(alpha), C.c_float(shift), _p(out), _DT[out.dtype], C.c_int64(ldo), _st(z)))
+    _check(lib().b200seq_act(_p(z), ldz, T, N, kind, limit, alpha, shift, _p(out), _DT[out.dtype], ldo, _st(z)))
 
 
 @_timed
@@ -339,15 +363,15 @@ def depth_norm(x_cur: torch.Tensor, out1: Optional[torch.Tensor], w1: Optional[t
     W = x_cur.shape[-1]
     R = x_cur.shape[0] if rows is None else rows.numel()
     o = out1 if out1 is not None else out2
-    _check(lib().b200seq_depth_norm(_p(hist), C.c_int64(hist.stride(0) if hist is not None else 0), n_prev, _p(dwa), _p(x_cur), _p(y1), _p(y2), _p(hist_out), _p(x_out), W,
-                                    C.c_float(eps), _p(w1), _p(w2), _p(rows), R, _p(out1), _p(out2), _DT[o.dtype] if o is not None else F32, _st(x_cur)))
+    _check(lib().b200seq_depth_norm(_p(hist), hist.stride(0) if hist is not None else 0, n_prev, _p(dwa), _p(x_cur), _p(y1), _p(y2), _p(hist_out), _p(x_out), W,
+                                    eps, _p(w1), _p(w2), _p(rows), R, _p(out1), _p(out2), _DT[o.dtype] if o is not None else F32, _st(x_cur)))
 
 
 @_timed
 def attn_prep_ex(proj: torch.Tensor, step: "StepDesc", d: "AttnDesc", kpool: Optional[torch.Tensor], vpool: Optional[torch.Tensor],
                  kpooled: Optional[torch.Tensor] = None, vpooled: Optional[torch.Tensor] = None):
     _, _, ld = _rows2d(proj)
-    _check(lib().b200seq_attn_prep_ex(_p(proj), C.c_int64(ld), C.byref(step), C.byref(d), _p(kpool), _p(vpool), _p(kpooled), _p(vpooled), _st(proj)))
+    _check(lib().b200seq_attn_prep_ex(_p(proj), ld, C.byref(step), C.byref(d), _p(kpool), _p(vpool), _p(kpooled), _p(vpooled), _st(proj)))
 
 
 @_timed
@@ -360,8 +384,8 @@ def attn_ex(proj: torch.Tensor, step: "StepDesc", d: "AttnDesc", kpool: torch.Te
         d2.gate, d2.gate_ld = gate.data_ptr(), gate.stride(0)
         d = d2
     assert out.is_contiguous() and (scratch is None or (scratch.dtype == torch.float32 and scratch.is_contiguous()))
-    _check(lib().b200seq_attn_ex(_p(proj), C.c_int64(ld), C.byref(step), C.byref(d), _p(kpool), _p(vpool), _p(kpooled), _p(vpooled), _p(out), _DT[out.dtype], _p(scratch),
-                                 C.c_size_t(scratch.numel() if scratch is not None else 0), _st(proj)))
+    _check(lib().b200seq_attn_ex(_p(proj), ld, C.byref(step), C.byref(d), _p(kpool), _p(vpool), _p(kpooled), _p(vpooled), _p(out), _DT[out.dtype], _p(scratch),
+                                 scratch.numel() if scratch is not None else 0, _st(proj)))
 
 
 @_timed
@@ -369,7 +393,7 @@ def moe_route(z: torch.Tensor, E: int, groups: int, keep: int, top: int, ids: to
     """z f32 [T, >= E] router logits -> ids int32 [T, top], wts f32 [T, top], counts int32 [E]"""
     T, _, ldz = _rows2d(z)
     assert ids.dtype == torch.int32 and wts.dtype == torch.float32 and ids.is_contiguous() and wts.is_contiguous() and ids.numel() >= T * top
-    _check(lib().b200seq_moe_route(_p(z), C.c_int64(ldz), T, E, groups, keep, top, _p(ids), _p(wts), _p(counts), _st(z)))
+    _check(lib().b200seq_moe_route(_p(z), ldz, T, E, groups, keep, top, _p(ids), _p(wts), _p(counts), _st(z)))
 
 
 @_timed
@@ -378,7 +402,7 @@ def moe_router(x: torch.Tensor, w: torch.Tensor, E: int, groups: int, keep: int,
     T, K, ldx = _rows2d(x)
     _, NR, ldz = _rows2d(z)
     assert w.dtype == torch.bfloat16 and w.is_contiguous() and tuple(w.shape) == (NR, K) and z.dtype == torch.float32 and z.shape[0] == T
-    _check(lib().b200seq_moe_router(_p(x), _DT[x.dtype], C.c_int64(ldx), _p(w), T, NR, K, E, groups, keep, top, _p(z), C.c_int64(ldz), _p(ids), _p(wts), _st(x)))
+    _check(lib().b200seq_moe_router(_p(x), _DT[x.dtype], ldx, _p(w), T, NR, K, E, groups, keep, top, _p(z), ldz, _p(ids), _p(wts), _st(x)))
 
 
 @_timed
@@ -402,8 +426,8 @@ def moe_linear(x: torch.Tensor, x_div: int, w: torch.Tensor, ids: torch.Tensor, 
     _, No, ldo = _rows2d(out)
     E, N = w.shape[0], w.shape[1]
     assert w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[2] == K and out.shape[0] >= pairs and No == (N // 2 if act in ACT_GATED else N)
-    _check(lib().b200seq_moe_linear_act(_p(x), _DT[x.dtype], C.c_int64(ldx), x_div, _p(w), _p(ids), _p(order), _p(offs), pairs, E, N, K, act, C.c_float(limit),
-                                        C.c_float(alpha), C.c_float(shift), _p(out), _DT[out.dtype], C.c_int64(ldo), _st(x)))
+    _check(lib().b200seq_moe_linear_act(_p(x), _DT[x.dtype], ldx, x_div, _p(w), _p(ids), _p(order), _p(offs), pairs, E, N, K, act, limit,
+                                        alpha, shift, _p(out), _DT[out.dtype], ldo, _st(x)))
 
 
 @_timed
@@ -414,7 +438,7 @@ def head_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ocol: int, 
     _, _, ldo = _rows2d(out)
     H, N, K = w.shape
     assert w.dtype == torch.bfloat16 and w.is_contiguous() and out.shape[0] == T and (act != ACT_NONE or out.dtype == torch.float32)
-    _check(lib().b200seq_head_linear(_p(x), _DT[x.dtype], C.c_int64(ldx), _p(w), T, H, N, K, act, _p(out), _DT[out.dtype], C.c_int64(ldo), C.c_int64(ocol), _st(x)))
+    _check(lib().b200seq_head_linear(_p(x), _DT[x.dtype], ldx, _p(w), T, H, N, K, act, _p(out), _DT[out.dtype], ldo, ocol, _st(x)))
 
 
 @_timed
@@ -423,7 +447,7 @@ def moe_gather(x: torch.Tensor, x_div: int, order: torch.Tensor, pairs: int, out
     _, K, ldx = _rows2d(x)
     _, _, ldo = _rows2d(out)
     assert x.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and out.shape[0] >= pairs and out.shape[1] == K
-    _check(lib().b200seq_moe_gather(_p(x), C.c_int64(ldx), _p(order), x_div, pairs, K, _p(out), C.c_int64(ldo), _st(x)))
+    _check(lib().b200seq_moe_gather(_p(x), ldx, _p(order), x_div, pairs, K, _p(out), ldo, _st(x)))
 
 
 @_timed
@@ -431,7 +455,7 @@ def moe_combine(ys: torch.Tensor, wts: torch.Tensor, slot_of: Optional[torch.Ten
                 y: torch.Tensor):
     W = y.shape[1]
     assert ys.is_contiguous() and y.is_contiguous() and (shared is None or shared.is_contiguous())
-    _check(lib().b200seq_moe_combine(_p(ys), _p(wts), _p(slot_of), T, top, W, _p(shared), _p(gate_z), C.c_int64(gate_z.stride(0) if gate_z is not None else 0), _p(y), _st(y)))
+    _check(lib().b200seq_moe_combine(_p(ys), _p(wts), _p(slot_of), T, top, W, _p(shared), _p(gate_z), gate_z.stride(0) if gate_z is not None else 0, _p(y), _st(y)))
 
 
 def tc_usable(x: torch.Tensor, K: int) -> bool:
@@ -442,7 +466,7 @@ def tc_usable(x: torch.Tensor, K: int) -> bool:
 @_timed
 def attn_prep(qkvg: torch.Tensor, step: "StepDesc", kpool: torch.Tensor, vpool: torch.Tensor, H: int, G: int, D: int, V: int, qk_eps: float):
     _, _, ld = _rows2d(qkvg)
-    _check(lib().b200seq_attn_prep(_p(qkvg), C.c_int64(ld), C.byref(step), _p(kpool), _p(vpool), H, G, D, V, C.c_float(qk_eps), _st(qkvg)))
+    _check(lib().b200seq_attn_prep(_p(qkvg), ld, C.byref(step), _p(kpool), _p(vpool), H, G, D, V, qk_eps, _st(qkvg)))
 
 
 def attn_scratch_floats(T: int, B: int, H: int, G: int, V: int, max_keys: int) -> int:
@@ -457,8 +481,8 @@ def attn(qkvg: torch.Tensor, step: "StepDesc", kpool: torch.Tensor, vpool: torch
          window: int, gated: bool, out: torch.Tensor, scratch: Optional[torch.Tensor] = None):
     _, _, ld = _rows2d(qkvg)
     assert out.is_contiguous() and (scratch is None or (scratch.dtype == torch.float32 and scratch.is_contiguous()))
-    _check(lib().b200seq_attn(_p(qkvg), C.c_int64(ld), C.byref(step), _p(kpool), _p(vpool), H, G, D, V, C.c_float(scale), chunk, window, int(gated),
-                              _p(out), _DT[out.dtype], _p(scratch), C.c_size_t(scratch.numel() if scratch is not None else 0), _st(qkvg)))
+    _check(lib().b200seq_attn(_p(qkvg), ld, C.byref(step), _p(kpool), _p(vpool), H, G, D, V, scale, chunk, window, int(gated),
+                              _p(out), _DT[out.dtype], _p(scratch), scratch.numel() if scratch is not None else 0, _st(qkvg)))
 
 
 @_timed
@@ -469,22 +493,22 @@ def latent_prep(proj: torch.Tensor, c_col: int, gate_col: int, q: torch.Tensor, 
     _, _, ldq = _rows2d(q)
     ldQ = _rows2d(Qp)[2] if Qp is not None else 0
     assert (qn is None or qn.is_contiguous()) and kpool.is_contiguous() and kpool.shape[-1] == R + Rd
-    _check(lib().b200seq_latent_prep(_p(proj), C.c_int64(ldp), c_col, gate_col, _p(q), C.c_int64(ldq), C.byref(step), H, Dn, Rd, R, _p(norm_w), C.c_float(eps),
-                                     _p(rot_freq), C.c_float(rot_scale), _p(kpool), _p(Qp), C.c_int64(ldQ), _p(qn), _DT[qn.dtype] if qn is not None else F32, _st(proj)))
+    _check(lib().b200seq_latent_prep(_p(proj), ldp, c_col, gate_col, _p(q), ldq, C.byref(step), H, Dn, Rd, R, _p(norm_w), eps,
+                                     _p(rot_freq), rot_scale, _p(kpool), _p(Qp), ldQ, _p(qn), _DT[qn.dtype] if qn is not None else F32, _st(proj)))
 
 
 @_timed
 def latent_gather(kpool: torch.Tensor, step: "StepDesc", R: int, ctx_rows: int, out: torch.Tensor):
     """out[r] = the latent (first R floats) of the r-th (entry, position) of the step's contexts, from the paged pool, in out's type"""
     assert kpool.is_contiguous() and out.is_contiguous() and out.shape[0] >= ctx_rows and out.shape[1] == R
-    _check(lib().b200seq_latent_gather(_p(kpool), C.c_int64(kpool.shape[-1]), C.byref(step), R, ctx_rows, _p(out), _DT[out.dtype], _st(kpool)))
+    _check(lib().b200seq_latent_gather(_p(kpool), kpool.shape[-1], C.byref(step), R, ctx_rows, _p(out), _DT[out.dtype], _st(kpool)))
 
 
 @_timed
 def rotary(x: torch.Tensor, col: int, nheads: int, D: int, step: "StepDesc", rot_freq: Optional[torch.Tensor], half: bool, rot_scale: float = 1.0, mult: float = 1.0):
     _, _, ld = _rows2d(x)
-    _check(lib().b200seq_rotary(_p(x), C.c_int64(ld), col, nheads, D, C.byref(step), 2 * rot_freq.numel() if rot_freq is not None else 0, int(half), _p(rot_freq),
-                                C.c_float(rot_scale), C.c_float(mult), _st(x)))
+    _check(lib().b200seq_rotary(_p(x), ld, col, nheads, D, C.byref(step), 2 * rot_freq.numel() if rot_freq is not None else 0, int(half), _p(rot_freq),
+                                rot_scale, mult, _st(x)))
 
 
 def retention_scratch_floats(T: int, B: int, H: int, D: int, V: int) -> int:
@@ -510,8 +534,8 @@ def retention(proj: torch.Tensor, step: "StepDesc", d: "RetentionDesc", state: t
         d2.sumsq = sumsq.data_ptr()
         d = d2
     assert out.is_contiguous() and state.is_contiguous() and (scratch is None or (scratch.dtype == torch.float32 and scratch.is_contiguous()))
-    _check(lib().b200seq_retention(_p(proj), C.c_int64(ld), C.byref(step), C.byref(d), _p(state), _p(out), _DT[out.dtype], _p(scratch),
-                                   C.c_size_t(scratch.numel() if scratch is not None else 0), _st(proj)))
+    _check(lib().b200seq_retention(_p(proj), ld, C.byref(step), C.byref(d), _p(state), _p(out), _DT[out.dtype], _p(scratch),
+                                   scratch.numel() if scratch is not None else 0, _st(proj)))
 
 
 @_timed
@@ -531,7 +555,7 @@ def post_norm(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], eps: 
     R = x.shape[0] if rows is None else rows.numel()
     o = a_out if a_out is not None else a_shift_out
     assert x.is_contiguous() and (y is None or y.is_contiguous())
-    _check(lib().b200seq_post_norm(_p(x), _p(y), _p(zg), C.c_int64(zg.stride(0) if zg is not None else 0), _p(gate_b), C.c_float(alpha), _p(w), _p(b), C.c_float(eps), W,
+    _check(lib().b200seq_post_norm(_p(x), _p(y), _p(zg), zg.stride(0) if zg is not None else 0, _p(gate_b), alpha, _p(w), _p(b), eps, W,
                                    _p(rows), R, _p(x_out), _p(a_out), _DT[o.dtype] if o is not None else F32, _p(state_out), _p(next_mu), _p(next_state), _p(a_shift_out),
                                    C.byref(step) if step is not None else None, _st(x)))
 
@@ -549,8 +573,8 @@ def ssm_scan(proj: torch.Tensor, z0: int, dt0: int, xbc: torch.Tensor, A_log: to
     _, _, ldp = _rows2d(proj)
     _, _, ldx = _rows2d(xbc)
     assert out.is_contiguous() and (scratch is None or (scratch.dtype == torch.float32 and scratch.is_contiguous()))
-    _check(lib().b200seq_ssm_scan(_p(proj), C.c_int64(ldp), z0, dt0, _p(xbc), C.c_int64(ldx), _p(A_log), _p(Dp), _p(dt_bias), _p(state), C.byref(step),
-                                  H, V, N, G, _p(out), _p(scratch), C.c_size_t(scratch.numel() if scratch is not None else 0), _st(proj)))
+    _check(lib().b200seq_ssm_scan(_p(proj), ldp, z0, dt0, _p(xbc), ldx, _p(A_log), _p(Dp), _p(dt_bias), _p(state), C.byref(step),
+                                  H, V, N, G, _p(out), _p(scratch), scratch.numel() if scratch is not None else 0, _st(proj)))
 
 
 @_timed
@@ -571,7 +595,7 @@ def moe_route_ex(z: torch.Tensor, E: int, groups: int, keep: int, top: int, kind
     T, _, ldz = _rows2d(z)
     assert ids.dtype == torch.int32 and wts.dtype == torch.float32 and ids.is_contiguous() and wts.is_contiguous() and ids.numel() >= T * top
     assert correction is None or (correction.dtype == torch.float32 and correction.numel() == E)
-    _check(lib().b200seq_moe_route_ex(_p(z), C.c_int64(ldz), T, E, groups, keep, top, kind, _p(correction), _p(ids), _p(wts), _p(counts), _st(z)))
+    _check(lib().b200seq_moe_route_ex(_p(z), ldz, T, E, groups, keep, top, kind, _p(correction), _p(ids), _p(wts), _p(counts), _st(z)))
 
 
 @_timed
@@ -581,7 +605,7 @@ def moe_router_ex(x: torch.Tensor, w: torch.Tensor, E: int, groups: int, keep: i
     T, K, ldx = _rows2d(x)
     _, NR, ldz = _rows2d(z)
     assert w.dtype == torch.bfloat16 and w.is_contiguous() and tuple(w.shape) == (NR, K) and z.dtype == torch.float32 and z.shape[0] == T
-    _check(lib().b200seq_moe_router_ex(_p(x), _DT[x.dtype], C.c_int64(ldx), _p(w), T, NR, K, E, groups, keep, top, kind, _p(correction), _p(z), C.c_int64(ldz), _p(ids),
+    _check(lib().b200seq_moe_router_ex(_p(x), _DT[x.dtype], ldx, _p(w), T, NR, K, E, groups, keep, top, kind, _p(correction), _p(z), ldz, _p(ids),
                                        _p(wts), _st(x)))
 
 
@@ -592,7 +616,7 @@ def moe_combine_ex(ys: torch.Tensor, wts: torch.Tensor, slot_of: Optional[torch.
     W = y.shape[1]
     assert ys.is_contiguous() and y.is_contiguous() and (shared is None or shared.is_contiguous()) and x_id.is_contiguous() and x_id.dtype == torch.float32
     _check(lib().b200seq_moe_combine_ex(_p(ys), _p(wts), _p(slot_of), _p(ids), E_real, _p(x_id), T, top, W, _p(shared), _p(gate_z),
-                                        C.c_int64(gate_z.stride(0) if gate_z is not None else 0), _p(y), _st(y)))
+                                        gate_z.stride(0) if gate_z is not None else 0, _p(y), _st(y)))
 
 
 @_timed
@@ -602,8 +626,8 @@ def causal_conv_ex(x: torch.Tensor, in_bias: Optional[torch.Tensor], w: torch.Te
     T, Cn, ldx = _rows2d(x)
     _, _, ldo = _rows2d(out)
     ldo2 = _rows2d(out2)[2] if out2 is not None else 0
-    _check(lib().b200seq_causal_conv_ex(_p(x), C.c_int64(ldx), _p(in_bias), _p(w), _p(bias), _p(state), C.byref(step), Cn, w.shape[1], mode, _p(out), _DT[out.dtype],
-                                        C.c_int64(ldo), _p(out2), _DT[out2.dtype] if out2 is not None else F32, C.c_int64(ldo2), _st(x)))
+    _check(lib().b200seq_causal_conv_ex(_p(x), ldx, _p(in_bias), _p(w), _p(bias), _p(state), C.byref(step), Cn, w.shape[1], mode, _p(out), _DT[out.dtype],
+                                        ldo, _p(out2), _DT[out2.dtype] if out2 is not None else F32, ldo2, _st(x)))
 
 
 @_timed
@@ -613,7 +637,7 @@ def embed_bigram(table: torch.Tensor, bigram: Optional[torch.Tensor], ids: torch
     W = x.shape[-1]
     assert table.dtype == torch.bfloat16 and table.is_contiguous() and x.is_contiguous() and x.dtype == torch.float32 and (a is None or a.is_contiguous())
     assert bigram is None or (bigram.dtype == torch.bfloat16 and bigram.is_contiguous() and tuple(bigram.shape) == (buckets + 1, W))
-    _check(lib().b200seq_embed_bigram(_p(table), _p(bigram), _p(ids), _p(ent_prev), C.byref(step), C.c_float(scale), buckets, mul_prev, mul_cur, W, _p(x), _p(a),
+    _check(lib().b200seq_embed_bigram(_p(table), _p(bigram), _p(ids), _p(ent_prev), C.byref(step), scale, buckets, mul_prev, mul_cur, W, _p(x), _p(a),
                                       _DT[a.dtype] if a is not None else F32, _st(x)))
 
 
@@ -625,7 +649,7 @@ def branch_norm(x: torch.Tensor, y1: torch.Tensor, w: torch.Tensor, eps: float, 
     W = x.shape[-1]
     R = x.shape[0] if rows is None else rows.numel()
     assert x.is_contiguous() and y1.is_contiguous() and (y2 is None or y2.is_contiguous()) and (a_out is None or a_out.is_contiguous())
-    _check(lib().b200seq_branch_norm(_p(x), _p(y1), _p(bias1), _p(w_b1), C.c_float(s1), _p(y2), _p(w_b2), C.c_float(s2), _p(w), C.c_float(eps), W, _p(rows), R, _p(x_out),
+    _check(lib().b200seq_branch_norm(_p(x), _p(y1), _p(bias1), _p(w_b1), s1, _p(y2), _p(w_b2), s2, _p(w), eps, W, _p(rows), R, _p(x_out),
                                      _p(a_out), _DT[a_out.dtype] if a_out is not None else F32, _p(fin_w), _st(x)))
 
 
@@ -635,13 +659,13 @@ def polynorm(z: torch.Tensor, coef: torch.Tensor, eps: float, out: torch.Tensor)
     T, F, ldz = _rows2d(z)
     _, _, ldo = _rows2d(out)
     assert coef.dtype == torch.float32 and coef.numel() == 4 and out.shape[1] == F
-    _check(lib().b200seq_polynorm(_p(z), C.c_int64(ldz), T, F, _p(coef), C.c_float(eps), _p(out), _DT[out.dtype], C.c_int64(ldo), _st(z)))
+    _check(lib().b200seq_polynorm(_p(z), ldz, T, F, _p(coef), eps, _p(out), _DT[out.dtype], ldo, _st(z)))
 
 
 @_timed
 def softcap(x: torch.Tensor, cap: float):
     assert x.is_contiguous() and x.dtype == torch.float32
-    _check(lib().b200seq_softcap(_p(x), C.c_int64(x.numel()), C.c_float(cap), _st(x)))
+    _check(lib().b200seq_softcap(_p(x), x.numel(), cap, _st(x)))
 
 
 @_timed
@@ -649,14 +673,14 @@ def diff_combine(a: torch.Tensor, H: int, G: int, V: int, lam: float, out_scale:
     """a f32 [T, 2 * H * V], the two maps per head in the order [key group][map][head of the group] -> out [T, H * V] = unit_rms(a1 - lam * a2) * out_scale"""
     T = a.shape[0]
     assert a.is_contiguous() and a.dtype == torch.float32 and a.shape[1] == 2 * H * V and out.is_contiguous() and tuple(out.shape) == (T, H * V)
-    _check(lib().b200seq_diff_combine(_p(a), T, H, G, V, C.c_float(lam), C.c_float(out_scale), C.c_float(eps), _p(out), _DT[out.dtype], _st(a)))
+    _check(lib().b200seq_diff_combine(_p(a), T, H, G, V, lam, out_scale, eps, _p(out), _DT[out.dtype], _st(a)))
 
 
 @_timed
 def min_gru(proj: torch.Tensor, z_col: int, x_col: int, g_col: int, bias: Optional[torch.Tensor], state: torch.Tensor, step: "StepDesc", Cn: int, out: torch.Tensor):
     _, _, ldp = _rows2d(proj)
     assert out.is_contiguous() and out.shape[1] == Cn and state.is_contiguous() and state.shape[1] == Cn
-    _check(lib().b200seq_min_gru(_p(proj), C.c_int64(ldp), z_col, x_col, g_col, _p(bias), _p(state), C.byref(step), Cn, _p(out), _DT[out.dtype], _st(proj)))
+    _check(lib().b200seq_min_gru(_p(proj), ldp, z_col, x_col, g_col, _p(bias), _p(state), C.byref(step), Cn, _p(out), _DT[out.dtype], _st(proj)))
 
 
 @_timed
@@ -666,7 +690,7 @@ def rg_lru(u: torch.Tensor, gates: torch.Tensor, gate_bias: Optional[torch.Tenso
     _, _, ldg = _rows2d(gates)
     _, _, ldp = _rows2d(proj)
     assert out.is_contiguous() and out.shape[1] == Cn and state.is_contiguous() and state.shape[1] == Cn and sp_lam.numel() == Cn
-    _check(lib().b200seq_rg_lru(_p(u), C.c_int64(ldu), _p(gates), C.c_int64(ldg), _p(gate_bias), _p(sp_lam), C.c_float(decay_c), _p(proj), C.c_int64(ldp), y_col, _p(bias),
+    _check(lib().b200seq_rg_lru(_p(u), ldu, _p(gates), ldg, _p(gate_bias), _p(sp_lam), decay_c, _p(proj), ldp, y_col, _p(bias),
                                 _p(state), C.byref(step), Cn, blocks, _p(out), _DT[out.dtype], _st(proj)))
 
 
@@ -683,8 +707,8 @@ def delta(proj: torch.Tensor, step: "StepDesc", d: "DeltaDesc", wz: Optional[tor
     """wz f32 [T, H * D]: low-rank branch output (steps with portions; None in steps of single tokens, where the kernel applies w2 itself)"""
     _, _, ld = _rows2d(proj)
     assert out.is_contiguous() and state.is_contiguous() and (scratch is None or (scratch.dtype == torch.float32 and scratch.is_contiguous()))
-    _check(lib().b200seq_delta(_p(proj), C.c_int64(ld), C.byref(step), C.byref(d), _p(wz), C.c_int64(wz.stride(0) if wz is not None else 0), _p(state), _p(out),
-                               _DT[out.dtype], _p(scratch), C.c_size_t(scratch.numel() if scratch is not None else 0), _st(proj)))
+    _check(lib().b200seq_delta(_p(proj), ld, C.byref(step), C.byref(d), _p(wz), wz.stride(0) if wz is not None else 0, _p(state), _p(out),
+                               _DT[out.dtype], _p(scratch), scratch.numel() if scratch is not None else 0, _st(proj)))
 
 
 def position_frequencies(width: int, base: float) -> torch.Tensor:
@@ -701,7 +725,7 @@ def embed_pos(table: torch.Tensor, ids: torch.Tensor, step: "StepDesc", scale: f
     """x[t] = table[ids[t]] * scale + sinusoid(pos) (+ add_vec); x0: the same without add_vec; a: x, normed with fin_w when given, in its own type"""
     W = x.shape[-1]
     assert table.dtype == torch.bfloat16 and table.is_contiguous() and x.is_contiguous() and (freq is None or tuple(freq.shape) == (2, (W + 1) // 2))
-    _check(lib().b200seq_embed_pos(_p(table), _p(ids), C.byref(step), C.c_float(scale), _p(freq), W, _p(x0), _p(add_vec), _p(x), _p(fin_w), C.c_float(eps), _p(a),
+    _check(lib().b200seq_embed_pos(_p(table), _p(ids), C.byref(step), scale, _p(freq), W, _p(x0), _p(add_vec), _p(x), _p(fin_w), eps, _p(a),
                                    _DT[a.dtype] if a is not None else F32, _st(x)))
 
 
@@ -713,7 +737,7 @@ def sandwich_norm(x: torch.Tensor, eps: float, *, y: Optional[torch.Tensor] = No
     W = x.shape[-1]
     R = x.shape[0] if rows is None else rows.numel()
     assert x.is_contiguous() and (y is None or y.is_contiguous()) and (a_out is None or a_out.is_contiguous()) and (add_row is None or add_row.is_contiguous())
-    _check(lib().b200seq_sandwich_norm(_p(x), _p(y), _p(w), C.c_float(eps), _p(add_row), _p(add_vec), W, _p(rows), R, _p(x_out), _p(a_out),
+    _check(lib().b200seq_sandwich_norm(_p(x), _p(y), _p(w), eps, _p(add_row), _p(add_vec), W, _p(rows), R, _p(x_out), _p(a_out),
                                        _DT[a_out.dtype] if a_out is not None else F32, _p(fin_w), _st(x)))
 
 
@@ -722,7 +746,7 @@ def token_gate(z: torch.Tensor, table: torch.Tensor, col: int, ids: torch.Tensor
     """out[t] = gelu_tanh(z[t]) * table[ids[t]][col : col + dim]"""
     T, dim, ldz = _rows2d(z)
     assert table.dtype == torch.bfloat16 and table.is_contiguous() and out.is_contiguous() and tuple(out.shape) == (T, dim)
-    _check(lib().b200seq_token_gate(_p(z), C.c_int64(ldz), T, dim, _p(table), C.c_int64(table.shape[1]), col, _p(ids), _p(out), _DT[out.dtype], _st(z)))
+    _check(lib().b200seq_token_gate(_p(z), ldz, T, dim, _p(table), table.shape[1], col, _p(ids), _p(out), _DT[out.dtype], _st(z)))
 
 
 @_timed
@@ -735,7 +759,7 @@ def side_close(x: torch.Tensor, y: torch.Tensor, w: torch.Tensor, eps: float, ga
     dim = gate.shape[0]
     assert x.is_contiguous() and y.is_contiguous() and tuple(gate.shape) == (dim, W) and tuple(proj.shape) == (W, dim) and gate.is_contiguous() and proj.is_contiguous()
     assert gate.dtype == proj.dtype == table.dtype == torch.bfloat16 and table.is_contiguous()
-    _check(lib().b200seq_side_close(_p(x), _p(y), _p(w), C.c_float(eps), _p(gate), _p(proj), _p(table), C.c_int64(table.shape[1]), col, dim, _p(ids), _p(side_w),
+    _check(lib().b200seq_side_close(_p(x), _p(y), _p(w), eps, _p(gate), _p(proj), _p(table), table.shape[1], col, dim, _p(ids), _p(side_w),
                                     _p(add_row), _p(add_vec), W, _p(rows), R, _p(x_out), _p(a_out), _DT[a_out.dtype] if a_out is not None else F32, _p(fin_w), _st(x)))
 
 
@@ -757,7 +781,7 @@ def route_desc(E: int, groups: int, keep: int, top: int, kind: int, *, group_bes
 def moe_route_rule(z: torch.Tensor, d: "RouteDesc", ids: torch.Tensor, wts: torch.Tensor, counts: Optional[torch.Tensor]):
     T, _, ldz = _rows2d(z)
     assert ids.dtype == torch.int32 and wts.dtype == torch.float32 and ids.is_contiguous() and wts.is_contiguous() and ids.numel() >= T * d.top
-    _check(lib().b200seq_moe_route_rule(_p(z), C.c_int64(ldz), T, C.byref(d), _p(ids), _p(wts), _p(counts), _st(z)))
+    _check(lib().b200seq_moe_route_rule(_p(z), ldz, T, C.byref(d), _p(ids), _p(wts), _p(counts), _st(z)))
 
 
 @_timed
@@ -766,7 +790,7 @@ def moe_router_rule(x: torch.Tensor, w: torch.Tensor, d: "RouteDesc", z: torch.T
     T, K, ldx = _rows2d(x)
     _, NR, ldz = _rows2d(z)
     assert w.dtype == torch.bfloat16 and w.is_contiguous() and tuple(w.shape) == (NR, K) and z.dtype == torch.float32 and z.shape[0] == T
-    _check(lib().b200seq_moe_router_rule(_p(x), _DT[x.dtype], C.c_int64(ldx), _p(w), T, NR, K, C.byref(d), _p(z), C.c_int64(ldz), _p(ids), _p(wts), _st(x)))
+    _check(lib().b200seq_moe_router_rule(_p(x), _DT[x.dtype], ldx, _p(w), T, NR, K, C.byref(d), _p(z), ldz, _p(ids), _p(wts), _st(x)))
 
 
 class ScanDesc(C.Structure):
@@ -798,8 +822,8 @@ def selective_scan(u: torch.Tensor, dbc: torch.Tensor, dtz: Optional[torch.Tenso
     assert u.is_contiguous() and u.shape[1] == d.C and out.is_contiguous() and out.shape[1] == d.C and state.is_contiguous() and tuple(state.shape[1:]) == (d.C, d.N)
     assert dbc.dtype == gate.dtype == state.dtype == torch.float32 and (dtz is None or (dtz.dtype == torch.float32 and dtz.is_contiguous() and dtz.shape[1] == d.C))
     assert scratch is None or (scratch.dtype == torch.float32 and scratch.is_contiguous())
-    _check(lib().b200seq_selective_scan(_p(u), _DT[u.dtype], _p(dbc), C.c_int64(ldd), _p(dtz), _p(gate), C.c_int64(ldg), C.byref(step), C.byref(d), _p(state), _p(out),
-                                        _DT[out.dtype], _p(scratch), C.c_size_t(scratch.numel() if scratch is not None else 0), _st(dbc)))
+    _check(lib().b200seq_selective_scan(_p(u), _DT[u.dtype], _p(dbc), ldd, _p(dtz), _p(gate), ldg, C.byref(step), C.byref(d), _p(state), _p(out),
+                                        _DT[out.dtype], _p(scratch), scratch.numel() if scratch is not None else 0, _st(dbc)))
 
 
 class ParallelDesc(C.Structure):
