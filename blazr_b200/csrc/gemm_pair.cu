@@ -36,18 +36,20 @@ static bool pair_plan(const b200q_weight* w, int64_t M, PairPlan* p) {
     return true;
 }
 
-// Which products take this kernel: those that the fused kernel does not cut along K (it then has fewer than half as many tiles as SMs), from 512 rows on, and
-// from 192 where the estimated waves are fewer.  Measured in loops of seconds (us, expanded once by gemm_wide.cu / fused / this): Q6_K 14336 x 4096, 2048 rows
-// 260 / 256 / 240, 1300 rows 193 / 167 / 153, 900 rows 148 / 136 / 112, 512 rows - / 68.5 / 65; Q4_K 16384 x 2048, 2048 rows 151 / 165 / 130, 1000 rows
-// - / 89 / 72; 2048 x 8192, 1536 rows 70 / 64 / 61; 10240 x 8192, 1000 rows 224 / 183 / 162; Q8_0 6144 x 4096, 1800 rows 121 / 110 / 95; AWQ 6144 x 4096, 1531
-// rows 89 / 76 / 72; 57344 x 8192, 250 rows - / 250 / 216.  Where it is the slower one it is so by 5 %: Q8_0 6144 x 4096, 600 rows - / 34 / 36; Q6_K 8192 x 8192,
-// 520 rows - / 92 / 97; Q4_K 8192 x 28672, 500 rows - / 215 / 227.
+// Which products take this kernel: those that the fused kernel does not cut along K (it then has fewer than half as many tiles as SMs), from 512 rows on where
+// that kernel needs two waves and more, else where the estimates say so, with a launch of staged rows and a set-up that cost 4 us more here, and something in
+// hand.  Measured in loops of seconds (us, expanded once by gemm_wide.cu / fused / this): Q6_K 14336 x 4096, 2048 rows 260 / 256 / 240, 1300 rows
+// 193 / 167 / 153, 900 rows 148 / 136 / 112, 512 rows - / 68.5 / 65; Q4_K 16384 x 2048, 2048 rows 151 / 165 / 130, 1000 rows - / 89 / 72; 2048 x 8192, 1536 rows
+// 70 / 64 / 61; 10240 x 8192, 1000 rows 224 / 183 / 162; Q8_0 6144 x 4096, 1800 rows 121 / 110 / 95; AWQ 6144 x 4096, 1531 rows 89 / 76 / 72; 57344 x 8192, 250
+// rows - / 250 / 216; the fused kernel in one wave: Q8_0 6144 x 4096, 600 rows - / 34 / 36; GPTQ 4096 x 4096, 887 rows - / 33 / 34; Q4_K 8192 x 28672, 500 rows
+// - / 215 / 227.  Where this one is taken and is the slower one it is so by 5 %: Q6_K 8192 x 8192, 520 rows - / 92 / 97.
 bool gemm_pair_wins(const b200q_weight* w, int64_t M) {
     PairPlan p;
     if (M < 192 || M > INT32_MAX / 2 || w->N % (2 * TILE_ROWS) != 0 || w->N > INT32_MAX || gemm_k_splits(w, M) > 1 || !pair_plan(w, M, &p)) return false;
-    if (M >= 512) return true;
-    const int64_t mt = (M + 255) / 256, rows = ((M + mt - 1) / mt + 31) / 32 * 32;
-    return (double)pair_waves(w, M, p.bt) * pair_wave_us(p.bt) < 0.95 * (double)((w->T * mt + w->num_sms - 1) / w->num_sms) * fused_wave_us(rows);
+    const int64_t mt = (M + 255) / 256, rows = ((M + mt - 1) / mt + 31) / 32 * 32, waves = (w->T * mt + w->num_sms - 1) / w->num_sms;
+    if (M >= 512 && waves > 1) return true;
+    const double deep = (double)w->K_pad / 4096.0;
+    return ((double)pair_waves(w, M, p.bt) * pair_wave_us(p.bt) * deep + 4.0) * (waves > 1 ? 1.03 : 1.09) < (double)waves * fused_wave_us(rows) * deep;
 }
 
 static cudaError_t pair_family(int family, const PairParams& p, const CUtensorMap& mx, int ctas, int smem, cudaStream_t st) {

@@ -44,7 +44,7 @@ def test_the_bits_of_the_fused_kernel(client, fmt, N, K, M):
     assert bool((y[M] == 7).all()) and bool((y[:, N:] == 7).all())
 
 
-@pytest.mark.parametrize("fmt,N,K,M", [("Q4_K", 256, 512, 512), ("Q6_K", 512, 256, 4099), ("Q8_0", 2560, 1056, 1537), ("GPTQ", 20480, 512, 1300), ("AWQ", 28672, 640, 260), ("Q6_K", 28672, 768, 250)])
+@pytest.mark.parametrize("fmt,N,K,M", [("Q4_K", 12800, 512, 512), ("Q6_K", 2560, 256, 4099), ("Q8_0", 5120, 1056, 1537), ("GPTQ", 20480, 512, 1300), ("AWQ", 28672, 4096, 250)])
 @pytest.mark.parametrize("dt", [torch.float32, torch.float16, torch.bfloat16])
 def test_against_the_dequantized_weight(client, fmt, N, K, M, dt):
     w, b = weight(client, fmt, N, K)
