@@ -41,6 +41,7 @@ __device__ __forceinline__ void pool_block(const b200seq_step& st, const int32_t
 // block that stores the last position of a pooled block also writes the block's mean -- the other rows are in the pool already.
 __global__ void attn_prep_kernel(float* __restrict__ proj, int64_t ld, b200seq_step st, const b200seq_attn_desc a, float* __restrict__ kpool,
                                  float* __restrict__ vpool, float* __restrict__ kpp, float* __restrict__ vpp, int fuse_pool, int* err) {
+    chain_enter();
     extern __shared__ float rot_sm[];
     const int t = blockIdx.x;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -389,6 +390,7 @@ __device__ __forceinline__ float dot4(const float4 a, const float4 b, float acc)
 
 template <int RT, int VPT>
 __global__ void __launch_bounds__(AT_NT, (VPT == 4) ? 3 : (VPT == 8 ? 2 : 1)) attn_tile_kernel(const AttnArgs a, const b200seq_step st) {
+    chain_enter();
     extern __shared__ __align__(16) float sm[];
     constexpr int RQ = 16 * RT, VS = 16 * VPT, PS = AT_KT + 4;
     const int D = a.D, V = a.V, H = a.H, G = a.G;
@@ -615,6 +617,7 @@ __global__ void __launch_bounds__(AT_NT, (VPT == 4) ? 3 : (VPT == 8 ? 2 : 1)) at
 
 // grid (T, H): merges the splits of one (token, head) in split order
 __global__ void attn_merge_kernel(const AttnArgs a) {
+    chain_enter();
     const int t = blockIdx.x, h = blockIdx.y;
     const int V = a.V, ns = a.nsplit;
     const float* pp = a.part + ((int64_t)t * a.H + h) * ns * (V + 2);
@@ -713,7 +716,7 @@ int b200seq_attn_prep_ex(float* proj, int64_t ld, const b200seq_step* st, const 
         return 0;
     }
     const int fuse_pool = d->pool > 0 && st->T == st->B;   // one token per entry: no other block of this step writes a row the mean reads
-    attn_prep_kernel<<<st->T, 256, (size_t)d->rot_dims * sizeof(float), (cudaStream_t)stream>>>(proj, ld, *st, *d, kpool, vpool, kpooled, vpooled, fuse_pool,
+    launch_chained(attn_prep_kernel, st->T, 256, (size_t)d->rot_dims * sizeof(float), (cudaStream_t)stream, proj, ld, *st, *d, kpool, vpool, kpooled, vpooled, fuse_pool,
                                                                                                  error_flag_dev());
     SEQ_LAUNCH_CHECK("attn_prep");
     if (d->pool > 0 && !fuse_pool) {
@@ -788,7 +791,7 @@ int b200seq_attn_ex(const float* qkvg, int64_t ld, const b200seq_step* st, const
     cudaStream_t cs = (cudaStream_t)stream;
     auto merge = [&]() -> int {
         if (a.nsplit > 1) {
-            attn_merge_kernel<<<dim3(st->T, H), V <= 64 ? 64 : 128, 0, cs>>>(a);
+            launch_chained(attn_merge_kernel, dim3(st->T, H), V <= 64 ? 64 : 128, 0, cs, a);
             SEQ_LAUNCH_CHECK("attn merge");
         }
         return 0;
@@ -814,7 +817,7 @@ int b200seq_attn_ex(const float* qkvg, int64_t ld, const b200seq_step* st, const
             e = cudaFuncSetAttribute(attn_tile_kernel<RT_, VPT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
             set_ = smem;                                                                                                        \
         }                                                                                                                       \
-        if (e == cudaSuccess) attn_tile_kernel<RT_, VPT_><<<grid, AT_NT, smem, cs>>>(a, *st);                                   \
+        if (e == cudaSuccess) launch_chained(attn_tile_kernel<RT_, VPT_>, grid, AT_NT, smem, cs, a, *st);                                   \
     } while (0)
     if (p.RT == 4) {
         if (VPT == 4) ATT_LAUNCH(4, 4);

@@ -132,6 +132,7 @@ __device__ __noinline__ void plain_row(const AttnArgs& a, const b200seq_step& st
 // 0.21 instructions per cycle) and took 860 us where it now takes 206 (4096 tokens, 32 heads of 64, chunks of 2048; the f32 tiles: 1 656).
 template <int MT, int VM, int DK, bool CAP>
 __global__ void __launch_bounds__((4 * MT + 12) * 32, 1) attn_tc_kernel(const __grid_constant__ AttnArgs a, const __grid_constant__ b200seq_step st) {
+    chain_enter();
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint32_t tmem_base;
     __shared__ int abort_sh;
@@ -559,7 +560,7 @@ cudaError_t run_cap(const AttnArgs& a, const b200seq_step& st, dim3 grid, cudaSt
         if (e != cudaSuccess) return e;
         if (dev < 16) ready[dev] = smem;
     }
-    attn_tc_kernel<MT, VM, DK, CAP><<<grid, (4 * MT + 12) * 32, smem, cs>>>(a, st);
+    launch_chained(attn_tc_kernel<MT, VM, DK, CAP>, grid, (4 * MT + 12) * 32, smem, cs, a, st);
     return cudaGetLastError();
 }
 

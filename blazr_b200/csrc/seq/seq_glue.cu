@@ -351,6 +351,7 @@ __global__ void group_rmsnorm_kernel(const float* __restrict__ x, int64_t ldx, c
 // F outputs per row; gated kinds read the pair (gate f, up f) from columns (2f, 2f + 1) (interleaved) or (f, F + f)
 __global__ void gated_act_kernel(const float* __restrict__ gu, int64_t ldg, int T, int F, const ActParams act, int interleaved, void* __restrict__ out,
                                  int out_dtype, int64_t ldo) {
+    chain_enter();
     const int64_t n = (int64_t)T * F;
     const bool gated = act_is_gated(act.kind);
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (int64_t)gridDim.x * blockDim.x) {
@@ -541,7 +542,7 @@ int b200seq_gated_act(const float* gu, int64_t ldg, int T, int F, float limit, f
     if (T == 0) return 0;
     const int64_t n = (int64_t)T * F;
     const int blocks = (int)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
-    gated_act_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(gu, ldg, T, F, ActParams{B200SEQ_ACT_SWISH_CLAMP, limit, alpha, up_shift}, interleaved, out, out_dtype, F);
+    launch_chained(gated_act_kernel, blocks, 256, 0, (cudaStream_t)stream, gu, ldg, T, F, ActParams{B200SEQ_ACT_SWISH_CLAMP, limit, alpha, up_shift}, interleaved, out, out_dtype, F);
     SEQ_LAUNCH_CHECK("gated_act");
     return 0;
 }
@@ -552,7 +553,7 @@ int b200seq_act(const float* z, int64_t ldz, int T, int N, int act, float limit,
     const int F = act_kind_gated(act) ? N / 2 : N;
     const int64_t n = (int64_t)T * F;
     const int blocks = (int)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
-    gated_act_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(z, ldz, T, F, ActParams{act, limit, alpha, shift}, 1, out, out_dtype, ldo);
+    launch_chained(gated_act_kernel, blocks, 256, 0, (cudaStream_t)stream, z, ldz, T, F, ActParams{act, limit, alpha, shift}, 1, out, out_dtype, ldo);
     SEQ_LAUNCH_CHECK("act");
     return 0;
 }

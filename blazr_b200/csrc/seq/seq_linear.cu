@@ -43,6 +43,7 @@ __device__ __forceinline__ float silu_range(float v, int n, int lo, int hi) { re
 template <typename XT, int MB, bool VEC>
 __global__ void __launch_bounds__(256) linear_rows_kernel(const XT* __restrict__ x, int64_t ldx, const __nv_bfloat16* __restrict__ w, int M, int N, int K,
                                                           float* __restrict__ y, int64_t ldy, int rows_per_warp, const GateEpi ge) {
+    chain_enter();
     const int lane = threadIdx.x & 31;
     const int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int n0 = warp * rows_per_warp;
@@ -117,6 +118,7 @@ constexpr int TM = 64, TN = 64, TK = 16;
 template <typename XT>
 __global__ void __launch_bounds__(256) linear_tiled_kernel(const XT* __restrict__ x, int64_t ldx, const __nv_bfloat16* __restrict__ w, int M, int N, int K,
                                                            float* __restrict__ y, int64_t ldy, int silu_lo, int silu_hi) {
+    chain_enter();
     __shared__ float xs[TK][TM + 4];
     __shared__ float ws[TK][TN + 4];
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
@@ -170,14 +172,14 @@ static void launch_rows(const XT* x, int64_t ldx, const __nv_bfloat16* w, int M,
     const int warps = (N + rpw - 1) / rpw;
     const int blocks = (warps + 7) / 8;
     if (M <= 1) {
-        if (vec) linear_rows_kernel<XT, 1, true><<<blocks, 256, 0, st>>>(x, ldx, w, M, N, K, y, ldy, rpw, ge);
-        else linear_rows_kernel<XT, 1, false><<<blocks, 256, 0, st>>>(x, ldx, w, M, N, K, y, ldy, rpw, ge);
+        if (vec) launch_chained(linear_rows_kernel<XT, 1, true>, blocks, 256, 0, st, x, ldx, w, M, N, K, y, ldy, rpw, ge);
+        else launch_chained(linear_rows_kernel<XT, 1, false>, blocks, 256, 0, st, x, ldx, w, M, N, K, y, ldy, rpw, ge);
     } else if (M <= 2) {
-        if (vec) linear_rows_kernel<XT, 2, true><<<blocks, 256, 0, st>>>(x, ldx, w, M, N, K, y, ldy, rpw, ge);
-        else linear_rows_kernel<XT, 2, false><<<blocks, 256, 0, st>>>(x, ldx, w, M, N, K, y, ldy, rpw, ge);
+        if (vec) launch_chained(linear_rows_kernel<XT, 2, true>, blocks, 256, 0, st, x, ldx, w, M, N, K, y, ldy, rpw, ge);
+        else launch_chained(linear_rows_kernel<XT, 2, false>, blocks, 256, 0, st, x, ldx, w, M, N, K, y, ldy, rpw, ge);
     } else {
-        if (vec) linear_rows_kernel<XT, 4, true><<<blocks, 256, 0, st>>>(x, ldx, w, M, N, K, y, ldy, rpw, ge);
-        else linear_rows_kernel<XT, 4, false><<<blocks, 256, 0, st>>>(x, ldx, w, M, N, K, y, ldy, rpw, ge);
+        if (vec) launch_chained(linear_rows_kernel<XT, 4, true>, blocks, 256, 0, st, x, ldx, w, M, N, K, y, ldy, rpw, ge);
+        else launch_chained(linear_rows_kernel<XT, 4, false>, blocks, 256, 0, st, x, ldx, w, M, N, K, y, ldy, rpw, ge);
     }
 }
 
@@ -210,8 +212,8 @@ extern "C" int b200seq_linear_silu(const void* x, int x_dtype, int64_t ldx, cons
         else launch_rows((const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, M, N, K, y, ldy, st, ge);
     } else if (path == B200SEQ_PATH_TILED) {
         dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM);
-        if (x_dtype == B200SEQ_F32) linear_tiled_kernel<<<grid, 256, 0, st>>>((const float*)x, ldx, (const __nv_bfloat16*)w, M, N, K, y, ldy, silu_lo, silu_hi);
-        else linear_tiled_kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, M, N, K, y, ldy, silu_lo, silu_hi);
+        if (x_dtype == B200SEQ_F32) launch_chained(linear_tiled_kernel<float>, grid, 256, 0, st, (const float*)x, ldx, (const __nv_bfloat16*)w, M, N, K, y, ldy, silu_lo, silu_hi);
+        else launch_chained(linear_tiled_kernel<__nv_bfloat16>, grid, 256, 0, st, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, M, N, K, y, ldy, silu_lo, silu_hi);
     } else {
         return fail(B200SEQ_ERR_INVALID_ARG, "linear: unknown path %d", path);
     }

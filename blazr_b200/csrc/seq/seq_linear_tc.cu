@@ -115,6 +115,7 @@ struct TcParams {
 constexpr int EPI_NONE = 0, EPI_GATED = 1, EPI_PLAIN_ACT = 2;
 
 __global__ void __launch_bounds__(128) linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const TcParams p) {
+    chain_enter();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t full[STAGES], empty[STAGES], acc_full;
@@ -362,7 +363,7 @@ template <class Epi>
 cudaError_t launch_pair(int bt, const void* x, int64_t ldx, const void* w, const TcParams& p, const Epi& epi, cudaStream_t st) {
     tcpair::Args a{};
     a.M = p.M, a.N = p.N, a.K = p.K, a.offs = p.offs, a.E = p.offs ? p.E : 1, a.bf16 = 1, a.bt = bt, a.err = p.err, a.err_bit = 2;
-    return tcpair::launch(w, p.offs ? (int64_t)p.E * p.N : p.N, p.K, x, ldx, a, epi, st);
+    return tcpair::launch(w, p.offs ? (int64_t)p.E * p.N : p.N, p.K, x, ldx, a, epi, st, true);
 }
 
 int launch(const void* x, int64_t ldx, const void* w, TcParams p, cudaStream_t st) {
@@ -405,7 +406,7 @@ int launch(const void* x, int64_t ldx, const void* w, TcParams p, cudaStream_t s
         attr_set = true;
     }
     dim3 grid((p.M + BM - 1) / BM + (p.offs ? p.E : 0), (p.N + BN - 1) / BN, p.heads ? p.heads : 1);
-    linear_tc_kernel<<<grid, 128, smem, st>>>(mw, mx, p);
+    launch_chained(linear_tc_kernel, grid, 128, smem, st, mw, mx, p);
     SEQ_LAUNCH_CHECK("linear tc");
     return 0;
 }

@@ -26,6 +26,7 @@ int launch_linear_tc_grouped_act(const void* x, int64_t ldx, const void* w, cons
 // grid (pairs): row r of the result = the activation row of the token behind the r-th sorted pair (contiguous rows for the tensor-core tiles)
 __global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const int32_t* __restrict__ sorted, int x_div, int K,
                                   __nv_bfloat16* __restrict__ out, int64_t ldo) {
+    chain_enter();
     const int r = blockIdx.x;
     const __nv_bfloat16* src = x + (int64_t)(sorted[r] / x_div) * ldx;
     __nv_bfloat16* dst = out + (int64_t)r * ldo;
@@ -39,6 +40,7 @@ __global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ x, int64_t l
 // the same with a warp per row and four 16-byte loads per lane in flight (K % 8 == 0, aligned rows): 16 384 rows of 1024 11.5 us with a block per row, now 8.5
 __global__ void __launch_bounds__(256) moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const int32_t* __restrict__ sorted, int x_div, int rows, int K8,
                                                               __nv_bfloat16* __restrict__ out, int64_t ldo) {
+    chain_enter();
     const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= rows) return;
     const uint4* src = reinterpret_cast<const uint4*>(x + (int64_t)(sorted[r] / x_div) * ldx);
@@ -160,6 +162,7 @@ __device__ __forceinline__ void route_token(const float* zr, float* sm, int t, i
 // with a block per token every choice was an atomic of its own on E addresses (4096 tokens, 4 of 32 experts: 13.6 us, now 8.6).
 __global__ void moe_route_kernel(const float* __restrict__ z, int64_t ldz, int T, const RouteRule rule, int32_t* __restrict__ ids, float* __restrict__ wts,
                                  int32_t* __restrict__ counts) {
+    chain_enter();
     extern __shared__ float sm[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, per = 2 * rule.E + rule.groups;
     const int t = blockIdx.x * nw + wid;
@@ -258,6 +261,7 @@ __global__ void __launch_bounds__(256) moe_router_rows_kernel(const XT* __restri
 constexpr int SORT_NT = 1024, SORT_W = SORT_NT / 32, SORT_U = 8;
 __global__ void __launch_bounds__(SORT_NT) moe_sort_kernel(const int32_t* __restrict__ ids, int pairs, int E, const int32_t* __restrict__ counts, int32_t* __restrict__ offs,
                                                            int32_t* __restrict__ sorted, int32_t* __restrict__ slot_of) {
+    chain_enter();
     __shared__ int seg[SORT_W], red[SORT_W];
     const int e = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int per = ((pairs + SORT_W - 1) / SORT_W + 31) & ~31;   // a warp's contiguous share of the pairs
@@ -362,6 +366,7 @@ __device__ __forceinline__ float moe_row_dot(const __nv_bfloat16* __restrict__ w
 // gated form of the per-pair rows: grid (blocks of 8 warps over N / 2, pairs): a warp = one (gate, up) pair of rows = one output of one pair
 template <typename XT, bool VEC>
 __global__ void __launch_bounds__(256) moe_rows_gated_kernel(const MoeLin a) {
+    chain_enter();
     const int lane = threadIdx.x & 31;
     const int f = blockIdx.x * 8 + (threadIdx.x >> 5);
     const int p = blockIdx.y;
@@ -378,6 +383,7 @@ __global__ void __launch_bounds__(256) moe_rows_gated_kernel(const MoeLin a) {
 // grid (blocks of 8 warps over N, pairs): a warp = one output of one pair
 template <typename XT, bool VEC>
 __global__ void __launch_bounds__(256) moe_rows_kernel(const MoeLin a) {
+    chain_enter();
     const int lane = threadIdx.x & 31;
     const int n = blockIdx.x * 8 + (threadIdx.x >> 5);
     const int p = blockIdx.y;
@@ -415,6 +421,7 @@ __global__ void __launch_bounds__(256) moe_rows_kernel(const MoeLin a) {
 constexpr int MT = 64, MTK = 16;
 template <typename XT>
 __global__ void __launch_bounds__(256) moe_tiled_kernel(const MoeLin a) {
+    chain_enter();
     __shared__ float xs[MTK][MT + 4];
     __shared__ float ws[MTK][MT + 4];
     __shared__ int rowsrc[MT];
@@ -574,6 +581,7 @@ __global__ void __launch_bounds__(256) head_tiled_kernel(const HeadLin a) {
 __global__ void moe_combine_kernel(const float* __restrict__ ys, const float* __restrict__ wts, const int32_t* __restrict__ slot_of, int top, int W,
                                    const float* __restrict__ shared, const float* __restrict__ gate_z, int64_t ldg, float* __restrict__ y,
                                    const int32_t* __restrict__ ids, int E_real, const float* __restrict__ x_id, int vec) {
+    chain_enter();
     const int64_t t = blockIdx.x;
     float gate = 1.f;
     if (shared && gate_z) gate = sigmoidf_acc(gate_z[t * ldg]);
@@ -656,8 +664,8 @@ int b200seq_moe_route_rule(const float* z, int64_t ldz, int T, const b200seq_rou
     if (T == 0) return 0;
     // eight tokens to a block where there are enough of them for every SM and their scores fit the default shared memory
     const size_t per = (size_t)(2 * E + rule.groups) * sizeof(float), block = 8 * per + (size_t)E * sizeof(int32_t);
-    if (T >= 1024 && block <= 48 * 1024) moe_route_kernel<<<(T + 7) / 8, 256, block, cs>>>(z, ldz, T, rule, ids, wts, counts);
-    else moe_route_kernel<<<T, 32, per, cs>>>(z, ldz, T, rule, ids, wts, counts);
+    if (T >= 1024 && block <= 48 * 1024) launch_chained(moe_route_kernel, (T + 7) / 8, 256, block, cs, z, ldz, T, rule, ids, wts, counts);
+    else launch_chained(moe_route_kernel, T, 32, per, cs, z, ldz, T, rule, ids, wts, counts);
     SEQ_LAUNCH_CHECK("moe_route");
     return 0;
 }
@@ -721,7 +729,7 @@ int b200seq_moe_router_rule(const void* x, int x_dtype, int64_t ldx_, const void
 
 int b200seq_moe_sort(const int32_t* ids, int pairs, int E, const int32_t* counts, int32_t* offs, int32_t* sorted, int32_t* slot_of, void* stream) {
     if (!ids || !counts || !offs || !sorted || !slot_of || pairs < 0 || E < 1) return fail(B200SEQ_ERR_INVALID_ARG, "moe_sort: bad arguments");
-    moe_sort_kernel<<<E, SORT_NT, 0, (cudaStream_t)stream>>>(ids, pairs, E, counts, offs, sorted, slot_of);
+    launch_chained(moe_sort_kernel, E, SORT_NT, 0, (cudaStream_t)stream, ids, pairs, E, counts, offs, sorted, slot_of);
     SEQ_LAUNCH_CHECK("moe_sort");
     return 0;
 }
@@ -751,11 +759,11 @@ int b200seq_moe_linear_act(const void* x, int x_dtype, int64_t ldx_, int x_div, 
         if (pairs > 65535) return fail(B200SEQ_ERR_UNSUPPORTED, "moe_linear: too many pairs for the row form");
         dim3 grid((N / 2 + 7) / 8, pairs);
         if (x_dtype == B200SEQ_F32) {
-            if (vec) moe_rows_gated_kernel<float, true><<<grid, 256, 0, cs>>>(a);
-            else moe_rows_gated_kernel<float, false><<<grid, 256, 0, cs>>>(a);
+            if (vec) launch_chained(moe_rows_gated_kernel<float, true>, grid, 256, 0, cs, a);
+            else launch_chained(moe_rows_gated_kernel<float, false>, grid, 256, 0, cs, a);
         } else {
-            if (vec) moe_rows_gated_kernel<__nv_bfloat16, true><<<grid, 256, 0, cs>>>(a);
-            else moe_rows_gated_kernel<__nv_bfloat16, false><<<grid, 256, 0, cs>>>(a);
+            if (vec) launch_chained(moe_rows_gated_kernel<__nv_bfloat16, true>, grid, 256, 0, cs, a);
+            else launch_chained(moe_rows_gated_kernel<__nv_bfloat16, false>, grid, 256, 0, cs, a);
         }
         SEQ_LAUNCH_CHECK("moe_linear gated rows");
         return 0;
@@ -766,11 +774,11 @@ int b200seq_moe_linear_act(const void* x, int x_dtype, int64_t ldx_, int x_div, 
         if (pairs > 65535) return fail(B200SEQ_ERR_UNSUPPORTED, "moe_linear: too many pairs for the row form");
         dim3 grid((N + 7) / 8, pairs);
         if (x_dtype == B200SEQ_F32) {
-            if (vec) moe_rows_kernel<float, true><<<grid, 256, 0, cs>>>(a);
-            else moe_rows_kernel<float, false><<<grid, 256, 0, cs>>>(a);
+            if (vec) launch_chained(moe_rows_kernel<float, true>, grid, 256, 0, cs, a);
+            else launch_chained(moe_rows_kernel<float, false>, grid, 256, 0, cs, a);
         } else {
-            if (vec) moe_rows_kernel<__nv_bfloat16, true><<<grid, 256, 0, cs>>>(a);
-            else moe_rows_kernel<__nv_bfloat16, false><<<grid, 256, 0, cs>>>(a);
+            if (vec) launch_chained(moe_rows_kernel<__nv_bfloat16, true>, grid, 256, 0, cs, a);
+            else launch_chained(moe_rows_kernel<__nv_bfloat16, false>, grid, 256, 0, cs, a);
         }
         SEQ_LAUNCH_CHECK("moe_linear rows");
         return 0;
@@ -782,8 +790,8 @@ int b200seq_moe_linear_act(const void* x, int x_dtype, int64_t ldx_, int x_div, 
     const int tiles = (pairs + MT - 1) / MT + E;
     if (tiles > 65535) return fail(B200SEQ_ERR_UNSUPPORTED, "moe_linear: too many row tiles");
     dim3 grid((N + MT - 1) / MT, tiles);
-    if (x_dtype == B200SEQ_F32) moe_tiled_kernel<float><<<grid, 256, 0, cs>>>(a);
-    else moe_tiled_kernel<__nv_bfloat16><<<grid, 256, 0, cs>>>(a);
+    if (x_dtype == B200SEQ_F32) launch_chained(moe_tiled_kernel<float>, grid, 256, 0, cs, a);
+    else launch_chained(moe_tiled_kernel<__nv_bfloat16>, grid, 256, 0, cs, a);
     SEQ_LAUNCH_CHECK("moe_linear tiles");
     return 0;
 }
@@ -825,8 +833,8 @@ int b200seq_moe_gather(const void* x_bf16, int64_t ldx_, const int32_t* sorted, 
     if (!x_bf16 || !sorted || !out_bf16 || x_div < 1 || pairs < 0 || K < 1 || ldx_ < K || ldo < K) return fail(B200SEQ_ERR_INVALID_ARG, "moe_gather: bad arguments");
     if (pairs == 0) return 0;
     if (pairs >= 1024 && ((K | ldx_ | ldo) & 7) == 0 && ((reinterpret_cast<uintptr_t>(x_bf16) | reinterpret_cast<uintptr_t>(out_bf16)) & 15) == 0)   // (fewer rows: a block each covers the chip)
-        moe_gather_rows_kernel<<<(pairs + 7) / 8, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x_bf16, ldx_, sorted, x_div, pairs, K / 8, (__nv_bfloat16*)out_bf16, ldo);
-    else moe_gather_kernel<<<pairs, K >= 2048 ? 256 : 128, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x_bf16, ldx_, sorted, x_div, K, (__nv_bfloat16*)out_bf16, ldo);
+        launch_chained(moe_gather_rows_kernel, (pairs + 7) / 8, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16*)x_bf16, ldx_, sorted, x_div, pairs, K / 8, (__nv_bfloat16*)out_bf16, ldo);
+    else launch_chained(moe_gather_kernel, pairs, K >= 2048 ? 256 : 128, 0, (cudaStream_t)stream, (const __nv_bfloat16*)x_bf16, ldx_, sorted, x_div, K, (__nv_bfloat16*)out_bf16, ldo);
     SEQ_LAUNCH_CHECK("moe_gather");
     return 0;
 }
@@ -841,7 +849,7 @@ int b200seq_moe_combine_ex(const float* ys, const float* wts, const int32_t* slo
     if (!ys || !wts || !y || T < 0 || top < 1 || W < 1 || (ids && !x_id)) return fail(B200SEQ_ERR_INVALID_ARG, "moe_combine: bad arguments");
     if (T == 0) return 0;
     auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    moe_combine_kernel<<<T, W >= 1024 ? 256 : 128, 0, (cudaStream_t)stream>>>(ys, wts, slot_of, top, W, shared, gate_z, ldg, y, ids, E_real, x_id,
+    launch_chained(moe_combine_kernel, T, W >= 1024 ? 256 : 128, 0, (cudaStream_t)stream, ys, wts, slot_of, top, W, shared, gate_z, ldg, y, ids, E_real, x_id,
         W % 4 == 0 && al(ys) && al(shared) && al(y) && al(x_id));
     SEQ_LAUNCH_CHECK("moe_combine");
     return 0;

@@ -21,6 +21,7 @@ namespace b200seq {
 // NPL: state floats per lane.  Lane -> (sub = lane / cpw, col = lane % cpw), cpw = 32 / NL; the lane holds n = sub * NPL + i.
 template <int NPL, int MODE>
 __global__ void __launch_bounds__(SSM_WARPS * 32) ssm_kernel(const SsmArgs a, const b200seq_step st) {
+    chain_enter();
     extern __shared__ __align__(16) float sm[];
     const int H = a.H, V = a.V, N = a.N, NL = a.NL;
     const int cpw = 32 / NL, cols = SSM_WARPS * cpw;       // value columns of this block (NL, cpw, cols and NPL are powers of two)
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(SSM_WARPS * 32) ssm_kernel(const SsmArgs a, co
 // another and are issued together (one at a time, each behind the store before it: 791 us for 33 segments of 64 x 128 x 64, now bound by memory).
 template <int VW>
 __global__ void ssm_combine_kernel(const SsmArgs a, const b200seq_step st) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // pass C may set up beside this one (the pass before is complete: a plain launch)
+    chain_enter();   // pass C may set up beside this one (the pass before is complete)
     const int64_t per = (int64_t)a.H * a.N * a.V;
     const int64_t idx = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * VW;
     const int e = blockIdx.y;
@@ -182,7 +183,7 @@ static cudaError_t ssm_launch(const SsmArgs& a, const b200seq_step& st, int nz, 
     const int cpw = 32 / a.NL, cols = SSM_WARPS * cpw;
     const size_t smem = ((size_t)2 * SSM_TT * a.NL * (NPL + 4) + 2 * SSM_TT * cols + 2 * SSM_TT + 4) * sizeof(float);
     dim3 grid((a.V + cols - 1) / cols, a.H, nz);
-    ssm_kernel<NPL, MODE><<<grid, SSM_WARPS * 32, smem, cs>>>(a, st);
+    launch_chained(ssm_kernel<NPL, MODE>, grid, SSM_WARPS * 32, smem, cs, a, st);
     return cudaGetLastError();
 }
 
@@ -236,8 +237,8 @@ extern "C" int b200seq_ssm_scan(const float* proj, int64_t ldp, int z0, int dt0,
     }
     if (e != cudaSuccess) return cuda_status(e, "ssm_scan local pass");
     const int64_t per = (int64_t)H * N * V;
-    if (tiles) ssm_combine_kernel<4><<<dim3((unsigned)((per / 4 + 255) / 256), st->B), 256, 0, cs>>>(a, *st);
-    else ssm_combine_kernel<1><<<dim3((unsigned)((per + 255) / 256), st->B), 256, 0, cs>>>(a, *st);
+    if (tiles) launch_chained(ssm_combine_kernel<4>, dim3((unsigned)((per / 4 + 255) / 256), st->B), 256, 0, cs, a, *st);
+    else launch_chained(ssm_combine_kernel<1>, dim3((unsigned)((per + 255) / 256), st->B), 256, 0, cs, a, *st);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e, "ssm_scan combine pass");
     if (tiles) e = launch_ssm_tiles_out(a, *st, segs, false, cs);
     else e = small ? ssm_launch<16, SSM_FINAL>(a, *st, segs, cs) : ssm_launch<32, SSM_FINAL>(a, *st, segs, cs);
