@@ -43,7 +43,7 @@ __host__ __device__ constexpr int stage_count(int bt) { return RING / stage_byte
 
 struct Args {
     int M, N, K;             // token rows, weight rows of one group, reduction length
-    int bt;                  // token rows per tile: a multiple of 32, at most 256
+    int bt;                  // token rows per tile: a multiple of 16, at most 256; grouped: the most that a tile has
     int MT, NT;              // token tiles (bound when grouped), weight tiles of 256
     int parts;               // PARTS (not grouped): K cut into this many runs of whole 256-k chunks, run i to the result rows i * M ..
     const int32_t* offs;     // grouped form: [E + 1] first token row of every group; group e uses the weight rows e * N ..
@@ -154,7 +154,8 @@ __device__ __forceinline__ void ld32(uint32_t taddr, float* v) {
 __device__ __forceinline__ void ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 struct Tile {
-    int m0, m_end, wrow, n0;   // first token row, end of its group's rows, first weight row in memory, first output column
+    int m0, m_end, wrow, n0;   // first token row, end of the tile's rows, first weight row in memory, first output column
+    int bt;                    // columns of the tile: a multiple of 16, m_end - m0 or more
     int kb0, kb1, out;         // slabs of k; result row of token row 0
 };
 
@@ -184,7 +185,7 @@ __device__ __forceinline__ Tile tile_of(const Args& p, const int32_t* first, int
     r.n0 = nt * 2 * ROWS;
     r.wrow = r.n0;
     if (!p.offs) {
-        r.m0 = mt * BT, r.m_end = p.M;
+        r.m0 = mt * BT, r.m_end = r.m0 + BT < p.M ? r.m0 + BT : p.M, r.bt = BT;
     } else {
         int lo = 0, hi = p.E;      // the last group whose first tile is <= mt (groups without rows have no tile)
         while (hi - lo > 1) {
@@ -192,7 +193,10 @@ __device__ __forceinline__ Tile tile_of(const Args& p, const int32_t* first, int
             if (first[mid] <= mt) lo = mid;
             else hi = mid;
         }
-        r.m0 = p.offs[lo] + (mt - first[lo]) * BT, r.m_end = p.offs[lo + 1];
+        // a group's rows are shared out evenly over its tiles: 32 groups of 512 rows, a few more or less, were 2 or 3 tiles of 256, a quarter of them padding
+        const int t0 = first[lo], tiles = first[lo + 1] - t0, row0 = p.offs[lo], end = p.offs[lo + 1];
+        r.bt = ((end - row0 + tiles - 1) / tiles + 15) & ~15;
+        r.m0 = row0 + (mt - t0) * r.bt, r.m_end = r.m0 + r.bt < end ? r.m0 + r.bt : end;
         r.wrow += lo * p.N;
     }
     return r;
@@ -261,7 +265,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             bool ok = true;
             for (int t = (int)blockIdx.x >> 1; t < tiles && ok; t += stride) {
                 const Tile tl = tile_of<PARTS>(p, first, MT, t);
-                const int wr = tl.wrow + (int)rank * ROWS, xr = tl.m0 + (int)rank * (BT / 2);
+                const int wr = tl.wrow + (int)rank * ROWS, xr = tl.m0 + (int)rank * (tl.bt / 2);   // (the copies are as long as the longest tile needs)
                 for (int kb = tl.kb0; kb < tl.kb1; ++kb) {
                     ok = bar_wait(empty + 8 * s, ph, abort_flag);
                     if (!ok) break;
@@ -282,7 +286,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         }
     } else if (warp == 1) {
         if (rank == 0 && elect()) {
-            const uint32_t idesc = (1u << 4) | (p.bf16 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(BT >> 3) << 17) | ((uint32_t)(2 * ROWS >> 4) << 24);
+            const uint32_t idesc0 = (1u << 4) | (p.bf16 ? (1u << 7) | (1u << 10) : 0u) | ((uint32_t)(2 * ROWS >> 4) << 24);
             int s = 0, b = 0;
             uint32_t ph = 0, eph = 1;
             bool ok = true;
@@ -291,9 +295,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
                 if (!ok) break;
                 fence_after();
                 const uint32_t d = tmem + b * ACC_STRIDE;
-                int kb0, kb1;
-                slabs_of<PARTS>(p, MT, t, kb0, kb1);
-                const int nk = kb1 - kb0;
+                const Tile tl = tile_of<PARTS>(p, first, MT, t);
+                const uint32_t idesc = idesc0 | ((uint32_t)(tl.bt >> 3) << 17);
+                const int nk = tl.kb1 - tl.kb0;
                 for (int kb = 0; kb < nk; ++kb) {
                     ok = bar_wait(full + 8 * s, ph, abort_flag);
                     if (!ok) break;
@@ -321,8 +325,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             const int n = tl.n0 + (int)rank * ROWS + q * 32 + lane;
             const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + b * ACC_STRIDE;
 #pragma unroll 1
-            for (int c = half * 32; c < BT; c += 64) {
-                if (tl.m0 + c >= tl.m_end) break;
+            for (int c = half * 32; tl.m0 + c < tl.m_end; c += 64) {
                 float v[32];
                 ld32(ta + c, v);
                 ld_wait();
@@ -393,7 +396,7 @@ template <class Tiles>
 inline int pick_bt(int64_t pairs, int64_t K, Tiles tiles) {
     int best = MAX_BT;
     double best_t = 0;
-    for (int bt = MAX_BT; bt >= 32; bt -= 32) {
+    for (int bt = MAX_BT; bt >= 32; bt -= 16) {
         const double t = (double)((tiles(bt) + pairs - 1) / pairs) * wave_us(bt, K);
         if (bt == MAX_BT || t < best_t) best = bt, best_t = t;
     }
