@@ -649,8 +649,8 @@ static int32_t fused_common(const b200q_weight* w, int64_t M, void* y, int32_t y
     return B200Q_OK;
 }
 
-int32_t b200q_matmul_norm(const b200q_weight* w, const float* h_in, const float* delta, float* h_out, const float* norm_w, float eps, int64_t M,
-                          void* y, int32_t y_dtype, int64_t ldy, void* workspace, size_t workspace_bytes, void* stream) {
+static int32_t matmul_norm(const b200q_weight* w, const float* h_in, const float* delta, float* h_out, const float* norm_w, float eps, int64_t M, void* y, int32_t y_dtype, int64_t ldy,
+                           void* workspace, size_t workspace_bytes, void* stream, int late) {
     int32_t rc = fused_common(w, M, y, y_dtype, ldy, workspace, workspace_bytes);
     if (rc) return rc;
     if (!h_in || !norm_w) return fail(B200Q_ERR_INVALID_ARG, "null h_in / norm_w");
@@ -660,8 +660,17 @@ int32_t b200q_matmul_norm(const b200q_weight* w, const float* h_in, const float*
     }
     if (delta && h_out == h_in) return fail(B200Q_ERR_INVALID_ARG, "h_out must not alias h_in when delta is given");
     FusedPrologue fp{1, h_in, delta, h_out, norm_w, eps, nullptr};
+    fp.late = late;
     CUDA_TRY(launch_matvec(w, nullptr, M, y, y_dtype, ldy, (uint8_t*)workspace, (cudaStream_t)stream, &fp));
     return B200Q_OK;
+}
+int32_t b200q_matmul_norm(const b200q_weight* w, const float* h_in, const float* delta, float* h_out, const float* norm_w, float eps, int64_t M,
+                          void* y, int32_t y_dtype, int64_t ldy, void* workspace, size_t workspace_bytes, void* stream) {
+    return matmul_norm(w, h_in, delta, h_out, norm_w, eps, M, y, y_dtype, ldy, workspace, workspace_bytes, stream, 0);
+}
+int32_t b200q_matmul_norm_first(const b200q_weight* w, const float* h_in, const float* delta, float* h_out, const float* norm_w, float eps, int64_t M,
+                                void* y, int32_t y_dtype, int64_t ldy, void* workspace, size_t workspace_bytes, void* stream) {
+    return matmul_norm(w, h_in, delta, h_out, norm_w, eps, M, y, y_dtype, ldy, workspace, workspace_bytes, stream, 1);
 }
 
 /* ---- fused SwiGLU epilogue: w = gate|up with rows interleaved per 128-row tile (b200q_gate_up_row); writes the quantised

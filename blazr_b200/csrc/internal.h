@@ -65,6 +65,7 @@ struct FusedPrologue {
     const void* x = nullptr;   // mode 3
     int x_dtype = 0;
     int64_t ldx = 0;
+    int late = 0;      // mode 1: MatvecParams::late
 };
 cudaError_t matvec_plan(const b200q_weight* w, int64_t M, MatvecPlan* plan, int pro = 0);
 bool matvec_quantises(const b200q_weight* w, int64_t M);   // launch_matvec takes FusedPrologue mode 3 (x itself) for M rows

@@ -187,6 +187,7 @@ cudaError_t launch_matvec(const b200q_weight* w, const uint8_t* xq, int64_t M, v
     p.h_out = fp ? fp->h_out : nullptr;
     p.norm_w = fp ? fp->norm_w : nullptr;
     p.eps = fp ? fp->eps : 0.0f;
+    p.late = fp ? fp->late : 0;
     p.gate_up = fp ? fp->gate_up : nullptr;
     p.x = fp ? fp->x : nullptr;
     p.x_dtype = fp ? fp->x_dtype : 0;

@@ -40,6 +40,8 @@ struct MatvecParams {
     float* h_out;
     const float* norm_w;
     float eps;
+    // pro 1: 1 = the launch behind this one may start only when what lies ahead is complete (b200q_matmul_norm_first)
+    int late;
     const float* gate_up;
     const void* x;         // pro 3: x[M][ldx] (x_dtype) of K columns, gathered through perm if there is one
     int x_dtype;

@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_kernel(const MatvecParam
     const int KC = (int)p.KC;
     const int nst = p.nstages;
     SkPlan& sp = *reinterpret_cast<SkPlan*>(smem + 2 * MV_MAX_STAGES * 8);       // shared plan (computed once)
-    pdl_launch_dependents();  // let the next kernel of the stream start its own weight prefetch
+    if (PRO != PRO_FUSED || !p.late) pdl_launch_dependents();  // let the next kernel of the stream start its own weight prefetch
 
     // The producer lane initialises the barriers and requests the first ring-full of weights BEFORE the CTA-wide barrier:
     // the TMA stream starts a few hundred cycles after the CTA lands on the SM, while thread 0 publishes the plan.
@@ -694,6 +694,7 @@ __global__ void __launch_bounds__(MV_THREADS, 1) matvec_kernel(const MatvecParam
                 case 2: { float nw[2]; load_nw<2>(p.norm_w, tid, nw); pdl_wait_again(); norm_prologue<MB, 2>(p, xhat, nw, tid, warp, lane, g == 0, s_red); break; }
                 default: { float nw[1]; load_nw<1>(p.norm_w, tid, nw); pdl_wait_again(); norm_prologue<MB, 1>(p, xhat, nw, tid, warp, lane, g == 0, s_red); break; }
             }
+            if (p.late) pdl_launch_dependents();
         } else {
             pdl_wait_again();
             fused_prologue<MB>(p, xhat, tid, warp, lane, g == 0);

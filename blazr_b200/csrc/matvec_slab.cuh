@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) matvec_slab_kernel(const Matv
     const int base = second ? p.T1 * TILE_ROWS : 0;                                             // output row of the weight's first
     const int N = second ? (int)p.N - base : (DUAL ? p.T1 * TILE_ROWS : (int)p.N);
     const int have = ((N + TILE_ROWS - 1) / TILE_ROWS) * TILE_ROWS - row0, rows = have < R ? have : R;
-    pdl_launch_dependents();
+    if (PRO != PRO_FUSED || !p.late) pdl_launch_dependents();
     // the weights are static: requested before anything is waited for
     if (second) slab_request<F2>(p.w2, KC, cb, row0, rows, R, gpc, slab, stride, wbar, warp, lane);
     else slab_request<F>(p.w, KC, cb, row0, rows, R, gpc, slab, stride, wbar, warp, lane);
@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) matvec_slab_kernel(const Matv
             case 2: { float nw[2]; load_nw<2>(p.norm_w, tid, nw); pdl_wait(); norm_prologue<MB, 2>(p, xhat, nw, tid, warp, lane, g == 0, s_red); break; }
             default: { float nw[1]; load_nw<1>(p.norm_w, tid, nw); pdl_wait(); norm_prologue<MB, 1>(p, xhat, nw, tid, warp, lane, g == 0, s_red); break; }
         }
+        if (p.late) pdl_launch_dependents();
     } else {
         pdl_wait();   // y and the bias may still be in use by the preceding kernel before this point
         if constexpr (PRO == PRO_QUANT) {

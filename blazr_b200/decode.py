@@ -180,6 +180,9 @@ class _Linear:
     fmt: str = ""
 
 
+CHAIN = 8   # steps of the larger of the two captured graphs (4-layer model, us a step on the device: 101.6 in a graph of its own, 98.1 of four, 97.4 of eight, 97.2 of sixteen)
+
+
 class Decoder:
     """One rank of a (tensor-parallel) decoder.  `host` gives exact weights (tests); otherwise weights are
     random blocks generated on the device (bench)."""
@@ -317,7 +320,8 @@ class Decoder:
         self.tp_finish = self.tp_finish and self.fused
         self.fused_swiglu = _os.environ.get("B200Q_FUSED_SWIGLU", "0") != "0" and not self.wide  # measured slower: 148x redundant SiLU
         self.pf_bytes = int(float(_os.environ.get("B200Q_PF_MB", "0")) * (1 << 20))
-        self.graph = None
+        self.graph = self.chain_graph = None
+        self.fed = self.chosen = None      # [max_ctx, M]: tokens that captured steps take instead of their own choice (-1: none), and their choices
         self._host_pos = 0
         # EXPERIMENTAL (B200Q_DSTEP=1, single GPU, M <= 4): persistent op-list kernel, 3 launches per layer instead of 8
         self.programs = None
@@ -569,8 +573,13 @@ class Decoder:
         """raises if a kernel refused an out-of-range position, or a prompt's GEMM gave up waiting, since the last check (synchronises the device)"""
         ops.check_device_errors()
 
-    def step(self):
-        """ids (device) -> next ids (device); positions advance on the device: graph-replayable."""
+    def _chained(self) -> bool:
+        """whether captured steps end with b200q_argmax_next (one GPU, fused norms): prompt tokens are fed on the device and steps follow one another in one graph"""
+        return self.fused and not self.wide and self.comm is None and self.world == 1 and self.programs is None and self.step_program is None and self.cfg.hidden % 2 == 0
+
+    def step(self, embedded: bool = False, chain: bool = False, more: bool = False):
+        """ids (device) -> next ids (device); positions advance on the device: graph-replayable.  In a chain of captured steps (`chain`): embedded, the step
+        before has left the embedded token in h; more, this one does so for the next."""
         if not torch.cuda.is_current_stream_capturing():
             self._advance()
         if self.step_program is not None:
@@ -580,7 +589,8 @@ class Decoder:
         L, cfg, M = ops.lib(), self.cfg, self.M
         st = ops._stream_ptr(self.dev)
         P = lambda t: C.c_void_p(t.data_ptr())
-        ops._check(L.b200q_embed(P(self.embed), P(self.ids), C.c_int64(cfg.hidden), C.c_int64(M), P(self.h), st))
+        if not embedded:
+            ops._check(L.b200q_embed(P(self.embed), P(self.ids), C.c_int64(cfg.hidden), C.c_int64(M), P(self.h), st))
         hin, hout = self.h, self.h2
         delta = None
         in_flight = False  # TP: the projection ahead left its partial sums in the exchange buffers (see _rowpar)
@@ -595,19 +605,20 @@ class Decoder:
                                                      P(self.xq_h) if self.wide else None, st))
             hin, hout = hout, hin
 
-        def matvec_norm(lins, w, out):
+        def matvec_norm(lins, w, out, first=False):
             """norm fused into the matvec prologue (one launch per fused weight group; the first writes h_out)"""
             nonlocal hin, hout
             for j, ln in enumerate(lins):
-                ops._check(L.b200q_matmul_norm(ln.w.handle, P(hin), P(delta) if delta is not None else None, P(hout) if j == 0 else None, P(w),
-                                               C.c_float(cfg.eps), C.c_int64(M), C.c_void_p(out.data_ptr() + 4 * ln.col0), C.c_int32(ops.F32),
-                                               C.c_int64(out.stride(0)), C.c_void_p(ln.ws.data_ptr()), C.c_size_t(ln.ws.numel()), st))
+                call = L.b200q_matmul_norm_first if first and j == 0 else L.b200q_matmul_norm
+                ops._check(call(ln.w.handle, P(hin), P(delta) if delta is not None else None, P(hout) if j == 0 else None, P(w),
+                                C.c_float(cfg.eps), C.c_int64(M), C.c_void_p(out.data_ptr() + 4 * ln.col0), C.c_int32(ops.F32),
+                                C.c_int64(out.stride(0)), C.c_void_p(ln.ws.data_ptr()), C.c_size_t(ln.ws.numel()), st))
             hin, hout = hout, hin
 
         fused = self.fused
         for li, lay in enumerate(self.layers):
             if fused:
-                matvec_norm(lay["qkv_mv"], lay["attn_norm"], self.qkv)
+                matvec_norm(lay["qkv_mv"], lay["attn_norm"], self.qkv, first=embedded and li == 0)
             else:
                 norm(lay["attn_norm"])
                 self._matvec(lay["qkv_mv"], self.xq_h, self.qkv)
@@ -666,6 +677,9 @@ class Decoder:
             full = self.logits.permute(1, 0, 2).reshape(M, -1).contiguous()  # column r * vs + j = vocabulary id (padding = -inf)
             ops._check(L.b200q_argmax(P(full), C.c_int64(full.shape[1]), C.c_int64(M), P(self.ids), P(self.pos), st))
             self._full_logits = full[:, :cfg.vocab]
+        elif chain:
+            ops._check(L.b200q_argmax_next(P(self.logits), C.c_int64(self.logits.shape[1]), C.c_int64(M), P(self.ids), P(self.pos), P(self.fed), P(self.chosen),
+                                           C.c_int64(self.max_ctx), P(self.embed) if more else None, C.c_int64(cfg.hidden), P(self.h) if more else None, st))
         else:
             ops._check(L.b200q_argmax(P(self.logits), C.c_int64(self.logits.shape[1]), C.c_int64(M), P(self.ids), P(self.pos), st))
 
@@ -696,13 +710,24 @@ class Decoder:
         self.pos.sub_(1)      # the warm-up forward is not part of any sequence: undo its position advance
         self._host_pos -= 1
         torch.cuda.synchronize(self.dev)
-        g = torch.cuda.CUDAGraph()
-        s = torch.cuda.Stream(self.dev)
-        s.wait_stream(torch.cuda.current_stream(self.dev))
-        with torch.cuda.stream(s):
-            with torch.cuda.graph(g, stream=s):
-                self.step()
-        torch.cuda.synchronize(self.dev)
+        chain = self._chained()
+        if chain and self.fed is None:
+            self.fed = torch.full((self.max_ctx, self.M), -1, dtype=torch.int64, device=self.dev)
+            self.chosen = torch.zeros_like(self.fed)
+
+        def record(steps):
+            g = torch.cuda.CUDAGraph()
+            s = torch.cuda.Stream(self.dev)
+            s.wait_stream(torch.cuda.current_stream(self.dev))
+            with torch.cuda.stream(s):
+                with torch.cuda.graph(g, stream=s):
+                    for i in range(steps):
+                        self.step(i > 0, chain, i + 1 < steps)
+            torch.cuda.synchronize(self.dev)
+            return g
+
+        g = record(1)
+        self.chain_graph = record(CHAIN) if chain else None
         self.graph = g
         return g
 
@@ -850,10 +875,27 @@ class Decoder:
         if use_graph and self.graph is None:
             self.capture()
         self.reset(prompt[:, 0])
-        run = self.replay if use_graph else self.step
+        steps = S + n_new - 1
         fed = torch.from_numpy(np.ascontiguousarray(prompt.T)).to(self.dev)   # one upload: a copy per step made the host wait for every step
+        if use_graph and self.fed is not None:
+            self.fed[:S].copy_(fed)
+            try:
+                left = steps
+                while left > 0:
+                    n = CHAIN if left >= CHAIN else 1
+                    for _ in range(n):
+                        self._advance()
+                    (self.chain_graph if n > 1 else self.graph).replay()
+                    left -= n
+            finally:
+                self.fed[:S].fill_(-1)
+            out = self.chosen[S - 1:steps].T.contiguous()
+            torch.cuda.synchronize(self.dev)
+            self.check_device_errors()
+            return out.cpu().numpy()
+        run = self.replay if use_graph else self.step
         out = []
-        for s_ in range(S + n_new - 1):
+        for s_ in range(steps):
             run()
             if s_ + 1 < S:
                 self.ids.copy_(fed[s_ + 1])  # teacher-force the prompt
