@@ -110,6 +110,7 @@ struct EpiOut {
 // four apart.  The gate's lane takes the first 16 tokens, the up's lane the others.  Same operations as swiglu_rows_kernel on the stored products, whose
 // 134 MB (2048 tokens, 2 x 8192) are neither written nor read again: product and activation 102 + 32 us, now 99.
 struct EpiGatedRows {
+    static constexpr int WARPS = 16;   // (eight: two to a scheduler, whose divisions and shuffles took as long as a tile's products; a prompt of 2048 tokens 2 % longer)
     __half* act;
     int64_t ld;
     const float* bias;

@@ -7,12 +7,12 @@
 // (128-byte swizzle); rows and k outside the matrices read as zero.
 //
 // The kernel is persistent (one pair per two SMs, tiles dealt round-robin, token tiles fastest so that a weight tile is read from HBM
-// once) and the accumulator is double-buffered in TMEM (2 x 256 columns): the eight epilogue warps drain tile i while the tensor cores run
+// once) and the accumulator is double-buffered in TMEM (2 x 256 columns): the epilogue warps drain tile i while the tensor cores run
 // tile i + 1.  What bounds it is the tensor pipe; the single-SM kernel it replaces for large steps stalled on L2 -> SM traffic (512 bytes
 // per 32 768 FLOPs against 1 024 per 131 072 here) and on a main loop that its epilogue interrupted.  Measured, 4096 tokens: 16384 x 2048 267 ->
 // 198 us (1.39 PFLOP/s), with the gated activation 478 -> 201 us; 2048 x 8192 128 -> 100 us; 8192 x 1024 91 -> 61 us.
 //
-// Warp roles: 0 = TMA producer (both CTAs), 1 = MMA issuer (leader CTA only), 2 = TMEM allocation, 4..11 = epilogue.
+// Warp roles: 0 = TMA producer (both CTAs), 1 = MMA issuer (leader CTA only), 2 = TMEM allocation, 4 and on = epilogue.
 // Barriers: full[s] lives in the leader and counts the bytes of both CTAs; empty[s] and acc_full are signalled in both CTAs by
 // multicast tcgen05.commit; acc_empty lives in the leader and collects the epilogue warps of both CTAs.
 // Every wait is bounded by a clock: one that runs out raises the abort flag, the role leaves its loop, and the CTA goes through the
@@ -21,13 +21,23 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 
 namespace tcpair {
 
 constexpr int ROWS = 128;        // weight rows per CTA
 constexpr int BK = 64;           // k per slab
-constexpr int EPI_WARPS = 8;
-constexpr int THREADS = (4 + EPI_WARPS) * 32;
+// Warps of an epilogue: eight, or as many as it names itself (a multiple of four)
+template <class Epi, class = void>
+struct EpiWarps {
+    static constexpr int value = 8;
+};
+template <class Epi>
+struct EpiWarps<Epi, std::void_t<decltype(Epi::WARPS)>> {
+    static constexpr int value = Epi::WARPS;
+};
+template <class Epi>
+constexpr int THREADS = (4 + EpiWarps<Epi>::value) * 32;
 constexpr int HDR = 1024;
 constexpr int MAX_GROUPS = 1024;
 constexpr unsigned long long WAIT_NS = 2000000000ull;
@@ -205,9 +215,10 @@ __device__ __forceinline__ Tile tile_of(const Args& p, const int32_t* first, int
 // Epi: struct with   __device__ void store(const float (&v)[32], int n, int m, int m_end, int lane) const
 //   v[j] = acc[n][m + j] of this lane's n (n may be >= N: nothing is stored); all 32 lanes of a warp call it with the same m
 template <class Epi, bool PARTS>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS<Epi>, 1)
     pair_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Args p, const Epi epi) {
     extern __shared__ uint8_t smem_raw[];
+    constexpr int EPI_WARPS = EpiWarps<Epi>::value;
     const int BT = p.bt, STAGE = stage_bytes(BT), STAGES = stage_count(BT);
     const uint32_t base = (sa(smem_raw) + 1023u) & ~1023u;
     const uint32_t full = base, empty = full + 8 * MAX_STAGES, acc_full = empty + 8 * MAX_STAGES, acc_empty = acc_full + 16;
@@ -314,7 +325,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             }
         }
     } else if (warp >= 4) {
-        const int q = warp & 3, half = (warp - 4) >> 2;     // TMEM lane quarter; every other group of 32 columns
+        const int q = warp & 3, share = (warp - 4) >> 2;    // TMEM lane quarter; one of every EPI_WARPS / 4 groups of 32 columns
         const uint32_t drained = map_leader(acc_empty);
         int b = 0;
         uint32_t ph = 0;
@@ -325,7 +336,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             const int n = tl.n0 + (int)rank * ROWS + q * 32 + lane;
             const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + b * ACC_STRIDE;
 #pragma unroll 1
-            for (int c = half * 32; tl.m0 + c < tl.m_end; c += 64) {
+            for (int c = share * 32; tl.m0 + c < tl.m_end; c += 8 * EPI_WARPS) {
                 float v[32];
                 ld32(ta + c, v);
                 ld_wait();
@@ -423,7 +434,7 @@ cudaError_t launch(const void* w, int64_t w_rows, int64_t ldw, const void* x, in
     const int sms = pair_sms();
     if (ctas > sms) ctas = sms;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ctas), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = SMEM, cfg.stream = st;
+    cfg.gridDim = dim3((unsigned)ctas), cfg.blockDim = dim3(THREADS<Epi>), cfg.dynamicSmemBytes = SMEM, cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization, attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr, cfg.numAttrs = pdl ? 1 : 0;
