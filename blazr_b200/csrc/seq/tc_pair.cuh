@@ -46,7 +46,7 @@ constexpr int MAX_BT = 256;
 constexpr int ACC_STRIDE = MAX_BT;       // TMEM columns between the two accumulator buffers
 constexpr int RING = 192 * 1024;         // bytes of operand stages
 constexpr int MAX_STAGES = 9;
-constexpr int SMEM = RING + HDR + 1024 + (MAX_GROUPS + 1) * 4;
+constexpr int SMEM = RING + HDR + 1024 + 2 * (MAX_GROUPS + 1) * 4;
 constexpr int TMEM_COLS = 2 * ACC_STRIDE;
 __host__ __device__ constexpr int stage_bytes(int bt) { return ROWS * BK * 2 + bt / 2 * BK * 2; }   // per CTA
 __host__ __device__ constexpr int stage_count(int bt) { return RING / stage_bytes(bt) < MAX_STAGES ? RING / stage_bytes(bt) : MAX_STAGES; }
@@ -179,9 +179,9 @@ __device__ __forceinline__ void slabs_of(const Args& p, int MT, int t, int& kb0,
     }
 }
 
-// tile t of the step (token tiles fastest).  first: grouped form, [E + 1] first token tile of every group
+// tile t of the step (token tiles fastest).  first, rows: grouped form, [E + 1] first token tile and first row of every group, in shared memory
 template <bool PARTS>
-__device__ __forceinline__ Tile tile_of(const Args& p, const int32_t* first, int MT, int t) {
+__device__ __forceinline__ Tile tile_of(const Args& p, const int32_t* first, const int32_t* rows, int MT, int t) {
     Tile r;
     const int BT = p.bt;
     const int mt = t % MT;
@@ -204,7 +204,7 @@ __device__ __forceinline__ Tile tile_of(const Args& p, const int32_t* first, int
             else hi = mid;
         }
         // a group's rows are shared out evenly over its tiles: 32 groups of 512 rows, a few more or less, were 2 or 3 tiles of 256, a quarter of them padding
-        const int t0 = first[lo], tiles = first[lo + 1] - t0, row0 = p.offs[lo], end = p.offs[lo + 1];
+        const int t0 = first[lo], tiles = first[lo + 1] - t0, row0 = rows[lo], end = rows[lo + 1];
         r.bt = ((end - row0 + tiles - 1) / tiles + 15) & ~15;
         r.m0 = row0 + (mt - t0) * r.bt, r.m_end = r.m0 + r.bt < end ? r.m0 + r.bt : end;
         r.wrow += lo * p.N;
@@ -226,6 +226,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS<Epi>, 1)
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(hdr + 512);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(hdr + 520);
     int32_t* first = reinterpret_cast<int32_t*>(hdr + HDR + RING);
+    int32_t* rows = first + MAX_GROUPS + 1;
     const uint32_t stages = base + HDR;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t rank;
@@ -244,8 +245,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS<Epi>, 1)
     if (p.offs && warp == 3) {   // first token tile of every group: an inclusive scan over the groups, 32 at a time
         int run = 0;
         for (int e0 = 0; e0 < p.E; e0 += 32) {
-            const int e = e0 + lane;
-            int n = e < p.E ? (p.offs[e + 1] - p.offs[e] + BT - 1) / BT : 0;
+            const int e = e0 + lane, row = e < p.E ? p.offs[e] : 0, end = e < p.E ? p.offs[e + 1] : 0;
+            if (e < p.E) rows[e] = row;
+            if (e == p.E - 1) rows[p.E] = end;
+            int n = (end - row + BT - 1) / BT;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const int u = __shfl_up_sync(0xffffffffu, n, o);
@@ -274,8 +277,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS<Epi>, 1)
             int s = 0;
             uint32_t ph = 1;
             bool ok = true;
+            Tile tl, next{};
+            if (((int)blockIdx.x >> 1) < tiles) next = tile_of<PARTS>(p, first, rows, MT, (int)blockIdx.x >> 1);
             for (int t = (int)blockIdx.x >> 1; t < tiles && ok; t += stride) {
-                const Tile tl = tile_of<PARTS>(p, first, MT, t);
+                tl = next;
                 const int wr = tl.wrow + (int)rank * ROWS, xr = tl.m0 + (int)rank * (tl.bt / 2);   // (the copies are as long as the longest tile needs)
                 for (int kb = tl.kb0; kb < tl.kb1; ++kb) {
                     ok = bar_wait(empty + 8 * s, ph, abort_flag);
@@ -285,6 +290,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS<Epi>, 1)
                     tma_pair(st, &map_w, kb * BK, wr, full_l + 8 * s);
                     tma_pair(st + ROWS * BK * 2, &map_x, kb * BK, xr, full_l + 8 * s);
                     if (++s == STAGES) s = 0, ph ^= 1u;
+                    if (kb == tl.kb0 && t + stride < tiles) next = tile_of<PARTS>(p, first, rows, MT, t + stride);   // (looked up beside the copies)
                 }
             }
             // every slab issued has been consumed before the CTA's shared memory goes away (a stage never used passes at once; after an
@@ -301,12 +307,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS<Epi>, 1)
             int s = 0, b = 0;
             uint32_t ph = 0, eph = 1;
             bool ok = true;
+            Tile tl, next{};
+            if (((int)blockIdx.x >> 1) < tiles) next = tile_of<PARTS>(p, first, rows, MT, (int)blockIdx.x >> 1);
             for (int t = (int)blockIdx.x >> 1; t < tiles && ok; t += stride) {
                 ok = bar_wait(acc_empty + 8 * b, eph, abort_flag);   // the epilogues of both CTAs have drained this buffer
                 if (!ok) break;
                 fence_after();
                 const uint32_t d = tmem + b * ACC_STRIDE;
-                const Tile tl = tile_of<PARTS>(p, first, MT, t);
+                tl = next;
                 const uint32_t idesc = idesc0 | ((uint32_t)(tl.bt >> 3) << 17);
                 const int nk = tl.kb1 - tl.kb0;
                 for (int kb = 0; kb < nk; ++kb) {
@@ -318,6 +326,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS<Epi>, 1)
                     for (int kk = 0; kk < BK / 16; ++kk) mma_pair(d, da + 2 * kk, db + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
                     commit_pair(empty + 8 * s);
                     if (++s == STAGES) s = 0, ph ^= 1u;
+                    if (kb == 0 && t + stride < tiles) next = tile_of<PARTS>(p, first, rows, MT, t + stride);
                 }
                 if (ok) commit_pair(acc_full + 8 * b);
                 b ^= 1;
@@ -330,7 +339,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS<Epi>, 1)
         int b = 0;
         uint32_t ph = 0;
         for (int t = (int)blockIdx.x >> 1; t < tiles; t += stride) {
-            const Tile tl = tile_of<PARTS>(p, first, MT, t);
+            const Tile tl = tile_of<PARTS>(p, first, rows, MT, t);
             if (!bar_wait(acc_full + 8 * b, ph, abort_flag)) break;
             fence_after();
             const int n = tl.n0 + (int)rank * ROWS + q * 32 + lane;
