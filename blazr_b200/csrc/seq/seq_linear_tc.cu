@@ -353,10 +353,20 @@ using tcpair::make_map;
 int pick_tile(const TcParams& p) {
     const int64_t pairs = tcpair::pair_sms() / 2;
     if (p.heads || pairs < 1 || (p.offs && p.E > tcpair::MAX_GROUPS)) return 0;
-    return tcpair::pick_bt(pairs, p.K, [&](int bt) {   // grouped: every group's last tile is half full on average
-        const int64_t mt = p.offs ? (p.M + bt / 2 * (int64_t)p.E + bt - 1) / bt : (p.M + bt - 1) / bt;
-        return mt * ((p.N + 255) / 256);
-    });
+    const int64_t NT = (p.N + 255) / 256;
+    if (!p.offs) return tcpair::pick_bt(pairs, p.K, [&](int bt) { return (p.M + bt - 1) / bt * NT; });
+    // Grouped: a group's last tile is half full on average, its rows are shared out evenly over its tiles, and few rows are a tile a group.  Of equal ones the
+    // smallest: the less a stage holds, the more of them there are.
+    int best = 0;
+    double best_t = 0;
+    for (int bt : {256, 192, 128, 64, 32}) {
+        int64_t tiles = (p.M + bt / 2 * (int64_t)p.E + bt - 1) / bt;
+        if (tiles < p.E) tiles = p.E;
+        const int64_t width = p.M / tiles + 16 < bt ? p.M / tiles + 16 : bt;
+        const double t = (double)((tiles * NT + pairs - 1) / pairs) * tcpair::wave_us((int)width, p.K);
+        if (best == 0 || t <= best_t) best = bt, best_t = t;
+    }
+    return best;
 }
 
 template <class Epi>

@@ -163,6 +163,10 @@ __device__ __forceinline__ void ld32(uint32_t taddr, float* v) {
 }
 __device__ __forceinline__ void ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// Rows of a copy of token rows.  Grouped: 32, as many of them as the tile needs (a copy as long as the longest tile's 128 rows is an eighth too much for a tile
+// of 176, and what bounds short products is 64 bytes a cycle from L2 to an SM), where they fill the longest tile's rows exactly; else all in one.
+__host__ __device__ __forceinline__ int x_box(const Args& p) { return p.offs && p.bt % 64 == 0 ? 32 : p.bt / 2; }
+
 struct Tile {
     int m0, m_end, wrow, n0;   // first token row, end of the tile's rows, first weight row in memory, first output column
     int bt;                    // columns of the tile: a multiple of 16, m_end - m0 or more
@@ -281,14 +285,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS<Epi>, 1)
             if (((int)blockIdx.x >> 1) < tiles) next = tile_of<PARTS>(p, first, rows, MT, (int)blockIdx.x >> 1);
             for (int t = (int)blockIdx.x >> 1; t < tiles && ok; t += stride) {
                 tl = next;
-                const int wr = tl.wrow + (int)rank * ROWS, xr = tl.m0 + (int)rank * (tl.bt / 2);   // (the copies are as long as the longest tile needs)
+                const int wr = tl.wrow + (int)rank * ROWS, xr = tl.m0 + (int)rank * (tl.bt / 2), box = x_box(p), copies = (tl.bt / 2 + box - 1) / box;
                 for (int kb = tl.kb0; kb < tl.kb1; ++kb) {
                     ok = bar_wait(empty + 8 * s, ph, abort_flag);
                     if (!ok) break;
-                    if (rank == 0) bar_expect(full + 8 * s, 2 * STAGE);
+                    if (rank == 0) bar_expect(full + 8 * s, 2 * (ROWS + copies * box) * BK * 2);
                     const uint32_t st = stages + s * STAGE;
                     tma_pair(st, &map_w, kb * BK, wr, full_l + 8 * s);
-                    tma_pair(st + ROWS * BK * 2, &map_x, kb * BK, xr, full_l + 8 * s);
+                    for (int i = 0; i < copies; ++i) tma_pair(st + (ROWS + i * box) * BK * 2, &map_x, kb * BK, xr + i * box, full_l + 8 * s);
                     if (++s == STAGES) s = 0, ph ^= 1u;
                     if (kb == tl.kb0 && t + stride < tiles) next = tile_of<PARTS>(p, first, rows, MT, t + stride);   // (looked up beside the copies)
                 }
@@ -427,7 +431,7 @@ inline int pick_bt(int64_t pairs, int64_t K, Tiles tiles) {
 template <bool PARTS = false, class Epi>
 cudaError_t launch(const void* w, int64_t w_rows, int64_t ldw, const void* x, int64_t ldx, Args p, const Epi& epi, cudaStream_t st, bool pdl = false) {
     CUtensorMap mw, mx;
-    if (!make_map(&mw, w, w_rows, p.K, ldw, ROWS, p.bf16 != 0) || !make_map(&mx, x, p.M, p.K, ldx, p.bt / 2, p.bf16 != 0)) return cudaErrorInvalidValue;
+    if (!make_map(&mw, w, w_rows, p.K, ldw, ROWS, p.bf16 != 0) || !make_map(&mx, x, p.M, p.K, ldx, x_box(p), p.bf16 != 0)) return cudaErrorInvalidValue;
     static bool ready[16] = {false};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
