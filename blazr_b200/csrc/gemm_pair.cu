@@ -42,7 +42,8 @@ static bool pair_plan(const b200q_weight* w, int64_t M, PairPlan* p) {
 // 193 / 167 / 153, 900 rows 148 / 136 / 112, 512 rows - / 68.5 / 65; Q4_K 16384 x 2048, 2048 rows 151 / 165 / 130, 1000 rows - / 89 / 72; 2048 x 8192, 1536 rows
 // 70 / 64 / 61; 10240 x 8192, 1000 rows 224 / 183 / 162; Q8_0 6144 x 4096, 1800 rows 121 / 110 / 95; AWQ 6144 x 4096, 1531 rows 89 / 76 / 72; 57344 x 8192, 250
 // rows - / 250 / 216; the fused kernel in one wave: Q8_0 6144 x 4096, 600 rows - / 34 / 36; GPTQ 4096 x 4096, 887 rows - / 33 / 34; Q4_K 8192 x 28672, 500 rows
-// - / 215 / 227.  Where this one is taken and is the slower one it is so by 5 %: Q6_K 8192 x 8192, 520 rows - / 92 / 97.
+// - / 215 / 227.  Where this one is taken and is the slower one it is so by 5 %: Q6_K 8192 x 8192, 520 rows - / 92 / 97; Q4_K
+// 2560 x 2048, 2048 rows 28.7 / - / 30.1.
 bool gemm_pair_wins(const b200q_weight* w, int64_t M) {
     PairPlan p;
     if (M < 192 || M > INT32_MAX / 2 || w->N % (2 * TILE_ROWS) != 0 || w->N > INT32_MAX || gemm_k_splits(w, M) > 1 || !pair_plan(w, M, &p)) return false;

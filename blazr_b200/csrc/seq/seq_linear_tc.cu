@@ -373,7 +373,8 @@ template <class Epi>
 cudaError_t launch_pair(int bt, const void* x, int64_t ldx, const void* w, const TcParams& p, const Epi& epi, cudaStream_t st) {
     tcpair::Args a{};
     a.M = p.M, a.N = p.N, a.K = p.K, a.offs = p.offs, a.E = p.offs ? p.E : 1, a.bf16 = 1, a.bt = bt, a.err = p.err, a.err_bit = 2;
-    return tcpair::launch(w, p.offs ? (int64_t)p.E * p.N : p.N, p.K, x, ldx, a, epi, st, true);
+    if (p.offs) return tcpair::launch<false, true>(w, (int64_t)p.E * p.N, p.K, x, ldx, a, epi, st, true);
+    return tcpair::launch(w, p.N, p.K, x, ldx, a, epi, st, true);
 }
 
 int launch(const void* x, int64_t ldx, const void* w, TcParams p, cudaStream_t st) {
