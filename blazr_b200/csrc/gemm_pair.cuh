@@ -5,8 +5,8 @@
 // would have written.  So a prompt's weight is neither expanded in a pass of its own nor written to and read back from L2 (2 bytes per weight each way), a
 // slab of 64 k costs an SM bt * 64 bytes of activations and 4.6 - 8.5 KB of packed weights, and the accumulator is double-buffered, so that an epilogue
 // runs under the next tile's products.  A weight is expanded once per bt token rows, 16 of 28 warps doing nothing else.  Bound by power in long runs (the clock
-// falls to 1.4 - 1.6 GHz; expansion and products together draw what the card may), by the expansion's latency per slab below about 200 rows a tile.  Measured: Q6_K
-// 14336 x 4096, 2048 rows 260 us -> 240; with the pass of its own and the product of expanded rows alone 211.
+// falls to 1.4 - 1.6 GHz; expansion and products together draw what the card may), by the expansion's latency per slab below about 200 rows a tile.  Measured, whole calls: Q6_K
+// 14336 x 4096, 2048 rows 263 us -> 232 (1.04 PFLOP/s), AWQ 6144 x 4096, 1531 rows 88 -> 73; the product of rows expanded before takes 200 of the former.
 //
 // Operands (f16 roundings of weights and activations), order of k and f32 accumulation are those of gemm_impl.cuh and gemm_wide.cu: the same results, bit for bit.
 //

@@ -179,10 +179,10 @@ static WidePlan wide_plan(const b200q_weight* w, int64_t M) {
 // (8192 x 8192, 800 rows: estimated 12 % faster, measured 3 % slower; 10240 x 8192, 300 to 640 rows: 10 to 25 % slower, 800: 8 to 14 % faster) and
 // not where K is cut.  Cut products, fused / expanded, us: 512 x 2048, 2048 rows 45.8 / 24.1; 1024 x 4096, 1280 rows 55.9 / 30.8; 1024 x 8192, 2048 rows
 // 120 / 67; 4096 x 4096, 512 rows 49.0 / 47.0.
-// The fused kernel's times are those from before all its warps stored results and its staging moved 16-byte pieces.  Now it would be the better one well
-// above these lines (fused / expanded in a loop of seconds, us: AWQ 6144 x 4096, 1531 rows 73 / 86; Q6_K 14336 x 4096, 1000 rows 130 / 151; 28672 x 4096, 1280
-// rows 287 / 320; 8192 x 8192, 1536 rows 195 / 230; 2048 x 8192, 2048 rows 76 / 84).  The lines are still those of the older
-// times, and stand to be drawn again.  A caller who brings the smaller workspace has the fused kernel; both give the same bits.
+// What these lines still decide: a prompt's products with the expansion taken out of them, weights whose N is not a multiple of 256, products cut along K, and int4
+// weights with f32 results; all else of this size takes gemm_pair.cuh first.  The fused kernel's times are those from before all its warps stored results, and it would
+// now be the better one above some of these lines (2048 x 8192, 2048 rows 76 / 84; 512 x 2048, 2048 rows 16 / 23).  A caller who brings the smaller workspace has the
+// fused kernel; all give the same bits.
 static bool wide_wins(const b200q_weight* w, int64_t M, const WidePlan& p) {
     const int64_t mt = (M + 255) / 256, rows = ((M + mt - 1) / mt + 31) / 32 * 32, items = w->T * mt;
     const double wave = (12.0 + 0.1 * (double)rows) * (double)w->K_pad / 4096.0;

@@ -321,6 +321,7 @@ class Decoder:
         self.fused_swiglu = _os.environ.get("B200Q_FUSED_SWIGLU", "0") != "0" and not self.wide  # measured slower: 148x redundant SiLU
         self.pf_bytes = int(float(_os.environ.get("B200Q_PF_MB", "0")) * (1 << 20))
         self.graph = self.chain_graph = None
+        self.chain_steps = 1               # steps of chain_graph
         self.fed = self.chosen = None      # [max_ctx, M]: tokens that captured steps take instead of their own choice (-1: none), and their choices
         self._host_pos = 0
         # EXPERIMENTAL (B200Q_DSTEP=1, single GPU, M <= 4): persistent op-list kernel, 3 launches per layer instead of 8
@@ -727,6 +728,7 @@ class Decoder:
             return g
 
         g = record(1)
+        self.chain_steps = CHAIN if chain else 1
         self.chain_graph = record(CHAIN) if chain else None
         self.graph = g
         return g
@@ -882,7 +884,7 @@ class Decoder:
             try:
                 left = steps
                 while left > 0:
-                    n = CHAIN if left >= CHAIN else 1
+                    n = self.chain_steps if left >= self.chain_steps else 1
                     for _ in range(n):
                         self._advance()
                     (self.chain_graph if n > 1 else self.graph).replay()
