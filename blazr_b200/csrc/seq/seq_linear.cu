@@ -163,11 +163,26 @@ __global__ void __launch_bounds__(256) linear_tiled_kernel(const XT* __restrict_
     }
 }
 
+// whole 16-byte pieces of a row of x and w
+static bool rows_vec(const void* x, int64_t es, int64_t ldx, const void* w, int K) {
+    return K % 8 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (ldx * es) % 16 == 0;
+}
+
+// Rows between the few of a decode step and the 32 of the tensor-core tiles: the streaming kernel passes over the weight once for every four of them, out of L1
+// and L2, which is less than the f32 tiles take with nearly all of their 64 rows empty.  Measured, us, streamed / tiled (error against 64 bits 0.8e-7 / 3.9e-7; the
+// tensor cores take 10 and are off by 2.1e-6): bf16 16384 x 2048, 9 rows 44 / 219, 31 rows 138 / 226; 2048 x 8192, 9 rows 74 / 565, 31 rows 236 / 566; 8192 x 1024,
+// 31 rows 73 / 73; f32 rows 16384 x 2048, 31 rows 208 / 219; 8192 x 1024, 9 rows 37 / 71, 16 rows of 32768 x 1024 102 / 216, but 31 rows
+// of 8192 x 1024 115 / 72.  Short rows leave lanes without a piece and every output its own sum over the warp: bf16 31 rows, 65536 x 512 165 / 188, 16384 x 512
+// 52 / 58, but 65536 x 256 121 / 95 and 131072 x 64 234 / 50.
+static bool streams_rows(const void* x, int x_dtype, int64_t ldx, const void* w, int M, int K) {
+    if (M <= 8) return true;
+    return M < 32 && K >= 512 && rows_vec(x, x_dtype == B200SEQ_F32 ? 4 : 2, ldx, w, K) && (x_dtype == B200SEQ_BF16 || M <= 16 || K >= 2048);
+}
+
 template <typename XT>
 static void launch_rows(const XT* x, int64_t ldx, const __nv_bfloat16* w, int M, int N, int K, float* y, int64_t ldy, cudaStream_t st,
                         const GateEpi ge) {
-    const bool vec = K % 8 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
-                     (ldx * (int64_t)sizeof(XT)) % 16 == 0;
+    const bool vec = rows_vec(x, sizeof(XT), ldx, w, K);
     const int rpw = ((ge.out && act_kind_gated(ge.act.kind)) || (N + 15) / 16 >= 4 * 148) ? 2 : 1;   // few rows: one per warp, so that every SM streams weights
     const int warps = (N + rpw - 1) / rpw;
     const int blocks = (warps + 7) / 8;
@@ -198,7 +213,7 @@ extern "C" int b200seq_linear_silu(const void* x, int x_dtype, int64_t ldx, cons
     if (M == 0) return 0;
     cudaStream_t st = (cudaStream_t)stream;
     if (path == B200SEQ_PATH_AUTO) {
-        if (M <= 8) path = B200SEQ_PATH_ROWS;
+        if (streams_rows(x, x_dtype, ldx, w, M, K)) path = B200SEQ_PATH_ROWS;
         else if (M >= 32 && linear_tc_usable(x_dtype, ldx, M, N, K, x, w)) path = B200SEQ_PATH_TC;
         else path = B200SEQ_PATH_TILED;
     }
