@@ -56,3 +56,20 @@ def test_against_the_dequantized_weight(client, fmt, N, K, M, dt):
         assert ((y.double() - ref).norm() / ref.norm()).item() < 8.3e-4 + {torch.float32: 0.0, torch.float16: 2 ** -11, torch.bfloat16: 2 ** -9}[out]
     from blazr_b200 import ops
     ops.check_device_errors()
+
+
+@pytest.mark.parametrize("fmt,N,K,M", [("Q8_0", 4096, 14336, 520), ("Q8_0", 4096, 8192, 1300), ("Q6_K", 4096, 14336, 520), ("AWQ", 8192, 8192, 560)])
+def test_a_chunk_is_read_before_its_slot_is_refilled(client, fmt, N, K, M):
+    """narrow token tiles over a long K: the expansion is the bound, two to four slots of packed chunks turn over as fast as they can, call behind call"""
+    w, _ = weight(client, fmt, N, K)
+    x = torch.randn((M, K), device="cuda:0", generator=torch.Generator(device="cuda:0").manual_seed(3)).half()
+    ref = x.double() @ client.dequantize(w).double().T
+    ws = w.workspace(M)
+    outs = [torch.empty((M, N), dtype=torch.float16, device="cuda:0") for _ in range(8)]
+    for _ in range(8):
+        for y in outs:
+            client.quant_matmul(x, w, out=y, workspace=ws)
+        for y in outs:
+            assert torch.equal(y, outs[0])
+    # one unit of 32 k that is another chunk's moves its row by sqrt(64 / K) of the result, 7 % and more; the roundings of 2^-11 each stay below 1 % at any element
+    assert ((outs[0].double() - ref).abs().max() / ref.square().mean().sqrt()).item() < 2e-2
