@@ -11,7 +11,8 @@
 // Operands (f16 roundings of weights and activations), order of k and f32 accumulation are those of gemm_impl.cuh and gemm_wide.cu: the same results, bit for bit.
 //
 // Warp roles: 0 = activation tiles (TMA, both CTAs), 1 = MMA issuer (leader CTA), 2 = TMEM allocation, 3 = packed chunks, 4..11 = epilogue, 12..27 = expansion.
-// Barriers: full[s] lives in the leader: the bytes of both CTAs' activation rows and one arrival per expanding warp of the stage; empty[s] and
+// Barriers: full[s] lives in the leader: the bytes of both CTAs' activation rows, one arrival per expanding warp of the leader's share of the stage and one for
+// the whole of the peer's: its warps arrive on expanded[s] in their own CTA, and its warp 1, which has no products to issue, passes that on; empty[s] and
 // acc_full are signalled in both CTAs by multicast tcgen05.commit; acc_empty lives in the leader; w_full / w_empty belong to the CTA's own chunk ring.
 // Every wait is bounded (tcpair::bar_wait): one that runs out raises the abort flag, the roles leave their loops, copies in flight are waited for, TMEM is freed.
 #pragma once
@@ -38,10 +39,12 @@ struct PairParams {
     int err_bit;
 };
 
-// The arrival of an expanding warp at the leader's barrier.  The stores are in this SM's shared memory, and known to the asynchronous proxy that reads them
-// there, since fence.proxy.async; the arrival needs no wider release of its own (one at cluster scope waits for all of the thread's memory operations and
-// doubles the kernel's time).
-__device__ __forceinline__ void arrive_leader(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
+// An arrival on another CTA's barrier that hands this CTA's shared memory over: what the thread has seen written there is ordered before it at cluster scope.
+// The fence is restricted to shared memory: mbarrier.arrive.release.cluster also waits for all else that is on its way to memory (2.2 times the kernel's time).
+__device__ __forceinline__ void arrive_cluster_shared(uint32_t bar) {
+    asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 
 __device__ __forceinline__ void sts128_sa(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
     asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
@@ -54,7 +57,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PG_THREADS, 1) pair_
     const int BT = p.bt, X_BYTES = BT / 2 * BK * 2, STAGE = PG_A_BYTES + X_BYTES, STAGES = p.stages;
     const uint32_t base = (sa(smem_raw) + 1023u) & ~1023u;
     const uint32_t full = base, empty = full + 8 * PG_MAX_STAGES, acc_full = empty + 8 * PG_MAX_STAGES, acc_empty = acc_full + 16, w_full = acc_empty + 16,
-                   w_empty = w_full + 8 * PG_MAX_NW;
+                   w_empty = w_full + 8 * PG_MAX_NW, expanded = w_empty + 8 * PG_MAX_NW;
     uint8_t* hdr = smem_raw + (base - sa(smem_raw));
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(hdr + 512);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(hdr + 520);
@@ -63,7 +66,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PG_THREADS, 1) pair_
     uint32_t rank;
     asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(rank));
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) bar_init(full + 8 * s, 1 + PG_DQ_WARPS), bar_init(empty + 8 * s, 1);   // a stage is expanded by half of the warps of both CTAs
+        for (int s = 0; s < STAGES; ++s) bar_init(full + 8 * s, 2 + PG_DQ_WARPS / 2), bar_init(empty + 8 * s, 1), bar_init(expanded + 8 * s, PG_DQ_WARPS / 2);   // (half of a CTA's warps expand a stage)
         for (int b = 0; b < 2; ++b) bar_init(acc_full + 8 * b, 1), bar_init(acc_empty + 8 * b, 2 * PG_EPI_WARPS);
         for (int s = 0; s < p.nw; ++s) bar_init(w_full + 8 * s, 1), bar_init(w_empty + 8 * s, PG_DQ_WARPS);
         *abort_flag = 0;
@@ -131,6 +134,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PG_THREADS, 1) pair_
                 b ^= 1;
                 if (b == 0) eph ^= 1u;
             }
+        } else if (rank != 0 && elect()) {
+            // The peer's share of a stage, handed to the leader's products: its warps' stores are ordered before this thread by arrivals at CTA scope, and one arrival
+            // at cluster scope passes all of them on (release is cumulative).  With a fence and an arrival of that kind in every expanding warp Q6_K 14336 x 4096, 2048
+            // rows took 241 us instead of 234.
+            const uint32_t full_l = map_leader(full);
+            int s = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int t = t0; t < tiles && ok; t += stride) {
+                for (int kb = 0; kb < 4 * KC; ++kb) {
+                    ok = bar_wait<false>(expanded + 8 * s, ph, abort_flag);
+                    if (!ok) break;
+                    arrive_cluster_shared(full_l + 8 * s);
+                    if (++s == STAGES) s = 0, ph ^= 1u;
+                }
+            }
         }
     } else if (warp == 3) {
         if (elect()) {
@@ -191,7 +210,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PG_THREADS, 1) pair_
         // ===================== expansion: thread = weight row; a warp makes one of the two units (32 k) of every other slab =====================
         const int d = warp - PG_DQ_WARP0, q = d & 3, g = (d >> 2) & 1, grp = d >> 3, r = 32 * q + lane;
         const FmtMeta meta{p.gpc};
-        const uint32_t full_l = map_leader(full), row = stages + r * 128;
+        const uint32_t made = rank == 0 ? full : expanded, row = stages + r * 128;
         uint32_t at[4];                             // the unit's four 16-byte pieces in a stage's row
 #pragma unroll
         for (int c = 0; c < 4; ++c) at[c] = row + (uint32_t)(((4 * g + c) ^ (r & 7)) << 4);
@@ -237,7 +256,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PG_THREADS, 1) pair_
                     else {
                         fence_proxy_async();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive_sa(w_empty + 8 * ws), arrive_leader(full_l + 8 * s0), arrive_leader(full_l + 8 * s);
+                        if (lane == 0) mbar_arrive_sa(w_empty + 8 * ws), mbar_arrive_sa(made + 8 * s0), mbar_arrive_sa(made + 8 * s);
                     }
                     if ((s += 2) >= STAGES) s -= STAGES, ph ^= 1u;
                 }
