@@ -20,13 +20,25 @@ int* error_flag_dev();   // device int: bit 0 = KV position outside the block ta
         count_launch();                                \
     } while (0)
 
+template <class T>
+__device__ __forceinline__ void behind_wait(T& p) {   // (through the global address, so that its loads stay global ones)
+    size_t g = __cvta_generic_to_global(p);
+    asm volatile("" : "+l"(g)::"memory");
+    p = static_cast<T>(__cvta_global_to_generic(g));
+}
+
 // Operators follow one another on a stream, many of them a few us long: their kernels are launched as programmatic successors (launch_chained), so that a
 // kernel's blocks are placed while the one ahead drains.  chain_enter is the first thing such a kernel does: all that was launched before it is complete
 // beyond the wait, and only then may the kernel behind it be placed, so that never more than one kernel waits and what lies two launches back is complete.
 // Measured, us a call: feed-forward of 2048 x 8192, 85 tokens 43.0 -> 39.4, 2 tokens of 1024 x 4096 22.3 -> 19.5; recurrence of 5 tokens 9.0 -> 7.5; routed experts of
 // 4096 tokens (seven launches) 192 -> 187.
-__device__ __forceinline__ void chain_enter() {
+// reads: the kernel's pointers to const that are __restrict__.  What they point to may be written while this kernel waits, so it is not constant for the whole of
+// it, as read-only loads (__ldg, or the compiler's own choice for such pointers) demand, and those may be moved ahead of the wait; beyond the empty statement
+// a pointer's origin is unknown, and its loads are ordinary ones.
+template <class... T>
+__device__ __forceinline__ void chain_enter(T&... reads) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    (behind_wait(reads), ...);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <class... P, class... A>

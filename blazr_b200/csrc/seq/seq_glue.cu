@@ -351,7 +351,7 @@ __global__ void group_rmsnorm_kernel(const float* __restrict__ x, int64_t ldx, c
 // F outputs per row; gated kinds read the pair (gate f, up f) from columns (2f, 2f + 1) (interleaved) or (f, F + f)
 __global__ void gated_act_kernel(const float* __restrict__ gu, int64_t ldg, int T, int F, const ActParams act, int interleaved, void* __restrict__ out,
                                  int out_dtype, int64_t ldo) {
-    chain_enter();
+    chain_enter(gu);
     const int64_t n = (int64_t)T * F;
     const bool gated = act_is_gated(act.kind);
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (int64_t)gridDim.x * blockDim.x) {

@@ -15,7 +15,7 @@ int launch_linear_tc_act(const void* x, int64_t ldx, const void* w, int M, int N
 template <typename XT>
 __device__ __forceinline__ float ld_x(const XT* p);
 template <>
-__device__ __forceinline__ float ld_x<float>(const float* p) { return __ldg(p); }
+__device__ __forceinline__ float ld_x<float>(const float* p) { return *p; }
 template <>
 __device__ __forceinline__ float ld_x<__nv_bfloat16>(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 
@@ -43,7 +43,7 @@ __device__ __forceinline__ float silu_range(float v, int n, int lo, int hi) { re
 template <typename XT, int MB, bool VEC>
 __global__ void __launch_bounds__(256) linear_rows_kernel(const XT* __restrict__ x, int64_t ldx, const __nv_bfloat16* __restrict__ w, int M, int N, int K,
                                                           float* __restrict__ y, int64_t ldy, int rows_per_warp, const GateEpi ge) {
-    chain_enter();
+    chain_enter(x, w);
     const int lane = threadIdx.x & 31;
     const int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int n0 = warp * rows_per_warp;
@@ -59,18 +59,18 @@ __global__ void __launch_bounds__(256) linear_rows_kernel(const XT* __restrict__
 #pragma unroll 4
             for (int k = lane * 8; k < K; k += 256) {
                 float a[8], b[8];
-                bf16x8_to_f32(__ldg(reinterpret_cast<const uint4*>(w0 + k)), a);
-                bf16x8_to_f32(__ldg(reinterpret_cast<const uint4*>(w1 + k)), b);
+                bf16x8_to_f32(*reinterpret_cast<const uint4*>(w0 + k), a);
+                bf16x8_to_f32(*reinterpret_cast<const uint4*>(w1 + k), b);
 #pragma unroll
                 for (int m = 0; m < MB; ++m) {
                     if (m0 + m < M) {
                         float xv[8];
                         const XT* xp = x + (int64_t)(m0 + m) * ldx + k;
                         if (sizeof(XT) == 4) {
-                            const float4 p = __ldg(reinterpret_cast<const float4*>(xp)), q = __ldg(reinterpret_cast<const float4*>(xp) + 1);
+                            const float4 p = *reinterpret_cast<const float4*>(xp), q = *(reinterpret_cast<const float4*>(xp) + 1);
                             xv[0] = p.x, xv[1] = p.y, xv[2] = p.z, xv[3] = p.w, xv[4] = q.x, xv[5] = q.y, xv[6] = q.z, xv[7] = q.w;
                         } else {
-                            bf16x8_to_f32(__ldg(reinterpret_cast<const uint4*>(xp)), xv);
+                            bf16x8_to_f32(*reinterpret_cast<const uint4*>(xp), xv);
                         }
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
@@ -118,7 +118,7 @@ constexpr int TM = 64, TN = 64, TK = 16;
 template <typename XT>
 __global__ void __launch_bounds__(256) linear_tiled_kernel(const XT* __restrict__ x, int64_t ldx, const __nv_bfloat16* __restrict__ w, int M, int N, int K,
                                                            float* __restrict__ y, int64_t ldy, int silu_lo, int silu_hi) {
-    chain_enter();
+    chain_enter(x, w);
     __shared__ float xs[TK][TM + 4];
     __shared__ float ws[TK][TN + 4];
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;

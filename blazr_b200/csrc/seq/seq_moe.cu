@@ -26,7 +26,7 @@ int launch_linear_tc_grouped_act(const void* x, int64_t ldx, const void* w, cons
 // grid (pairs): row r of the result = the activation row of the token behind the r-th sorted pair (contiguous rows for the tensor-core tiles)
 __global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const int32_t* __restrict__ sorted, int x_div, int K,
                                   __nv_bfloat16* __restrict__ out, int64_t ldo) {
-    chain_enter();
+    chain_enter(x, sorted);
     const int r = blockIdx.x;
     const __nv_bfloat16* src = x + (int64_t)(sorted[r] / x_div) * ldx;
     __nv_bfloat16* dst = out + (int64_t)r * ldo;
@@ -40,7 +40,7 @@ __global__ void moe_gather_kernel(const __nv_bfloat16* __restrict__ x, int64_t l
 // the same with a warp per row and four 16-byte loads per lane in flight (K % 8 == 0, aligned rows): 16 384 rows of 1024 11.5 us with a block per row, now 8.5
 __global__ void __launch_bounds__(256) moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const int32_t* __restrict__ sorted, int x_div, int rows, int K8,
                                                               __nv_bfloat16* __restrict__ out, int64_t ldo) {
-    chain_enter();
+    chain_enter(x, sorted);
     const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= rows) return;
     const uint4* src = reinterpret_cast<const uint4*>(x + (int64_t)(sorted[r] / x_div) * ldx);
@@ -162,7 +162,7 @@ __device__ __forceinline__ void route_token(const float* zr, float* sm, int t, i
 // with a block per token every choice was an atomic of its own on E addresses (4096 tokens, 4 of 32 experts: 13.6 us, now 8.6).
 __global__ void moe_route_kernel(const float* __restrict__ z, int64_t ldz, int T, const RouteRule rule, int32_t* __restrict__ ids, float* __restrict__ wts,
                                  int32_t* __restrict__ counts) {
-    chain_enter();
+    chain_enter(z);
     extern __shared__ float sm[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, per = 2 * rule.E + rule.groups;
     const int t = blockIdx.x * nw + wid;
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(256) moe_router_rows_kernel(const XT* __restri
 constexpr int SORT_NT = 1024, SORT_W = SORT_NT / 32, SORT_U = 8;
 __global__ void __launch_bounds__(SORT_NT) moe_sort_kernel(const int32_t* __restrict__ ids, int pairs, int E, const int32_t* __restrict__ counts, int32_t* __restrict__ offs,
                                                            int32_t* __restrict__ sorted, int32_t* __restrict__ slot_of) {
-    chain_enter();
+    chain_enter(ids, counts);
     __shared__ int seg[SORT_W], red[SORT_W];
     const int e = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int per = ((pairs + SORT_W - 1) / SORT_W + 31) & ~31;   // a warp's contiguous share of the pairs
@@ -320,7 +320,7 @@ __device__ __forceinline__ void bf16x8_f32(const uint4 v, float* f) {
 template <typename XT>
 __device__ __forceinline__ float ldx(const XT* p);
 template <>
-__device__ __forceinline__ float ldx<float>(const float* p) { return __ldg(p); }
+__device__ __forceinline__ float ldx<float>(const float* p) { return *p; }
 template <>
 __device__ __forceinline__ float ldx<__nv_bfloat16>(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 
@@ -331,12 +331,12 @@ __device__ __forceinline__ float moe_row_dot(const __nv_bfloat16* __restrict__ w
 #pragma unroll 4
         for (int k = lane * 8; k < K; k += 256) {
             float wv[8], xv[8];
-            bf16x8_f32(__ldg(reinterpret_cast<const uint4*>(wr + k)), wv);
+            bf16x8_f32(*reinterpret_cast<const uint4*>(wr + k), wv);
             if (sizeof(XT) == 4) {
-                const float4 q0 = __ldg(reinterpret_cast<const float4*>(xr + k)), q1 = __ldg(reinterpret_cast<const float4*>(xr + k) + 1);
+                const float4 q0 = *reinterpret_cast<const float4*>(xr + k), q1 = *(reinterpret_cast<const float4*>(xr + k) + 1);
                 xv[0] = q0.x, xv[1] = q0.y, xv[2] = q0.z, xv[3] = q0.w, xv[4] = q1.x, xv[5] = q1.y, xv[6] = q1.z, xv[7] = q1.w;
             } else {
-                bf16x8_f32(__ldg(reinterpret_cast<const uint4*>(xr + k)), xv);
+                bf16x8_f32(*reinterpret_cast<const uint4*>(xr + k), xv);
             }
 #pragma unroll
             for (int i = 0; i < 8; ++i) acc = fmaf(wv[i], xv[i], acc);
@@ -397,12 +397,12 @@ __global__ void __launch_bounds__(256) moe_rows_kernel(const MoeLin a) {
 #pragma unroll 4
         for (int k = lane * 8; k < a.K; k += 256) {
             float wv[8], xv[8];
-            bf16x8_f32(__ldg(reinterpret_cast<const uint4*>(wr + k)), wv);
+            bf16x8_f32(*reinterpret_cast<const uint4*>(wr + k), wv);
             if (sizeof(XT) == 4) {
-                const float4 q0 = __ldg(reinterpret_cast<const float4*>(xr + k)), q1 = __ldg(reinterpret_cast<const float4*>(xr + k) + 1);
+                const float4 q0 = *reinterpret_cast<const float4*>(xr + k), q1 = *(reinterpret_cast<const float4*>(xr + k) + 1);
                 xv[0] = q0.x, xv[1] = q0.y, xv[2] = q0.z, xv[3] = q0.w, xv[4] = q1.x, xv[5] = q1.y, xv[6] = q1.z, xv[7] = q1.w;
             } else {
-                bf16x8_f32(__ldg(reinterpret_cast<const uint4*>(xr + k)), xv);
+                bf16x8_f32(*reinterpret_cast<const uint4*>(xr + k), xv);
             }
 #pragma unroll
             for (int i = 0; i < 8; ++i) acc = fmaf(wv[i], xv[i], acc);
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(256) head_tiled_kernel(const HeadLin a) {
 __global__ void moe_combine_kernel(const float* __restrict__ ys, const float* __restrict__ wts, const int32_t* __restrict__ slot_of, int top, int W,
                                    const float* __restrict__ shared, const float* __restrict__ gate_z, int64_t ldg, float* __restrict__ y,
                                    const int32_t* __restrict__ ids, int E_real, const float* __restrict__ x_id, int vec) {
-    chain_enter();
+    chain_enter(ys, wts, slot_of, shared, gate_z, ids, x_id);
     const int64_t t = blockIdx.x;
     float gate = 1.f;
     if (shared && gate_z) gate = sigmoidf_acc(gate_z[t * ldg]);
