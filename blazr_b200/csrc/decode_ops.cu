@@ -625,6 +625,9 @@ __global__ void __launch_bounds__(1024) argmax_kernel(const float* __restrict__ 
     }
 }
 
+// row of an embedding table of V rows: ids outside it (the choice of a row without a number is 2^31 - 1) take row 0, whichever kernel embeds them
+__device__ __forceinline__ size_t table_row(int64_t id, int64_t V) { return (uint64_t)id < (uint64_t)V ? (size_t)id : 0; }
+
 // The end of a step that another one follows: the choice at position p goes to chosen[p][M], the token at position p + 1 is fed[p + 1][M] where that is not
 // negative, else the choice; with a table its row is the next step's h.  In a chain of captured steps the copy of the next token, the embedding's launch and
 // the start of the first product behind it stood between two steps: a token of the 4-layer model 106.9 us -> 100.3 in graphs of eight steps.
@@ -649,7 +652,7 @@ __global__ void __launch_bounds__(1024) argmax_next_kernel(const float* __restri
     }
     if (!table) return;
     __syncthreads();
-    const __half2* row = reinterpret_cast<const __half2*>(table + (size_t)(next < V ? next : 0) * H);   // (no logit was a number: no column)
+    const __half2* row = reinterpret_cast<const __half2*>(table + table_row(next, V) * H);
     for (int k = t; k < H / 2; k += 1024) *reinterpret_cast<float2*>(h + (size_t)m * H + 2 * k) = __half22float2(row[k]);
 }
 
@@ -711,25 +714,25 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restric
     out[(size_t)t * H + h] = acc;
 }
 
-// embedding gather: h[m, :] = table[ids[m], :] (f16 table -> f32)
+// embedding gather: h[m, :] = table[table_row(ids[m]), :] (f16 table -> f32)
 // First kernel of a decode step: it releases its dependents only AFTER its own dependency wait, which breaks the
 // programmatic chain at the step boundary -- nothing of step s+1 (in particular the attention prologue, which reads
 // pos[] ahead of its wait) can start before step s's argmax has advanced pos[] and written the token ids.
-__global__ void embed_kernel(const __half* __restrict__ table, const int64_t* __restrict__ ids, int H, float* __restrict__ h) {
+__global__ void embed_kernel(const __half* __restrict__ table, int64_t V, const int64_t* __restrict__ ids, int H, float* __restrict__ h) {
     pdl_wait();
     pdl_launch_dependents();
     const int m = blockIdx.y;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < H) h[(size_t)m * H + k] = __half2float(table[(size_t)ids[m] * H + k]);
+    if (k < H) h[(size_t)m * H + k] = __half2float(table[table_row(ids[m], V) * H + k]);
 }
 
 // the same, eight columns per thread (whole 16-byte pieces): 2048 rows of 2048 19.7 us, now 9.1
-__global__ void __launch_bounds__(256) embed8_kernel(const __half* __restrict__ table, const int64_t* __restrict__ ids, int H, float* __restrict__ h) {
+__global__ void __launch_bounds__(256) embed8_kernel(const __half* __restrict__ table, int64_t V, const int64_t* __restrict__ ids, int H, float* __restrict__ h) {
     pdl_wait();
     pdl_launch_dependents();
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
     if (k >= H) return;
-    const uint4 u = *reinterpret_cast<const uint4*>(table + (size_t)ids[blockIdx.y] * H + k);
+    const uint4 u = *reinterpret_cast<const uint4*>(table + table_row(ids[blockIdx.y], V) * H + k);
     const uint32_t wd[4] = {u.x, u.y, u.z, u.w};
     float4* o = reinterpret_cast<float4*>(h + (size_t)blockIdx.y * H + k);
 #pragma unroll
@@ -1001,16 +1004,19 @@ int32_t b200q_moe_combine(const float* y, const float* gate_w, int64_t T, int64_
     return e == cudaSuccess ? B200Q_OK : B200Q_ERR_CUDA;
 }
 
-int32_t b200q_embed(const void* table_f16, const int64_t* ids, int64_t H, int64_t M, float* h, void* stream) {
-    if (!table_f16 || !ids || !h || H <= 0 || M <= 0) return B200Q_ERR_INVALID_ARG;
+int32_t b200q_embed_rows(const void* table_f16, int64_t V, const int64_t* ids, int64_t H, int64_t M, float* h, void* stream) {
+    if (!table_f16 || !ids || !h || V <= 0 || H <= 0 || M <= 0) return B200Q_ERR_INVALID_ARG;
     if (M > 1 && H % 8 == 0 && aligned16(table_f16) && aligned16(h)) {   // (one row: eight blocks of single columns start sooner)
         const unsigned nt = H >= 2048 ? 256 : 128;
-        cudaError_t e8 = launch_pdl(embed8_kernel, dim3((unsigned)((H / 8 + nt - 1) / nt), (unsigned)M), dim3(nt), 0, (cudaStream_t)stream, (const __half*)table_f16, ids, (int)H, h);
+        cudaError_t e8 = launch_pdl(embed8_kernel, dim3((unsigned)((H / 8 + nt - 1) / nt), (unsigned)M), dim3(nt), 0, (cudaStream_t)stream, (const __half*)table_f16, V, ids, (int)H, h);
         return e8 == cudaSuccess ? B200Q_OK : B200Q_ERR_CUDA;
     }
     cudaError_t e = launch_pdl(embed_kernel, dim3((unsigned)((H + 255) / 256), (unsigned)M), dim3(256), 0, (cudaStream_t)stream,
-                               (const __half*)table_f16, ids, (int)H, h);
+                               (const __half*)table_f16, V, ids, (int)H, h);
     return e == cudaSuccess ? B200Q_OK : B200Q_ERR_CUDA;
+}
+int32_t b200q_embed(const void* table_f16, const int64_t* ids, int64_t H, int64_t M, float* h, void* stream) {
+    return b200q_embed_rows(table_f16, INT64_MAX, ids, H, M, h, stream);
 }
 
 }  // extern "C"

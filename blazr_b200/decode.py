@@ -480,7 +480,7 @@ class Decoder:
         L, cfg, M = ops.lib(), self.cfg, self.M
         st = ops._stream_ptr(self.dev)
         P = lambda t: C.c_void_p(t.data_ptr())
-        ops._check(L.b200q_embed(P(self.embed), P(self.ids), C.c_int64(cfg.hidden), C.c_int64(M), P(self.h), st))
+        ops._check(L.b200q_embed_rows(P(self.embed), cfg.vocab, P(self.ids), cfg.hidden, M, P(self.h), st))
         progs, pf = self.programs
         for lay, (p1, p2) in zip(self.layers, progs):
             p1.launch()
@@ -591,7 +591,7 @@ class Decoder:
         st = ops._stream_ptr(self.dev)
         P = lambda t: C.c_void_p(t.data_ptr())
         if not embedded:
-            ops._check(L.b200q_embed(P(self.embed), P(self.ids), C.c_int64(cfg.hidden), C.c_int64(M), P(self.h), st))
+            ops._check(L.b200q_embed_rows(P(self.embed), cfg.vocab, P(self.ids), cfg.hidden, M, P(self.h), st))
         hin, hout = self.h, self.h2
         delta = None
         in_flight = False  # TP: the projection ahead left its partial sums in the exchange buffers (see _rowpar)
@@ -774,7 +774,7 @@ class Decoder:
             b["logits1"] = torch.full((1, self.logits_local.shape[1]), float("-inf"), **f32)
             self._pf = b
         ids_d = torch.from_numpy(ids_h).to(dev)
-        ops._check(L.b200q_embed(P(self.embed), P(ids_d), H, S, P(b["h"]), st))
+        ops._check(L.b200q_embed_rows(P(self.embed), cfg.vocab, P(ids_d), H, S, P(b["h"]), st))
         hin, hout = b["h"], b["h2"]
         delta = None
         def expand(i):
@@ -872,6 +872,8 @@ class Decoder:
         """prompt: int64 [M, S].  Greedy: feeds the prompt token by token (decode steps), then n_new tokens."""
         prompt = np.asarray(prompt, dtype=np.int64).reshape(self.M, -1)
         S = prompt.shape[1]
+        if S and not 0 <= prompt.min() <= prompt.max() < self.cfg.vocab:
+            raise ValueError(f"prompt holds token ids outside [0, {self.cfg.vocab})")
         if S + n_new - 1 > self.max_ctx:
             raise ValueError(f"prompt ({S}) + new tokens ({n_new}) - 1 = {S + n_new - 1} positions exceed max_ctx={self.max_ctx}")
         if use_graph and self.graph is None:

@@ -53,7 +53,7 @@ EXPORTS = [
     "b200q_weight_set_bias", "b200q_weight_set_next", "b200q_weight_set_pair", "b200q_shard_range", "b200q_shard_range_blocks", "b200q_workspace_bytes", "b200q_matmul",
     "b200q_act_bytes", "b200q_quantize_act", "b200q_matmul_q8", "b200q_matmul_path", "b200q_dequantize", "b200q_act_unpack",
     "b200q_int_partials", "b200q_launch_count", "b200q_add_rmsnorm_quant", "b200q_swiglu_quant", "b200q_attn_decode", "b200q_attn_decode_paged",
-    "b200q_argmax", "b200q_argmax_next", "b200q_matmul_norm_first", "b200q_decode_error", "b200q_embed", "b200q_weight_prefetch_l2", "b200q_matmul_norm", "b200q_matmul_swiglu",
+    "b200q_argmax", "b200q_argmax_next", "b200q_matmul_norm_first", "b200q_decode_error", "b200q_embed", "b200q_embed_rows", "b200q_weight_prefetch_l2", "b200q_matmul_norm", "b200q_matmul_swiglu",
     "b200q_add_rmsnorm_f16", "b200q_swiglu_f16", "b200q_rope_kv_prefill", "b200q_expand_bytes", "b200q_expand", "b200q_gated_rows_ok", "b200q_matmul_rows", "b200q_swiglu_f32", "b200q_swiglu_f32_interleaved", "b200q_gate_up_row", "b200q_matmul_q8_swiglu", "b200q_matmul_norm_swiglu", "b200q_moe_matmul_q8_swiglu", "b200q_program_create", "b200q_program_add_normq", "b200q_program_add_matvec", "b200q_program_add_swigluq", "b200q_program_add_attn", "b200q_program_add_argmax", "b200q_program_add_embed",
     "b200q_program_finalize", "b200q_program_launch", "b200q_program_free", "b200q_comm_create", "b200q_comm_handle", "b200q_comm_connect", "b200q_allreduce_f64", "b200q_comm_free", "b200q_comm_gather_ptr",
     "b200q_matmul_q8_rowpar", "b200q_allreduce_add_rmsnorm_quant", "b200q_allreduce_finish", "b200q_matmul_q8_gather", "b200q_argmax_gathered", "b200q_allreduce",
@@ -65,7 +65,7 @@ EXPORTS = [
 _ARG = dict(p=C.c_void_p, i=C.c_int32, l=C.c_int64, z=C.c_size_t, f=C.c_float)
 SIGNATURES = {
     "matmul": "ppillpilpzp", "matmul_q8": "pplpilpzp", "matmul_rows": "ppillppplpzp", "expand": "plpip", "expand_bytes": "pl", "gated_rows_ok": "pl",
-    "embed": "ppllpp", "add_rmsnorm_f16": "ppppfllpp", "add_rmsnorm_quant": "ppppfllppp", "rope_kv_prefill": "ppiiilppppppip", "swiglu_f16": "pllipp",
+    "embed": "ppllpp", "embed_rows": "plpllpp", "add_rmsnorm_f16": "ppppfllpp", "add_rmsnorm_quant": "ppppfllppp", "rope_kv_prefill": "ppiiilppppppip", "swiglu_f16": "pllipp",
     "swiglu_f32": "pllpp", "swiglu_f32_interleaved": "pllpp", "quantize_act": "pilllppp", "moe_matmul_q8": "pplpllpilpzp", "moe_matmul_q8_swiglu": "pplpllppzp",
     "moe_combine": "pplllpp", "matmul_path": "pipillpilpzp"
 }

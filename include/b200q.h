@@ -334,14 +334,15 @@ int32_t b200q_decode_error(int32_t* out_flags);
 /* greedy token: argmax over V, lowest index wins ties; pos_inc (nullable) is incremented per row (graph replay) */
 int32_t b200q_argmax(const float* logits, int64_t V, int64_t M, int64_t* out_ids, int32_t* pos_inc, void* stream);
 /* the end of a step that another one follows: the choice at position p = pos[m] goes to chosen[p][M], ids[m] is fed[p + 1][M] where that is not negative and the choice
- * otherwise, pos[m] = p + 1; with table_f16 (else null, and h null), h[M][H] = table[ids[m]].  fed and chosen have max_ctx rows.  The step behind it then begins with
+ * otherwise, pos[m] = p + 1; with table_f16 (V rows; else null, and h null), h[M][H] = table[ids[m]] as b200q_embed_rows.  fed and chosen have max_ctx rows.  The step behind it then begins with
  * b200q_matmul_norm_first on h: b200q_matmul_norm whose successors in the stream (the attention, which reads pos as it starts) start only when this launch is complete. */
 int32_t b200q_argmax_next(const float* logits, int64_t V, int64_t M, int64_t* ids, int32_t* pos, const int64_t* fed, int64_t* chosen, int64_t max_ctx, const void* table_f16,
                           int64_t H, float* h, void* stream);
 int32_t b200q_matmul_norm_first(const b200q_weight* w, const float* h_in, const float* delta, float* h_out, const float* norm_w, float eps, int64_t M,
                                 void* y, int32_t y_dtype, int64_t ldy, void* workspace, size_t workspace_bytes, void* stream);
-/* h[m,:] = f16 table[ids[m],:] */
+/* h[m,:] = f16 table[ids[m],:]; b200q_embed_rows: of a table of V rows, where an id outside it takes row 0 (b200q_argmax's choice in a row without a number is 2^31 - 1) */
 int32_t b200q_embed(const void* table_f16, const int64_t* ids, int64_t H, int64_t M, float* h, void* stream);
+int32_t b200q_embed_rows(const void* table_f16, int64_t V, const int64_t* ids, int64_t H, int64_t M, float* h, void* stream);
 
 /* number of kernels the library has launched on this process (all threads); for bench accounting */
 int64_t b200q_launch_count(void);
