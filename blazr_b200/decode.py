@@ -872,6 +872,8 @@ class Decoder:
         """prompt: int64 [M, S].  Greedy: feeds the prompt token by token (decode steps), then n_new tokens."""
         prompt = np.asarray(prompt, dtype=np.int64).reshape(self.M, -1)
         S = prompt.shape[1]
+        if n_new < 1:
+            raise ValueError(f"{n_new} new tokens: at least one is chosen")
         if S and not 0 <= prompt.min() <= prompt.max() < self.cfg.vocab:
             raise ValueError(f"prompt holds token ids outside [0, {self.cfg.vocab})")
         if S + n_new - 1 > self.max_ctx:

@@ -85,3 +85,11 @@ def test_generate_refuses_ids_without_a_row(host, use_graph):
             with pytest.raises(ValueError, match="outside"):
                 a.generate(prompt, 2, use_graph)
     assert a.generate(np.array([[0, vocab - 1]]), 2, use_graph).shape == (1, 2)
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_generate_refuses_no_new_tokens(host, use_graph):
+    a = _decoder(host, 1, False)
+    for n_new in (0, -2):
+        with pytest.raises(ValueError, match="at least one"):
+            a.generate(np.array([[1, 2, 3, 4]]), n_new, use_graph)
