@@ -572,12 +572,12 @@ int32_t b200q_matmul_path(const b200q_weight* w, int32_t path, const void* x, in
     if (path == 2) {
         size_t need = align256(gemm_ws_bytes(w, M));
         if (workspace_bytes < need) return fail(B200Q_ERR_WORKSPACE, "workspace too small: %zu < %zu", workspace_bytes, need);
-        // The paired kernel needs no more scratch than the fused one.  Int4 weights whose results leave as f32 keep the expansion where it stands (its launches are
-        // what test_gpu_gemm_wide.py holds these calls to; they would be as much faster as those that leave in 16 bits: 89 us to 72, figures at gemm_pair_wins).
-        const bool pair = gemm_pair_wins(w, M), hold = w->family == B200Q_FAM_G4 && y_dtype == B200Q_F32;
-        const size_t wide = pair && !hold ? 0 : gemm_wide_ws_bytes(w, M);   // large steps; a workspace sized for less keeps the fused kernel
+        const size_t wide = gemm_wide_ws_bytes(w, M);   // large steps; a workspace sized for less keeps the fused or the paired kernel (staged rows only)
         const bool expands = wide > 0 && workspace_bytes >= wide;
-        if (pair && !(hold && expands)) {
+        // Int4 weights whose results leave as f32 keep the expansion where it stands (its launches are what test_gpu_gemm_wide.py holds these calls to; they would
+        // be as much faster as those that leave in 16 bits: AWQ 6144 x 4096, 1531 rows 89 us to 72).
+        const bool hold = expands && w->family == B200Q_FAM_G4 && y_dtype == B200Q_F32;
+        if (!hold && gemm_pair_wins(w, M, expands)) {
             CUDA_TRY(launch_gemm_pair(w, x, x_dtype, M, ldx, y, y_dtype, ldy, (uint8_t*)workspace, st));
             return B200Q_OK;
         }

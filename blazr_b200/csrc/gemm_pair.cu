@@ -8,10 +8,8 @@ struct PairPlan {
     int bt, nw, stages, w_stage_bytes, smem;
 };
 
-// Estimated time of one wave of tiles at K = 4096 (us, at the clock that a second of such products runs at): 29.5 for 256 token rows, 28 for 240, 23.6 for
-// 176 measured; the fused kernel of gemm_tc.cu: 31 for 256, 22 to 24 for 192.
+// Widths of a token tile: one wave of tiles of bt rows at K = 4096 against another (relative: what a call takes is pair_us)
 static double pair_wave_us(int bt) { return 5.5 + 0.092 * bt; }
-static double fused_wave_us(int64_t rows) { return 0.125 * rows; }
 
 static int64_t pair_waves(const b200q_weight* w, int64_t M, int bt) {
     const int64_t pairs = tcpair::pair_sms() / 2;
@@ -36,21 +34,53 @@ static bool pair_plan(const b200q_weight* w, int64_t M, PairPlan* p) {
     return true;
 }
 
-// Which products take this kernel: those that the fused kernel does not cut along K (it then has fewer than half as many tiles as SMs), from 512 rows on where
-// that kernel needs two waves and more, else where the estimates say so, with a launch of staged rows and a set-up that cost 4 us more here, and something in
-// hand.  Measured in loops of seconds (us, expanded once by gemm_wide.cu / fused / this): Q6_K 14336 x 4096, 2048 rows 260 / 256 / 240, 1300 rows
-// 193 / 167 / 153, 900 rows 148 / 136 / 112, 512 rows - / 68.5 / 65; Q4_K 16384 x 2048, 2048 rows 151 / 165 / 130, 1000 rows - / 89 / 72; 2048 x 8192, 1536 rows
-// 70 / 64 / 61; 10240 x 8192, 1000 rows 224 / 183 / 162; Q8_0 6144 x 4096, 1800 rows 121 / 110 / 95; AWQ 6144 x 4096, 1531 rows 89 / 76 / 72; 57344 x 8192, 250
-// rows - / 250 / 216; the fused kernel in one wave: Q8_0 6144 x 4096, 600 rows - / 34 / 36; GPTQ 4096 x 4096, 887 rows - / 33 / 34; Q4_K 8192 x 28672, 500 rows
-// - / 215 / 227.  Where this one is taken and is the slower one it is so by 5 %: Q6_K 8192 x 8192, 520 rows - / 92 / 97; Q4_K
-// 2560 x 2048, 2048 rows 28.7 / - / 30.1.
-bool gemm_pair_wins(const b200q_weight* w, int64_t M) {
+// us of a whole call, runs of it back to back: this kernel and the fused one of gemm_tc.cu (the third way, an expansion ahead of the product: gemm_wide_us).  Fitted
+// to 965 measured calls (twelve formats; 2560 to 28672 rows of weights, K 256 to 14336, 200 to 4096 tokens), off by 4 to 6 % (rms).  A wave of tiles takes
+// a part for the weights, which the formats' expansion decides, and parts for its token rows, as waves of the chip and, power being what bounds them, as work.
+struct FormatUs {
+    double pair, fused;   // per wave of tiles at K = 4096
+};
+static FormatUs format_us(int family) {
+    switch (family) {
+        case B200Q_FAM_Q4_K: return {10.2, 5.4};
+        case B200Q_FAM_Q6_K: return {11.3, 5.9};
+        case B200Q_FAM_Q5_K: return {11.4, 6.7};
+        case B200Q_FAM_Q4_1: return {9.2, 5.0};
+        case B200Q_FAM_Q5_1: return {10.3, 6.1};
+        case B200Q_FAM_Q2_K: return {8.8, 5.0};
+        case B200Q_FAM_Q3_K: return {9.9, 5.4};
+        case B200Q_FAM_IQ4_XS: return {16.0, 13.3};
+        case B200Q_FAM_TQ2_0: return {7.2, 4.0};
+        case B200Q_FAM_G4: return {8.9, 5.1};
+        default: return {12.0, 6.3};   // Q8_0 (measured), I8S
+    }
+}
+static double pair_us(const b200q_weight* w, int64_t M, int bt) {
+    const double deep = (double)w->K_pad / 4096.0, rows = bt / 256.0, waves = (double)pair_waves(w, M, bt);
+    const double work = (double)((w->T / 2) * ((M + bt - 1) / bt)) / (double)(tcpair::pair_sms() / 2);
+    return 6.3 + 4.0 * waves * rows + deep * (waves * (format_us(w->family).pair + 4.7 * rows) + 14.1 * work * rows);
+}
+static double fused_us(const b200q_weight* w, int64_t M) {
+    const int64_t mt = (M + 255) / 256, items = w->T * mt;
+    const double deep = (double)w->K_pad / 4096.0, rows = (double)(((M + mt - 1) / mt + 31) / 32 * 32) / 256.0;
+    const double waves = (double)((items + w->num_sms - 1) / w->num_sms), work = (double)items / (double)w->num_sms;
+    return 2.8 + 6.7 * waves * rows + deep * (waves * (format_us(w->family).fused + 9.6 * rows) + 13.1 * work * rows);
+}
+
+// Which products take this kernel: those that the fused kernel does not cut along K (it then has fewer than half as many tiles as SMs) where the estimates put it
+// ahead of the kernel that the caller's workspace would have otherwise, by what they are off for calls alike.  Measured (us, expanded / fused / this): Q6_K 14336 x 4096,
+// 2048 rows 260 / 284 / 235, 900 rows 146 / 145 / 117, 700 rows - / 100 / 101, 520 rows - / 78 / 91; 8192 x 8192, 520 rows - / 92 / 97, 1536 rows 233 / 201 / 221; Q4_K 16384 x 2048, 700
+// rows - / 73 / 64; 2560 x 2048, 2048 rows 29.3 / 39.7 / 30.9; AWQ 6144 x 4096, 1531 rows 88 / 77 / 71; IQ4_XS 14336 x 4096, 2048 rows 245 / 325 / 255.  (With one wave time
+// for all formats and every product of 512 rows and two waves, 98 of 704 of these calls were slower than without this kernel, by up to 21 %; now
+// none of 720 by more than 3 %.)  K of at most 1024: the expansion's second pass over the weight costs a call whose operands are not in L2 more than the loop shows (Q6_K
+// 10240 x 1024, 785 rows 31.7 / 36.4 / 29.6 in a loop, 44 / 44 / 36 cold; IQ4_XS 30.9 / 43.2 / 33.7 and 42 / 50 / 42), so the line lies 12 % on this kernel's side.
+bool gemm_pair_wins(const b200q_weight* w, int64_t M, bool expands) {
     PairPlan p;
     if (M < 192 || M > INT32_MAX / 2 || w->N % (2 * TILE_ROWS) != 0 || w->N > INT32_MAX || gemm_k_splits(w, M) > 1 || !pair_plan(w, M, &p)) return false;
-    const int64_t mt = (M + 255) / 256, rows = ((M + mt - 1) / mt + 31) / 32 * 32, waves = (w->T * mt + w->num_sms - 1) / w->num_sms;
-    if (M >= 512 && waves > 1) return true;
-    const double deep = (double)w->K_pad / 4096.0;
-    return ((double)pair_waves(w, M, p.bt) * pair_wave_us(p.bt) * deep + 4.0) * (waves > 1 ? 1.03 : 1.09) < (double)waves * fused_wave_us(rows) * deep;
+    const double us = pair_us(w, M, p.bt);
+    // (rows gathered through a permutation: 2.5 us a million values more to stage in rows than in the fused kernel's tiles; GPTQ 8192 x 8192, 520 rows - / 95 / 104)
+    if (!expands) return us * 1.02 + (w->perm ? 2.5e-6 * (double)M * (double)w->K_pad : 0.0) < fused_us(w, M);
+    return us * (w->K_pad <= 1024 && M <= 2048 ? 0.88 : 1.01) < gemm_wide_us(w, M);
 }
 
 static cudaError_t pair_family(int family, const PairParams& p, const CUtensorMap& mx, int ctas, int smem, cudaStream_t st) {

@@ -177,12 +177,12 @@ static WidePlan wide_plan(const b200q_weight* w, int64_t M) {
 // projections of hidden sizes 2048, 4096 and 8192; it cuts K when there are at most half as many tiles as SMs, which costs a pass over the partial
 // sums, here as there).  Lines drawn from the same measurements: never below 512 rows; weights of several panels from 768 rows, with 14 % in hand
 // (8192 x 8192, 800 rows: estimated 12 % faster, measured 3 % slower; 10240 x 8192, 300 to 640 rows: 10 to 25 % slower, 800: 8 to 14 % faster) and
-// not where K is cut.  Cut products, fused / expanded, us: 512 x 2048, 2048 rows 45.8 / 24.1; 1024 x 4096, 1280 rows 55.9 / 30.8; 1024 x 8192, 2048 rows
-// 120 / 67; 4096 x 4096, 512 rows 49.0 / 47.0.
-// What these lines still decide: a prompt's products with the expansion taken out of them, weights whose N is not a multiple of 256, products cut along K, and int4
-// weights with f32 results; all else of this size takes gemm_pair.cuh first.  The fused kernel's times are those from before all its warps stored results, and it would
-// now be the better one above some of these lines (2048 x 8192, 2048 rows 76 / 84; 512 x 2048, 2048 rows 16 / 23).  A caller who brings the smaller workspace has the
-// fused kernel; all give the same bits.
+// not where K is cut.  Cut products, fused / expanded, us, when the lines were drawn: 512 x 2048, 2048 rows 45.8 / 24.1; 1024 x 4096, 1280 rows 55.9 / 30.8; 1024 x 8192,
+// 2048 rows 120 / 67; 4096 x 4096, 512 rows 49.0 / 47.0.
+// The fused kernel's times are those from before all its warps stored results, and it would now be the better one above some of these lines (2048 x 8192, 2048 rows
+// 76 / 84; 512 x 2048, 2048 rows 16 / 23).  They say what a step is expanded for where the paired kernel does not take it: gemm_pair_wins of gemm_pair.cu compares with today's
+// times.  They alone decide a prompt's products with the expansion taken out of them, weights whose N is not a multiple of 256, products cut along K, and int4 weights
+// with f32 results.  A caller who brings the smaller workspace has the fused kernel; all give the same bits.
 static bool wide_wins(const b200q_weight* w, int64_t M, const WidePlan& p) {
     const int64_t mt = (M + 255) / 256, rows = ((M + mt - 1) / mt + 31) / 32 * 32, items = w->T * mt;
     const double wave = (12.0 + 0.1 * (double)rows) * (double)w->K_pad / 4096.0;
@@ -198,6 +198,16 @@ size_t gemm_wide_ws_bytes(const b200q_weight* w, int64_t M) {
     if (M < GEMM_WIDE_MIN_M || M > INT32_MAX / 2) return 0;
     const WidePlan p = wide_plan(w, M);
     return wide_wins(w, M, p) ? p.bytes() : 0;
+}
+
+// us of a whole call, not cut along K, runs of it back to back (fitted to 460 measured calls beside pair_us of gemm_pair.cu; the plan's own estimate above is a wave's
+// relative one): every panel costs its launches, the longest panel's expansion is not hidden, and the products follow their waves.
+double gemm_wide_us(const b200q_weight* w, int64_t M) {
+    const WidePlan p = wide_plan(w, M);
+    const int64_t pairs = w->num_sms / 2, NT = (w->T + 1) / 2, MT = (M + p.bt - 1) / p.bt, full = NT / p.per, rest = NT - full * p.per;
+    const double waves = (double)(full * ((p.per * MT + pairs - 1) / pairs) + (rest * MT + pairs - 1) / pairs), rows = p.bt / 256.0, deep = (double)w->K_pad / 4096.0;
+    const double panel = (double)p.per * 256.0 * (double)w->K_pad / 1e7, packed = (double)w->chunk_bytes / (TILE_ROWS * CHUNK_K);
+    return -13.3 + 20.0 * p.panels + panel * (3.3 + 3.2 * packed) + waves * (2.3 * rows + deep * (1.25 + 28.1 * rows));
 }
 
 size_t gemm_wide_panel_bytes(const b200q_weight* w, int64_t M) { return gemm_wide_ws_bytes(w, M) ? wide_plan(w, M).buf_bytes : 0; }

@@ -93,18 +93,17 @@ size_t gemm_wide_ws_bytes(const b200q_weight* w, int64_t M);   // 0: this M stay
 // panel: the first panel's expansion, made ahead (null: made here); x_ready: f16 rows without infinities, read in place; act: gated f16 rows instead of y
 cudaError_t launch_gemm_wide(const b200q_weight* w, const void* x, int x_dtype, int64_t M, int64_t ldx, void* y, int y_dtype, int64_t ldy, uint8_t* ws, cudaStream_t st,
                              const void* panel = nullptr, bool x_ready = false, void* act = nullptr);
+double gemm_wide_us(const b200q_weight* w, int64_t M);
 size_t gemm_wide_panel_bytes(const b200q_weight* w, int64_t M);   // of the first panel; 0: this M stays on the fused kernel
 bool gemm_wide_gated_ok(const b200q_weight* w, int64_t M);
 cudaError_t launch_expand(const b200q_weight* w, int64_t M, void* panel, bool beside, cudaStream_t st);
 constexpr int B200Q_DECODE_ERR_GEMM_WAIT = 2;   // a bounded wait of the paired GEMM ran out: rows of its result are unwritten
 int* decode_error_dev();   // the device error word of b200q_decode_error (decode_ops.cu)
 
-cudaError_t launch_stage_rows(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, const int32_t* perm, int64_t K_pad, void* out, cudaStream_t st);   // f16 rows [M][K_pad]
-
 cudaError_t launch_stage_rows(const void* x, int x_dtype, int64_t M, int64_t K, int64_t ldx, const int32_t* perm, int64_t K_pad, void* rows, cudaStream_t st);   // f16 rows [M][K_pad]
 
 // ---- gemm_pair.cu ----
-bool gemm_pair_wins(const b200q_weight* w, int64_t M);   // M rows of this weight take it; its scratch (staged rows) is no more than the fused kernel's
+bool gemm_pair_wins(const b200q_weight* w, int64_t M, bool expands);   // M rows take it, where the expansion (expands) or the fused kernel would have them; scratch: staged rows, no more than the fused kernel's
 cudaError_t launch_gemm_pair(const b200q_weight* w, const void* x, int x_dtype, int64_t M, int64_t ldx, void* y, int y_dtype, int64_t ldy, uint8_t* ws, cudaStream_t st);
 
 // ---- gemm_tc.cu ----
