@@ -575,7 +575,7 @@ int32_t b200q_matmul_path(const b200q_weight* w, int32_t path, const void* x, in
         const size_t wide = gemm_wide_ws_bytes(w, M);   // large steps; a workspace sized for less keeps the fused or the paired kernel (staged rows only)
         const bool expands = wide > 0 && workspace_bytes >= wide;
         // Int4 weights whose results leave as f32 keep the expansion where it stands (its launches are what test_gpu_gemm_wide.py holds these calls to; they would
-        // be as much faster as those that leave in 16 bits: AWQ 6144 x 4096, 1531 rows 89 us to 72).
+        // be as much faster as those that leave in 16 bits: AWQ 6144 x 4096, 1531 rows 89 us to 75).
         const bool hold = expands && w->family == B200Q_FAM_G4 && y_dtype == B200Q_F32;
         if (!hold && gemm_pair_wins(w, M, expands)) {
             CUDA_TRY(launch_gemm_pair(w, x, x_dtype, M, ldx, y, y_dtype, ldy, (uint8_t*)workspace, st));

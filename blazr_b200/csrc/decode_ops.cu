@@ -430,10 +430,10 @@ __global__ void __launch_bounds__(ATT_NT) attn_decode_kernel(const float* __rest
     __shared__ float s_redf[NW];
     __shared__ double s_redd[NW];
     // ---- before griddepcontrol.wait: everything that does not depend on the qkv matvec running just ahead of this
-    // kernel -- pos (advanced by the previous step's argmax; stable here because embed_kernel, the first kernel of
-    // every step, releases its dependents only after that argmax completed), the RoPE row and the cached K / V rows
-    // j < p (written by earlier steps) -- is pulled into registers, so only the new q/k/v load remains on the
-    // critical path after it.
+    // kernel -- pos (advanced by the previous step's argmax; stable here because the first kernel of every step,
+    // embed_kernel or, behind a step of the same graph, the product of b200q_matmul_norm_first, releases its dependents
+    // only after that argmax completed), the RoPE row and the cached K / V rows j < p (written by earlier steps) -- is
+    // pulled into registers, so only the new q/k/v load remains on the critical path after it.
     constexpr int QE = HD / 4;          // score pass: elements per thread (4 threads per position)
     constexpr int EG = HD / 4;          // output pass: element groups of 4
     constexpr int JG = ATT_NT / EG;     // output pass: position groups (16 for hd 128, 32 for hd 64)

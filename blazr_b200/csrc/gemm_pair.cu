@@ -68,9 +68,10 @@ static double fused_us(const b200q_weight* w, int64_t M) {
 }
 
 // Which products take this kernel: those that the fused kernel does not cut along K (it then has fewer than half as many tiles as SMs) where the estimates put it
-// ahead of the kernel that the caller's workspace would have otherwise, by what they are off for calls alike.  Measured (us, expanded / fused / this): Q6_K 14336 x 4096,
-// 2048 rows 260 / 284 / 235, 900 rows 146 / 145 / 117, 700 rows - / 100 / 101, 520 rows - / 78 / 91; 8192 x 8192, 520 rows - / 92 / 97, 1536 rows 233 / 201 / 221; Q4_K 16384 x 2048, 700
-// rows - / 73 / 64; 2560 x 2048, 2048 rows 29.3 / 39.7 / 30.9; AWQ 6144 x 4096, 1531 rows 88 / 77 / 71; IQ4_XS 14336 x 4096, 2048 rows 245 / 325 / 255.  (With one wave time
+// ahead of the kernel that the caller's workspace would have otherwise, by what they are off for calls alike.  Measured (us, expanded / fused / this, f16 rows): Q6_K
+// 14336 x 4096, 2048 rows 247 / 275 / 226, 900 rows 142 / 141 / 112, 700 rows - / 98 / 101, 520 rows - / 78 / 91; 8192 x 8192, 520 rows - / 91 / 97, 1536 rows 233 / 201 / 221;
+// Q4_K 16384 x 2048, 700 rows - / 60 / 53; 2560 x 2048, 2048 rows 29.3 / 39.7 / 30.9; AWQ 6144 x 4096, 1536 rows 89 / 75 / 72; IQ4_XS 14336 x 4096, 2048 rows 245 / 325 / 255.
+// (With one wave time
 // for all formats and every product of 512 rows and two waves, 98 of 704 of these calls were slower than without this kernel, by up to 21 %; now
 // none of 720 by more than 3 %.)  K of at most 1024: the expansion's second pass over the weight costs a call whose operands are not in L2 more than the loop shows (Q6_K
 // 10240 x 1024, 785 rows 31.7 / 36.4 / 29.6 in a loop, 44 / 44 / 36 cold; IQ4_XS 30.9 / 43.2 / 33.7 and 42 / 50 / 42), so the line lies 12 % on this kernel's side.

@@ -6,7 +6,7 @@
 // slab of 64 k costs an SM bt * 64 bytes of activations and 4.6 - 8.5 KB of packed weights, and the accumulator is double-buffered, so that an epilogue
 // runs under the next tile's products.  A weight is expanded once per bt token rows, 16 of 28 warps doing nothing else.  Bound by power in long runs (the clock
 // falls to 1.4 - 1.6 GHz; expansion and products together draw what the card may), by the expansion's latency per slab below about 200 rows a tile.  Measured, whole calls: Q6_K
-// 14336 x 4096, 2048 f32 rows 260 us expanded ahead, 235 here (1.02 PFLOP/s), AWQ 6144 x 4096, 1531 rows 88 and 71; the product of rows expanded before takes 200 of the 260.
+// 14336 x 4096, 2048 f32 rows 265 us expanded ahead, 239 here (1.01 PFLOP/s), AWQ 6144 x 4096, 1531 rows 89 and 75; the product of rows expanded before takes 200 of the 265.
 //
 // Operands (f16 roundings of weights and activations), order of k and f32 accumulation are those of gemm_impl.cuh and gemm_wide.cu: the same results, bit for bit.
 //
@@ -136,8 +136,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PG_THREADS, 1) pair_
             }
         } else if (rank != 0 && elect()) {
             // The peer's share of a stage, handed to the leader's products: its warps' stores are ordered before this thread by arrivals at CTA scope, and one arrival
-            // at cluster scope passes all of them on (release is cumulative).  With a fence and an arrival of that kind in every expanding warp Q6_K 14336 x 4096, 2048
-            // rows took 241 us instead of 235.
+            // at cluster scope passes all of them on (release is cumulative).  With a fence and an arrival of that kind in every expanding warp Q6_K 14336 x 4096 took 3 % longer
+            // with 2048 rows and 6 % with 900 (AWQ 6144 x 4096, 1531 rows: 2 % less).
             const uint32_t full_l = map_leader(full);
             int s = 0;
             uint32_t ph = 0;

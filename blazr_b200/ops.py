@@ -281,7 +281,7 @@ class B200Client:
     def quant_matmul(self, x: torch.Tensor, w: QuantWeight, out: Optional[torch.Tensor] = None, out_dtype=None,
                      path: int = PATH_AUTO, workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Y[..., N] = X[..., K] @ dequant(W)[N, K]^T (+bias).  x: f32 / f16 / bf16 on this device.  The call does not wait for the device: what its
-        kernels report (a wait that ran out in a step of 512 rows and more) is raised by check_device_errors()."""
+        kernels report (a wait that ran out in a step of 192 rows and more) is raised by check_device_errors()."""
         shape = x.shape
         assert x.is_cuda and shape[-1] == w.K, (shape, w.K)
         x2 = x if len(shape) == 2 else x.reshape(-1, w.K)

@@ -329,7 +329,7 @@ int32_t b200q_attn_decode_paged(const float* qkv, const int32_t* pos, float* k_p
 /* A position pos[m] outside [0, max_ctx) makes b200q_attn_decode write nothing and raise a sticky per-device error
  * word instead of indexing past the KV cache.  b200q_decode_error reads and clears it for the current device
  * (synchronises the device: not capturable; call it after a generate loop).  bit 0 = position out of range.
- * bit 1 = a bounded wait of the large-step GEMM (b200q_matmul, 512 rows and more) ran out: the call that raised it left rows unwritten. */
+ * bit 1 = a bounded wait of a large-step GEMM (b200q_matmul, 192 rows and more) ran out: the call that raised it left rows unwritten. */
 int32_t b200q_decode_error(int32_t* out_flags);
 /* greedy token: argmax over V, lowest index wins ties; pos_inc (nullable) is incremented per row (graph replay) */
 int32_t b200q_argmax(const float* logits, int64_t V, int64_t M, int64_t* out_ids, int32_t* pos_inc, void* stream);

@@ -21,6 +21,16 @@ def _decoder(host, M, paged):
     return decode.Decoder(ops.B200Client(0), decode.PRESETS["tiny"], "Q4_K_M", batch=M, max_ctx=32, host=host, **(dict(paged=True, block_size=4) if paged else {}))
 
 
+class _Counted:
+    """a captured graph that counts its replays"""
+    def __init__(self, graph):
+        self.graph, self.n = graph, 0
+
+    def replay(self):
+        self.n += 1
+        self.graph.replay()
+
+
 @pytest.mark.parametrize("M,paged", [(1, False), (1, True), (3, False)])
 @pytest.mark.parametrize("S,n_new", [(1, 1), (7, 1), (8, 1), (9, 1), (5, 4), (3, 17), (17, 16)])
 def test_generate_in_one_graph(host, M, paged, S, n_new):
@@ -28,7 +38,11 @@ def test_generate_in_one_graph(host, M, paged, S, n_new):
     vocab = decode.PRESETS["tiny"].vocab
     a, b = _decoder(host, M, paged), _decoder(host, M, paged)
     prompt = np.random.default_rng(S).integers(0, vocab, (M, S))
+    a.capture()
+    assert a.chain_steps == decode.CHAIN > 1
+    a.graph, a.chain_graph = _Counted(a.graph), _Counted(a.chain_graph)
     got, want = a.generate(prompt, n_new), b.generate(prompt, n_new, use_graph=False)
+    assert (a.chain_graph.n, a.graph.n) == divmod(S + n_new - 1, decode.CHAIN) and bool((a.fed == -1).all())
     assert got.dtype == want.dtype and got.shape == (M, n_new) and (got == want).all()
     for _ in range(2):
         assert torch.equal(a.full_logits(), b.full_logits()) and torch.equal(a.ids, b.ids) and torch.equal(a.pos, b.pos)

@@ -44,6 +44,21 @@ def test_the_bits_of_the_fused_kernel(client, fmt, N, K, M):
     assert bool((y[M] == 7).all()) and bool((y[:, N:] == 7).all())
 
 
+@pytest.mark.parametrize("fmt", FORMATS)
+def test_the_bits_of_the_fused_kernel_in_f32(client, fmt):
+    """unrounded: the sums themselves are the same (int4 weights with f32 results are expanded where the workspace has room: they bring staged rows' worth)"""
+    from blazr_b200 import ops
+    N, K, M = 10240, 1024, 785
+    w, _ = weight(client, fmt, N, K)
+    x = torch.randn((M, K), device="cuda:0", generator=torch.Generator(device="cuda:0").manual_seed(4))
+    ws = torch.zeros(1024 * w.K_pad * 2, dtype=torch.uint8, device="cuda:0")      # what the fused kernel asks for: four tiles of up to 256 rows
+    n0 = ops.launch_count()
+    y = client.quant_matmul(x, w, workspace=ws)
+    assert ops.launch_count() - n0 == 2
+    for a in range(0, M, 160):
+        assert torch.equal(y[a:a + 160], client.quant_matmul(x[a:a + 160], w))
+
+
 @pytest.mark.parametrize("fmt,N,K,M", [("Q4_K", 12800, 512, 512), ("Q6_K", 2560, 256, 4099), ("Q8_0", 5120, 1056, 1537), ("GPTQ", 20480, 512, 1300), ("AWQ", 28672, 4096, 250)])
 @pytest.mark.parametrize("dt", [torch.float32, torch.float16, torch.bfloat16])
 def test_against_the_dequantized_weight(client, fmt, N, K, M, dt):
